@@ -11,6 +11,7 @@ from . import abi
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libsimnets_b200.so")
 _lib = None
+_ops = None
 
 _P = C.c_void_p
 
@@ -64,6 +65,20 @@ def lib():
         l.get_mex_offsets_nregions.restype = C.c_int
         _lib = l
     return _lib
+
+
+def ops():
+    """The PyTorch front end of the library (_torch_ops.so): the operators on tensors, wired into autograd."""
+    global _ops
+    if _ops is None:
+        lib()
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        try:
+            from . import _torch_ops
+        except ImportError as e:
+            raise ImportError("simnets_tf_b200/_torch_ops.so cannot be loaded (%s): build it with `python -m simnets_tf_b200.build`" % e)
+        _ops = _torch_ops
+    return _ops
 
 
 def check(status):

@@ -1,11 +1,9 @@
-"""Plumbing between torch tensors and the C ABI: dtype codes, pointers, the current stream and a
-per-(device, stream) scratch workspace that grows on demand."""
+"""Plumbing between torch tensors and the library: dtype codes, the current stream, the plans of recent calls and per-op
+timing."""
 
 import torch
 
-from . import abi
-
-_WORKSPACES = {}
+from . import _lib, abi
 
 # Descriptor flags OR-ed into every op call of this process; 0 unless a program sets it (an A/B measurement that
 # wants, say, abi.FLAG_MEX_NO_PAIR_TILES on every layer assigns it before the first call).
@@ -36,57 +34,49 @@ def stream_ptr(dev):
     return torch.cuda.current_stream(dev).cuda_stream
 
 
-def workspace(dev, nbytes):
-    """A scratch buffer of at least `nbytes` for the current stream of `dev` (contents undefined)."""
-    key = (dev.index, stream_ptr(dev))
-    buf = _WORKSPACES.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)
-        _WORKSPACES[key] = buf
-    return buf
+def sequence_key(v):
+    """`v` as part of a dictionary key: lists and tuples by value."""
+    return tuple(v) if isinstance(v, (list, tuple)) else v
+
+
+class PlanCache(object):
+    """The native plans (descriptor, geometry) of the calls seen last, by everything that determines them.  Bounded: a
+    program that keeps changing shapes starts over after `limit` of them."""
+
+    def __init__(self, limit=1024):
+        self.limit, self.plans = limit, {}
+
+    def get(self, key, make):
+        try:
+            plan = self.plans.get(key)
+        except TypeError:                   # an attribute that cannot be hashed (an array, say): no caching
+            return make()
+        if plan is None:
+            plan = make()
+            if len(self.plans) >= self.limit:
+                self.plans.clear()
+            self.plans[key] = plan
+        return plan
 
 
 class OpProfile(object):
     """Optional per-op device timing: when enabled, every operator call is bracketed by CUDA events on
     the stream it launches on, together with the algorithmic bytes and term count of that call."""
 
-    def __init__(self):
-        self.enabled = False
-        self.rows = {}
-
     def start(self):
-        self.enabled, self.rows = True, {}
+        _lib.ops().profile_start()
 
     def stop(self):
         """Stop recording and return {key: dict(calls, ms, bytes, terms)} (synchronises)."""
-        self.enabled = False
         torch.cuda.synchronize()
         out = {}
-        for key, recs in self.rows.items():
-            out[key] = dict(calls=len(recs), ms=sum(s.elapsed_time(e) for s, e, _, _ in recs),
-                            bytes=sum(r[2] for r in recs), terms=sum(r[3] for r in recs))
-        self.rows = {}
+        for key, ms, nbytes, terms in _lib.ops().profile_stop():
+            r = out.setdefault(key, dict(calls=0, ms=0.0, bytes=0, terms=0))
+            r["calls"] += 1
+            r["ms"] += ms
+            r["bytes"] += int(nbytes)
+            r["terms"] += int(terms)
         return out
 
 
 PROFILE = OpProfile()
-
-
-class timed(object):
-    """`with timed(op, signature, algorithmic_bytes, terms):` around one C-ABI call."""
-
-    def __init__(self, op, sig, nbytes, terms):
-        self.key, self.nbytes, self.terms = "%s[%s]" % (op, sig), nbytes, terms
-
-    def __enter__(self):
-        if PROFILE.enabled:
-            self.s = torch.cuda.Event(enable_timing=True)
-            self.e = torch.cuda.Event(enable_timing=True)
-            self.s.record()
-        return self
-
-    def __exit__(self, *exc):
-        if PROFILE.enabled and exc[0] is None:
-            self.e.record()
-            PROFILE.rows.setdefault(self.key, []).append((self.s, self.e, self.nbytes, self.terms))
-        return False

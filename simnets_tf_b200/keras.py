@@ -13,12 +13,10 @@ import numpy as np
 import torch
 
 from . import _lib, abi
-from .ops.mex import _expand_dim_specification, _mex_dims_helper
-from .ops.mex import mex as _mex
-from .ops.mex import mex_sum_pool2 as _mex_sum_pool2
-from .ops.mex import mex_in_workspace as _mex_in_workspace, mex_layer_workspace_for as _mex_layer_workspace_for
-from .ops.mex import mex_workspace_maxima as _mex_workspace_maxima
-from .ops.similarity import similarity_of_raw_weights as _similarity_of_raw_weights
+from . import _torch_glue
+from .ops.mex import _attrs as _mex_attrs, _expand_dim_specification, _mex_dims_helper
+from .ops.mex import mex_plan as _mex_plan, mex_with_plan as _mex_with_plan
+from .ops.similarity import similarity_of_raw_weights as _similarity_of_raw_weights, _attrs as _similarity_attrs, similarity_plan as _similarity_plan
 
 
 def _sinks(*params):
@@ -98,6 +96,17 @@ class Similarity(torch.nn.Module):
         out = [shape[0], self.num_instances, oh.value, ow.value]
         return tuple([out[0], out[2], out[3], out[1]] if self.channels_last else out)
 
+    def _op_attrs(self):
+        return dict(similarity_function=self.similarity_function, blocks=self.blocks, strides=self.strides, padding=self.padding,
+                    normalization_term=self.normalization_term, normalization_term_fudge=self.normalization_term_fudge,
+                    ignore_nan_input=self.ignore_nan_input, out_of_bounds_value=self.out_of_bounds_value)
+
+    def output_shape_for(self, x):
+        """Shape of `forward(x)` for a channels-first tensor (the layer is built on first use, as in `forward`)."""
+        if self.templates is None:
+            self.build(tuple(x.shape), x.device, x.dtype)
+        return _similarity_plan(x, self.templates, self.sweights, _similarity_attrs(**self._op_attrs())).out_shape
+
     def forward(self, x, extrema=None):
         """extrema=(max_address, min_address): also write the per-pixel maximum / minimum of the output over the
         templates to those device addresses (see Mex.extrema_slot)."""
@@ -106,12 +115,8 @@ class Similarity(torch.nn.Module):
         if self.channels_last:
             x = x.permute(0, 3, 1, 2)
         # |weights| and its gradient are taken inside the op's kernels
-        y = _similarity_of_raw_weights(x, self.templates, self.sweights, similarity_function=self.similarity_function,
-                                       blocks=self.blocks, strides=self.strides, padding=self.padding,
-                                       normalization_term=self.normalization_term,
-                                       normalization_term_fudge=self.normalization_term_fudge,
-                                       ignore_nan_input=self.ignore_nan_input, out_of_bounds_value=self.out_of_bounds_value,
-                                       extrema=extrema, grad_sinks=_sinks(self.templates, self.sweights))
+        y = _similarity_of_raw_weights(x, self.templates, self.sweights, extrema=extrema, grad_sinks=_sinks(self.templates, self.sweights),
+                                       **self._op_attrs())
         return y.permute(0, 2, 3, 1) if self.channels_last else y
 
     def get_config(self):
@@ -254,7 +259,6 @@ class Mex(torch.nn.Module):
         # with respect to the raw values); otherwise effective_offsets() does it in front of the op
         fused = self.normalize_offsets and dtype == torch.float32 and device.type == "cuda" and self.offsets is not None and \
             self.offsets.dtype == torch.float32 and self.offsets.is_cuda
-        from . import _torch_glue
         if _torch_glue.DEFAULT_FLAGS & (abi.FLAG_FORCE_DIRECT | abi.FLAG_MEX_EXACT):
             fused = False           # those routes run without a workspace, which the fused normalisation needs
         return abi.FLAG_MEX_NORMALIZED_OFFSETS if fused else 0
@@ -272,10 +276,14 @@ class Mex(torch.nn.Module):
         b, c, h, w = [int(e) for e in input_shape]
         if list(self.blocks) != [c, 1, 1] or list(self.strides)[1:] != [1, 1] or any(int(p) != 0 for p in self.padding) or b == 0:
             return None
-        ws = _mex_layer_workspace_for((b, c, h, w), dtype, device, self.num_instances, pooled=sum_pool2, flags=self._op_flags(dtype, device),
-                                      **self._op_attrs())
-        ptr = _mex_workspace_maxima((b, c, h, w), dtype, self.num_instances, ws, flags=self._op_flags(dtype, device), **self._op_attrs())
-        return None if ptr is None else (ws, ptr, float(self.epsilon) > 0)
+        op_flags = self._op_flags(dtype, device)
+        plan = self._plan((b, c, h, w), dtype)
+        ws = plan.layer_workspace(op_flags, sum_pool2, device)
+        ptr = plan.maxima(op_flags, ws)
+        return (ws, ptr, float(self.epsilon) > 0) if ptr else None
+
+    def _plan(self, shape, dtype):
+        return _mex_plan(shape, dtype, self.num_instances, _mex_attrs(**self._op_attrs()))
 
     def forward(self, x, sum_pool2=False, layer_ws=None, maxima_given=False):
         """sum_pool2=True returns the 2x2 sum pooling of the layer's output (pooling gradient fused into the
@@ -285,20 +293,11 @@ class Mex(torch.nn.Module):
         if self.channels_last:
             x = x.permute(0, 3, 1, 2)
         op_flags = self._op_flags(x.dtype, x.device) if x.shape[0] > 0 else 0
-        if layer_ws is not None or op_flags:
-            sink = _sinks(self.offsets) if op_flags else None       # (the raw offsets are the op's own input only when it normalises them)
-            y = _mex_in_workspace(x, self.offsets if op_flags else self.effective_offsets(), self.num_instances, layer_ws,
-                                  fwd_flags=abi.FLAG_MEX_MAXIMA_GIVEN if maxima_given else 0, op_flags=op_flags, sum_pool2=sum_pool2,
-                                  grad_sink=sink[0] if sink else None, **self._op_attrs())
-            return y.permute(0, 2, 3, 1) if self.channels_last else y
-        op = _mex_sum_pool2 if sum_pool2 else _mex
-        y = op(x, self.effective_offsets(), self.num_instances, blocks=self.blocks, padding=self.padding,
-                 strides=self.strides, use_unshared_regions=self.use_unshared_regions,
-                 shared_offset_region=self.shared_offset_region,
-                 blocks_out_of_bounds_value=self.blocks_out_of_bounds_value,
-                 blocks_round_down=self.blocks_round_down,
-                 unshared_offset_region=self.unshared_offset_region,
-                 epsilon=self.epsilon, softmax_mode=self.softmax_mode)
+        _torch_glue.dtype_code(x)                   # (rejects anything but float32 / float64)
+        # (the raw offsets are the op's own input, and a gradient bucket its target, only when the op normalises them)
+        sink = _sinks(self.offsets) if op_flags else None
+        y = _mex_with_plan(self._plan(x.shape, x.dtype), x, self.offsets if op_flags else self.effective_offsets(), layer_ws,
+                           abi.FLAG_MEX_MAXIMA_GIVEN if maxima_given else 0, op_flags, sum_pool2, sink[0] if sink else None)
         return y.permute(0, 2, 3, 1) if self.channels_last else y
 
     def get_config(self):

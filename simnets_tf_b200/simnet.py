@@ -108,7 +108,7 @@ class SimNet(torch.nn.Module):
                 # Similarity -> MEX over the channels of each pixel: the Similarity kernel leaves the per-pixel extrema of its
                 # output in the MEX layer's workspace, and the MEX forward pass skips its pass over that tensor
                 nxt = plan[i + 1][1]
-                slot = nxt.extrema_slot(mod.compute_output_shape(tuple(x.shape)), x.dtype, x.device, sum_pool2=pooled_next(i + 1))
+                slot = None if mod.channels_last else nxt.extrema_slot(mod.output_shape_for(x), x.dtype, x.device, sum_pool2=pooled_next(i + 1))
                 if slot is not None:
                     ws, ptr, up = slot
                     x = mod(x, extrema=(ptr, None) if up else (None, ptr))
