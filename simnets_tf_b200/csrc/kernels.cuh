@@ -1,5 +1,6 @@
 // Internal launch interface between the C ABI layer (api.cu) and the kernel translation units.
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include "simnets_b200.h"
@@ -53,6 +54,13 @@ cudaError_t launch_sim_fwd_tc(const SimGeo&, const float* x, const float* planes
 cudaError_t launch_sim_dx_tiled(const SimGeo&, const float* x, const float* t, const float* w, const float* dy, float* dx, void* ws, cudaStream_t);
 cudaError_t launch_sim_dparams_tiled(const SimGeo&, const float* x, const float* t, const float* w, const float* dy,
                                      float* dt, float* dw, bool accumulate, void* ws, cudaStream_t);
+// sim_dparams.cu
+int sim_dparams_splits(const SimGeo&);
+cudaError_t launch_sim_dparams(const SimGeo&, const float* x, const float* t, const float* w, const float* dy, float* dt, float* dw,
+                               bool accumulate, float* part, cudaStream_t);
+// sim_dx.cu
+size_t sim_dx_scratch_floats(const SimGeo&);
+cudaError_t launch_sim_dx(const SimGeo&, const float* x, const float* t, const float* w, const float* dy, float* dx, float* dxp, cudaStream_t);
 // sim_smallk.cu -- forward for short patches (K <= 32): patches in registers, two positions per thread
 bool sim_smallk_shape(const SimGeo&);
 cudaError_t launch_sim_fwd_smallk(const SimGeo&, const float* x, const float* planes, const float* cm, const int2* taps, float* y,

@@ -1,0 +1,322 @@
+// Similarity parameter gradients (float32): per template m and tap k, over all output positions of the batch,
+//
+//     sT = sum a d,   sW = sum a d^2   (L1: sum a sign(d), sum a |d|),   sN = sum a [x is a number],   a = dy, d = x - t
+//
+// as a generalized GEMM with rows m, columns k and positions as the reduction index (the reference's element functors:
+// HUJI-Deep/simnets-tf include/utils/similarity_utils.hpp:64-119; no patch matrix).
+//
+// Bound: the FP32 pipe, 4 lane operations per term (5 with missing data).  A CTA of 256 threads owns 32 templates x up to
+// 64 taps, a thread 4 x 2 of them with all its sums in registers: few enough registers for 16 warps per SM, which the chain
+// difference -> product -> sums needs (4 x 4 per thread at 12 warps stalled on that chain: FP32 pipe 53 % busy).
+// Both operands are contiguous along positions in memory and stay that way in shared memory ([row][position], rows padded by
+// four floats so that eight rows of one 16-byte read hit 32 different banks): nothing is transposed, and the packed FP32
+// instructions pair two positions, so that no operand needs to be duplicated into both halves.  When the patch is short, the
+// threads cover the tile several times over and the copies split the positions of a chunk among themselves (K = 4: sixteen
+// ways).  Partial sums of the splits are added in split order.
+#include "kernels.cuh"
+#include "tile.cuh"
+
+namespace simnets {
+namespace {
+
+constexpr int kDpThreads = 256, kDpMaxK2 = 32, kDpCtasPerSm = 2;
+
+struct DpTile { int k2, groups, tm, kc; };       // tap columns / 2, copies of the tile per CTA, templates per tile, positions per chunk
+
+// Tile of a patch of K taps: the patch in n equal tiles of at most 64 taps, n the smallest that keeps nearly as many threads
+// busy as the best does (K = 36: one tile would leave 112 of 256 threads idle, three of 12 none).  Up to 32 taps a tile takes
+// 64 templates, so that a thread still stages few values per term (K = 27 at 32 templates: 906 us instead of the figure
+// below).  The chunk is long enough that every copy of the tile gets a quad of positions.
+__host__ inline DpTile dp_tile(const SimGeo& g) {
+    DpTile best = {1, 1, 32, 64};
+    double best_busy = 0;
+    const int first = (g.K + 2 * kDpMaxK2 - 1) / (2 * kDpMaxK2), last = std::max(first, std::min(first + 3, (g.K + 11) / 12));
+    for (int n = first; n <= last; ++n) {
+        DpTile t;
+        t.k2 = ((g.K + n - 1) / n + 1) / 2;
+        t.tm = g.M > 32 && t.k2 >= 2 && t.k2 <= 16 ? 64 : 32;
+        t.kc = t.tm == 32 && t.k2 <= 8 ? 64 : 32;
+        const int one = t.tm / 4 * t.k2;
+        t.groups = std::min(kDpThreads / one, t.kc / 4);
+        const int quads = t.kc / 4, rounds = (quads + t.groups - 1) / t.groups;
+        const double busy = double(g.K) / (2.0 * t.k2 * n) * (double(one) * quads) / (double(rounds) * kDpThreads);
+        if (busy > 1.05 * best_busy) { best_busy = busy; best = t; }
+    }
+    return best;
+}
+__host__ inline int dp_tiles(const SimGeo& g, const DpTile& t) { return ((g.M + t.tm - 1) / t.tm) * ((g.K + 2 * t.k2 - 1) / (2 * t.k2)); }
+
+__device__ __forceinline__ float2 dp_abs2(float2 v) { return make_float2(fabsf(v.x), fabsf(v.y)); }
+// sign of d, 0 for 0 and NaN as in the reference: 1.0 with d's sign bit, or 0 (two conversions of comparisons cost twice this)
+__device__ __forceinline__ float dp_sign(float d) { return fabsf(d) > 0.f ? __uint_as_float(0x3f800000u | (__float_as_uint(d) & 0x80000000u)) : 0.f; }
+
+template <int MODE, int KC, int MAXK, int TM>
+__global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g, FastDiv f_N, FastDiv f_ow, DpTile tile, const float* __restrict__ x,
+                                                             const float* __restrict__ tm, const float* __restrict__ dy,
+                                                             float* __restrict__ part, int splits) {
+    constexpr bool MASKED = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
+    constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
+    constexpr int LD = KC + 4, TI = TM / 4;                                           // row stride, floats
+    constexpr int A_PER = TM * KC / kDpThreads, B_PER = MAXK * KC / kDpThreads, ROWS = kDpThreads / KC;
+    constexpr int A_FLOATS = TM * LD, B_FLOATS = MAXK * LD, STAGE = A_FLOATS + (MASKED ? 2 : 1) * B_FLOATS;
+    static_assert(2 * STAGE >= 3 * TM * MAXK || MAXK == 64, "the copies' sums are added up in the stages");
+    __shared__ __align__(16) float smem[2 * STAGE];
+    __shared__ int2 taps[MAXK];                                          // {byte offset inside a sample, kh << 16 | kw}
+
+    const long long P = (long long)g.B * g.N;
+    const int TK = 2 * tile.k2, ktiles = (g.K + TK - 1) / TK, mtiles = (g.M + TM - 1) / TM;
+    int bid = blockIdx.x;
+    const int kt = bid % ktiles; bid /= ktiles;
+    const int mt = bid % mtiles, split = bid / mtiles;
+    const int m0 = mt * TM, k0 = kt * TK;
+    const long long chunks = (P + KC - 1) / KC;
+    const long long c_begin = chunks * split / splits, c_end = chunks * (split + 1) / splits;
+
+    for (int i = threadIdx.x; i < MAXK; i += kDpThreads) {
+        const int k = k0 + i;
+        const int kw = k % g.bw, kh = (k / g.bw) % g.bh, c = k / (g.bw * g.bh);
+        taps[i] = k < g.K ? make_int2(4 * ((c * g.H + kh) * g.W + kw), (kh << 16) | kw) : make_int2(0, 0);     // (columns past K: any tap)
+    }
+
+    const int G = TI * tile.k2, group = threadIdx.x / G, lid = threadIdx.x - group * G;
+    const bool worker = group < tile.groups;
+    const int ti = lid & (TI - 1), tj = lid / TI;                        // rows ti + TI r, columns tj + k2 c
+    float2 tt[4][2], sT[4][2], sW[4][2], sN[4][MASKED ? 2 : 1];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int m = m0 + ti + TI * r, k = k0 + tj + tile.k2 * c;
+            tt[r][c] = splat2((worker && m < g.M && k < g.K) ? -tm[(size_t)m * g.K + k] : 0.f);
+            sT[r][c] = sW[r][c] = make_float2(0.f, 0.f);
+            sN[r][MASKED ? c : 0] = make_float2(0.f, 0.f);
+        }
+
+    // staging: this thread brings position q of every chunk, rows e, e + ROWS, ...
+    const int q = threadIdx.x % KC, e = threadIdx.x / KC;
+    const float oob = float(g.oob);
+    float ra[A_PER], rb[B_PER];
+    // rows of dy this thread brings (bit s: row e + ROWS s exists) and the first of them
+    uint32_t a_rows = 0;
+#pragma unroll
+    for (int s = 0; s < A_PER; ++s) a_rows |= uint32_t(m0 + e + ROWS * s < g.M) << s;
+    const char* dy0 = reinterpret_cast<const char*>(dy) + 4 * (long long)(m0 + e) * g.N;
+    const size_t a_step = 4 * (size_t)ROWS * g.N;
+    auto fetch = [&](long long chunk) {
+        const long long j = chunk * KC + q;
+        const bool live = j < P;
+        int n = 0, pos = 0;
+        if (live) {
+            if (P <= 0x7fffffffLL) { n = int(fast_div(uint32_t(j), f_N)); pos = int(j) - n * g.N; }
+            else { n = int(j / g.N); pos = int(j - (long long)n * g.N); }
+        }
+        const int ho = int(fast_div(uint32_t(pos), f_ow)), wo = pos - ho * g.ow;
+        const char* a = dy0 + 4 * ((long long)n * g.M * g.N + pos);
+        const uint32_t rows = live ? a_rows : 0u;
+#pragma unroll
+        for (int s = 0; s < A_PER; ++s, a += a_step) {
+            ra[s] = 0.f;
+            if ((rows >> s) & 1u) ra[s] = __ldg(reinterpret_cast<const float*>(a));
+        }
+        // dead positions (dy = 0) and columns past K (sums nobody reads) pair with any finite value: they look outside the image
+        const int h0 = ho * g.sh - g.ph, w0 = wo * g.sw - g.pw, h_seen = live ? h0 : -0x10000;
+        const char* xc = reinterpret_cast<const char*>(x + (size_t)n * g.C * g.H * g.W + h0 * g.W + w0);
+        const float outside = live ? oob : 0.f;
+#pragma unroll
+        for (int s = 0; s < B_PER; ++s) {
+            if (MAXK > 4 && ROWS * s >= TK) { rb[s] = 0.f; continue; }
+            const int2 t = taps[e + ROWS * s];
+            rb[s] = outside;
+            if (uint32_t(h_seen + (t.y >> 16)) < uint32_t(g.H) && uint32_t(w0 + (t.y & 0xffff)) < uint32_t(g.W))
+                rb[s] = __ldg(reinterpret_cast<const float*>(xc + t.x));
+        }
+    };
+    auto commit = [&](float* stage) {
+#pragma unroll
+        for (int s = 0; s < A_PER; ++s) stage[(e + ROWS * s) * LD + q] = ra[s];
+        float* B = stage + A_FLOATS;
+#pragma unroll
+        for (int s = 0; s < B_PER; ++s) {
+            const int o = (e + ROWS * s) * LD + q;
+            if (MASKED) {
+                const bool nan = rb[s] != rb[s];
+                B[o] = nan ? 0.f : rb[s];
+                B[B_FLOATS + o] = nan ? 0.f : 1.f;
+            } else {
+                B[o] = rb[s];
+            }
+        }
+    };
+    auto compute = [&](const float* stage) {
+        const float* A = stage + ti * LD;
+        const float* B = stage + A_FLOATS + tj * LD;
+#pragma unroll 1
+        for (int qd = group; qd < KC / 4; qd += tile.groups) {
+            float4 a[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + TI * r * LD + qd * 4);
+            if (MODE == SIM_L2N) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    // (sum of dy per template: the normalisation term's, the same for every tap)
+                    sN[r][0] = add2(sN[r][0], add2(make_float2(a[r].x, a[r].y), make_float2(a[r].z, a[r].w)));
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float4 b = *reinterpret_cast<const float4*>(B + c * tile.k2 * LD + qd * 4);
+                float4 k4v;
+                if (MASKED) k4v = *reinterpret_cast<const float4*>(B + B_FLOATS + c * tile.k2 * LD + qd * 4);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const float2 b2 = half ? make_float2(b.z, b.w) : make_float2(b.x, b.y);
+                    float2 k2;
+                    if (MASKED) k2 = half ? make_float2(k4v.z, k4v.w) : make_float2(k4v.x, k4v.y);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const float2 a2 = half ? make_float2(a[r].z, a[r].w) : make_float2(a[r].x, a[r].y);
+                        const float2 d = MASKED ? fma2(tt[r][c], k2, b2) : add2(b2, tt[r][c]);
+                        if (L1) {
+                            sT[r][c] = fma2(a2, make_float2(dp_sign(d.x), dp_sign(d.y)), sT[r][c]);
+                            sW[r][c] = fma2(a2, dp_abs2(d), sW[r][c]);
+                        } else {
+                            const float2 u = mul2(a2, d);
+                            sT[r][c] = add2(sT[r][c], u);
+                            sW[r][c] = fma2(u, d, sW[r][c]);
+                            if (MASKED) sN[r][MASKED ? c : 0] = fma2(a2, k2, sN[r][MASKED ? c : 0]);
+                        }
+                    }
+                }
+            }
+        }
+    };
+
+    __syncthreads();                                                     // the tap table
+    const int n_chunks = int(c_end - c_begin);
+    if (n_chunks > 0) {
+        fetch(c_begin);
+        commit(smem);
+        __syncthreads();
+        for (int i = 0; i < n_chunks; ++i) {
+            float* now = smem + (i & 1) * STAGE;
+            float* next = smem + ((i + 1) & 1) * STAGE;
+            const bool more = i + 1 < n_chunks;
+            if (more) fetch(c_begin + i + 1);
+            if (worker) compute(now);
+            if (more) commit(next);
+            __syncthreads();
+        }
+    }
+
+    // the copies' sums, one after the other; then this split's partial sums
+    const size_t mk = (size_t)g.M * g.K;
+    float* dst = part + (size_t)split * 3 * mk;
+    const int last = tile.groups - 1;
+    for (int grp = 0; grp <= last; ++grp) {
+        if (group == grp) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float v[3] = {sT[r][c].x + sT[r][c].y, sW[r][c].x + sW[r][c].y, 0.f};
+                    if (MASKED && !L1) v[2] = sN[r][MASKED ? c : 0].x + sN[r][MASKED ? c : 0].y;
+                    else if (!L1) v[2] = sN[r][0].x + sN[r][0].y;
+                    const int row = ti + TI * r, col = tj + tile.k2 * c, m = m0 + row, k = k0 + col;
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        float* s = smem + (p * TM + row) * TK + col;
+                        if (grp > 0) v[p] += *s;
+                        if (grp < last) *s = v[p];
+                        else if (m < g.M && k < g.K) dst[p * mk + (size_t)m * g.K + k] = v[p];
+                    }
+                }
+        }
+        if (grp < last) __syncthreads();
+    }
+}
+
+// Sums the splits' partial sums in split order and applies the per-parameter factors of the backward functors.  512 threads =
+// `slices` slices of the splits x 512 / slices consecutive outputs; the slices are added in a fixed order (same sums on every
+// run).  Many splits (short patches: K = 27, 222 splits): 64 slices, so that the few outputs still spread over a couple of
+// hundred CTAs; few splits (K = 576: 6): 8 slices, 64 outputs per CTA.
+__global__ void __launch_bounds__(512) sim_dparams_reduce(SimGeo g, int splits, int slices, const float* __restrict__ part,
+                                                          const float* __restrict__ wt, float* __restrict__ dt, float* __restrict__ dw,
+                                                          int accumulate) {
+    __shared__ float red[3][512];
+    const int mk = g.M * g.K, lanes = 512 / slices;
+    const float fudge = float(g.fudge);
+    const bool third = g.mode == SIM_L2N || g.mode == SIM_L2N_NAN;
+    const int lane = threadIdx.x & (lanes - 1), slice = threadIdx.x / lanes;
+    for (int first = blockIdx.x * lanes; first < mk; first += gridDim.x * lanes) {
+        const int i = first + lane;
+        float a = 0.f, b = 0.f, c = 0.f;
+        if (i < mk) {
+#pragma unroll 4
+            for (int s = slice; s < splits; s += slices) {
+                const float* p = part + (size_t)s * 3 * mk;
+                a += p[i]; b += p[mk + i];
+                if (third) c += p[2 * mk + i];
+            }
+        }
+        red[0][threadIdx.x] = a; red[1][threadIdx.x] = b; red[2][threadIdx.x] = c;
+        __syncthreads();
+        if (slice == 0 && i < mk) {
+#pragma unroll 8
+            for (int q = 1; q < slices; ++q) { a += red[0][q * lanes + lane]; b += red[1][q * lanes + lane]; c += red[2][q * lanes + lane]; }
+            const float wraw = wt[i], w = g.absw ? fabsf(wraw) : wraw;
+            float gt, gw;
+            if (g.mode == SIM_L1 || g.mode == SIM_L1_SKIP) { gt = w * a; gw = -b; }
+            else if (g.mode == SIM_L2) { gt = 2.f * w * a; gw = -b; }
+            else { gt = w * a; gw = 0.5f * (c / (w + fudge) - b); }
+            if (g.absw) gw *= wraw > 0.f ? 1.f : (wraw < 0.f ? -1.f : 0.f);          // d|w|/dw, 0 at w = 0
+            dt[i] = accumulate ? dt[i] + gt : gt;
+            dw[i] = accumulate ? dw[i] + gw : gw;
+        }
+        __syncthreads();
+    }
+}
+
+}  // namespace
+
+// How many ways the positions are split: one wave of the CTAs that fit the GPU at once, fewer where a split would hold under 256
+// positions (its partial sums are 3 M K floats written and read again).
+int sim_dparams_splits(const SimGeo& g) {
+    const DpTile t = dp_tile(g);
+    const long long P = (long long)g.B * g.N, chunks = (P + t.kc - 1) / t.kc, tiles = dp_tiles(g, t);
+    long long s = (device_sm_count() * kDpCtasPerSm) / tiles;
+    s = std::min(s, std::max<long long>(1, P / 256));
+    return int(std::max<long long>(1, std::min(s, chunks)));
+}
+
+cudaError_t launch_sim_dparams(const SimGeo& g, const float* x, const float* t, const float* w, const float* dy, float* dt, float* dw,
+                               bool accumulate, float* part, cudaStream_t s) {
+    if ((long long)g.C * g.H * g.W >= (1LL << 29)) return launch_sim_dparams_direct(g, false, x, t, w, dy, dt, dw, accumulate, s);    // (32-bit byte offsets)
+    const DpTile tile = dp_tile(g);
+    const int splits = sim_dparams_splits(g);
+    const long long blocks = (long long)dp_tiles(g, tile) * splits;
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    const FastDiv f_N = make_fastdiv(g.N), f_ow = make_fastdiv(g.ow);
+#define DP_TILE(MODE, KC, MAXK, TM) sim_dparams<MODE, KC, MAXK, TM><<<int(blocks), kDpThreads, 0, s>>>(g, f_N, f_ow, tile, x, t, dy, part, splits)
+#define DP(MODE)                                            \
+    do {                                                    \
+        if (tile.tm == 64) DP_TILE(MODE, 32, 32, 64);       \
+        else if (tile.kc == 64) DP_TILE(MODE, 64, 16, 32);  \
+        else if (tile.k2 <= 16) DP_TILE(MODE, 32, 32, 32);  \
+        else DP_TILE(MODE, 32, 64, 32);                     \
+    } while (0)
+    switch (g.mode) {
+    case SIM_L1: DP(SIM_L1); break;
+    case SIM_L1_SKIP: DP(SIM_L1_SKIP); break;
+    case SIM_L2: DP(SIM_L2); break;
+    case SIM_L2N: DP(SIM_L2N); break;
+    default: DP(SIM_L2N_NAN); break;
+    }
+#undef DP
+#undef DP_TILE
+    const int mk = g.M * g.K, slices = splits >= 64 ? 64 : 8, lanes = 512 / slices;
+    sim_dparams_reduce<<<std::min((mk + lanes - 1) / lanes, device_sm_count() * 8), 512, 0, s>>>(g, splits, slices, part, w, dt, dw, accumulate);
+    count_launch(2);
+    return cudaGetLastError();
+}
+
+}  // namespace simnets
