@@ -61,10 +61,10 @@ cudaError_t launch_sim_dparams(const SimGeo&, const float* x, const float* t, co
 // sim_dx.cu
 size_t sim_dx_scratch_floats(const SimGeo&);
 cudaError_t launch_sim_dx(const SimGeo&, const float* x, const float* t, const float* w, const float* dy, float* dx, float* dxp, cudaStream_t);
-// sim_smallk.cu -- forward for short patches (K <= 32): patches in registers, two positions per thread
+// sim_smallk.cu -- forward for short patches (K <= 32): patches in registers; extrema_done: ch_max / ch_min were written too
 bool sim_smallk_shape(const SimGeo&);
-cudaError_t launch_sim_fwd_smallk(const SimGeo&, const float* x, const float* planes, const float* cm, const int2* taps, float* y,
-                                  float* ch_max, float* ch_min, cudaStream_t);
+cudaError_t launch_sim_fwd_smallk(const SimGeo&, const float* x, const float* t, const float* w, float* y, float* ch_max, float* ch_min,
+                                  bool* extrema_done, int* flag, cudaStream_t);
 bool mex_use_tiled(const MexGeo&, bool f64, uint32_t flags);
 size_t mex_workspace_bytes(const MexGeo&, bool f64, uint32_t flags);
 // pooled: when given, the 2x2 sum pooling of y is produced as well (fused into the pair-tile kernel, a pooling launch behind the others)

@@ -10,6 +10,7 @@
 // the NaN itself is staged and propagates through the arithmetic exactly as in the reference.
 // Per-(m,k) constants (0.5*log(w + fudge) - 0.5*log(2*pi), -w, -0.5*w) are computed once by a prepass,
 // which also lays the parameters out tap-major so that the forward kernel's loads are contiguous.
+#include <cmath>
 #include "kernels.cuh"
 #include "tile.cuh"
 
@@ -114,12 +115,20 @@ template <int MODE> struct FwdPlanes {
 
 __device__ __forceinline__ float2 abs2(float2 v) { return make_float2(fabsf(v.x), fabsf(v.y)); }
 
-template <int TM, int MODE>
-__global__ void __launch_bounds__(256, TM == 128 ? 2 : 1) sim_fwd_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ planes,
+// Tile TM x TN, 8 x 8, 4 x 8 or 4 x 4 outputs per thread; small tiles walk 16 taps per chunk (their chunks are short, and every
+// chunk costs a round trip to L2).
+template <int TM, int TN> struct FwdTile {
+    static constexpr int RM = TM == 128 ? 8 : 4, RN = TN == 128 ? 8 : 4, KC = TM * TN <= 2048 ? 16 : 8, THREADS = (TM / RM) * (TN / RN);
+    static constexpr int PER_SM = TM == 128 ? 2 : (TN == 128 ? 1 : 512 / THREADS);
+};
+
+template <int TM, int TN, int MODE>
+__global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER_SM) sim_fwd_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ planes,
                                                      const float* __restrict__ cm, const int2* __restrict__ taps, float* __restrict__ y) {
     constexpr int NA = FwdPlanes<MODE>::NA, NB = FwdPlanes<MODE>::NB;
-    using Cfg = TileCfg<TM, 128, 8, TM / 16, 8, NA, NB>;
-    static_assert(Cfg::THREADS == 256, "256 threads");
+    using Cfg = TileCfg<TM, TN, FwdTile<TM, TN>::KC, FwdTile<TM, TN>::RM, FwdTile<TM, TN>::RN, NA, NB>;
+    constexpr int QSTEP = Cfg::THREADS / TN;                     // threads along the taps when a chunk is staged
+    static_assert(QSTEP >= 1 && Cfg::THREADS % TN == 0, "a thread stages one column");
     __shared__ __align__(16) float smem[Cfg::SMEM_FLOATS];
     __shared__ long long col_base[Cfg::TN];
     const long long P = (long long)g.B * g.N;
@@ -133,7 +142,7 @@ __global__ void __launch_bounds__(256, TM == 128 ? 2 : 1) sim_fwd_tiled(SimGeo g
     const float oob = float(g.oob);
     const int ldm = pad4(g.M);
     const size_t plane = (size_t)g.K * ldm;
-    const int s_lane = threadIdx.x % 128, s_k = threadIdx.x / 128;
+    const int s_lane = threadIdx.x % TN, s_k = threadIdx.x / TN;
     const SimColumn sc = sim_column(g, j0 + s_lane, P);
     if (s_k == 0) col_base[s_lane] = sc.base;
     const bool live = sc.base >= 0;
@@ -157,7 +166,7 @@ __global__ void __launch_bounds__(256, TM == 128 ? 2 : 1) sim_fwd_tiled(SimGeo g
     auto fetchB = [&](int chunk, float*) {
 #pragma unroll
         for (int s = 0; s < Cfg::B_PER; ++s) {
-            const int k = chunk * Cfg::KC + s_k + s * 2;
+            const int k = chunk * Cfg::KC + s_k + s * QSTEP;
             // rows past K pair a zero scale / zero constant with a finite value: the term is exactly 0
             if (k >= g.K || !live) rb[s] = 0.f;
             else if (inside) rb[s] = __ldg(xc + __ldg(taps + k).x);
@@ -168,7 +177,7 @@ __global__ void __launch_bounds__(256, TM == 128 ? 2 : 1) sim_fwd_tiled(SimGeo g
     auto commitB = [&](float* Bs) {
 #pragma unroll
         for (int s = 0; s < Cfg::B_PER; ++s) {
-            const int o = (s_k + s * 2) * Cfg::TN + s_lane;
+            const int o = (s_k + s * QSTEP) * Cfg::TN + s_lane;
             if (NB == 2) {
                 const bool nan = rb[s] != rb[s];
                 Bs[o] = nan ? 0.f : rb[s];
@@ -243,6 +252,7 @@ cudaError_t launch_sim_fwd_tiled(const SimGeo& g, const float* x, const float* t
 static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const float* t, const float* w, float* y, void* ws, uint32_t flags,
                                       cudaStream_t s, float* ch_max, float* ch_min, bool* extrema_done) {
     const SimWs W = carve(g, ws);
+    if (!sim_tc_shape(g, flags) && sim_smallk_shape(g)) return launch_sim_fwd_smallk(g, x, t, w, y, ch_max, ch_min, extrema_done, W.flag, s);
     launch_prep(g, W, t, w, s);
     if (sim_tc_shape(g, flags)) {
         // opt-in: the expanded square on the tensor cores; behind it the term-by-term kernel, which runs only if a
@@ -251,21 +261,31 @@ static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const flo
         if (e != cudaSuccess) return e;
         return launch_sim_fwd_direct(g, false, x, t, w, y, s, W.flag);
     }
-    if (sim_smallk_shape(g)) { *extrema_done = true; return launch_sim_fwd_smallk(g, x, W.planes, W.cm, W.taps, y, ch_max, ch_min, s); }
     const long long P = (long long)g.B * g.N;
-    const bool wide = g.M > 64;
-    const long long blocks = ((P + 127) / 128) * ((g.M + (wide ? 127 : 63)) / (wide ? 128 : 64));
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-#define FWD(TM, MODE) sim_fwd_tiled<TM, MODE><<<int(blocks), 256, 0, s>>>(g, x, W.planes, W.cm, W.taps, y)
-#define FWD_MODES(TM)                                        \
-    switch (g.mode) {                                        \
-    case SIM_L1: FWD(TM, SIM_L1); break;                     \
-    case SIM_L1_SKIP: FWD(TM, SIM_L1_SKIP); break;           \
-    case SIM_L2: FWD(TM, SIM_L2); break;                     \
-    case SIM_L2N: FWD(TM, SIM_L2N); break;                   \
-    default: FWD(TM, SIM_L2N_NAN); break;                    \
+    // The tile with the least estimated time: tiles per SM (rounded up) x outputs per tile x the relative cost of a term at
+    // that tile's register blocking, stretched where too few warps are resident to keep the FP32 pipe fed (the larger tiles on
+    // small inputs: 16 x 20 x 20 inputs under 48 templates fill 56 tiles of 64 x 128 on 148 SMs).
+    struct { int tm, tn, threads; double cost; } const tiles[] = {{128, 128, 256, 1.0}, {64, 128, 256, 1.05}, {32, 64, 128, 1.6}, {16, 32, 32, 2.0}};
+    int pick = 0;
+    double best = 0;
+    for (int i = 0; i < 4; ++i) {
+        const double ctas = double((P + tiles[i].tn - 1) / tiles[i].tn) * ((g.M + tiles[i].tm - 1) / tiles[i].tm);
+        const double per_sm = std::ceil(ctas / device_sm_count()), warps = per_sm * tiles[i].threads / 32;
+        const double t = per_sm * tiles[i].tm * tiles[i].tn * tiles[i].cost * (warps < 8 ? 8 / warps : 1.0);
+        if (i == 0 || t < best) { best = t; pick = i; }
     }
-    if (wide) { FWD_MODES(128) } else { FWD_MODES(64) }
+    const long long blocks = ((P + tiles[pick].tn - 1) / tiles[pick].tn) * ((g.M + tiles[pick].tm - 1) / tiles[pick].tm);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+#define FWD(TM, TN, MODE) sim_fwd_tiled<TM, TN, MODE><<<int(blocks), FwdTile<TM, TN>::THREADS, 0, s>>>(g, x, W.planes, W.cm, W.taps, y)
+#define FWD_MODES(TM, TN)                                        \
+    switch (g.mode) {                                            \
+    case SIM_L1: FWD(TM, TN, SIM_L1); break;                     \
+    case SIM_L1_SKIP: FWD(TM, TN, SIM_L1_SKIP); break;           \
+    case SIM_L2: FWD(TM, TN, SIM_L2); break;                     \
+    case SIM_L2N: FWD(TM, TN, SIM_L2N); break;                   \
+    default: FWD(TM, TN, SIM_L2N_NAN); break;                    \
+    }
+    if (pick == 0) { FWD_MODES(128, 128) } else if (pick == 1) { FWD_MODES(64, 128) } else if (pick == 2) { FWD_MODES(32, 64) } else { FWD_MODES(16, 32) }
 #undef FWD_MODES
 #undef FWD
     count_launch();
