@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     __shared__ long long col_base[2][kResTN];
     __shared__ float row_const[TM];
     __shared__ int2 tp[kResMaxK];
-    __shared__ float red[TI][kResTN];
+    __shared__ __align__(16) float red[2][TI][kResTN];             // the extrema of each thread row, two tiles' worth
     const int K = g.K, i0 = blockIdx.y * TM;
     float* As = sm;
     float* Bs = sm + NA * TM * K;
@@ -229,6 +229,17 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
             }
         }
     };
+    // per-pixel extrema over the instances, for a consumer that stabilises a log-sum-exp over them (NaN ignored); a tile's are
+    // reduced over the thread rows and stored one iteration later, behind the barrier that is there anyway
+    const bool extrema = ch_max != nullptr || ch_min != nullptr, up = ch_max != nullptr;       // (only when one tile of rows holds all templates)
+    auto store_extrema = [&](long long of_tile, int from) {
+        const long long j = of_tile * kResTN + threadIdx.x;
+        if (threadIdx.x >= kResTN || j >= P) return;
+        float v = red[from][0][threadIdx.x];
+#pragma unroll
+        for (int i = 1; i < TI; ++i) v = up ? fmaxf(v, red[from][i][threadIdx.x]) : fminf(v, red[from][i][threadIdx.x]);
+        (up ? ch_max : ch_min)[j] = v;
+    };
     long long tile = blockIdx.x;
     int buf = 0;
     if (tile < tiles) { fetch(tile); commit(0); }
@@ -236,6 +247,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     for (; tile < tiles; tile += gridDim.x, buf ^= 1) {
         const bool more = tile + gridDim.x < tiles;
         if (more) fetch(tile + gridDim.x);
+        if (extrema && tile >= gridDim.x) store_extrema(tile - gridDim.x, buf ^ 1);
         float2 acc[4][4];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
@@ -276,9 +288,9 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
             long long cb[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) cb[u] = col_base[buf][h * (kResTN / 2) + t.tj * 4 + u];
-            float vmax[4], vmin[4];
+            float ext[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) { vmax[u] = -CUDART_INF_F; vmin[u] = CUDART_INF_F; }
+            for (int u = 0; u < 4; ++u) ext[u] = up ? -CUDART_INF_F : CUDART_INF_F;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int m = i0 + t.row(r);
@@ -290,8 +302,10 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
                         v[u] += row_const[m - i0];
                         if (g.batch_quirk) v[u] += quirk_c * float(g.B - 1 - int(cb[u] / ((long long)g.M * g.N)));
                     }
-                    vmax[u] = fmaxf(vmax[u], v[u]);
-                    vmin[u] = fminf(vmin[u], v[u]);
+                }
+                if (extrema) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) ext[u] = up ? fmaxf(ext[u], v[u]) : fminf(ext[u], v[u]);
                 }
                 float* row = y + (long long)m * g.N;
                 if (vec && cb[0] >= 0) {
@@ -301,23 +315,12 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
                     for (int u = 0; u < 4; ++u) if (cb[u] >= 0) __stcs(row + cb[u], v[u]);
                 }
             }
-            if (ch_max != nullptr || ch_min != nullptr) {        // (only when one tile of rows holds all templates)
-#pragma unroll
-                for (int u = 0; u < 4; ++u) red[t.ti][h * (kResTN / 2) + t.tj * 4 + u] = ch_max ? vmax[u] : vmin[u];
-            }
-        }
-        if (ch_max != nullptr || ch_min != nullptr) {
-            __syncthreads();
-            if (threadIdx.x < kResTN && tile * kResTN + threadIdx.x < P) {
-                float v = red[0][threadIdx.x];
-#pragma unroll
-                for (int i = 1; i < TI; ++i) v = ch_max ? fmaxf(v, red[i][threadIdx.x]) : fminf(v, red[i][threadIdx.x]);
-                (ch_max ? ch_max : ch_min)[tile * kResTN + threadIdx.x] = v;
-            }
+            if (extrema) *reinterpret_cast<float4*>(&red[buf][t.ti][h * (kResTN / 2) + t.tj * 4]) = make_float4(ext[0], ext[1], ext[2], ext[3]);
         }
         if (more) commit(buf ^ 1);
         __syncthreads();
     }
+    if (extrema && tile > blockIdx.x) store_extrema(tile - gridDim.x, buf ^ 1);
 }
 
 // The same extrema from a finished output tensor, for the forward kernels that do not produce them on the way
@@ -365,7 +368,7 @@ cudaError_t launch_resident(const SimGeo& g, const float* x, const float* t, con
         opted.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
     }
     const long long tiles = ((long long)g.B * g.N + kResTN - 1) / kResTN;
-    const int mtiles = (g.M + TM - 1) / TM, per_sm = std::min(TM == 64 ? 2 : 4, 220 * 1024 / (smem + 12 * 1024));
+    const int mtiles = (g.M + TM - 1) / TM, per_sm = std::min(TM == 64 ? 2 : 4, 220 * 1024 / (smem + 2 * (TM / 4) * kResTN * int(sizeof(float)) + 4096));
     const int resident = std::max(1, device_sm_count() * per_sm / mtiles);
     const long long rounds = (tiles + resident - 1) / resident;          // equal rounds: as few CTAs as finish in the same number
     const dim3 grid(unsigned((tiles + rounds - 1) / rounds), unsigned(mtiles));
