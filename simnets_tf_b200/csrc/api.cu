@@ -180,7 +180,8 @@ int get_mex_offsets_nregions(int n_input_dim, const int* input_dim, int n_paddin
 size_t simnets_mex_workspace_bytes(const simnets_mex_desc* d) {
     MexGeo g;
     if (mex_geometry(d, nullptr, &g)) return 0;
-    return mex_workspace_bytes(g, d->dtype == SIMNETS_F64, d->flags);
+    if (d->dtype == SIMNETS_F64) return mex_use_f64(g, d->flags) ? mex_f64_workspace_bytes(g) : 256;
+    return mex_workspace_bytes(g, false, d->flags);
 }
 
 int simnets_mex_forward(const simnets_mex_desc* d, const void* x, const void* off, void* y, void* ws, size_t ws_bytes, void* stream) {
@@ -189,7 +190,11 @@ int simnets_mex_forward(const simnets_mex_desc* d, const void* x, const void* of
     if (rc) return rc;
     if (!off || (g.B > 0 && (!x || !y))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
+    if (f64 && mex_use_f64(g, d->flags)) {
+        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_fwd_f64(g, (const double*)x, (const double*)off, (double*)y, ws, d->flags, as_stream(stream)));
+    }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
         return from_cuda(launch_mex_fwd_tiled(g, (const float*)x, (const float*)off, (float*)y, ws, d->flags, as_stream(stream)));
@@ -255,7 +260,11 @@ int simnets_mex_input_grad(const simnets_mex_desc* d, const void* x, const void*
     if (rc) return rc;
     if (!off || (g.B > 0 && (!x || !y || !dy || !dx))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
+    if (f64 && mex_use_f64(g, d->flags)) {
+        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_bwd_f64(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, nullptr, false, ws, d->flags, as_stream(stream)));
+    }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
         return from_cuda(launch_mex_dx_tiled(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx,
@@ -271,8 +280,12 @@ int simnets_mex_offsets_grad(const simnets_mex_desc* d, const void* x, const voi
     if (rc) return rc;
     if (!off || !doff || (g.B > 0 && (!x || !y || !dy))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
     const bool acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
+    if (f64 && mex_use_f64(g, d->flags)) {
+        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_bwd_f64(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, nullptr, (double*)doff, acc, ws, d->flags, as_stream(stream)));
+    }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
         return from_cuda(launch_mex_doff_tiled(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy,
@@ -288,8 +301,12 @@ int simnets_mex_backward(const simnets_mex_desc* d, const void* x, const void* o
     if (rc) return rc;
     if (!off || !doff || (g.B > 0 && (!x || !y || !dy || !dx))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
     const bool acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
+    if (f64 && mex_use_f64(g, d->flags)) {
+        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_bwd_f64(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, (double*)doff, acc, ws, d->flags, as_stream(stream)));
+    }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
         return from_cuda(launch_mex_backward_tiled(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy,

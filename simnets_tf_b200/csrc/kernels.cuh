@@ -123,6 +123,13 @@ cudaError_t launch_mex_dx_pair(const MexGeo&, const float* x, const float* tiles
                                const float* dy, float* dx, int* flag, cudaStream_t);
 cudaError_t launch_mex_doff_pair(const MexGeo&, const float* x, const float* mo, const float* mx, const float* y, const float* dy,
                                  float* part, int* splits_out, int* flag, cudaStream_t);
+// mex_f64.cu -- the factorised passes in double precision
+bool mex_use_f64(const MexGeo&, uint32_t flags);
+size_t mex_f64_workspace_bytes(const MexGeo&);
+cudaError_t launch_mex_fwd_f64(const MexGeo&, const double* x, const double* off, double* y, void* ws, uint32_t flags, cudaStream_t);
+// dx or doff may be null
+cudaError_t launch_mex_bwd_f64(const MexGeo&, const double* x, const double* off, const double* y, const double* dy, double* dx, double* doff,
+                               bool accumulate, void* ws, uint32_t flags, cudaStream_t);
 // number of multiprocessors of the current device (148 when no device answers)
 int device_sm_count();
 

@@ -255,10 +255,10 @@ class Mex(torch.nn.Module):
                     epsilon=self.epsilon, softmax_mode=self.softmax_mode)
 
     def _op_flags(self, dtype, device):
-        # float32 on the GPU: the op takes the raw offsets and normalises them in its own prepass (and its gradient comes back
+        # on the GPU the op takes the raw offsets and normalises them in its own prepass (and its gradient comes back
         # with respect to the raw values); otherwise effective_offsets() does it in front of the op
-        fused = self.normalize_offsets and dtype == torch.float32 and device.type == "cuda" and self.offsets is not None and \
-            self.offsets.dtype == torch.float32 and self.offsets.is_cuda
+        fused = self.normalize_offsets and device.type == "cuda" and self.offsets is not None and self.offsets.dtype == dtype and \
+            self.offsets.is_cuda and (dtype == torch.float32 or (dtype == torch.float64 and math.isfinite(self.epsilon)))
         if _torch_glue.DEFAULT_FLAGS & (abi.FLAG_FORCE_DIRECT | abi.FLAG_MEX_EXACT):
             fused = False           # those routes run without a workspace, which the fused normalisation needs
         return abi.FLAG_MEX_NORMALIZED_OFFSETS if fused else 0
