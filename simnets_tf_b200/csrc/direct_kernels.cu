@@ -45,6 +45,7 @@ __device__ __forceinline__ T block_sum(T v, T* smem) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads) sim_fwd_direct(SimGeo g, const T* __restrict__ x, const T* __restrict__ tm,
                                                            const T* __restrict__ wt, T* __restrict__ y, const int* __restrict__ gate) {
+    stream_order();
     if (gate && gate[1] == 0) return;
     const long long total = (long long)g.B * g.M * g.N;
     const T oob = T(g.oob), fudge = T(g.fudge);
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(kThreads) sim_fwd_direct(SimGeo g, const T* __
 template <typename T>
 __global__ void __launch_bounds__(kThreads) sim_dx_direct(SimGeo g, const T* __restrict__ x, const T* __restrict__ tm,
                                                           const T* __restrict__ wt, const T* __restrict__ dy, T* __restrict__ dx) {
+    stream_order();
     const long long total = (long long)g.B * g.C * g.H * g.W;
     for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads) {
         const int w0 = int(idx % g.W);
@@ -129,6 +131,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T* __restrict__ x, const T* __restrict__ tm,
                                                                const T* __restrict__ wt, const T* __restrict__ dy,
                                                                T* __restrict__ dt, T* __restrict__ dw, int accumulate) {
+    stream_order();
     __shared__ T smem[kThreads];
     const int mk = blockIdx.x;
     const int m = mk / g.K, k = mk % g.K;
@@ -171,6 +174,7 @@ __device__ __forceinline__ T mex_tap(const MexGeo& g, const T* __restrict__ xs, 
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) mex_fwd_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off, T* __restrict__ y, const int* __restrict__ gate) {
+    stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.M * g.N;
     const T oob = T(g.oob), eps = T(g.eps), cst = T(g.cst);
@@ -206,6 +210,7 @@ __device__ __forceinline__ T mex_weight(const MexGeo& g, T eps, T cst, T data, T
 template <typename T>
 __global__ void __launch_bounds__(kThreads) mex_dx_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off,
                                                           const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx, const int* __restrict__ gate) {
+    stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.C * g.H * g.W;
     const T eps = T(g.eps), cst = T(g.cst);
@@ -249,6 +254,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) mex_doff_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off,
                                                             const T* __restrict__ y, const T* __restrict__ dy,
                                                             T* __restrict__ doff, int accumulate, const int* __restrict__ gate) {
+    stream_order();
     __shared__ T smem[kThreads];
     if (gate && (gate[0] | gate[1]) == 0) return;
     const T oob = T(g.oob), eps = T(g.eps), cst = T(g.cst);
@@ -289,8 +295,8 @@ cudaError_t launch_sim_fwd_direct(const SimGeo& g, bool f64, const void* x, cons
     const long long total = (long long)g.B * g.M * g.N;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (sim_fwd_direct<float><<<grid_for(total), kThreads, 0, s>>>(g, (const float*)x, (const float*)t, (const float*)w, (float*)y, gate)),
-        (sim_fwd_direct<double><<<grid_for(total), kThreads, 0, s>>>(g, (const double*)x, (const double*)t, (const double*)w, (double*)y, gate)));
+        (in_stream_order(sim_fwd_direct<float>, grid_for(total), kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (float*)y, gate)),
+        (in_stream_order(sim_fwd_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (double*)y, gate)));
     count_launch();
     return cudaGetLastError();
 }
@@ -299,8 +305,8 @@ cudaError_t launch_sim_dx_direct(const SimGeo& g, bool f64, const void* x, const
     const long long total = (long long)g.B * g.C * g.H * g.W;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (sim_dx_direct<float><<<grid_for(total), kThreads, 0, s>>>(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dx)),
-        (sim_dx_direct<double><<<grid_for(total), kThreads, 0, s>>>(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dx)));
+        (in_stream_order(sim_dx_direct<float>, grid_for(total), kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dx)),
+        (in_stream_order(sim_dx_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dx)));
     count_launch();
     return cudaGetLastError();
 }
@@ -309,8 +315,8 @@ cudaError_t launch_sim_dparams_direct(const SimGeo& g, bool f64, const void* x, 
                                       void* dt, void* dw, bool accumulate, cudaStream_t s) {
     const int blocks = g.M * g.K;
     SIMNETS_DTYPE_SWITCH(f64,
-        (sim_dparams_direct<float><<<blocks, kThreads, 0, s>>>(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dt, (float*)dw, accumulate)),
-        (sim_dparams_direct<double><<<blocks, kThreads, 0, s>>>(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dt, (double*)dw, accumulate)));
+        (in_stream_order(sim_dparams_direct<float>, blocks, kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dt, (float*)dw, accumulate)),
+        (in_stream_order(sim_dparams_direct<double>, blocks, kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dt, (double*)dw, accumulate)));
     count_launch();
     return cudaGetLastError();
 }
@@ -319,8 +325,8 @@ cudaError_t launch_mex_fwd_direct(const MexGeo& g, bool f64, const void* x, cons
     const long long total = (long long)g.B * g.M * g.N;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (mex_fwd_direct<float><<<grid_for(total, gate != nullptr), kThreads, 0, s>>>(g, (const float*)x, (const float*)off, (float*)y, gate)),
-        (mex_fwd_direct<double><<<grid_for(total), kThreads, 0, s>>>(g, (const double*)x, (const double*)off, (double*)y, gate)));
+        (in_stream_order(mex_fwd_direct<float>, grid_for(total, gate != nullptr), kThreads, 0, s)(g, (const float*)x, (const float*)off, (float*)y, gate)),
+        (in_stream_order(mex_fwd_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)off, (double*)y, gate)));
     count_launch();
     return cudaGetLastError();
 }
@@ -329,8 +335,8 @@ cudaError_t launch_mex_dx_direct(const MexGeo& g, bool f64, const void* x, const
     const long long total = (long long)g.B * g.C * g.H * g.W;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (mex_dx_direct<float><<<grid_for(total, gate != nullptr), kThreads, 0, s>>>(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx, gate)),
-        (mex_dx_direct<double><<<grid_for(total), kThreads, 0, s>>>(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, gate)));
+        (in_stream_order(mex_dx_direct<float>, grid_for(total, gate != nullptr), kThreads, 0, s)(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx, gate)),
+        (in_stream_order(mex_dx_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, gate)));
     count_launch();
     return cudaGetLastError();
 }
@@ -341,8 +347,8 @@ cudaError_t launch_mex_doff_direct(const MexGeo& g, bool f64, const void* x, con
     const long long cap = (long long)device_sm_count() * 16;
     const int blocks = int(triples < cap ? triples : cap);
     SIMNETS_DTYPE_SWITCH(f64,
-        (mex_doff_direct<float><<<blocks, kThreads, 0, s>>>(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)doff, accumulate, gate)),
-        (mex_doff_direct<double><<<blocks, kThreads, 0, s>>>(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)doff, accumulate, gate)));
+        (in_stream_order(mex_doff_direct<float>, blocks, kThreads, 0, s)(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)doff, accumulate, gate)),
+        (in_stream_order(mex_doff_direct<double>, blocks, kThreads, 0, s)(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)doff, accumulate, gate)));
     count_launch();
     return cudaGetLastError();
 }

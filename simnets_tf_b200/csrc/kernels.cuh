@@ -5,6 +5,7 @@
 #include <math_constants.h>
 #include "simnets_b200.h"
 #include "geometry.cuh"
+#include "launch.cuh"
 
 namespace simnets {
 

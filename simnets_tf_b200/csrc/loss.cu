@@ -26,6 +26,7 @@ __device__ __forceinline__ float loss_warp_sum(float v) {
 __global__ void __launch_bounds__(kLossThreads) softmax_xent(int batch, int classes, float scale, const float* __restrict__ logits,
                                                             const long long* __restrict__ labels, float* __restrict__ loss,
                                                             float* __restrict__ dlogits, float* __restrict__ partial, unsigned* __restrict__ ticket) {
+    stream_order();
     __shared__ float rows[kLossRows];
     __shared__ bool last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -80,7 +81,7 @@ cudaError_t launch_softmax_xent(int batch, int classes, float scale, const float
     float* partial = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
     const cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
-    softmax_xent<<<loss_grid(batch), kLossThreads, 0, s>>>(batch, classes, scale, logits, labels, loss, dlogits, partial, ticket);
+    in_stream_order(softmax_xent, loss_grid(batch), kLossThreads, 0, s)(batch, classes, scale, logits, labels, loss, dlogits, partial, ticket);
     count_launch();
     return cudaGetLastError();
 }

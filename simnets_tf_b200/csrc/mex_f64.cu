@@ -81,6 +81,7 @@ __device__ __forceinline__ double block_reduce(double v, double* red, bool sum) 
 // One CTA per (region, instance): reference value, Eo, log-sum-exp and normalised row of raw offsets, the safety verdict.
 __global__ void __launch_bounds__(256) mex_prep64(MexGeo g, const double* __restrict__ off, double* __restrict__ mo, double* __restrict__ eo,
                                                   double* __restrict__ offn, double* __restrict__ lse_out, int* __restrict__ flag, int normalize) {
+    stream_order();
     __shared__ double red[256];
     const size_t row = (size_t)blockIdx.x * g.K;
     double hi = -CUDART_INF, lo = -CUDART_INF;            // (lo: maximum of the negated values)
@@ -132,6 +133,7 @@ __device__ __forceinline__ long long tap_address(const MexGeo& g, const Col64& c
 
 // Largest (eps > 0) or smallest tap of every patch, NaN ignored; `lanes` positions per CTA of 256 threads, 256 / lanes slices of the taps.
 __global__ void __launch_bounds__(256) mex_colmax64(MexGeo g, const double* __restrict__ x, double* __restrict__ mx, int lanes) {
+    stream_order();
     __shared__ double red[256];
     const int slices = 256 / lanes, lane = threadIdx.x % lanes, slice = threadIdx.x / lanes;
     const long long total = (long long)g.B * g.N;
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(kThreads64) mex_gemm64(MexGeo g, Split64 sp, c
                                                          const double* __restrict__ mo, const double* __restrict__ mx, const double* __restrict__ y,
                                                          const double* __restrict__ dy, double* __restrict__ out, double* __restrict__ part,
                                                          const int* __restrict__ flag) {
+    stream_order();
     if (*flag) return;
     __shared__ __align__(16) double As[2][kQ][kLd], Bs[2][kQ][kLd];
     const long long P = (long long)g.B * g.rs;
@@ -277,6 +280,7 @@ template <int OP>
 __global__ void __launch_bounds__(256) mex_finish64(MexGeo g, int splits, const double* __restrict__ x, const double* __restrict__ mo,
                                                     const double* __restrict__ mx, const double* __restrict__ part, double* __restrict__ out,
                                                     const int* __restrict__ flag) {
+    stream_order();
     if (*flag) return;
     const long long P = (long long)g.B * g.rs, rows = OP == kDx ? g.K : g.M, per = (long long)g.R * rows * P;
     for (long long idx = blockIdx.x * 256LL + threadIdx.x; idx < per; idx += (long long)gridDim.x * 256) {
@@ -301,6 +305,7 @@ __global__ void __launch_bounds__(256) mex_finish64(MexGeo g, int splits, const 
 __global__ void __launch_bounds__(256) mex_doff_finish64(MexGeo g, int splits, double* __restrict__ part, const double* __restrict__ eo,
                                                          const double* __restrict__ raw, const double* __restrict__ lse, double* __restrict__ doff,
                                                          int normalize, int accumulate, const int* __restrict__ flag) {
+    stream_order();
     __shared__ double red[256];
     const bool exact = *flag != 0;
     const size_t n = (size_t)g.R * g.M * g.K, row = (size_t)blockIdx.x * g.K;
@@ -326,10 +331,10 @@ bool norm64(uint32_t flags) { return (flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSET
 cudaError_t prepare64(const MexGeo& g, const Ws64& w, const double* x, const double* off, uint32_t flags, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(w.flag, 0, 2 * sizeof(int), s);
     if (e != cudaSuccess) return e;
-    mex_prep64<<<g.R * g.M, 256, 0, s>>>(g, off, w.mo, w.eo, w.offn, w.lse, w.flag, norm64(flags));
+    in_stream_order(mex_prep64, g.R * g.M, 256, 0, s)(g, off, w.mo, w.eo, w.offn, w.lse, w.flag, norm64(flags));
     const long long total = (long long)g.B * g.N;
     const int lanes = g.K >= 512 ? 1 : (g.K >= 32 ? 32 : 256);
-    mex_colmax64<<<int(std::min<long long>((total + lanes - 1) / lanes, 16LL * device_sm_count())), 256, 0, s>>>(g, x, w.mx, lanes);
+    in_stream_order(mex_colmax64, int(std::min<long long>((total + lanes - 1) / lanes, 16LL * device_sm_count())), 256, 0, s)(g, x, w.mx, lanes);
     count_launch(2);
     return cudaGetLastError();
 }
@@ -338,12 +343,12 @@ template <int OP>
 cudaError_t gemm64(const MexGeo& g, const Ws64& w, const double* x, const double* y, const double* dy, double* out, int* splits, cudaStream_t s) {
     const Split64 sp = split_of(g, Op64(OP));
     if (sp.it * sp.jt * g.R > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    mex_gemm64<OP><<<dim3(unsigned(sp.it * sp.jt * g.R), unsigned(sp.splits)), kThreads64, 0, s>>>(g, sp, x, w.eo, w.mo, w.mx, y, dy, out, w.part, w.flag);
+    in_stream_order(mex_gemm64<OP>, dim3(unsigned(sp.it * sp.jt * g.R), unsigned(sp.splits)), kThreads64, 0, s)(g, sp, x, w.eo, w.mo, w.mx, y, dy, out, w.part, w.flag);
     count_launch();
     *splits = sp.splits;
     if (OP != kDoff && sp.splits > 1) {
         const long long per = (long long)g.R * (OP == kDx ? g.K : g.M) * ((long long)g.B * g.rs);
-        mex_finish64<OP><<<int(std::min<long long>((per + 255) / 256, 16LL * device_sm_count())), 256, 0, s>>>(g, sp.splits, x, w.mo, w.mx, w.part, out, w.flag);
+        in_stream_order(mex_finish64<OP>, int(std::min<long long>((per + 255) / 256, 16LL * device_sm_count())), 256, 0, s)(g, sp.splits, x, w.mo, w.mx, w.part, out, w.flag);
         count_launch();
     }
     return cudaGetLastError();
@@ -393,7 +398,7 @@ cudaError_t launch_mex_bwd_f64(const MexGeo& g, const double* x, const double* o
     if (e != cudaSuccess) return e;
     e = launch_mex_doff_direct(g, true, x, rows, y, dy, w.part, false, s, w.flag);
     if (e != cudaSuccess) return e;
-    mex_doff_finish64<<<g.R * g.M, 256, 0, s>>>(g, splits, w.part, w.eo, off, w.lse, doff, norm64(flags), accumulate, w.flag);
+    in_stream_order(mex_doff_finish64, g.R * g.M, 256, 0, s)(g, splits, w.part, w.eo, off, w.lse, doff, norm64(flags), accumulate, w.flag);
     count_launch();
     return cudaGetLastError();
 }

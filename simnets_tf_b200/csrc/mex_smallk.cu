@@ -48,6 +48,7 @@ __device__ __forceinline__ void load_offsets_chunk(const MexGeo& g, const float*
 template <int KP, int C, bool SPATIAL1>
 __global__ void __launch_bounds__(kT, 2) mex_fwd_smallk(MexGeo g, const float* __restrict__ x, const float* __restrict__ eo,
                                                      const float* __restrict__ mo, float* __restrict__ y, const int* __restrict__ flag) {
+    stream_order();
     __shared__ __align__(16) float eo_s[kMC * KP];
     __shared__ float mo_s[kMC];
     if (*flag) return;
@@ -107,6 +108,7 @@ template <int KP, int C, bool SPATIAL1>
 __global__ void __launch_bounds__(kT, 2) mex_dx_smallk(MexGeo g, const float* __restrict__ x, const float* __restrict__ eo,
                                                     const float* __restrict__ mo, const float* __restrict__ y, const float* __restrict__ dy,
                                                     float* __restrict__ dx, const int* __restrict__ flag) {
+    stream_order();
     __shared__ __align__(16) float eo_s[kMC * KP];
     __shared__ float mo_s[kMC];
     if (*flag) return;
@@ -191,6 +193,7 @@ template <int KP, bool SPATIAL1>
 __global__ void __launch_bounds__(kT, 2) mex_doff_smallk(MexGeo g, const float* __restrict__ x, const float* __restrict__ mo,
                                                       const float* __restrict__ y, const float* __restrict__ dy,
                                                       float* __restrict__ part, int slabs, const int* __restrict__ flag) {
+    stream_order();
     constexpr int SUP = KP <= 16 ? 128 : 64;                 // positions whose Ex are prepared together
     __shared__ float q_s[kPT][kT + 1];
     __shared__ __align__(16) float ex_s[SUP][KP];
@@ -276,12 +279,13 @@ __global__ void __launch_bounds__(kT, 2) mex_doff_smallk(MexGeo g, const float* 
 
 }  // namespace
 
+#define SMALLK_RUN(KERNEL, K_, C_, SP) in_stream_order(KERNEL<K_, C_, SP>, int(blocks), kT, 0, s)
 #define SMALLK_DISPATCH(KERNEL, C_, ...)                                                            \
     do {                                                                                            \
         const bool sp1 = g.bh == 1 && g.bw == 1;                                                    \
-        if (g.K <= 8) { if (sp1) KERNEL<8, C_, true> __VA_ARGS__; else KERNEL<8, C_, false> __VA_ARGS__; }          \
-        else if (g.K <= 16) { if (sp1) KERNEL<16, C_, true> __VA_ARGS__; else KERNEL<16, C_, false> __VA_ARGS__; }  \
-        else { if (sp1) KERNEL<32, C_, true> __VA_ARGS__; else KERNEL<32, C_, false> __VA_ARGS__; }                 \
+        if (g.K <= 8) { if (sp1) SMALLK_RUN(KERNEL, 8, C_, true)(__VA_ARGS__); else SMALLK_RUN(KERNEL, 8, C_, false)(__VA_ARGS__); }          \
+        else if (g.K <= 16) { if (sp1) SMALLK_RUN(KERNEL, 16, C_, true)(__VA_ARGS__); else SMALLK_RUN(KERNEL, 16, C_, false)(__VA_ARGS__); }  \
+        else { if (sp1) SMALLK_RUN(KERNEL, 32, C_, true)(__VA_ARGS__); else SMALLK_RUN(KERNEL, 32, C_, false)(__VA_ARGS__); }                 \
     } while (0)
 
 cudaError_t launch_mex_fwd_smallk(const MexGeo& g, const float* x, const float* eo, const float* mo, float* y, const int* flag, cudaStream_t s) {
@@ -289,11 +293,11 @@ cudaError_t launch_mex_fwd_smallk(const MexGeo& g, const float* x, const float* 
     if (g.K <= 16) {
         const long long blocks = ((P + kT * 4 - 1) / (kT * 4)) * g.R;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        SMALLK_DISPATCH(mex_fwd_smallk, 4, <<<int(blocks), kT, 0, s>>>(g, x, eo, mo, y, flag));
+        SMALLK_DISPATCH(mex_fwd_smallk, 4, g, x, eo, mo, y, flag);
     } else {
         const long long blocks = ((P + kT * 2 - 1) / (kT * 2)) * g.R;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        SMALLK_DISPATCH(mex_fwd_smallk, 2, <<<int(blocks), kT, 0, s>>>(g, x, eo, mo, y, flag));
+        SMALLK_DISPATCH(mex_fwd_smallk, 2, g, x, eo, mo, y, flag);
     }
     count_launch();
     return cudaGetLastError();
@@ -305,11 +309,11 @@ cudaError_t launch_mex_dx_smallk(const MexGeo& g, const float* x, const float* e
     if (g.K <= 16) {
         const long long blocks = ((P + kT * 2 - 1) / (kT * 2)) * g.R;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        SMALLK_DISPATCH(mex_dx_smallk, 2, <<<int(blocks), kT, 0, s>>>(g, x, eo, mo, y, dy, dx, flag));
+        SMALLK_DISPATCH(mex_dx_smallk, 2, g, x, eo, mo, y, dy, dx, flag);
     } else {
         const long long blocks = ((P + kT - 1) / kT) * g.R;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        SMALLK_DISPATCH(mex_dx_smallk, 1, <<<int(blocks), kT, 0, s>>>(g, x, eo, mo, y, dy, dx, flag));
+        SMALLK_DISPATCH(mex_dx_smallk, 1, g, x, eo, mo, y, dy, dx, flag);
     }
     count_launch();
     return cudaGetLastError();
@@ -319,8 +323,8 @@ cudaError_t launch_mex_doff_smallk(const MexGeo& g, const float* x, const float*
                                    float* part, int slabs, const int* flag, cudaStream_t s) {
     const int blocks = ((g.M + kT - 1) / kT) * g.R * slabs;
     const bool sp1 = g.bh == 1 && g.bw == 1;
-#define DOFFK(KP) do { if (sp1) mex_doff_smallk<KP, true><<<blocks, kT, 0, s>>>(g, x, mo, y, dy, part, slabs, flag); \
-                       else mex_doff_smallk<KP, false><<<blocks, kT, 0, s>>>(g, x, mo, y, dy, part, slabs, flag); } while (0)
+#define DOFFK(KP) do { if (sp1) in_stream_order(mex_doff_smallk<KP, true>, blocks, kT, 0, s)(g, x, mo, y, dy, part, slabs, flag); \
+                       else in_stream_order(mex_doff_smallk<KP, false>, blocks, kT, 0, s)(g, x, mo, y, dy, part, slabs, flag); } while (0)
     if (g.K <= 8) DOFFK(8); else if (g.K <= 16) DOFFK(16); else DOFFK(32);
 #undef DOFFK
     count_launch();

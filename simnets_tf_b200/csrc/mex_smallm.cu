@@ -61,6 +61,7 @@ __device__ __forceinline__ float block_patch_extreme(const MexGeo& g, const floa
 
 template <bool SPATIAL1>
 __global__ void __launch_bounds__(kT) mex_colmax_wide(MexGeo g, const float* __restrict__ x, float* __restrict__ mx, const int* __restrict__ flag) {
+    stream_order();
     __shared__ float red[kT / 32];
     if (*flag) return;
     const long long idx = blockIdx.x;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(kT) mex_colmax_wide(MexGeo g, const float* __r
 template <bool SPATIAL1>
 __global__ void __launch_bounds__(kT) mex_fwd_smallm(MexGeo g, const float* __restrict__ x, const float* __restrict__ eot,
                                                      const float* __restrict__ mo, float* __restrict__ y, const int* __restrict__ flag) {
+    stream_order();
     __shared__ float red[kT / 32];
     __shared__ float racc[kT / 32][kMaxM];
     if (*flag) return;
@@ -120,6 +122,7 @@ template <bool SPATIAL1>
 __global__ void __launch_bounds__(kT) mex_dx_smallm(MexGeo g, const float* __restrict__ x, const float* __restrict__ eo,
                                                     const float* __restrict__ mo, const float* __restrict__ y, const float* __restrict__ dy,
                                                     float* __restrict__ dx, const int* __restrict__ flag) {
+    stream_order();
     __shared__ float red[kT / 32];
     __shared__ float Q[kMaxM];
     if (*flag) return;
@@ -160,6 +163,7 @@ template <bool SPATIAL1>
 __global__ void __launch_bounds__(kT) mex_doff_smallm(MexGeo g, const float* __restrict__ x, const float* __restrict__ mo,
                                                       const float* __restrict__ mx, const float* __restrict__ y, const float* __restrict__ dy,
                                                       float* __restrict__ part, int splits, const int* __restrict__ flag) {
+    stream_order();
     __shared__ Column cols[kGroup];
     __shared__ float Qs[kGroup][kMaxM];
     if (*flag) return;
@@ -229,6 +233,7 @@ template <int MP>
 __global__ void __launch_bounds__(kT) mex_fwd_head(MexGeo g, int pb, int slices, const float* __restrict__ x, const float* __restrict__ eot,
                                                    const float* __restrict__ mo, float* __restrict__ mx, float* __restrict__ y,
                                                    float* __restrict__ partial, int* __restrict__ tickets, const int* __restrict__ flag) {
+    stream_order();
     __shared__ float red[kT / 32][kHeadPB];
     __shared__ float racc[kT / 32][kHeadPB][MP];
     __shared__ float mxs[kHeadPB];
@@ -363,6 +368,7 @@ template <int MP>
 __global__ void __launch_bounds__(kT, 2) mex_fwd_head_wide(MexGeo g, int slices, const float* __restrict__ x, const float* __restrict__ eo,
                                                            const float* __restrict__ mo, float* __restrict__ mx, float* __restrict__ y,
                                                            float* __restrict__ partial, int* __restrict__ tickets, const int* __restrict__ flag) {
+    stream_order();
     extern __shared__ __align__(16) float seo[];                   // [MP][kWideSlice]
     __shared__ int last;
     if (*flag) return;
@@ -480,6 +486,7 @@ __global__ void __launch_bounds__(kT) mex_bwd_head(MexGeo g, const float* __rest
                                                    const float* __restrict__ y, const float* __restrict__ dy,
                                                    float* __restrict__ dx, float* __restrict__ part, int splits,
                                                    const int* __restrict__ flag) {
+    stream_order();
     constexpr int GP = 8;                                           // positions staged together
     __shared__ float Qs[2][GP][kMaxM + 1];                          // Q of a group's positions and, in the last column, their maxima
     if (*flag) return;
@@ -572,8 +579,8 @@ __global__ void __launch_bounds__(kT) mex_bwd_head(MexGeo g, const float* __rest
 cudaError_t launch_mex_colmax_wide(const MexGeo& g, const float* x, float* mx, const int* flag, cudaStream_t s) {
     const long long total = (long long)g.B * g.N;
     if (total > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if (g.bh == 1 && g.bw == 1) mex_colmax_wide<true><<<int(total), kT, 0, s>>>(g, x, mx, flag);
-    else mex_colmax_wide<false><<<int(total), kT, 0, s>>>(g, x, mx, flag);
+    if (g.bh == 1 && g.bw == 1) in_stream_order(mex_colmax_wide<true>, int(total), kT, 0, s)(g, x, mx, flag);
+    else in_stream_order(mex_colmax_wide<false>, int(total), kT, 0, s)(g, x, mx, flag);
     count_launch();
     return cudaGetLastError();
 }
@@ -581,8 +588,8 @@ cudaError_t launch_mex_colmax_wide(const MexGeo& g, const float* x, float* mx, c
 cudaError_t launch_mex_fwd_smallm(const MexGeo& g, const float* x, const float* eot, const float* mo, float* y, const int* flag, cudaStream_t s) {
     const long long blocks = (long long)g.B * g.rs * g.R;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if (g.bh == 1 && g.bw == 1) mex_fwd_smallm<true><<<int(blocks), kT, 0, s>>>(g, x, eot, mo, y, flag);
-    else mex_fwd_smallm<false><<<int(blocks), kT, 0, s>>>(g, x, eot, mo, y, flag);
+    if (g.bh == 1 && g.bw == 1) in_stream_order(mex_fwd_smallm<true>, int(blocks), kT, 0, s)(g, x, eot, mo, y, flag);
+    else in_stream_order(mex_fwd_smallm<false>, int(blocks), kT, 0, s)(g, x, eot, mo, y, flag);
     count_launch();
     return cudaGetLastError();
 }
@@ -591,8 +598,8 @@ cudaError_t launch_mex_dx_smallm(const MexGeo& g, const float* x, const float* e
                                  float* dx, const int* flag, cudaStream_t s) {
     const long long blocks = (long long)g.B * g.rs * g.R;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if (g.bh == 1 && g.bw == 1) mex_dx_smallm<true><<<int(blocks), kT, 0, s>>>(g, x, eo, mo, y, dy, dx, flag);
-    else mex_dx_smallm<false><<<int(blocks), kT, 0, s>>>(g, x, eo, mo, y, dy, dx, flag);
+    if (g.bh == 1 && g.bw == 1) in_stream_order(mex_dx_smallm<true>, int(blocks), kT, 0, s)(g, x, eo, mo, y, dy, dx, flag);
+    else in_stream_order(mex_dx_smallm<false>, int(blocks), kT, 0, s)(g, x, eo, mo, y, dy, dx, flag);
     count_launch();
     return cudaGetLastError();
 }
@@ -600,8 +607,8 @@ cudaError_t launch_mex_dx_smallm(const MexGeo& g, const float* x, const float* e
 cudaError_t launch_mex_doff_smallm(const MexGeo& g, const float* x, const float* mo, const float* mx, const float* y, const float* dy,
                                    float* part, int splits, const int* flag, cudaStream_t s) {
     const int blocks = ((g.K + kT - 1) / kT) * g.R * splits;
-    if (g.bh == 1 && g.bw == 1) mex_doff_smallm<true><<<blocks, kT, 0, s>>>(g, x, mo, mx, y, dy, part, splits, flag);
-    else mex_doff_smallm<false><<<blocks, kT, 0, s>>>(g, x, mo, mx, y, dy, part, splits, flag);
+    if (g.bh == 1 && g.bw == 1) in_stream_order(mex_doff_smallm<true>, blocks, kT, 0, s)(g, x, mo, mx, y, dy, part, splits, flag);
+    else in_stream_order(mex_doff_smallm<false>, blocks, kT, 0, s)(g, x, mo, mx, y, dy, part, splits, flag);
     count_launch();
     return cudaGetLastError();
 }
@@ -655,7 +662,7 @@ cudaError_t launch_mex_fwd_head(const MexGeo& g, const float* x, const float* eo
                 if (e != cudaSuccess) return e;                                                                         \
                 attr_done = true;                                                                                       \
             }                                                                                                           \
-            mex_fwd_head_wide<MP><<<blocks, kT, smem, s>>>(g, slices, x, eo, mo, mx, y, partial, tickets, flag);        \
+            in_stream_order(mex_fwd_head_wide<MP>, blocks, kT, smem, s)(g, slices, x, eo, mo, mx, y, partial, tickets, flag);        \
         } while (0)
         switch (pad4(g.M)) {
         case 4: HEAD_WIDE(4); break;
@@ -680,10 +687,10 @@ cudaError_t launch_mex_fwd_head(const MexGeo& g, const float* x, const float* eo
     if (e != cudaSuccess) return e;
     const int blocks = int(groups * slices);
     switch (pad4(g.M)) {
-    case 4: mex_fwd_head<4><<<blocks, kT, 0, s>>>(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
-    case 8: mex_fwd_head<8><<<blocks, kT, 0, s>>>(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
-    case 12: mex_fwd_head<12><<<blocks, kT, 0, s>>>(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
-    default: mex_fwd_head<16><<<blocks, kT, 0, s>>>(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
+    case 4: in_stream_order(mex_fwd_head<4>, blocks, kT, 0, s)(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
+    case 8: in_stream_order(mex_fwd_head<8>, blocks, kT, 0, s)(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
+    case 12: in_stream_order(mex_fwd_head<12>, blocks, kT, 0, s)(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
+    default: in_stream_order(mex_fwd_head<16>, blocks, kT, 0, s)(g, pb, slices, x, eot, mo, mx, y, partial, tickets, flag); break;
     }
     count_launch();
     return cudaGetLastError();
@@ -696,9 +703,9 @@ cudaError_t launch_mex_bwd_head(const MexGeo& g, bool want_dx, bool want_doff, c
     const int blocks = ktiles * splits;
 #define HEAD_BWD(MP)                                                                                                          \
     do {                                                                                                                      \
-        if (want_dx && want_doff) mex_bwd_head<MP, true, true><<<blocks, kT, 0, s>>>(g, x, eo, mo, mx, y, dy, dx, part, splits, flag); \
-        else if (want_dx) mex_bwd_head<MP, true, false><<<blocks, kT, 0, s>>>(g, x, eo, mo, mx, y, dy, dx, part, splits, flag);        \
-        else mex_bwd_head<MP, false, true><<<blocks, kT, 0, s>>>(g, x, eo, mo, mx, y, dy, dx, part, splits, flag);                     \
+        if (want_dx && want_doff) in_stream_order(mex_bwd_head<MP, true, true>, blocks, kT, 0, s)(g, x, eo, mo, mx, y, dy, dx, part, splits, flag); \
+        else if (want_dx) in_stream_order(mex_bwd_head<MP, true, false>, blocks, kT, 0, s)(g, x, eo, mo, mx, y, dy, dx, part, splits, flag);        \
+        else in_stream_order(mex_bwd_head<MP, false, true>, blocks, kT, 0, s)(g, x, eo, mo, mx, y, dy, dx, part, splits, flag);                     \
     } while (0)
     switch (pad4(g.M)) {
     case 4: HEAD_BWD(4); break;

@@ -27,6 +27,7 @@ namespace {
 // tiles[r][row tile of NT][chunk of 16 along red][plane][NT * 16 floats]; out-of-range entries are zero.
 // Forward: rows = instances, red = taps (source Eo[r][m][ld]); input gradient: rows = taps, red = instances (Eo^T).
 __global__ void __launch_bounds__(256) mex_tc_prep(int R, int rows, int red, int ld, int NT, const float* __restrict__ src, float* __restrict__ tiles) {
+    stream_order();
     const int chunks = (red + kTcKT - 1) / kTcKT, rtiles = (rows + NT - 1) / NT;
     const long long total = (long long)R * rtiles * chunks * NT * kTcKT;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
@@ -50,6 +51,7 @@ template <int NT, bool SPATIAL1, bool INTERIOR>
 __global__ void __launch_bounds__(kTcThreads) mex_fwd_tc(MexGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
                                                         const float* __restrict__ mo, const float* __restrict__ mx,
                                                         float* __restrict__ y, int* __restrict__ flag) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ TcShared sh;
     __shared__ float mo_s[NT];
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kTcThreads, NT == 256 ? 2 : 3) mex_dx_tc(MexGe
                                                        const float* __restrict__ mo, const float* __restrict__ mx,
                                                        const float* __restrict__ y, const float* __restrict__ dy,
                                                        float* __restrict__ dx, int* __restrict__ flag) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ TcShared sh;
     __shared__ int tap_tab[SPATIAL1 ? 1 : kTapTable];
@@ -284,6 +287,7 @@ __global__ void __launch_bounds__(kTcThreads, NT == 64 ? 3 : 2) mex_doff_tc(MexG
                                                          const float* __restrict__ mx, const float* __restrict__ y,
                                                          const float* __restrict__ dy, float* __restrict__ part, int splits,
                                                          int* __restrict__ flag) {
+    stream_order();
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ TcShared sh;
     __shared__ float amo_s[128];                        // mo of this CTA's instances
@@ -406,7 +410,7 @@ cudaError_t set_smem_once(Kernel kernel, int smem, bool& done) {
         static bool attr_done = false;                                         \
         const cudaError_t e_ = set_smem_once(KERNEL, SMEM, attr_done);          \
         if (e_ != cudaSuccess) return e_;                                      \
-        KERNEL<<<GRID, kTcThreads, SMEM, s>>>(__VA_ARGS__);                     \
+        in_stream_order(KERNEL, GRID, kTcThreads, SMEM, s)(__VA_ARGS__);                     \
     } while (0)
 
 template <int NT>
@@ -441,7 +445,7 @@ cudaError_t launch_dx_nt(const MexGeo& g, const float* x, const float* tiles, co
         static bool attr_done = false;                                                              \
         const cudaError_t e_ = set_smem_once(KERNEL, smem_max, attr_done);                          \
         if (e_ != cudaSuccess) return e_;                                                           \
-        KERNEL<<<int(blocks), kTcThreads, smem, s>>>(g, x, tiles, mo, mx, y, dy, dx, flag);         \
+        in_stream_order(KERNEL, int(blocks), kTcThreads, smem, s)(g, x, tiles, mo, mx, y, dy, dx, flag);         \
     } while (0)
     if (g.bh == 1 && g.bw == 1) {
         if (patches_inside_input(g) && (long long)NT * g.H * g.W < 0x7fffffffLL) DX_RUN((mex_dx_tc<NT, true, true>));
@@ -500,7 +504,7 @@ int mex_tc_doff_splits(const MexGeo& g) {
 cudaError_t launch_mex_tc_prep(const MexGeo& g, bool transposed, const float* src, float* tiles, cudaStream_t s, int nt) {
     const int rows = transposed ? g.K : g.M, red = transposed ? g.M : g.K, NT = nt > 0 ? nt : pick_nt(rows);
     const long long total = (long long)g.R * ((rows + NT - 1) / NT) * ((red + kTcKT - 1) / kTcKT) * NT * kTcKT;
-    mex_tc_prep<<<int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s>>>(g.R, rows, red, pad4(red), NT, src, tiles);
+    in_stream_order(mex_tc_prep, int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(g.R, rows, red, pad4(red), NT, src, tiles);
     count_launch();
     return cudaGetLastError();
 }

@@ -286,6 +286,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) mex_fwd_pair(MexGeo g, const 
                                                                const float* __restrict__ mo, const float* __restrict__ mx,
                                                                float* __restrict__ y, float* __restrict__ pooled, WsPlan plan,
                                                                int* __restrict__ flag, int test_expire) {
+    stream_order();
     constexpr int STAGES = pair_stages<NT>();
     constexpr int STAGE_BYTES = pair_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 4 * NT;
@@ -472,6 +473,7 @@ __global__ void __launch_bounds__(kDxThreads, 1) mex_dx_pair(MexGeo g, const flo
                                                             const float* __restrict__ mo, const float* __restrict__ mx,
                                                             const float* __restrict__ y, const float* __restrict__ dy,
                                                             float* __restrict__ dx, WsPlan plan, int* __restrict__ flag) {
+    stream_order();
     constexpr int STAGES = pair_stages<NT>(), DEPTH = dx_depth<POOLED>(), kDxSlotBytes = dx_slot_bytes<POOLED>();
     constexpr int STAGE_BYTES = pair_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 4 * NT;
@@ -725,6 +727,7 @@ __global__ void __launch_bounds__(do_pair_threads(LOAD), 1) mex_doff_pair(MexGeo
                                                                   const float* __restrict__ dy, float* __restrict__ part,
                                                                   DoPairPlan plan, int* __restrict__ flag,
                                                                   const __grid_constant__ DoMaps maps) {
+    stream_order();
     constexpr bool WIDE = LOAD == 1;
     using Cfg = DoCfg<MT, NT, CP, POOLED>;
     constexpr int kDoDepth = Cfg::DEPTH;
@@ -1007,7 +1010,7 @@ __global__ void __launch_bounds__(do_pair_threads(LOAD), 1) mex_doff_pair(MexGeo
         static bool attr_done = false;                                          \
         const cudaError_t e_ = ws_set_smem(KERNEL, SMEM, attr_done);            \
         if (e_ != cudaSuccess) return e_;                                       \
-        KERNEL<<<GRID, THREADS, SMEM, s>>>(__VA_ARGS__);                         \
+        in_stream_order(KERNEL, GRID, THREADS, SMEM, s)(__VA_ARGS__);                         \
     } while (0)
 
 // two neighbouring pixel pairs of a tile are 16 contiguous, 16-byte aligned bytes in every tensor

@@ -25,6 +25,7 @@ template <int NT, bool SPATIAL1, bool INTERIOR>
 __global__ void __launch_bounds__(kWsThreads, 1) mex_fwd_ws(MexGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
                                                            const float* __restrict__ mo, const float* __restrict__ mx,
                                                            float* __restrict__ y, WsPlan plan, int* __restrict__ flag) {
+    stream_order();
     constexpr int STAGES = ws_stages<NT>();
     constexpr int A_BYTES = kTcPos * kTcKT * 4, STAGE_BYTES = ws_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 2 * NT < 32 ? 32 : 2 * NT;
@@ -203,6 +204,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mex_dx_ws(MexGeo g, const float
                                                           const float* __restrict__ mo, const float* __restrict__ mx,
                                                           const float* __restrict__ y, const float* __restrict__ dy,
                                                           float* __restrict__ dx, WsPlan plan, int* __restrict__ flag) {
+    stream_order();
     constexpr int STAGES = ws_stages<NT>();
     constexpr int A_BYTES = kTcPos * kTcKT * 4, STAGE_BYTES = ws_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 2 * NT < 32 ? 32 : 2 * NT;

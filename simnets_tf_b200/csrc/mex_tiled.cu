@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(512) mex_prep_offsets(MexGeo g, int Mp, const 
                                                         float* __restrict__ eo, float* __restrict__ eot, int* __restrict__ flag,
                                                         float* __restrict__ tf, int ntf, float* __restrict__ td, int ntd,
                                                         float* __restrict__ offn, float* __restrict__ lse_out) {
+    stream_order();
     __shared__ float s_hi[512], s_lo[512];
     __shared__ int s_bad[512];
     const int nt = blockDim.x;                       // 128, or 512 for long rows
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(512) mex_prep_offsets(MexGeo g, int Mp, const 
 template <bool SPATIAL1>
 __global__ void __launch_bounds__(256) mex_colmax(MexGeo g, const float* __restrict__ x, float* __restrict__ mx, const int* __restrict__ flag,
                                                   int interior) {
+    stream_order();
     if (*flag) return;
     const long long total = (long long)g.B * g.N;
     const bool up = g.eps > 0;
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(256) mex_colmax(MexGeo g, const float* __restr
 // tap with a division each.  Same values: max and min are associative and skip NaN taps either way.
 template <int BW>
 __global__ void __launch_bounds__(256) mex_colmax_rows(MexGeo g, const float* __restrict__ x, float* __restrict__ mx, const int* __restrict__ flag) {
+    stream_order();
     if (*flag) return;
     const long long total = (long long)g.B * g.N;
     const bool up = g.eps > 0;
@@ -197,6 +200,7 @@ __global__ void __launch_bounds__(256) mex_colmax_rows(MexGeo g, const float* __
 template <bool SPATIAL1>
 __global__ void __launch_bounds__(256) mex_colmax_sliced(MexGeo g, const float* __restrict__ x, float* __restrict__ mx, const int* __restrict__ flag,
                                                          int interior) {
+    stream_order();
     __shared__ float part[8][32];
     if (*flag) return;
     const long long total = (long long)g.B * g.N;
@@ -245,6 +249,7 @@ template <int TM, bool SPATIAL1, bool INTERIOR>
 __global__ void __launch_bounds__(256) mex_fwd_tiled(MexGeo g, const float* __restrict__ x, const float* __restrict__ eot,
                                                      const float* __restrict__ mo, const float* __restrict__ mx,
                                                      float* __restrict__ y, const int* __restrict__ flag) {
+    stream_order();
     using Cfg = TileCfg<TM, 128, 8, TM / 16, 8, 1, 1>;
     static_assert(Cfg::THREADS == 256, "256 threads");
     if (*flag) return;
@@ -326,6 +331,7 @@ __global__ void __launch_bounds__(256) mex_dx_tiled(MexGeo g, const float* __res
                                                     const float* __restrict__ mo, const float* __restrict__ mx,
                                                     const float* __restrict__ y, const float* __restrict__ dy,
                                                     float* __restrict__ dx, const int* __restrict__ flag) {
+    stream_order();
     using Cfg = TileCfg<TM, 128, 8, TM / 16, 8, 1, 1>;
     if (*flag) return;
     __shared__ __align__(16) float smem[Cfg::SMEM_FLOATS];
@@ -403,6 +409,7 @@ __global__ void __launch_bounds__(256) mex_doff_tiled(MexGeo g, const float* __r
                                                       const float* __restrict__ mx, const float* __restrict__ y,
                                                       const float* __restrict__ dy, float* __restrict__ part, int splits,
                                                       const int* __restrict__ flag) {
+    stream_order();
     using Cfg = TileCfg<TILE, TILE, KC, TILE / 16, TILE / 16, 1, 1>;
     static_assert(Cfg::THREADS == 256, "256 threads");
     constexpr int ROWS = 256 / KC;                                  // tile rows one staging pass covers
@@ -484,6 +491,7 @@ __global__ void __launch_bounds__(256) mex_doff_tiled(MexGeo g, const float* __r
 // doff[r][m][k] (+)= Eo[r][m][k] * sum over splits, in split order (deterministic)
 __global__ void __launch_bounds__(256) mex_doff_reduce(long long n, int K, int splits, const float* __restrict__ part, const float* __restrict__ eo,
                                                        float* __restrict__ doff, int accumulate, const int* __restrict__ flag) {
+    stream_order();
     if (flag[0] | flag[1]) return;               // unsafe spread, or a tensor-core launch gave up on a wait: the exact kernel behind does the work
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
         float s = 0.f;
@@ -502,6 +510,7 @@ template <int EPT>
 __global__ void __launch_bounds__(128) mex_doff_reduce_norm(int K, int splits, long long n, const float* __restrict__ part, const float* __restrict__ eo,
                                                             const float* __restrict__ raw, const float* __restrict__ lse,
                                                             float* __restrict__ doff, int accumulate, const int* __restrict__ flag) {
+    stream_order();
     __shared__ float red[128];
     const bool exact = (flag[0] | flag[1]) != 0;
     const long long row = blockIdx.x;
@@ -545,6 +554,7 @@ __global__ void __launch_bounds__(128) mex_doff_reduce_norm(int K, int splits, l
 // row pass.  `tmp` = gradient with respect to the normalised rows.
 __global__ void __launch_bounds__(256) mex_doff_reduce_tmp(long long n, int K, int splits, const float* __restrict__ part, const float* __restrict__ eo,
                                                            float* __restrict__ tmp, const int* __restrict__ flag) {
+    stream_order();
     const bool exact = (flag[0] | flag[1]) != 0;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
         if (exact) { tmp[i] = part[i]; continue; }
@@ -556,6 +566,7 @@ __global__ void __launch_bounds__(256) mex_doff_reduce_tmp(long long n, int K, i
 
 __global__ void __launch_bounds__(256) mex_doff_norm_rows(int K, const float* __restrict__ tmp, const float* __restrict__ raw, const float* __restrict__ lse,
                                                           float* __restrict__ doff, int accumulate) {
+    stream_order();
     __shared__ float red[256];
     const long long row = blockIdx.x;
     const float* t = tmp + row * K;
@@ -587,19 +598,19 @@ cudaError_t finish_doff(const MexGeo& g, const MexWs& w, int splits, const float
         cudaError_t e = launch_mex_doff_direct(g, false, x, w.offn, y, dy, w.part, false, s, w.flag);
         if (e != cudaSuccess) return e;
         const int rows = g.R * g.M;
-        if (g.K <= 128) mex_doff_reduce_norm<1><<<rows, 128, 0, s>>>(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else if (g.K <= 256) mex_doff_reduce_norm<2><<<rows, 128, 0, s>>>(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else if (g.K <= 512) mex_doff_reduce_norm<4><<<rows, 128, 0, s>>>(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else if (g.K <= 1024) mex_doff_reduce_norm<8><<<rows, 128, 0, s>>>(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        if (g.K <= 128) in_stream_order(mex_doff_reduce_norm<1>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        else if (g.K <= 256) in_stream_order(mex_doff_reduce_norm<2>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        else if (g.K <= 512) in_stream_order(mex_doff_reduce_norm<4>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        else if (g.K <= 1024) in_stream_order(mex_doff_reduce_norm<8>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
         else {
-            mex_doff_reduce_tmp<<<int(std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s>>>(n, g.K, splits, w.part, w.eo, w.dtmp, w.flag);
-            mex_doff_norm_rows<<<rows, 256, 0, s>>>(g.K, w.dtmp, off, w.lse, doff, accumulate);
+            in_stream_order(mex_doff_reduce_tmp, int(std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(n, g.K, splits, w.part, w.eo, w.dtmp, w.flag);
+            in_stream_order(mex_doff_norm_rows, rows, 256, 0, s)(g.K, w.dtmp, off, w.lse, doff, accumulate);
             count_launch();
         }
         count_launch();
         return cudaGetLastError();
     }
-    mex_doff_reduce<<<int(std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s>>>(n, g.K, splits, w.part, w.eo, doff, accumulate, w.flag);
+    in_stream_order(mex_doff_reduce, int(std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(n, g.K, splits, w.part, w.eo, doff, accumulate, w.flag);
     count_launch();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -632,10 +643,10 @@ cudaError_t run_prepasses(const MexGeo& g, const MexWs& w, const float* x, const
         // the pair-tile kernels' operand tiles (forward and input gradient) come out of the same launch
         const int ntf = mex_pair_nt_fwd(g), ntd = mex_pair_nt_dx(g);
         const int Mp = std::max(((g.M + ntf - 1) / ntf) * ntf, ((g.M + 15) / 16) * 16);
-        mex_prep_offsets<<<g.R * Mp, g.K >= 2048 ? 512 : 128, 0, s>>>(g, Mp, off, w.mo, w.eo, w.eot, w.flag, w.tc_tiles, ntf, w.tc_tiles_dx, ntd,
+        in_stream_order(mex_prep_offsets, g.R * Mp, g.K >= 2048 ? 512 : 128, 0, s)(g, Mp, off, w.mo, w.eo, w.eot, w.flag, w.tc_tiles, ntf, w.tc_tiles_dx, ntd,
                                                                       normalize ? w.offn : nullptr, w.lse);
     } else {
-        mex_prep_offsets<<<g.R * g.M, g.K >= 2048 ? 512 : 128, 0, s>>>(g, g.M, off, w.mo, w.eo, w.eot, w.flag, nullptr, 0, nullptr, 0,
+        in_stream_order(mex_prep_offsets, g.R * g.M, g.K >= 2048 ? 512 : 128, 0, s)(g, g.M, off, w.mo, w.eo, w.eot, w.flag, nullptr, 0, nullptr, 0,
                                                                        normalize ? w.offn : nullptr, w.lse);
     }
     if (!need_mx) { count_launch(); return cudaGetLastError(); }
@@ -647,18 +658,18 @@ cudaError_t run_prepasses(const MexGeo& g, const MexWs& w, const float* x, const
     // long patches while one thread per position would not fill the GPU's thread slots: 2048 per multiprocessor)
     if (g.K >= 128 && total < (long long)device_sm_count() * 2048) {
         const int grid = int(std::min<long long>((total + 31) / 32, (long long)device_sm_count() * 32));
-        if (g.bh == 1 && g.bw == 1) mex_colmax_sliced<true><<<grid, 256, 0, s>>>(g, x, w.mx, w.flag, inside);
-        else mex_colmax_sliced<false><<<grid, 256, 0, s>>>(g, x, w.mx, w.flag, inside);
+        if (g.bh == 1 && g.bw == 1) in_stream_order(mex_colmax_sliced<true>, grid, 256, 0, s)(g, x, w.mx, w.flag, inside);
+        else in_stream_order(mex_colmax_sliced<false>, grid, 256, 0, s)(g, x, w.mx, w.flag, inside);
     } else if ((g.bw == 2 || g.bw == 4) && g.sw == g.bw && g.W % g.bw == 0 && inside &&
                (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
         // every vector load is aligned: rows start at multiples of W floats, W and the sample stride are multiples of bw
         const int grid = int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 16));
-        if (g.bw == 2) mex_colmax_rows<2><<<grid, 256, 0, s>>>(g, x, w.mx, w.flag);
-        else mex_colmax_rows<4><<<grid, 256, 0, s>>>(g, x, w.mx, w.flag);
+        if (g.bw == 2) in_stream_order(mex_colmax_rows<2>, grid, 256, 0, s)(g, x, w.mx, w.flag);
+        else in_stream_order(mex_colmax_rows<4>, grid, 256, 0, s)(g, x, w.mx, w.flag);
     } else {
         const int grid = int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 16));
-        if (g.bh == 1 && g.bw == 1) mex_colmax<true><<<grid, 256, 0, s>>>(g, x, w.mx, w.flag, inside);
-        else mex_colmax<false><<<grid, 256, 0, s>>>(g, x, w.mx, w.flag, inside);
+        if (g.bh == 1 && g.bw == 1) in_stream_order(mex_colmax<true>, grid, 256, 0, s)(g, x, w.mx, w.flag, inside);
+        else in_stream_order(mex_colmax<false>, grid, 256, 0, s)(g, x, w.mx, w.flag, inside);
     }
     count_launch(2);
     return cudaGetLastError();
@@ -749,7 +760,7 @@ static cudaError_t mex_fwd_tiled_body(const MexGeo& g, const float* x, const flo
     const long long blocks = jtiles * ((g.M + (wide ? 127 : 63)) / (wide ? 128 : 64)) * g.R;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const bool interior = patches_inside_input(g);
-#define FWD(TM, SP, IN) mex_fwd_tiled<TM, SP, IN><<<int(blocks), 256, 0, s>>>(g, x, w.eot, w.mo, w.mx, y, w.flag)
+#define FWD(TM, SP, IN) in_stream_order(mex_fwd_tiled<TM, SP, IN>, int(blocks), 256, 0, s)(g, x, w.eot, w.mo, w.mx, y, w.flag)
 #define FWD_TM(TM)                                                                         \
     if (sp1) { if (interior) FWD(TM, true, true); else FWD(TM, true, false); }            \
     else { if (interior) FWD(TM, false, true); else FWD(TM, false, false); }
@@ -855,7 +866,7 @@ cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* of
     const bool wide = g.K > 64;
     const long long blocks = ((P + 127) / 128) * ((g.K + (wide ? 127 : 63)) / (wide ? 128 : 64)) * g.R;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-#define DX(TM, SP) mex_dx_tiled<TM, SP><<<int(blocks), 256, 0, s>>>(g, x, w.eo, w.mo, w.mx, y, dy, dx, w.flag)
+#define DX(TM, SP) in_stream_order(mex_dx_tiled<TM, SP>, int(blocks), 256, 0, s)(g, x, w.eo, w.mo, w.mx, y, dy, dx, w.flag)
     if (wide) { if (sp1) DX(128, true); else DX(128, false); }
     else { if (sp1) DX(64, true); else DX(64, false); }
 #undef DX
@@ -897,7 +908,7 @@ cudaError_t launch_mex_doff_tiled(const MexGeo& g, const float* x, const float* 
     const int tile = doff_big(g) ? 128 : 64;
     const long long blocks = (long long)((g.M + tile - 1) / tile) * ((g.K + tile - 1) / tile) * g.R * splits;
     const bool sp1 = g.bh == 1 && g.bw == 1;
-#define DOFF(T, KC, SP) mex_doff_tiled<T, KC, SP><<<int(blocks), 256, 0, s>>>(g, x, w.mo, w.mx, y, dy, w.part, splits, w.flag)
+#define DOFF(T, KC, SP) in_stream_order(mex_doff_tiled<T, KC, SP>, int(blocks), 256, 0, s)(g, x, w.mo, w.mx, y, dy, w.part, splits, w.flag)
     if (doff_big(g)) { if (sp1) DOFF(128, 16, true); else DOFF(128, 16, false); }
     else { if (sp1) DOFF(64, 32, true); else DOFF(64, 32, false); }
 #undef DOFF

@@ -27,6 +27,7 @@ __device__ __forceinline__ float block_reduce(float v, bool is_max, float* red) 
 
 // out[row][k] = off[row][k] - logsumexp_k(off[row][:])
 __global__ void __launch_bounds__(kNormThreads) normalize_offsets_fwd(int K, const float* __restrict__ off, float* __restrict__ out) {
+    stream_order();
     __shared__ float red[kNormThreads / 32];
     const float* o = off + (size_t)blockIdx.x * K;
     float mx = -CUDART_INF_F;
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(kNormThreads) normalize_offsets_fwd(int K, con
 // doff[row][k] = dout[row][k] - softmax(off[row][:])[k] * sum_k dout[row][:]
 __global__ void __launch_bounds__(kNormThreads) normalize_offsets_bwd(int K, const float* __restrict__ off, const float* __restrict__ dout,
                                                                       float* __restrict__ doff) {
+    stream_order();
     __shared__ float red[kNormThreads / 32];
     const float* o = off + (size_t)blockIdx.x * K;
     const float* g = dout + (size_t)blockIdx.x * K;
@@ -65,7 +67,7 @@ __global__ void __launch_bounds__(kNormThreads) normalize_offsets_bwd(int K, con
 cudaError_t launch_normalize_offsets_fwd(long long rows, int K, const float* off, float* out, cudaStream_t s) {
     if (rows == 0 || K == 0) return cudaSuccess;
     if (rows > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    normalize_offsets_fwd<<<int(rows), kNormThreads, 0, s>>>(K, off, out);
+    in_stream_order(normalize_offsets_fwd, int(rows), kNormThreads, 0, s)(K, off, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -73,7 +75,7 @@ cudaError_t launch_normalize_offsets_fwd(long long rows, int K, const float* off
 cudaError_t launch_normalize_offsets_bwd(long long rows, int K, const float* off, const float* dout, float* doff, cudaStream_t s) {
     if (rows == 0 || K == 0) return cudaSuccess;
     if (rows > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    normalize_offsets_bwd<<<int(rows), kNormThreads, 0, s>>>(K, off, dout, doff);
+    in_stream_order(normalize_offsets_bwd, int(rows), kNormThreads, 0, s)(K, off, dout, doff);
     count_launch();
     return cudaGetLastError();
 }

@@ -10,6 +10,7 @@ namespace {
 // the four addends are summed in window order, ((a + b) + c) + d, like a sequential pooling loop
 __global__ void __launch_bounds__(256) sum_pool2_vec4(long long total, int Ho, int W4, int W, const float* __restrict__ x, float* __restrict__ y,
                                                       const int* __restrict__ gate) {
+    stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
         const int w4 = int(i % W4);
@@ -26,6 +27,7 @@ __global__ void __launch_bounds__(256) sum_pool2_vec4(long long total, int Ho, i
 
 __global__ void __launch_bounds__(256) sum_pool2_scalar(long long total, int Wo, int W, const float* __restrict__ x, float* __restrict__ y,
                                                         const int* __restrict__ gate) {
+    stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
         const int w = int(i % Wo);
@@ -45,8 +47,8 @@ cudaError_t launch_sum_pool2(long long planes, int H, int W, const float* x, flo
     const long long total = vec ? planes * Ho * (W / 4) : planes * Ho * Wo;
     // (a gated launch almost always returns at once: one wave of CTAs is enough)
     const int grid = int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * (gate ? 4 : 16)));
-    if (vec) sum_pool2_vec4<<<grid, 256, 0, s>>>(total, Ho, W / 4, W, x, y, gate);
-    else sum_pool2_scalar<<<grid, 256, 0, s>>>(total, Wo, W, x, y, gate);
+    if (vec) in_stream_order(sum_pool2_vec4, grid, 256, 0, s)(total, Ho, W / 4, W, x, y, gate);
+    else in_stream_order(sum_pool2_scalar, grid, 256, 0, s)(total, Wo, W, x, y, gate);
     count_launch();
     return cudaGetLastError();
 }

@@ -10,6 +10,7 @@ namespace {
 // two-lane instruction; nothing touches memory inside the loop.
 template <bool PACKED>
 __global__ void __launch_bounds__(1024) fp32_fma_probe(int iters, float seed, float* __restrict__ out) {
+    stream_order();
     float2 a[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = make_float2(seed + j, seed - j);
@@ -30,8 +31,8 @@ __global__ void __launch_bounds__(1024) fp32_fma_probe(int iters, float seed, fl
 }  // namespace
 
 cudaError_t launch_fp32_probe(bool packed, int blocks, int iters, float* out, cudaStream_t s) {
-    if (packed) fp32_fma_probe<true><<<blocks, 1024, 0, s>>>(iters, 1.f, out);
-    else fp32_fma_probe<false><<<blocks, 1024, 0, s>>>(iters, 1.f, out);
+    if (packed) in_stream_order(fp32_fma_probe<true>, blocks, 1024, 0, s)(iters, 1.f, out);
+    else in_stream_order(fp32_fma_probe<false>, blocks, 1024, 0, s)(iters, 1.f, out);
     count_launch();
     return cudaGetLastError();
 }

@@ -54,6 +54,7 @@ template <int MODE, int KC, int MAXK, int TM>
 __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g, FastDiv f_N, FastDiv f_ow, DpTile tile, const float* __restrict__ x,
                                                              const float* __restrict__ tm, const float* __restrict__ dy,
                                                              float* __restrict__ part, int splits) {
+    stream_order();
     constexpr bool MASKED = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     constexpr int LD = KC + 4, TI = TM / 4;                                           // row stride, floats
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
 __global__ void __launch_bounds__(512) sim_dparams_reduce(SimGeo g, int splits, int slices, const float* __restrict__ part,
                                                           const float* __restrict__ wt, float* __restrict__ dt, float* __restrict__ dw,
                                                           int accumulate) {
+    stream_order();
     __shared__ float red[3][512];
     const int mk = g.M * g.K, lanes = 512 / slices;
     const float fudge = float(g.fudge);
@@ -296,7 +298,7 @@ cudaError_t launch_sim_dparams(const SimGeo& g, const float* x, const float* t, 
     const long long blocks = (long long)dp_tiles(g, tile) * splits;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const FastDiv f_N = make_fastdiv(g.N), f_ow = make_fastdiv(g.ow);
-#define DP_TILE(MODE, KC, MAXK, TM) sim_dparams<MODE, KC, MAXK, TM><<<int(blocks), kDpThreads, 0, s>>>(g, f_N, f_ow, tile, x, t, dy, part, splits)
+#define DP_TILE(MODE, KC, MAXK, TM) in_stream_order(sim_dparams<MODE, KC, MAXK, TM>, int(blocks), kDpThreads, 0, s)(g, f_N, f_ow, tile, x, t, dy, part, splits)
 #define DP(MODE)                                            \
     do {                                                    \
         if (tile.tm == 64) DP_TILE(MODE, 32, 32, 64);       \
@@ -314,7 +316,7 @@ cudaError_t launch_sim_dparams(const SimGeo& g, const float* x, const float* t, 
 #undef DP
 #undef DP_TILE
     const int mk = g.M * g.K, slices = splits >= 64 ? 64 : 8, lanes = 512 / slices;
-    sim_dparams_reduce<<<std::min((mk + lanes - 1) / lanes, device_sm_count() * 8), 512, 0, s>>>(g, splits, slices, part, w, dt, dw, accumulate);
+    in_stream_order(sim_dparams_reduce, std::min((mk + lanes - 1) / lanes, device_sm_count() * 8), 512, 0, s)(g, splits, slices, part, w, dt, dw, accumulate);
     count_launch(2);
     return cudaGetLastError();
 }

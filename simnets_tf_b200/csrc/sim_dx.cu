@@ -72,6 +72,7 @@ struct DxPixel {
 
 // (t, s w)[tap][m][Cp], channel-contiguous, for the tile kernel
 __global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, const float* __restrict__ tm, const float* __restrict__ wt, float* __restrict__ dxp) {
+    stream_order();
     const int taps = g.bh * g.bw, cp = dx_pad4(g.C);
     const long long total = (long long)taps * g.M * cp;
     const float s = g.mode == SIM_L2 ? 2.f : 1.f;
@@ -94,6 +95,7 @@ template <int TM> struct DxCfg {
 template <int TM, int MODE>
 __global__ void __launch_bounds__(DxCfg<TM>::Cfg::THREADS, DxCfg<TM>::Cfg::THREADS == 256 ? (TM == 128 ? 1 : 2) : 3)
 sim_dx_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ dxp, const float* __restrict__ dy, float* __restrict__ dx) {
+    stream_order();
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     constexpr bool SKIP_NAN = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
     using Cfg = typename DxCfg<TM>::Cfg;
@@ -219,6 +221,7 @@ constexpr int kNarrowThreads = 128, kNarrowQ = 64;
 template <int CT, int PP, int MODE>
 __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(SimGeo g, const float* __restrict__ x, const float* __restrict__ tm,
                                                                 const float* __restrict__ wt, const float* __restrict__ dy, float* __restrict__ dx) {
+    stream_order();
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     constexpr bool SKIP_NAN = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
     __shared__ __align__(16) float s_t[kNarrowQ * CT], s_w[kNarrowQ * CT];
@@ -305,8 +308,8 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
         const dim3 grid{unsigned(blocks), unsigned(phases)};
 #define NARROW(CT, MODE)                                                                                          \
     do {                                                                                                          \
-        if (many) sim_dx_narrow<CT, 4, MODE><<<grid, kNarrowThreads, 0, s>>>(g, x, t, w, dy, dx);                  \
-        else sim_dx_narrow<CT, 1, MODE><<<grid, kNarrowThreads, 0, s>>>(g, x, t, w, dy, dx);                       \
+        if (many) in_stream_order(sim_dx_narrow<CT, 4, MODE>, grid, kNarrowThreads, 0, s)(g, x, t, w, dy, dx);                  \
+        else in_stream_order(sim_dx_narrow<CT, 1, MODE>, grid, kNarrowThreads, 0, s)(g, x, t, w, dy, dx);                       \
     } while (0)
 #define NARROW_1(MODE) NARROW(1, MODE)
 #define NARROW_2(MODE) NARROW(2, MODE)
@@ -317,7 +320,7 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
         return cudaGetLastError();
     }
     const long long total = (long long)g.bh * g.bw * g.M * dx_pad4(g.C);
-    sim_dx_prep<<<int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s>>>(g, t, w, dxp);
+    in_stream_order(sim_dx_prep, int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(g, t, w, dxp);
     // the tile height that pads the channels least; of two equal ones the taller (its dy values serve more rows)
     const auto padded = [&](int tm) { return (g.C + tm - 1) / tm * tm; };
     int tm = 128;
@@ -327,7 +330,7 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
     const long long blocks = ((pixels + tn - 1) / tn) * ((g.C + tm - 1) / tm);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const dim3 grid{unsigned(blocks), unsigned(phases)};
-#define DX(TM, MODE) sim_dx_tiled<TM, MODE><<<grid, DxCfg<TM>::Cfg::THREADS, 0, s>>>(g, x, dxp, dy, dx)
+#define DX(TM, MODE) in_stream_order(sim_dx_tiled<TM, MODE>, grid, DxCfg<TM>::Cfg::THREADS, 0, s)(g, x, dxp, dy, dx)
 #define DX_16(MODE) DX(16, MODE)
 #define DX_32(MODE) DX(32, MODE)
 #define DX_64(MODE) DX(64, MODE)

@@ -87,6 +87,7 @@ template <int MODE, int KT>
 __global__ void __launch_bounds__(kSkThreads, 4) sim_fwd_smallk(SimGeo g, int slice, const float* __restrict__ x, const float* __restrict__ tm,
                                                                 const float* __restrict__ wt, float* __restrict__ y, float* __restrict__ ch_max,
                                                                 float* __restrict__ ch_min, int* __restrict__ flag) {
+    stream_order();
     constexpr bool MASKED = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     extern __shared__ __align__(16) float sm[];
@@ -172,6 +173,7 @@ template <int MODE, int TM>
 __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(SimGeo g, const float* __restrict__ x, const float* __restrict__ tm,
                                                                              const float* __restrict__ wt, float* __restrict__ y,
                                                                              float* __restrict__ ch_max, float* __restrict__ ch_min, int* __restrict__ flag) {
+    stream_order();
     constexpr int NA = ResidentPlanes<MODE>::NA, NB = ResidentPlanes<MODE>::NB, T = TM * 4, QSTEP = T / kResTN, PER = kResMaxK / QSTEP, TI = TM / 4;
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     using Cfg = TileCfg<TM, kResTN, 8, 4, 8, 1, 1>;
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
 
 // The same extrema from a finished output tensor, for the forward kernels that do not produce them on the way
 __global__ void __launch_bounds__(256) sim_extrema(long long P, int M, int N, const float* __restrict__ y, float* __restrict__ ch_max, float* __restrict__ ch_min) {
+    stream_order();
     for (long long q = blockIdx.x * 256LL + threadIdx.x; q < P; q += (long long)gridDim.x * 256) {
         const long long n = q / N;
         const float* p = y + n * (long long)M * N + (q - n * N);
@@ -342,7 +345,7 @@ cudaError_t launch_sk(const SimGeo& g, int slice, const float* x, const float* t
     const dim3 grid(unsigned(std::min<long long>(want, std::max(1, device_sm_count() * 4 / slices))), unsigned(slices));
     const int rows = (slice + 3) & ~3;
     const size_t smem = sizeof(float) * (KT * rows * (g.mode == SIM_L2N_NAN ? 3 : 2) + (g.mode == SIM_L2N ? rows : 0));
-#define SK(MODE) sim_fwd_smallk<MODE, KT><<<grid, kSkThreads, smem, s>>>(g, slice, x, t, w, y, ch_max, ch_min, flag)
+#define SK(MODE) in_stream_order(sim_fwd_smallk<MODE, KT>, grid, kSkThreads, smem, s)(g, slice, x, t, w, y, ch_max, ch_min, flag)
     switch (g.mode) {
     case SIM_L1: SK(SIM_L1); break;
     case SIM_L1_SKIP: SK(SIM_L1_SKIP); break;
@@ -372,7 +375,7 @@ cudaError_t launch_resident(const SimGeo& g, const float* x, const float* t, con
     const int resident = std::max(1, device_sm_count() * per_sm / mtiles);
     const long long rounds = (tiles + resident - 1) / resident;          // equal rounds: as few CTAs as finish in the same number
     const dim3 grid(unsigned((tiles + rounds - 1) / rounds), unsigned(mtiles));
-    sim_fwd_resident<MODE, TM><<<grid, TM * 4, smem, s>>>(g, x, t, w, y, ch_max, ch_min, flag);
+    in_stream_order(sim_fwd_resident<MODE, TM>, grid, TM * 4, smem, s)(g, x, t, w, y, ch_max, ch_min, flag);
     count_launch();
     return cudaGetLastError();
 }
@@ -426,7 +429,7 @@ cudaError_t launch_sim_fwd_smallk(const SimGeo& g, const float* x, const float* 
 cudaError_t launch_sim_extrema(const SimGeo& g, const float* y, float* ch_max, float* ch_min, cudaStream_t s) {
     const long long P = (long long)g.B * g.N;
     if (P == 0 || (ch_max == nullptr && ch_min == nullptr)) return cudaSuccess;
-    sim_extrema<<<int(std::min<long long>((P + 255) / 256, (long long)device_sm_count() * 16)), 256, 0, s>>>(P, g.M, g.N, y, ch_max, ch_min);
+    in_stream_order(sim_extrema, int(std::min<long long>((P + 255) / 256, (long long)device_sm_count() * 16)), 256, 0, s)(P, g.M, g.N, y, ch_max, ch_min);
     count_launch();
     return cudaGetLastError();
 }

@@ -47,6 +47,7 @@ __device__ __forceinline__ int sim_tc_core(int row, int k) { return (row >> 3) *
 // tiles[mt][chunk][hi, lo][NT x 16] and bias[m] = sum_k s t^2 + c[m].  planes, cm: as sim_prep leaves them.
 __global__ void __launch_bounds__(128) sim_tc_prep(SimGeo g, int NT, const float* __restrict__ planes, const float* __restrict__ cm,
                                                    float* __restrict__ tiles, float* __restrict__ bias) {
+    stream_order();
     __shared__ float red[128];
     const int m = blockIdx.x, ldm = (g.M + 3) & ~3;
     const int kchunks = (g.K + kSimTcTaps - 1) / kSimTcTaps;
@@ -78,6 +79,7 @@ template <int NT>
 __global__ void __launch_bounds__(kWsThreads, 1) sim_fwd_tc(SimGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
                                                            const float* __restrict__ bias, const int2* __restrict__ taps,
                                                            float* __restrict__ y, WsPlan plan, int* __restrict__ flag) {
+    stream_order();
     constexpr int STAGES = ws_stages<NT>();
     constexpr int A_BYTES = kTcPos * kTcKT * 4, STAGE_BYTES = ws_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 2 * NT < 32 ? 32 : 2 * NT;
@@ -206,7 +208,7 @@ size_t sim_tc_tile_floats(const SimGeo& g) {
 cudaError_t launch_sim_fwd_tc(const SimGeo& g, const float* x, const float* planes, const float* cm, const int2* taps, float* tiles,
                               float* bias, int* flag, float* y, cudaStream_t s) {
     const int NT = sim_tc_nt(g), mtiles = (g.M + NT - 1) / NT;
-    sim_tc_prep<<<mtiles * NT, 128, 0, s>>>(g, NT, planes, cm, tiles, bias);      // (sim_prep has cleared the flag words)
+    in_stream_order(sim_tc_prep, mtiles * NT, 128, 0, s)(g, NT, planes, cm, tiles, bias);      // (sim_prep has cleared the flag words)
     count_launch();
     const long long P = (long long)g.B * g.N;
     const long long items = ((P + kTcPos - 1) / kTcPos) * mtiles;

@@ -56,6 +56,7 @@ __host__ SimWs carve(const SimGeo& g, void* base) {
 __global__ void __launch_bounds__(128) sim_prep(SimGeo g, const float* __restrict__ tm, const float* __restrict__ wt,
                                                 float* __restrict__ planes, float* __restrict__ cm, int2* __restrict__ taps,
                                                 int* __restrict__ flag) {
+    stream_order();
     __shared__ float red[128];
     const int m = blockIdx.x;
     if (m == 0 && threadIdx.x < 2) flag[threadIdx.x] = 0;
@@ -125,6 +126,7 @@ template <int TM, int TN> struct FwdTile {
 template <int TM, int TN, int MODE>
 __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER_SM) sim_fwd_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ planes,
                                                      const float* __restrict__ cm, const int2* __restrict__ taps, float* __restrict__ y) {
+    stream_order();
     constexpr int NA = FwdPlanes<MODE>::NA, NB = FwdPlanes<MODE>::NB;
     using Cfg = TileCfg<TM, TN, FwdTile<TM, TN>::KC, FwdTile<TM, TN>::RM, FwdTile<TM, TN>::RN, NA, NB>;
     constexpr int QSTEP = Cfg::THREADS / TN;                     // threads along the taps when a chunk is staged
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER
 }
 
 void launch_prep(const SimGeo& g, const SimWs& w, const float* t, const float* wt, cudaStream_t s) {
-    sim_prep<<<g.M, 128, 0, s>>>(g, t, wt, w.planes, w.cm, w.taps, w.flag);
+    in_stream_order(sim_prep, g.M, 128, 0, s)(g, t, wt, w.planes, w.cm, w.taps, w.flag);
     count_launch();
 }
 
@@ -276,7 +278,7 @@ static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const flo
     }
     const long long blocks = ((P + tiles[pick].tn - 1) / tiles[pick].tn) * ((g.M + tiles[pick].tm - 1) / tiles[pick].tm);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-#define FWD(TM, TN, MODE) sim_fwd_tiled<TM, TN, MODE><<<int(blocks), FwdTile<TM, TN>::THREADS, 0, s>>>(g, x, W.planes, W.cm, W.taps, y)
+#define FWD(TM, TN, MODE) in_stream_order(sim_fwd_tiled<TM, TN, MODE>, int(blocks), FwdTile<TM, TN>::THREADS, 0, s)(g, x, W.planes, W.cm, W.taps, y)
 #define FWD_MODES(TM, TN)                                        \
     switch (g.mode) {                                            \
     case SIM_L1: FWD(TM, TN, SIM_L1); break;                     \

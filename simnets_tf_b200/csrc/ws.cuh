@@ -183,7 +183,7 @@ cudaError_t ws_set_smem(Kernel kernel, int smem, bool& done) {
         static bool attr_done = false;                                          \
         const cudaError_t e_ = ws_set_smem(KERNEL, SMEM, attr_done);            \
         if (e_ != cudaSuccess) return e_;                                       \
-        KERNEL<<<GRID, kWsThreads, SMEM, s>>>(__VA_ARGS__);                      \
+        in_stream_order(KERNEL, GRID, kWsThreads, SMEM, s)(__VA_ARGS__);                      \
     } while (0)
 
 
