@@ -75,6 +75,11 @@ enum { SIMNETS_SIM_L1 = 0, SIMNETS_SIM_L2 = 1 };
  * otherwise run on kernels that read and write pixel pairs); same results, kept for comparison measurements. */
 #define SIMNETS_FLAG_MEX_NO_PAIR_TILES (1u << 9)
 
+/* MEX only, float32: never run small layers on the small-contraction kernels (three launches per call instead of the
+ * tensor-core kernels' seven); same results, for comparison measurements and so that tests reach the tensor-core
+ * kernels at small sizes. */
+#define SIMNETS_FLAG_MEX_NO_SMALL_TILES (1u << 15)
+
 /* Test hook, simnets_mex_forward on a pair-tile shape only: the kernel's MMA role withholds the completion signal of
  * its first accumulator and every bounded wait is shortened to a fraction of a millisecond, so that one wait runs out.
  * Nothing hangs or faults: the roles leave their loops, tensor memory is freed, word 1 of the workspace status is set
@@ -99,12 +104,12 @@ enum { SIMNETS_SIM_L1 = 0, SIMNETS_SIM_L2 = 1 };
  * (see simnets_mex_workspace_maxima); ignored by shapes for which that function returns NULL. */
 #define SIMNETS_FLAG_MEX_MAXIMA_GIVEN  (1u << 13)
 
-/* MEX entry points that take a workspace, float32: `offsets` holds raw values and the op works on each (region,
+/* MEX entry points that take a workspace: `offsets` holds raw values and the op works on each (region,
  * instance) row minus its log-sum-exp, as the reference's Keras layer does with `normalize_offsets=True` in front of the
  * op (python/simnets/keras.py:155-160); the offsets-gradient entry points then return the gradient with respect to
  * the raw values, d - softmax(row) * sum(d).  Saves the separate normalisation kernels in both directions.  Not accepted
- * (SIMNETS_E_UNSUPPORTED) by calls that run without a workspace: float64, SIMNETS_FLAG_FORCE_DIRECT, SIMNETS_FLAG_MEX_EXACT,
- * simnets_mex_forward_static_scratch. */
+ * (SIMNETS_E_UNSUPPORTED) by calls that run without a workspace: infinite epsilon, SIMNETS_FLAG_FORCE_DIRECT,
+ * SIMNETS_FLAG_MEX_EXACT, simnets_mex_forward_static_scratch. */
 #define SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS (1u << 14)
 
 /* MEX gradient entry points only: dy is given at half resolution, dy[batch, M * channels_out, height_out / 2,

@@ -1,5 +1,6 @@
 // C ABI of the library (include/simnets_b200.h): validates descriptors, picks a kernel family and
 // enqueues it on the caller's stream.  No entry point here allocates, frees or synchronises.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -101,6 +102,7 @@ int simnets_similarity_forward_extrema(const simnets_sim_desc* d, const void* x,
 void* simnets_mex_workspace_maxima(const simnets_mex_desc* d, void* workspace) {
     MexGeo g;
     if (!d || !workspace || mex_geometry(d, nullptr, &g)) return nullptr;
+    if (d->dtype == SIMNETS_F32 && mex_use_gemm(g, false, d->flags)) return mex_gemm_maxima(g, false, workspace);
     if (!mex_use_tiled(g, d->dtype == SIMNETS_F64, d->flags)) return nullptr;
     return mex_workspace_maxima(g, workspace, d->flags);
 }
@@ -180,8 +182,9 @@ int get_mex_offsets_nregions(int n_input_dim, const int* input_dim, int n_paddin
 size_t simnets_mex_workspace_bytes(const simnets_mex_desc* d) {
     MexGeo g;
     if (mex_geometry(d, nullptr, &g)) return 0;
-    if (d->dtype == SIMNETS_F64) return mex_use_f64(g, d->flags) ? mex_f64_workspace_bytes(g) : 256;
-    return mex_workspace_bytes(g, false, d->flags);
+    const bool f64 = d->dtype == SIMNETS_F64;
+    // (room for either family: a caller may size a workspace once and pass other flags later)
+    return std::max(mex_workspace_bytes(g, f64, d->flags), mex_use_gemm(g, f64, d->flags) ? mex_gemm_workspace_bytes(g, f64) : size_t(256));
 }
 
 int simnets_mex_forward(const simnets_mex_desc* d, const void* x, const void* off, void* y, void* ws, size_t ws_bytes, void* stream) {
@@ -190,10 +193,10 @@ int simnets_mex_forward(const simnets_mex_desc* d, const void* x, const void* of
     if (rc) return rc;
     if (!off || (g.B > 0 && (!x || !y))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
-    if (f64 && mex_use_f64(g, d->flags)) {
-        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_fwd_f64(g, (const double*)x, (const double*)off, (double*)y, ws, d->flags, as_stream(stream)));
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if (mex_use_gemm(g, f64, d->flags)) {
+        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_fwd_gemm(g, f64, x, off, y, ws, d->flags, as_stream(stream)));
     }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
@@ -221,6 +224,12 @@ int simnets_mex_forward_pool2x2(const simnets_mex_desc* d, const void* x, const 
     if (d->dtype != SIMNETS_F32 || g.Ho % 2 || g.Wo % 2) return SIMNETS_E_UNSUPPORTED;
     if (!off || (g.B > 0 && (!x || !y || !y_pooled))) return SIMNETS_E_NULL;
     if (g.B == 0) return SIMNETS_OK;
+    if (mex_use_gemm(g, false, d->flags)) {
+        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, false)) return SIMNETS_E_WORKSPACE;
+        const cudaError_t e = launch_mex_fwd_gemm(g, false, x, off, y, ws, d->flags, as_stream(stream));
+        if (e != cudaSuccess) return from_cuda(e);
+        return from_cuda(launch_sum_pool2((long long)g.B * g.M * g.Co, g.Ho, g.Wo, (const float*)y, (float*)y_pooled, as_stream(stream)));
+    }
     if (mex_use_tiled(g, false, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, false, d->flags)) return SIMNETS_E_WORKSPACE;
         return from_cuda(launch_mex_fwd_tiled(g, (const float*)x, (const float*)off, (float*)y, ws, d->flags, as_stream(stream), (float*)y_pooled));
@@ -260,10 +269,10 @@ int simnets_mex_input_grad(const simnets_mex_desc* d, const void* x, const void*
     if (rc) return rc;
     if (!off || (g.B > 0 && (!x || !y || !dy || !dx))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
-    if (f64 && mex_use_f64(g, d->flags)) {
-        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_bwd_f64(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, nullptr, false, ws, d->flags, as_stream(stream)));
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if (mex_use_gemm(g, f64, d->flags)) {
+        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, nullptr, false, ws, d->flags, as_stream(stream)));
     }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
@@ -280,11 +289,11 @@ int simnets_mex_offsets_grad(const simnets_mex_desc* d, const void* x, const voi
     if (rc) return rc;
     if (!off || !doff || (g.B > 0 && (!x || !y || !dy))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
     const bool acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
-    if (f64 && mex_use_f64(g, d->flags)) {
-        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_bwd_f64(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, nullptr, (double*)doff, acc, ws, d->flags, as_stream(stream)));
+    if (mex_use_gemm(g, f64, d->flags)) {
+        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, nullptr, doff, acc, ws, d->flags, as_stream(stream)));
     }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
@@ -301,11 +310,11 @@ int simnets_mex_backward(const simnets_mex_desc* d, const void* x, const void* o
     if (rc) return rc;
     if (!off || !doff || (g.B > 0 && (!x || !y || !dy || !dx))) return SIMNETS_E_NULL;
     const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !(f64 ? mex_use_f64(g, d->flags) : mex_use_tiled(g, false, d->flags))) return SIMNETS_E_UNSUPPORTED;
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
     const bool acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
-    if (f64 && mex_use_f64(g, d->flags)) {
-        if (!ws || ws_bytes < mex_f64_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_bwd_f64(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, (double*)doff, acc, ws, d->flags, as_stream(stream)));
+    if (mex_use_gemm(g, f64, d->flags)) {
+        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
+        return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, doff, acc, ws, d->flags, as_stream(stream)));
     }
     if (mex_use_tiled(g, f64, d->flags)) {
         if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;

@@ -7,6 +7,7 @@
 // include/utils/similarity_utils.hpp:17-150 and include/utils/mex_utils.hpp:10-56), accumulation
 // order follows its CPU kernels where a thread owns the whole sum.
 #include "kernels.cuh"
+#include "mex_exact.cuh"
 
 namespace simnets {
 
@@ -17,13 +18,8 @@ constexpr int kThreads = 256;
 template <typename T> __device__ __forceinline__ bool is_nan(T v) { return v != v; }
 template <typename T> __device__ __forceinline__ T sign_of(T v) { return T((T(0) < v) - (v < T(0))); }
 
-__device__ __forceinline__ float dev_exp(float v) { return expf(v); }
-__device__ __forceinline__ double dev_exp(double v) { return exp(v); }
-__device__ __forceinline__ float dev_log(float v) { return logf(v); }
-__device__ __forceinline__ double dev_log(double v) { return log(v); }
 __device__ __forceinline__ float dev_abs(float v) { return fabsf(v); }
 __device__ __forceinline__ double dev_abs(double v) { return fabs(v); }
-template <typename T> __device__ __forceinline__ T pos_inf() { return T(CUDART_INF); }
 
 constexpr double kLog2Pi = 1.8378770664093454835606594728112;
 
@@ -166,45 +162,12 @@ __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T
 
 // ------------------------------------------------------------------------- MEX
 template <typename T>
-__device__ __forceinline__ T mex_tap(const MexGeo& g, const T* __restrict__ xs, int c, int h, int w, int k, T oob) {
-    const int kw = k % g.bw, kh = (k / g.bw) % g.bh, kc = k / (g.bw * g.bh);
-    const int cc = c * g.sc - g.pc + kc, hh = h * g.sh - g.ph + kh, ww = w * g.sw - g.pw + kw;
-    return (cc >= 0 && cc < g.C && hh >= 0 && hh < g.H && ww >= 0 && ww < g.W) ? xs[((size_t)cc * g.H + hh) * g.W + ww] : oob;
-}
-
-template <typename T>
 __global__ void __launch_bounds__(kThreads) mex_fwd_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off, T* __restrict__ y, const int* __restrict__ gate) {
     stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.M * g.N;
-    const T oob = T(g.oob), eps = T(g.eps), cst = T(g.cst);
-    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads) {
-        const int j = int(idx % g.N);
-        const long long q = idx / g.N;
-        const int m = int(q % g.M), n = int(q / g.M);
-        const int w = j % g.Wo, h = (j / g.Wo) % g.Ho, c = j / (g.Wo * g.Ho);
-        const T* xs = x + (size_t)n * g.C * g.H * g.W;
-        const T* o = off + ((size_t)mex_region_of(g, c, h, w) * g.M + m) * g.K;
-        T mx = eps > T(0) ? -pos_inf<T>() : pos_inf<T>();
-        for (int k = 0; k < g.K; ++k) {
-            const T v = o[k] + mex_tap(g, xs, c, h, w, k, oob);
-            // comparisons written as the host library's max/min: a NaN operand never replaces mx
-            if (eps > T(0)) { if (mx < v) mx = v; } else { if (v < mx) mx = v; }
-        }
-        T out = mx;
-        if (g.finite) {
-            T sum = T(0);
-            for (int k = 0; k < g.K; ++k) sum += dev_exp(eps * (mex_tap(g, xs, c, h, w, k, oob) + o[k] - mx) + cst);
-            out = mx + dev_log(sum) / eps;
-        }
-        y[idx] = out;
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ T mex_weight(const MexGeo& g, T eps, T cst, T data, T offset, T top, T top_diff) {
-    if (g.finite) return top_diff * dev_exp(eps * (data + offset - top) + cst);
-    return top_diff * T((data + offset) == top);
+    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads)
+        y[idx] = mex_exact_y(g, x, off, idx);
 }
 
 template <typename T>
@@ -213,38 +176,8 @@ __global__ void __launch_bounds__(kThreads) mex_dx_direct(MexGeo g, const T* __r
     stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.C * g.H * g.W;
-    const T eps = T(g.eps), cst = T(g.cst);
-    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads) {
-        const int w0 = int(idx % g.W);
-        long long q = idx / g.W;
-        const int h0 = int(q % g.H); q /= g.H;
-        const int c0 = int(q % g.C), n = int(q / g.C);
-        const T v = x[idx];
-        const T* y_n = y + (size_t)n * g.M * g.N;
-        T total_sum = T(0);
-        for (int kc = 0; kc < g.bc; ++kc) {
-            const int cp = c0 + g.pc - kc;
-            if (cp < 0 || cp % g.sc != 0 || cp / g.sc >= g.Co) continue;
-            for (int kh = 0; kh < g.bh; ++kh) {
-                const int hp = h0 + g.ph - kh;
-                if (hp < 0 || hp % g.sh != 0 || hp / g.sh >= g.Ho) continue;
-                for (int kw = 0; kw < g.bw; ++kw) {
-                    const int wp_ = w0 + g.pw - kw;
-                    if (wp_ < 0 || wp_ % g.sw != 0 || wp_ / g.sw >= g.Wo) continue;
-                    const int c = cp / g.sc, h = hp / g.sh, w = wp_ / g.sw;
-                    const int k = (kc * g.bh + kh) * g.bw + kw;
-                    const int j = (c * g.Ho + h) * g.Wo + w;
-                    const T* o = off + (size_t)mex_region_of(g, c, h, w) * g.M * g.K + k;
-                    const T* g_j = dy + mex_dy_base(g, n, j);
-                    T sum = T(0);
-                    for (int m = 0; m < g.M; ++m)
-                        sum += mex_weight(g, eps, cst, v, o[(size_t)m * g.K], y_n[(size_t)m * g.N + j], g_j[(size_t)m * g.Ng]);
-                    total_sum += sum;
-                }
-            }
-        }
-        dx[idx] = total_sum;
-    }
+    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads)
+        dx[idx] = mex_exact_dx(g, x, off, y, dy, idx);
 }
 
 // One block at a time per (region r, instance m, tap k): reduces over batch and the region's positions.
@@ -257,7 +190,6 @@ __global__ void __launch_bounds__(kThreads) mex_doff_direct(MexGeo g, const T* _
     stream_order();
     __shared__ T smem[kThreads];
     if (gate && (gate[0] | gate[1]) == 0) return;
-    const T oob = T(g.oob), eps = T(g.eps), cst = T(g.cst);
     const long long triples = (long long)g.R * g.M * g.K;
     for (long long rmk = blockIdx.x; rmk < triples; rmk += gridDim.x) {
         const int k = int(rmk % g.K), m = int((rmk / g.K) % g.M), r = int(rmk / ((long long)g.K * g.M));
@@ -265,13 +197,7 @@ __global__ void __launch_bounds__(kThreads) mex_doff_direct(MexGeo g, const T* _
         T sum = T(0);
         const long long total = (long long)g.B * g.rs;
         for (long long i = threadIdx.x; i < total; i += kThreads) {
-            const int l = int(i % g.rs), n = int(i / g.rs);
-            const int j = mex_region_position(g, r, l);
-            if (j < 0) continue;
-            const int w = j % g.Wo, h = (j / g.Wo) % g.Ho, c = j / (g.Wo * g.Ho);
-            const T v = mex_tap(g, x + (size_t)n * g.C * g.H * g.W, c, h, w, k, oob);
-            const size_t oi = ((size_t)n * g.M + m) * g.N + j;
-            sum += mex_weight(g, eps, cst, v, o, y[oi], dy[mex_dy_base(g, n, j) + (long long)m * g.Ng]);
+            sum += mex_exact_doff_term(g, x, o, y, dy, r, m, k, i);
         }
         const T rsum = block_sum(sum, smem);
         if (threadIdx.x == 0) doff[rmk] = accumulate ? doff[rmk] + rsum : rsum;

@@ -124,13 +124,14 @@ cudaError_t launch_mex_dx_pair(const MexGeo&, const float* x, const float* tiles
                                const float* dy, float* dx, int* flag, cudaStream_t);
 cudaError_t launch_mex_doff_pair(const MexGeo&, const float* x, const float* mo, const float* mx, const float* y, const float* dy,
                                  float* part, int* splits_out, int* flag, cudaStream_t);
-// mex_f64.cu -- the factorised passes in double precision
-bool mex_use_f64(const MexGeo&, uint32_t flags);
-size_t mex_f64_workspace_bytes(const MexGeo&);
-cudaError_t launch_mex_fwd_f64(const MexGeo&, const double* x, const double* off, double* y, void* ws, uint32_t flags, cudaStream_t);
+// mex_gemm.cu -- the factorised passes as small contractions: float64, small float32 layers, input gradients of overlapping blocks
+bool mex_use_gemm(const MexGeo&, bool f64, uint32_t flags);
+size_t mex_gemm_workspace_bytes(const MexGeo&, bool f64);
+void* mex_gemm_maxima(const MexGeo&, bool f64, void* ws);
+cudaError_t launch_mex_fwd_gemm(const MexGeo&, bool f64, const void* x, const void* off, void* y, void* ws, uint32_t flags, cudaStream_t);
 // dx or doff may be null
-cudaError_t launch_mex_bwd_f64(const MexGeo&, const double* x, const double* off, const double* y, const double* dy, double* dx, double* doff,
-                               bool accumulate, void* ws, uint32_t flags, cudaStream_t);
+cudaError_t launch_mex_bwd_gemm(const MexGeo&, bool f64, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff,
+                                bool accumulate, void* ws, uint32_t flags, cudaStream_t);
 // number of multiprocessors of the current device (148 when no device answers)
 int device_sm_count();
 

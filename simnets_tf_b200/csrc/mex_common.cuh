@@ -21,6 +21,7 @@ struct MexWs {           // workspace carve-up, every part 256-byte aligned
     float* offn;         // [R][M][K] offsets minus their row's log-sum-exp, when the caller passes raw offsets
     float* lse;          // [R][M] that log-sum-exp
     float* dtmp;         // [R][M][K] offsets gradient with respect to the normalised rows (rows longer than 1024 taps only)
+    void* overlap;       // workspace of the input gradient of overlapping blocks (mex_gemm.cu)
     size_t bytes;
     size_t fwd_bytes;    // bytes the forward pass touches (everything before `part`)
 };
@@ -42,7 +43,7 @@ __host__ inline bool smallk_shape(const MexGeo& g) { return g.gp == 1 && g.K <= 
 // (M and N bounds: the kernels keep one value per instance in shared memory and address the instances of a chunk
 // with 32-bit offsets of up to 16 N elements; the same for 32 H W input elements.)
 __host__ inline bool tc_shape(const MexGeo& g) {
-    return !smallk_shape(g) && !smallm_shape(g) && g.M >= 48 && g.K >= 48 && g.M <= 2048 && g.N < (1 << 26) &&
+    return g.K > 32 && !smallm_shape(g) && g.M >= 48 && g.K >= 48 && g.M <= 2048 && g.N < (1 << 26) &&
            (long long)g.H * g.W < (1 << 25);
 }
 
@@ -50,7 +51,7 @@ __host__ inline bool tc_shape(const MexGeo& g) {
 // element; on the tensor cores the K multiply-adds per element disappear from the instruction stream, which the
 // streaming kernels of mex_smallk.cu cannot match (measured on a 4x2x2-block, 256-instance layer).
 __host__ inline bool tc_smallk_shape(const MexGeo& g) {
-    return smallk_shape(g) && g.K >= 8 && g.M >= 48 && g.M <= 2048 && g.N < (1 << 26) && (long long)g.H * g.W < (1 << 25);
+    return g.K <= 32 && g.K >= 8 && g.M >= 48 && g.M <= 2048 && g.N < (1 << 26) && (long long)g.H * g.W < (1 << 25);
 }
 
 // no patch reaches outside the input: no padding, and the last patch along each axis ends inside
@@ -137,6 +138,7 @@ __host__ inline MexWs carve(const MexGeo& g_in, void* base) {
     w.offn = reinterpret_cast<float*>(take(sizeof(float) * (size_t)g.R * g.M * g.K));
     w.lse = reinterpret_cast<float*>(take(sizeof(float) * g.R * g.M));
     w.dtmp = reinterpret_cast<float*>(take(g.K > 1024 ? sizeof(float) * (size_t)g.R * g.M * g.K : 0));
+    w.overlap = take(g.sc < g.bc || g.sh < g.bh || g.sw < g.bw ? mex_gemm_workspace_bytes(g, false) : 0);
     w.bytes = off;
     return w;
 }

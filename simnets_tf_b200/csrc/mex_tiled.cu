@@ -813,13 +813,9 @@ int launch_mex_fwd_static(const MexGeo& g, const float* x, const float* off, flo
 cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx,
                                 void* ws, uint32_t flags, cudaStream_t s, bool prepped) {
     const MexWs w = carve(g, ws);
-    if (!blocks_disjoint(g)) {           // overlapping blocks: the exact kernel (on the normalised rows, if the offsets came raw)
-        if (mex_norm(flags) && !(prepped || forward_primes_workspace(g, flags))) {
-            const cudaError_t e0 = run_prepasses(g, w, x, off, s, false, false, true);
-            if (e0 != cudaSuccess) return e0;
-        }
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, nullptr);
-    }
+    if (!blocks_disjoint(g))             // several positions add to one input value: gathered from their products, in a workspace part of its own
+        return launch_mex_bwd_gemm(g, false, x, off, y, dy, dx, nullptr, false, w.overlap,
+                                   flags & ~uint32_t(SIMNETS_FLAG_MEX_WORKSPACE_PRIMED | SIMNETS_FLAG_MEX_MAXIMA_GIVEN), s);
     const bool small = smallm_shape(g) || use_smallk_kernels(g, flags);
     cudaError_t e = (prepped || forward_primes_workspace(g, flags)) ? cudaSuccess : run_prepasses(g, w, x, off, s, !small, pair_prep(g, flags), mex_norm(flags));
     if (e != cudaSuccess) return e;

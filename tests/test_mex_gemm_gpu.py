@@ -1,0 +1,70 @@
+"""The small-contraction MEX kernels (float64 layers, small float32 layers, input gradients of overlapping blocks) at the
+edges of their tiles, and the tensor-core kernels at the small sizes that would otherwise run on them."""
+import importlib
+
+import numpy as np
+import pytest
+import torch
+
+import cases
+import gpu_util
+from simnets_tf_b200 import abi
+
+mex_ops = importlib.import_module("simnets_tf_b200.ops.mex")
+pytestmark = pytest.mark.gpu
+
+# row counts around the tile heights 16, 32 and 64, tap counts around the 16-step chunks and the 64 columns, position counts
+# around 64, reductions long enough to be split, overlapping and padded blocks, gaps between blocks
+EDGES = [
+    cases.mex_case("one_of_each", (1, 1, 1, 1), 1, (1, 1, 1), softmax=True, seed=501),
+    cases.mex_case("rows_15_taps_17", (3, 17, 5, 5), 15, (17, 1, 1), (17, 1, 1), softmax=True, seed=502, normalize=True),
+    cases.mex_case("rows_33_taps_65", (2, 65, 8, 9), 33, (65, 1, 1), (65, 1, 1), eps=0.5, softmax=True, unshared_region=(2,), seed=503, normalize=True),
+    cases.mex_case("rows_65_split", (2, 130, 2, 2), 65, (130, 1, 1), (130, 1, 1), eps=-0.8, unshared_region=(2,), seed=504),
+    cases.mex_case("positions_63", (1, 9, 9, 7), 20, (9, 1, 1), (9, 1, 1), softmax=True, unshared=False, shared_region=(-1,), seed=505),
+    cases.mex_case("long_row", (2, 80, 4, 4), 3, (80, 4, 4), (80, 4, 4), softmax=True, seed=506, normalize=True),
+    cases.mex_case("overlap_padded", (3, 5, 7, 8), 9, (3, 3, 2), (2, 1, 1), (1, 1, 1), oob=0.4, softmax=True, unshared_region=(2,), seed=507, normalize=True),
+    cases.mex_case("overlap_strided", (2, 4, 11, 10), 18, (4, 5, 3), (4, 2, 2), (0, 2, 1), eps=1.5, unshared=False, shared_region=(2,), seed=508),
+    cases.mex_case("gaps", (2, 6, 9, 9), 5, (2, 2, 2), (3, 3, 4), softmax=True, seed=509),
+]
+
+
+@pytest.mark.parametrize("dtype", [abi.F32, abi.F64], ids=["f32", "f64"])
+@pytest.mark.parametrize("c", EDGES, ids=lambda c: c["name"])
+def test_tile_edges(port, c, dtype):
+    gpu_util.check_mex(port, c, dtype=dtype, tol=1e-5 if dtype == abi.F32 else 1e-12, f64_tiebreak=dtype == abi.F32)
+
+
+@pytest.mark.parametrize("c", cases.MEX_PAIR + cases.MEX_CONFIGS + cases.MEX_HEAD + cases.MEX_ROWS + [c for c in cases.MEX_SMALL if c["name"].startswith(("tc_", "tiled_", "head_"))],
+                         ids=lambda c: c["name"])
+def test_large_layer_kernels_at_small_sizes(port, c):
+    gpu_util.check_mex(port, c, flags=abi.FLAG_MEX_NO_SMALL_TILES, f64_tiebreak=True)
+    gpu_util.check_mex_pooled_dy(port, c, flags=abi.FLAG_MEX_NO_SMALL_TILES, tol=2e-5)
+
+
+@pytest.mark.parametrize("flags", [0, abi.FLAG_MEX_NO_SMALL_TILES], ids=["small", "large"])
+def test_overlapping_input_gradient_in_parts(flags):
+    """More products than the workspace holds at a time: the batch is walked in parts, with the results of single samples."""
+    x, off = torch.randn(12, 16, 128, 128, device="cuda"), torch.randn(1, 4, 16, 5, 5, device="cuda")
+    attrs = dict(blocks=[16, 5, 5], strides=[16, 1, 1], padding=[0, 2, 2], softmax_mode=True, use_unshared_regions=False, shared_offset_region=[-1])
+    y = mex_ops.mex_forward(x, off, 4, flags=flags, **attrs)
+    dy = torch.randn_like(y)
+    dx = mex_ops.mex_input_grad(x, off, y, dy, 4, flags=flags, **attrs)
+    for n in (0, 9, 10, 11):
+        one = mex_ops.mex_input_grad(x[n:n + 1], off, y[n:n + 1], dy[n:n + 1], 4, flags=flags, **attrs)
+        assert torch.allclose(dx[n:n + 1], one, rtol=1e-5, atol=1e-5 * float(one.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
+def test_offsets_beyond_the_safe_spread_are_evaluated_term_by_term(port, dtype):
+    c = cases.mex_case("spread", (3, 12, 6, 6), 10, (12, 1, 1), (12, 1, 1), softmax=True, unshared_region=(2,), seed=520)
+    code = abi.F32 if dtype == torch.float32 else abi.F64
+    d = cases.mex_desc(c, dtype=code)
+    x, off, dy = cases.mex_inputs(c, port.mex_offsets_shape(d), port.mex_out_shape(d), np.float32 if code == abi.F32 else np.float64)
+    off[2, 3, 5] = -500.0
+    xd, od, dyd = (gpu_util.dev(a, dtype) for a in (x, off, dy))
+    attrs = cases.mex_attrs(c)
+    ry = port.mex_forward(d, x, off)
+    cases.assert_parity(mex_ops.mex_forward(xd, od, c["M"], **attrs).cpu().numpy(), ry, what="y")
+    dx, doff = mex_ops.mex_backward(xd, od, gpu_util.dev(ry, dtype), dyd, c["M"], **attrs)
+    cases.assert_parity(dx.cpu().numpy(), port.mex_input_grad(d, x, off, ry, dy), what="dx")
+    cases.assert_parity(doff.cpu().numpy(), port.mex_offsets_grad(d, x, off, ry, dy), tol=2e-5, what="doff")
