@@ -20,7 +20,7 @@ struct MexWs {           // workspace carve-up, every part 256-byte aligned
     float* tc_tiles_dx;  // the same for the input gradient of the pair-tile kernels (rows = taps), written together with tc_tiles
     float* offn;         // [R][M][K] offsets minus their row's log-sum-exp, when the caller passes raw offsets
     float* lse;          // [R][M] that log-sum-exp
-    float* dtmp;         // [R][M][K] offsets gradient with respect to the normalised rows (rows longer than 1024 taps only)
+    float* dtmp;         // [R][M][K] offsets gradient with respect to the normalised rows
     void* overlap;       // workspace of the input gradient of overlapping blocks (mex_gemm.cu)
     size_t bytes;
     size_t fwd_bytes;    // bytes the forward pass touches (everything before `part`)
@@ -116,6 +116,7 @@ __host__ inline MexWs carve(const MexGeo& g_in, void* base) {
     auto splits_of = [](const MexGeo& q) {
         int s = (tc_shape(q) || tc_smallk_shape(q)) ? std::max(doff_splits(q), mex_tc_doff_splits(q)) : doff_splits(q);
         if ((tc_shape(q) || tc_smallk_shape(q)) && mex_pair_shape(q)) s = std::max(s, mex_pair_doff_splits(q));
+        if (tc_smallk_shape(q) && mex_short_shape(q)) s = std::max(s, mex_short_splits(q));
         if (mex_head_shape(q)) s = std::max(s, mex_head_splits(q));
         return s;
     };
@@ -137,7 +138,7 @@ __host__ inline MexWs carve(const MexGeo& g_in, void* base) {
     // raw offsets (SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS): the normalised rows for the exact kernels and each row's log-sum-exp
     w.offn = reinterpret_cast<float*>(take(sizeof(float) * (size_t)g.R * g.M * g.K));
     w.lse = reinterpret_cast<float*>(take(sizeof(float) * g.R * g.M));
-    w.dtmp = reinterpret_cast<float*>(take(g.K > 1024 ? sizeof(float) * (size_t)g.R * g.M * g.K : 0));
+    w.dtmp = reinterpret_cast<float*>(take(sizeof(float) * (size_t)g.R * g.M * g.K));
     w.overlap = take(g.sc < g.bc || g.sh < g.bh || g.sw < g.bw ? mex_gemm_workspace_bytes(g, false) : 0);
     w.bytes = off;
     return w;

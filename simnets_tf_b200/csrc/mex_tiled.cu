@@ -488,16 +488,35 @@ __global__ void __launch_bounds__(256) mex_doff_tiled(MexGeo g, const float* __r
     }
 }
 
-// doff[r][m][k] (+)= Eo[r][m][k] * sum over splits, in split order (deterministic)
-__global__ void __launch_bounds__(256) mex_doff_reduce(long long n, int K, int splits, const float* __restrict__ part, const float* __restrict__ eo,
-                                                       float* __restrict__ doff, int accumulate, const int* __restrict__ flag) {
+// out[r][m][k] (+)= Eo[r][m][k] * sum over splits, in a fixed order.  512 threads = `slices` slices of the splits x 512 / slices
+// consecutive outputs: with hundreds of splits of a small offsets table (256 instances of 16 taps, 296 splits) one thread per
+// output would fill 16 CTAs and walk the splits alone.  When a status word is set (unsafe spread, or a tensor-core launch gave
+// up on a wait) the exact kernel does the work: `keep_exact` copies what it left in `part`, else nothing is written.
+__global__ void __launch_bounds__(512) mex_doff_reduce(long long n, int K, int splits, int slices, const float* __restrict__ part, const float* __restrict__ eo,
+                                                       float* __restrict__ out, int accumulate, int keep_exact, const int* __restrict__ flag) {
     stream_order();
-    if (flag[0] | flag[1]) return;               // unsafe spread, or a tensor-core launch gave up on a wait: the exact kernel behind does the work
-    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    __shared__ float red[512];
+    const bool exact = (flag[0] | flag[1]) != 0;
+    if (exact && !keep_exact) return;
+    const int lanes = 512 / slices, lane = threadIdx.x & (lanes - 1), slice = threadIdx.x / lanes;
+    for (long long first = (long long)blockIdx.x * lanes; first < n; first += (long long)gridDim.x * lanes) {
+        const long long i = first + lane;
         float s = 0.f;
-        for (int p = 0; p < splits; ++p) s += part[(size_t)p * n + i];
-        s *= eo[(i / K) * pad4(K) + i % K];
-        doff[i] = accumulate ? doff[i] + s : s;
+        if (i < n) {
+            if (exact) s = slice == 0 ? part[i] : 0.f;
+            else {
+#pragma unroll 8
+                for (int p = slice; p < splits; p += slices) s += part[(size_t)p * n + i];
+            }
+        }
+        red[threadIdx.x] = s;
+        __syncthreads();
+        if (slice == 0 && i < n) {
+            for (int q = 1; q < slices; ++q) s += red[q * lanes + lane];
+            if (!exact) s *= eo[(i / K) * pad4(K) + i % K];
+            out[i] = accumulate ? out[i] + s : s;
+        }
+        __syncthreads();
     }
 }
 
@@ -525,6 +544,7 @@ __global__ void __launch_bounds__(128) mex_doff_reduce_norm(int K, int splits, l
             if (exact) sk[e] = part[i];
             else {
                 float a = 0.f;
+#pragma unroll 8
                 for (int p = 0; p < splits; ++p) a += part[(size_t)p * n + i];
                 sk[e] = a * eo[row * pad4(K) + k];
             }
@@ -550,20 +570,8 @@ __global__ void __launch_bounds__(128) mex_doff_reduce_norm(int K, int splits, l
     }
 }
 
-// Longer rows (the classifier head: 10 rows of 8192 taps): the element-parallel reduction into a scratch row set, then the
-// row pass.  `tmp` = gradient with respect to the normalised rows.
-__global__ void __launch_bounds__(256) mex_doff_reduce_tmp(long long n, int K, int splits, const float* __restrict__ part, const float* __restrict__ eo,
-                                                           float* __restrict__ tmp, const int* __restrict__ flag) {
-    stream_order();
-    const bool exact = (flag[0] | flag[1]) != 0;
-    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-        if (exact) { tmp[i] = part[i]; continue; }
-        float s = 0.f;
-        for (int p = 0; p < splits; ++p) s += part[(size_t)p * n + i];
-        tmp[i] = s * eo[(i / K) * pad4(K) + i % K];
-    }
-}
-
+// Longer rows, and few rows of many splits (the classifier head: 10 rows of 8192 taps): mex_doff_reduce into a scratch row set
+// (`tmp` = gradient with respect to the normalised rows), then the row pass.
 __global__ void __launch_bounds__(256) mex_doff_norm_rows(int K, const float* __restrict__ tmp, const float* __restrict__ raw, const float* __restrict__ lse,
                                                           float* __restrict__ doff, int accumulate) {
     stream_order();
@@ -594,23 +602,29 @@ inline bool mex_norm(uint32_t flags) { return (flags & SIMNETS_FLAG_MEX_NORMALIZ
 cudaError_t finish_doff(const MexGeo& g, const MexWs& w, int splits, const float* x, const float* off, const float* y, const float* dy,
                         float* doff, bool accumulate, uint32_t flags, cudaStream_t s) {
     const long long n = (long long)g.R * g.M * g.K;
+    const auto reduce_splits = [&](float* out, int add, int keep_exact) {
+        const int slices = splits >= 64 ? 32 : (splits >= 8 ? 8 : 1), lanes = 512 / slices;
+        in_stream_order(mex_doff_reduce, int(std::min<long long>((n + lanes - 1) / lanes, (long long)device_sm_count() * 8)), 512, 0, s)(
+            n, g.K, splits, slices, w.part, w.eo, out, add, keep_exact, w.flag);
+    };
     if (mex_norm(flags)) {
         cudaError_t e = launch_mex_doff_direct(g, false, x, w.offn, y, dy, w.part, false, s, w.flag);
         if (e != cudaSuccess) return e;
         const int rows = g.R * g.M;
-        if (g.K <= 128) in_stream_order(mex_doff_reduce_norm<1>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else if (g.K <= 256) in_stream_order(mex_doff_reduce_norm<2>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else if (g.K <= 512) in_stream_order(mex_doff_reduce_norm<4>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else if (g.K <= 1024) in_stream_order(mex_doff_reduce_norm<8>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
-        else {
-            in_stream_order(mex_doff_reduce_tmp, int(std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(n, g.K, splits, w.part, w.eo, w.dtmp, w.flag);
+        const bool few_rows = rows < device_sm_count() && splits >= 32;         // (one CTA per row would leave most of the GPU idle)
+        if (g.K > 1024 || few_rows) {
+            reduce_splits(w.dtmp, 0, 1);
             in_stream_order(mex_doff_norm_rows, rows, 256, 0, s)(g.K, w.dtmp, off, w.lse, doff, accumulate);
             count_launch();
         }
+        else if (g.K <= 128) in_stream_order(mex_doff_reduce_norm<1>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        else if (g.K <= 256) in_stream_order(mex_doff_reduce_norm<2>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        else if (g.K <= 512) in_stream_order(mex_doff_reduce_norm<4>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
+        else in_stream_order(mex_doff_reduce_norm<8>, rows, 128, 0, s)(g.K, splits, n, w.part, w.eo, off, w.lse, doff, accumulate, w.flag);
         count_launch();
         return cudaGetLastError();
     }
-    in_stream_order(mex_doff_reduce, int(std::min<long long>((n + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(n, g.K, splits, w.part, w.eo, doff, accumulate, w.flag);
+    reduce_splits(doff, accumulate, 0);
     count_launch();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -633,6 +647,12 @@ bool blocks_disjoint(const MexGeo& g) { return g.sc >= g.bc && g.sh >= g.bh && g
 bool blocks_cover_input(const MexGeo& g) {
     auto full = [](int dim, int block, int stride, int pad) { return stride == block && pad == 0 && dim % block == 0; };
     return full(g.C, g.bc, g.sc, g.pc) && full(g.H, g.bh, g.sh, g.ph) && full(g.W, g.bw, g.sw, g.pw);
+}
+
+// Gradients of short patches from one read of y and dy (mex_short.cu).  Layers whose unshared regions alternate along the width
+// keep the pair-tile kernels: a tile of one region would use every other float of a sector.
+bool use_short_bwd(const MexGeo& g, uint32_t flags, const void* a, const void* b, const void* c, const void* d) {
+    return use_tc_kernels(g, flags) && !(flags & SIMNETS_FLAG_MEX_TC_ONE_TILE) && mex_short_shape(g) && !use_pair_kernels(g, flags, a, b, c, d);
 }
 
 cudaError_t run_prepasses(const MexGeo& g, const MexWs& w, const float* x, const float* off, cudaStream_t s, bool need_mx = true,
@@ -828,6 +848,13 @@ cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* of
         if (e != cudaSuccess) return e;
         return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
     }
+    // (the input gradient alone: the one-tile kernel pads the taps to 16 or 32 columns of its tile but fills the GPU as well with
+    // many positions: 200 instances over 8x2x2 blocks at 0.4 GB of y 320 us there, 395 here; 64 over 2x2x2 176 there, 93 here)
+    if (use_short_bwd(g, flags, x, y, dy, dx) && (g.K <= 12 || (long long)g.B * g.rs * g.R <= 512LL * device_sm_count())) {
+        e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, dx, nullptr, w.flag, s);
+        if (e != cudaSuccess) return e;
+        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+    }
     if (use_tc_kernels(g, flags) && use_pair_kernels(g, flags, x, y, dy, dx)) {
         e = launch_mex_dx_pair(g, x, w.tc_tiles_dx, w.mo, w.mx, y, dy, dx, w.flag, s);
         if (e != cudaSuccess) return e;
@@ -877,6 +904,11 @@ cudaError_t launch_mex_doff_tiled(const MexGeo& g, const float* x, const float* 
     const MexWs w = carve(g, ws);
     cudaError_t e = (prepped || forward_primes_workspace(g, flags)) ? cudaSuccess : run_prepasses(g, w, x, off, s, !use_smallk_kernels(g, flags), pair_prep(g, flags), mex_norm(flags));
     if (e != cudaSuccess) return e;
+    if (use_short_bwd(g, flags, x, y, dy, dy)) {
+        e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, nullptr, w.part, w.flag, s);
+        if (e != cudaSuccess) return e;
+        return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s);
+    }
     if (use_tc_kernels(g, flags)) {
         int tsplits = mex_tc_doff_splits(g);
         e = use_pair_kernels(g, flags, x, y, dy, dy) ? launch_mex_doff_pair(g, x, w.mo, w.mx, y, dy, w.part, &tsplits, w.flag, s)
@@ -932,6 +964,17 @@ cudaError_t launch_mex_backward_tiled(const MexGeo& g, const float* x, const flo
         e = launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
         if (e != cudaSuccess) return e;
         return finish_doff(g, w, hs, x, off, y, dy, doff, accumulate, flags, s);
+    }
+    if (use_short_bwd(g, flags, x, y, dy, dx)) {
+        if (!blocks_cover_input(g)) {
+            e = cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)g.B * g.C * g.H * g.W, s);
+            if (e != cudaSuccess) return e;
+        }
+        e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, dx, w.part, w.flag, s);
+        if (e != cudaSuccess) return e;
+        e = launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        if (e != cudaSuccess) return e;
+        return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s);
     }
     e = launch_mex_dx_tiled(g, x, off, y, dy, dx, ws, flags, s, true);
     if (e != cudaSuccess) return e;
