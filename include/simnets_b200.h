@@ -350,6 +350,19 @@ SIMNETS_API int simnets_mex_backward(const simnets_mex_desc* d,
  * No counterpart in the reference. */
 SIMNETS_API int64_t simnets_fp32_fma_probe(int32_t packed, int32_t iters, void* scratch, void* stream);
 
+/* ---- diagonal Gaussian mixture over patches ------------------------------- */
+/* One EM step of the reference's unsupervised initialisation (python/simnets/unsupervised/gmm.py:37-71) over the patches that
+ * the descriptor's Similarity op would see (float32, L2 without normalisation, no flags; num_instances = components, uniform
+ * mixing weights).  simnets_mixture_statistics writes stats = { sum r (p - mean) [k][patch], sum r (p - mean)^2 [k][patch],
+ * sum r [k] } for responsibilities r under the current parameters; a data-parallel job adds its ranks' stats.
+ * simnets_mixture_parameters: mean + shift / mass, and the second moment about the new mean plus min_var.  A workspace size of 0
+ * means that the shape is not supported (double precision, hundreds of components). */
+SIMNETS_API size_t simnets_mixture_workspace_bytes(const simnets_sim_desc* desc);
+SIMNETS_API int simnets_mixture_statistics(const simnets_sim_desc* desc, const void* x, const void* means, const void* covs, void* stats,
+                                           void* workspace, size_t workspace_bytes, void* stream);
+SIMNETS_API int simnets_mixture_parameters(int32_t k, int32_t taps, float min_var, const float* stats, const float* means,
+                                           float* new_means, float* new_covs, void* stream);
+
 /* ---- sum pooling ----------------------------------------------------------- */
 /* y[p, h, w] = x[p, 2h, 2w] + x[p, 2h, 2w+1] + x[p, 2h+1, 2w] + x[p, 2h+1, 2w+1] over a dense float32 tensor
  * [planes, height, width] (planes = batch * channels); height and width even, else SIMNETS_E_UNSUPPORTED.

@@ -338,6 +338,28 @@ int simnets_normalize_offsets_backward(int64_t rows, int32_t k, const void* off,
     return from_cuda(launch_normalize_offsets_bwd(rows, k, (const float*)off, (const float*)dout, (float*)doff, as_stream(stream)));
 }
 
+size_t simnets_mixture_workspace_bytes(const simnets_sim_desc* d) {
+    SimGeo g;
+    if (sim_geometry(d, &g) || !mixture_shape(g, d->dtype == SIMNETS_F64, d->flags)) return 0;
+    return mixture_workspace_bytes(g);
+}
+
+int simnets_mixture_statistics(const simnets_sim_desc* d, const void* x, const void* means, const void* covs, void* stats, void* ws, size_t ws_bytes, void* stream) {
+    SimGeo g;
+    const int rc = sim_geometry(d, &g);
+    if (rc) return rc;
+    if (!mixture_shape(g, d->dtype == SIMNETS_F64, d->flags)) return SIMNETS_E_UNSUPPORTED;
+    if (!x || !means || !covs || !stats) return SIMNETS_E_NULL;
+    if (!ws || ws_bytes < mixture_workspace_bytes(g)) return SIMNETS_E_WORKSPACE;
+    return from_cuda(launch_mixture_statistics(g, (const float*)x, (const float*)means, (const float*)covs, (float*)stats, ws, as_stream(stream)));
+}
+
+int simnets_mixture_parameters(int32_t k, int32_t taps, float min_var, const float* stats, const float* means, float* new_means, float* new_covs, void* stream) {
+    if (k < 1 || taps < 1 || (long long)k * taps > (1LL << 30)) return SIMNETS_E_DESC;
+    if (!stats || !means || !new_means || !new_covs) return SIMNETS_E_NULL;
+    return from_cuda(launch_mixture_parameters(k, taps, min_var, stats, means, new_means, new_covs, as_stream(stream)));
+}
+
 int64_t simnets_fp32_fma_probe(int32_t packed, int32_t iters, void* scratch, void* stream) {
     if (iters < 1 || !scratch) return SIMNETS_E_DESC;
     const int blocks = device_sm_count() * 2;                       // two CTAs of 1024 threads fill an SM

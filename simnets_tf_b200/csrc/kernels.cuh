@@ -62,6 +62,11 @@ cudaError_t launch_sim_dparams(const SimGeo&, const float* x, const float* t, co
 // sim_dx.cu
 size_t sim_dx_scratch_floats(const SimGeo&);
 cudaError_t launch_sim_dx(const SimGeo&, const float* x, const float* t, const float* w, const float* dy, float* dx, float* dxp, cudaStream_t);
+// mixture.cu -- one EM step of a diagonal mixture over patches
+bool mixture_shape(const SimGeo&, bool f64, uint32_t flags);
+size_t mixture_workspace_bytes(const SimGeo&);
+cudaError_t launch_mixture_statistics(const SimGeo&, const float* x, const float* means, const float* covs, float* stats, void* ws, cudaStream_t);
+cudaError_t launch_mixture_parameters(int k, int taps, float min_var, const float* stats, const float* means, float* new_means, float* new_covs, cudaStream_t);
 // sim_smallk.cu -- forward for short patches (K <= 32): patches in registers; extrema_done: ch_max / ch_min were written too
 bool sim_smallk_shape(const SimGeo&);
 cudaError_t launch_sim_fwd_smallk(const SimGeo&, const float* x, const float* t, const float* w, float* y, float* ch_max, float* ch_min,

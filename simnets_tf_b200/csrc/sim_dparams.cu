@@ -265,9 +265,10 @@ __global__ void __launch_bounds__(512) sim_dparams_reduce(SimGeo g, int splits, 
         if (slice == 0 && i < mk) {
 #pragma unroll 8
             for (int q = 1; q < slices; ++q) { a += red[0][q * lanes + lane]; b += red[1][q * lanes + lane]; c += red[2][q * lanes + lane]; }
-            const float wraw = wt[i], w = g.absw ? fabsf(wraw) : wraw;
+            const float wraw = wt ? wt[i] : 1.f, w = g.absw ? fabsf(wraw) : wraw;
             float gt, gw;
-            if (g.mode == SIM_L1 || g.mode == SIM_L1_SKIP) { gt = w * a; gw = -b; }
+            if (wt == nullptr) { gt = a; gw = b; }           // no weights: the plain sums (the statistics of mixture.cu)
+            else if (g.mode == SIM_L1 || g.mode == SIM_L1_SKIP) { gt = w * a; gw = -b; }
             else if (g.mode == SIM_L2) { gt = 2.f * w * a; gw = -b; }
             else { gt = w * a; gw = 0.5f * (c / (w + fudge) - b); }
             if (g.absw) gw *= wraw > 0.f ? 1.f : (wraw < 0.f ? -1.f : 0.f);          // d|w|/dw, 0 at w = 0

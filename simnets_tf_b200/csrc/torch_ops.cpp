@@ -426,6 +426,32 @@ Tensor sim_apply(const SimPlanPtr& p, const Tensor& x, const Tensor& t, const Te
     return y;
 }
 
+// ----------------------------------------------------------------------------------------------------------------- mixture
+// Flat statistics of one EM step, or nothing where the library has no kernels for the shape.
+OptTensor mixture_statistics(const SimPlanPtr& p, const Tensor& x_in, const Tensor& means_in, const Tensor& covs_in) {
+    require_cuda_all(x_in, means_in, covs_in);
+    p->check_tensors(x_in, means_in, covs_in);
+    const size_t n = simnets_mixture_workspace_bytes(&p->d);
+    if (n == 0) return std::nullopt;
+    const Tensor x = x_in.contiguous(), means = means_in.contiguous(), covs = covs_in.contiguous();
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor stats = at::empty({2 * means.numel() + means.size(0)}, means.options());
+    const Tensor ws = scratch(x, n);
+    check(simnets_mixture_statistics(&p->d, ptr(x), ptr(means), ptr(covs), ptr(stats), ptr(ws), ws.numel(), stream_of(x)));
+    return stats;
+}
+
+std::pair<Tensor, Tensor> mixture_parameters(const Tensor& stats, const Tensor& means_in, double min_var) {
+    require_cuda_all(stats, means_in);
+    const Tensor means = means_in.contiguous();
+    TORCH_CHECK(stats.scalar_type() == at::kFloat && stats.is_contiguous() && stats.numel() == 2 * means.numel() + means.size(0), "stats do not belong to these means");
+    const c10::cuda::CUDAGuard guard(means.device());
+    Tensor new_means = at::empty(means.sizes(), means.options()), new_covs = at::empty(means.sizes(), means.options());
+    check(simnets_mixture_parameters(int32_t(means.size(0)), int32_t(means.numel() / means.size(0)), float(min_var), stats.data_ptr<float>(), means.data_ptr<float>(),
+                                     new_means.data_ptr<float>(), new_covs.data_ptr<float>(), stream_of(means)));
+    return {new_means, new_covs};
+}
+
 // ---------------------------------------------------------------------------------------------------- softmax cross-entropy
 std::pair<Tensor, Tensor> xent_with_grad(const Tensor& logits_in, const Tensor& labels_in, double scale) {
     require_cuda_all(logits_in);
@@ -511,6 +537,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sim_input_grad", &sim_input_grad);
     m.def("sim_params_grad", &sim_params_grad);
     m.def("sim_apply", &sim_apply);
+    m.def("mixture_statistics", &mixture_statistics);
+    m.def("mixture_parameters", &mixture_parameters);
     m.def("xent_with_grad", &xent_with_grad);
     m.def("xent_apply", &xent_apply);
     m.def("profile_start", [] { py::list dropped = profile_take(); g_profiling = true; });

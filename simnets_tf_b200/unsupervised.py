@@ -29,6 +29,8 @@ import importlib
 import numpy as np
 import torch
 
+from . import _lib
+
 _sim = importlib.import_module(__package__ + ".ops.similarity")     # the module: `ops.similarity` itself is the op function
 
 MIN_VAR = 1e-3      # variance floor added to every diagonal covariance by an EM step
@@ -50,6 +52,13 @@ class LibraryPatchOps(object):
         """(sum r (p - c), sum r (p - c)^2), each shaped like `centres`, for resp [batch, k, out_h, out_w]."""
         dt, dw = _sim.similarity_parameters_grad(x, centres, torch.ones_like(centres), resp, flags=self.flags, **self.attrs)
         return dt.mul_(0.5), dw.neg_()
+
+    def mixture_statistics(self, x, means, covs):
+        """sum r (p - mean), sum r (p - mean)^2 and sum r of a mixture's responsibilities r, in one flat tensor, by the
+        library's own kernels; None where it has none (float64, an empty batch, hundreds of components)."""
+        if x.dtype != torch.float32 or x.shape[0] == 0 or self.flags:
+            return None
+        return _lib.ops().mixture_statistics(_sim.similarity_plan(x, means, covs, _sim._attrs(**self.attrs)), x, means, covs)
 
 
 def _patch_grid(x, blocks, strides):
@@ -176,6 +185,11 @@ class DiagonalGMM(_Estimator):
 
     def update(self, x):
         x = self._check(x)
+        stats = self.ops.mixture_statistics(x, self.means, self.covs) if isinstance(self.ops, LibraryPatchOps) else None
+        if stats is not None:
+            stats, = _all_reduce(self.group, stats)
+            self.means, self.covs = _lib.ops().mixture_parameters(stats, self.means, self.min_var)
+            return self.means, self.covs
         half_mahalanobis = self.ops.neg_scaled_sqdist(x, self.means, (1.0 / self.covs).contiguous())
         logdet = self.covs.log().sum(dim=(1, 2, 3))
         resp = torch.softmax(0.5 * (half_mahalanobis - logdet.view(1, -1, 1, 1)), dim=1)
