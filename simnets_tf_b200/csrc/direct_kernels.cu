@@ -204,6 +204,49 @@ __global__ void __launch_bounds__(kThreads) mex_doff_direct(MexGeo g, const T* _
     }
 }
 
+// The term-by-term redo behind a factorised forward pass whose 2x2 sum pooling was produced with it: a thread redoes the four
+// outputs of one pooling window and their sum (added in window order).
+__global__ void __launch_bounds__(kThreads) mex_redo_fwd_pool(MexGeo g, const float* __restrict__ x, const float* __restrict__ off, float* __restrict__ y,
+                                                              float* __restrict__ pooled, const int* __restrict__ gate) {
+    stream_order();
+    if ((gate[0] | gate[1]) == 0) return;
+    const int Hp = g.Ho / 2, Wp = g.Wo / 2;
+    const long long total = (long long)g.B * g.M * g.Co * Hp * Wp;
+    for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < total; i += (long long)gridDim.x * kThreads) {
+        const int w = int(i % Wp);
+        const long long ph = i / Wp, at = (ph / Hp * g.Ho + 2 * (ph % Hp)) * g.Wo + 2 * w;
+        float s = 0.f;
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+            const long long idx = at + (u >> 1) * g.Wo + (u & 1);
+            const float v = mex_exact_y(g, x, off, idx);
+            y[idx] = v;
+            s = u == 0 ? v : s + v;
+        }
+        pooled[i] = s;
+    }
+}
+
+// The same behind both gradients of a layer: one launch redoes dx and doff.
+__global__ void __launch_bounds__(kThreads) mex_redo_bwd(MexGeo g, const float* __restrict__ x, const float* __restrict__ off, const float* __restrict__ y,
+                                                         const float* __restrict__ dy, float* __restrict__ dx, float* __restrict__ doff, int accumulate,
+                                                         const int* __restrict__ gate) {
+    stream_order();
+    __shared__ float smem[kThreads];
+    if ((gate[0] | gate[1]) == 0) return;
+    const long long total = (long long)g.B * g.C * g.H * g.W;
+    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads)
+        dx[idx] = mex_exact_dx(g, x, off, y, dy, idx);
+    const long long triples = (long long)g.R * g.M * g.K;
+    for (long long rmk = blockIdx.x; rmk < triples; rmk += gridDim.x) {
+        const int k = int(rmk % g.K), m = int((rmk / g.K) % g.M), r = int(rmk / ((long long)g.K * g.M));
+        float sum = 0.f;
+        for (long long i = threadIdx.x; i < (long long)g.B * g.rs; i += kThreads) sum += mex_exact_doff_term(g, x, off[rmk], y, dy, r, m, k, i);
+        const float rsum = block_sum(sum, smem);
+        if (threadIdx.x == 0) doff[rmk] = accumulate ? doff[rmk] + rsum : rsum;
+    }
+}
+
 // gated: the launch follows a factorised kernel and does work only if that one raised the safety flag; a grid that
 // just fills the GPU keeps the usual case (every CTA reads the flag and returns) at a few microseconds
 inline int grid_for(long long total, bool gated = false) {
@@ -253,6 +296,19 @@ cudaError_t launch_mex_fwd_direct(const MexGeo& g, bool f64, const void* x, cons
     SIMNETS_DTYPE_SWITCH(f64,
         (in_stream_order(mex_fwd_direct<float>, grid_for(total, gate != nullptr), kThreads, 0, s)(g, (const float*)x, (const float*)off, (float*)y, gate)),
         (in_stream_order(mex_fwd_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)off, (double*)y, gate)));
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mex_redo_fwd_pool(const MexGeo& g, const float* x, const float* off, float* y, float* pooled, cudaStream_t s, const int* gate) {
+    in_stream_order(mex_redo_fwd_pool, grid_for((long long)g.B * g.M * g.N / 4, true), kThreads, 0, s)(g, x, off, y, pooled, gate);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mex_redo_bwd(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx, float* doff, bool accumulate,
+                                cudaStream_t s, const int* gate) {
+    in_stream_order(mex_redo_bwd, device_sm_count() * 8, kThreads, 0, s)(g, x, off, y, dy, dx, doff, int(accumulate), gate);
     count_launch();
     return cudaGetLastError();
 }

@@ -36,6 +36,11 @@ cudaError_t launch_mex_dx_direct(const MexGeo&, bool f64, const void* x, const v
 cudaError_t launch_mex_doff_direct(const MexGeo&, bool f64, const void* x, const void* off, const void* y, const void* dy,
                                    void* doff, bool accumulate, cudaStream_t, const int* gate = nullptr);
 
+// one gated launch for a forward pass and its pooling, one for both gradients
+cudaError_t launch_mex_redo_fwd_pool(const MexGeo&, const float* x, const float* off, float* y, float* pooled, cudaStream_t, const int* gate);
+cudaError_t launch_mex_redo_bwd(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* dx, float* doff, bool accumulate,
+                                cudaStream_t, const int* gate);
+
 }  // namespace simnets
 
 namespace simnets {
@@ -122,7 +127,8 @@ int mex_pair_nt_fwd(const MexGeo&);
 int mex_pair_nt_dx(const MexGeo&);
 int mex_pair_doff_splits(const MexGeo&);
 size_t mex_pair_tile_floats(const MexGeo&);      // floats of one set of pre-split operand tiles as the pair-tile prepass writes them
-// pooled: when given, also the 2x2 sum pooling of y ([B, M * Co, Ho / 2, Wo / 2]; Ho and Wo even), added up by the epilogue
+// pooled: when given, also the 2x2 sum pooling of y ([B, M * Co, Ho / 2, Wo / 2]; Ho and Wo even), added up by the epilogue onto
+// the zeros that the caller has put there
 cudaError_t launch_mex_fwd_pair(const MexGeo&, const float* x, const float* tiles, const float* mo, const float* mx, float* y,
                                 float* pooled, int* flag, int test_expire, cudaStream_t);
 cudaError_t launch_mex_dx_pair(const MexGeo&, const float* x, const float* tiles, const float* mo, const float* mx, const float* y,
@@ -151,9 +157,9 @@ cudaError_t launch_softmax_xent(int batch, int classes, float scale, const float
 // forward on the library's fixed device scratch; returns a status code of simnets_b200.h
 int launch_mex_fwd_static(const MexGeo&, const float* x, const float* off, float* y, uint32_t flags, cudaStream_t);
 cudaError_t launch_mex_dx_tiled(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* dx,
-                                void* ws, uint32_t flags, cudaStream_t, bool prepped = false);
+                                void* ws, uint32_t flags, cudaStream_t, bool prepped = false, bool redo = true);
 cudaError_t launch_mex_backward_tiled(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* dx,
                                       float* doff, bool accumulate, void* ws, uint32_t flags, cudaStream_t);
 cudaError_t launch_mex_doff_tiled(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* doff,
-                                  bool accumulate, void* ws, uint32_t flags, cudaStream_t, bool prepped = false);
+                                  bool accumulate, void* ws, uint32_t flags, cudaStream_t, bool prepped = false, float* redo_dx = nullptr);
 }  // namespace simnets

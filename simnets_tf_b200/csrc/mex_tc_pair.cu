@@ -1186,10 +1186,6 @@ size_t mex_pair_tile_floats(const MexGeo& g) {
 
 cudaError_t launch_mex_fwd_pair(const MexGeo& g, const float* x, const float* tiles, const float* mo, const float* mx, float* y,
                                 float* pooled, int* flag, int test_expire, cudaStream_t s) {
-    if (pooled != nullptr) {           // the epilogue adds the two halves of every pooling window onto zeros
-        const cudaError_t e = cudaMemsetAsync(pooled, 0, sizeof(float) * (size_t)g.B * g.M * (g.N >> 2), s);
-        if (e != cudaSuccess) return e;
-    }
     if (pair_nt(g.M) == 128) return launch_fwd_pair_nt<128>(g, x, tiles, mo, mx, y, pooled, flag, test_expire, s);
     return launch_fwd_pair_nt<64>(g, x, tiles, mo, mx, y, pooled, flag, test_expire, s);
 }

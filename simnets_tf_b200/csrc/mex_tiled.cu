@@ -32,7 +32,7 @@ namespace simnets {
 namespace {
 
 // ------------------------------------------------------------------ prepasses
-// One block per (region, instance): stabiliser mo, Eo in both layouts, and the safety flag.  With tile pointers the block
+// One row of offsets (region, instance): stabiliser mo, Eo in both layouts, and the safety flag.  With tile pointers the block
 // also writes its part of the tensor-core operand tiles (Eo split into TF32 hi / lo, laid out as the MMA reads it: what
 // mex_tc_prep produces in a launch of its own): tf = forward tiles, rows = instances in tiles of ntf, reduction = taps;
 // td = input-gradient tiles, rows = taps in tiles of ntd, reduction = instances.  The grid then also covers the rows that
@@ -40,34 +40,37 @@ namespace {
 __device__ __forceinline__ float prep_tf32_hi(float v) { uint32_t r; asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v)); return __uint_as_float(r); }
 __device__ __forceinline__ int prep_core_offset(int row, int k) { return (row >> 3) * 128 + (k >> 2) * 32 + (row & 7) * 4 + (k & 3); }   // floats, 16-wide chunks
 
-__global__ void __launch_bounds__(512) mex_prep_offsets(MexGeo g, int Mp, const float* __restrict__ off, float* __restrict__ mo,
-                                                        float* __restrict__ eo, float* __restrict__ eot, int* __restrict__ flag,
-                                                        float* __restrict__ tf, int ntf, float* __restrict__ td, int ntd,
-                                                        float* __restrict__ offn, float* __restrict__ lse_out) {
-    stream_order();
-    __shared__ float s_hi[512], s_lo[512];
-    __shared__ int s_bad[512];
-    const int nt = blockDim.x;                       // 128, or 512 for long rows
-    const int r = blockIdx.x / Mp, m = blockIdx.x % Mp;
-    const bool real = m < g.M;
+struct PrepArgs {        // what the parameter prepass writes (see MexWs); tf / td / offn may be null
+    int Mp, ntf, ntd;
+    float *mo, *eo, *eot, *tf, *td, *offn, *lse;
+    int* flag;
+};
+
+// nt threads (t = 0 .. nt - 1) work on one row; every thread of the CTA calls this, with the row of its group
+__device__ __forceinline__ void prep_row(const MexGeo& g, int row, int t, int nt, float* s_hi, float* s_lo, int* s_bad, const float* __restrict__ off, const PrepArgs& a) {
+    const int Mp = a.Mp, ntf = a.ntf, ntd = a.ntd;
+    float *mo = a.mo, *eo = a.eo, *eot = a.eot, *tf = a.tf, *td = a.td, *offn = a.offn, *lse_out = a.lse;
+    int* flag = a.flag;
+    const int r = row / Mp, m = row % Mp;
+    const bool exists = row < g.R * Mp, real = exists && m < g.M;
     const int rm = r * g.M + m;
     const float* o = off + (size_t)rm * g.K;
     float hi = -CUDART_INF_F, lo = CUDART_INF_F;
     int bad = 0;
     if (real) {
-        for (int k = threadIdx.x; k < g.K; k += nt) {
+        for (int k = t; k < g.K; k += nt) {
             const float v = o[k];
             if (!isfinite(v)) bad = 1;
             hi = fmaxf(hi, v); lo = fminf(lo, v);
         }
     }
-    s_hi[threadIdx.x] = hi; s_lo[threadIdx.x] = lo; s_bad[threadIdx.x] = bad;
+    s_hi[t] = hi; s_lo[t] = lo; s_bad[t] = bad;
     __syncthreads();
     for (int s = nt / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            s_hi[threadIdx.x] = fmaxf(s_hi[threadIdx.x], s_hi[threadIdx.x + s]);
-            s_lo[threadIdx.x] = fminf(s_lo[threadIdx.x], s_lo[threadIdx.x + s]);
-            s_bad[threadIdx.x] |= s_bad[threadIdx.x + s];
+        if (t < s) {
+            s_hi[t] = fmaxf(s_hi[t], s_hi[t + s]);
+            s_lo[t] = fminf(s_lo[t], s_lo[t + s]);
+            s_bad[t] |= s_bad[t + s];
         }
         __syncthreads();
     }
@@ -81,30 +84,30 @@ __global__ void __launch_bounds__(512) mex_prep_offsets(MexGeo g, int Mp, const 
         __syncthreads();
         const float base = (hi == CUDART_INF_F || hi == -CUDART_INF_F) ? 0.f : hi;      // as a stable log-sum-exp treats infinite maxima
         float sum = 0.f;
-        if (real) for (int k = threadIdx.x; k < g.K; k += nt) sum += expf(o[k] - base);
-        s_hi[threadIdx.x] = sum;
+        if (real) for (int k = t; k < g.K; k += nt) sum += expf(o[k] - base);
+        s_hi[t] = sum;
         __syncthreads();
         for (int s = nt / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) s_hi[threadIdx.x] += s_hi[threadIdx.x + s];
+            if (t < s) s_hi[t] += s_hi[t + s];
             __syncthreads();
         }
         lse = base + logf(s_hi[0]);
         if (real) {
-            for (int k = threadIdx.x; k < g.K; k += nt) offn[(size_t)rm * g.K + k] = o[k] - lse;
-            if (threadIdx.x == 0) lse_out[rm] = lse;
+            for (int k = t; k < g.K; k += nt) offn[(size_t)rm * g.K + k] = o[k] - lse;
+            if (t == 0) lse_out[rm] = lse;
         }
     }
-    if (real && threadIdx.x == 0) {
+    if (real && t == 0) {
         mo[rm] = ref - lse;
         if (bad || !(fabsf(eps) * (hi - lo) <= kSafeSpread)) atomicOr(flag, 1);
     }
     // taps up to the padding of the tiles: chunks of 16 for the forward tiles, whole tap tiles for the input-gradient tiles
     const int kchunks = (g.K + 15) / 16, mchunks = (g.M + 15) / 16;
     const int mtiles = tf ? (g.M + ntf - 1) / ntf : 0, ktiles = td ? (g.K + ntd - 1) / ntd : 0;
-    int kend = g.K;
-    if (tf && m < mtiles * ntf) kend = max(kend, kchunks * 16);
-    if (td && m < mchunks * 16) kend = max(kend, ktiles * ntd);
-    for (int k = threadIdx.x; k < kend; k += nt) {
+    int kend = exists ? g.K : 0;
+    if (tf && exists && m < mtiles * ntf) kend = max(kend, kchunks * 16);
+    if (td && exists && m < mchunks * 16) kend = max(kend, ktiles * ntd);
+    for (int k = t; k < kend; k += nt) {
         const float e = (real && k < g.K) ? fast_exp(eps * (o[k] - ref)) : 0.f;
         if (real && k < g.K) {
             eo[(size_t)rm * pad4(g.K) + k] = e;
@@ -122,6 +125,63 @@ __global__ void __launch_bounds__(512) mex_prep_offsets(MexGeo g, int Mp, const 
             tile[q] = eh; tile[ntd * 16 + q] = el;
         }
     }
+}
+
+__global__ void __launch_bounds__(512) mex_prep_offsets(MexGeo g, const float* __restrict__ off, PrepArgs a) {
+    stream_order();
+    __shared__ float s_hi[512], s_lo[512];
+    __shared__ int s_bad[512];
+    prep_row(g, blockIdx.x, threadIdx.x, blockDim.x, s_hi, s_lo, s_bad, off, a);
+}
+
+// Everything a layer's main kernel needs, in one launch (small layers are bound by their launches): CTAs [0, prep_ctas) two rows
+// of offsets each; the next max_ctas the per-pixel extrema of 1x1 blocks inside the input, four consecutive pixels per thread,
+// `slices` threads sharing the channels of a pixel where pixels are few; the rest zeros for the sum pooling that the main kernel
+// adds up (134 MB: a memset of its own takes 46 us).
+__global__ void __launch_bounds__(256) mex_prepare(MexGeo g, const float* __restrict__ off, PrepArgs a, int prep_ctas, const float* __restrict__ x, float* __restrict__ mx,
+                                                   int max_ctas, int slices, float4* __restrict__ zero, long long n_zero) {
+    stream_order();
+    __shared__ __align__(16) float red[1024];
+    __shared__ int bad[256];
+    const int b = blockIdx.x;
+    if (b < prep_ctas) {
+        const int half = threadIdx.x >> 7;
+        prep_row(g, b * 2 + half, threadIdx.x & 127, 128, red + half * 128, red + 256 + half * 128, bad + half * 128, off, a);
+        return;
+    }
+    if (b < prep_ctas + max_ctas) {
+        const bool up = g.eps > 0;
+        const int lanes = 256 / slices, lane = threadIdx.x % lanes, slice = threadIdx.x / lanes;
+        const int hw4 = (g.H * g.W) >> 2;
+        const long long total = (long long)g.B * g.Co * hw4, i = (long long)(b - prep_ctas) * lanes + lane;
+        const float none = up ? -CUDART_INF_F : CUDART_INF_F;
+        float4 v = make_float4(none, none, none, none);
+        if (i < total) {
+            const long long nc = i / hw4;
+            const int q = int(i - nc * hw4), n = int(nc / g.Co), c = int(nc - (long long)n * g.Co);
+            const float4* p = reinterpret_cast<const float4*>(x) + ((long long)n * g.C + c * g.sc) * hw4 + q;
+#pragma unroll 8
+            for (int k = slice; k < g.K; k += slices) {
+                const float4 t = __ldg(p + (long long)k * hw4);
+                if (up) { v.x = fmaxf(v.x, t.x); v.y = fmaxf(v.y, t.y); v.z = fmaxf(v.z, t.z); v.w = fmaxf(v.w, t.w); }
+                else { v.x = fminf(v.x, t.x); v.y = fminf(v.y, t.y); v.z = fminf(v.z, t.z); v.w = fminf(v.w, t.w); }
+            }
+        }
+        float4* r4 = reinterpret_cast<float4*>(red);
+        r4[threadIdx.x] = v;
+        __syncthreads();
+        if (slice == 0 && i < total) {
+            for (int s = 1; s < slices; ++s) {
+                const float4 t = r4[s * lanes + lane];
+                if (up) { v.x = fmaxf(v.x, t.x); v.y = fmaxf(v.y, t.y); v.z = fmaxf(v.z, t.z); v.w = fmaxf(v.w, t.w); }
+                else { v.x = fminf(v.x, t.x); v.y = fminf(v.y, t.y); v.z = fminf(v.z, t.z); v.w = fminf(v.w, t.w); }
+            }
+            reinterpret_cast<float4*>(mx)[i] = v;
+        }
+        return;
+    }
+    const long long step = (long long)(gridDim.x - prep_ctas - max_ctas) * 256;
+    for (long long i = (long long)(b - prep_ctas - max_ctas) * 256 + threadIdx.x; i < n_zero; i += step) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // mx[n][pos] = max (eps > 0) or min (eps < 0) over the K taps of the patch at pos; NaN taps are ignored,
@@ -600,7 +660,7 @@ inline bool mex_norm(uint32_t flags) { return (flags & SIMNETS_FLAG_MEX_NORMALIZ
 // The tail of every offsets-gradient path: the split partial sums become doff, and the exact kernel behind acts only when a
 // status word is set.  With raw offsets the exact kernel goes first, into `part`, and one launch reduces and normalises.
 cudaError_t finish_doff(const MexGeo& g, const MexWs& w, int splits, const float* x, const float* off, const float* y, const float* dy,
-                        float* doff, bool accumulate, uint32_t flags, cudaStream_t s) {
+                        float* doff, bool accumulate, uint32_t flags, cudaStream_t s, float* redo_dx = nullptr) {
     const long long n = (long long)g.R * g.M * g.K;
     const auto reduce_splits = [&](float* out, int add, int keep_exact) {
         const int slices = splits >= 64 ? 32 : (splits >= 8 ? 8 : 1), lanes = 512 / slices;
@@ -608,7 +668,8 @@ cudaError_t finish_doff(const MexGeo& g, const MexWs& w, int splits, const float
             n, g.K, splits, slices, w.part, w.eo, out, add, keep_exact, w.flag);
     };
     if (mex_norm(flags)) {
-        cudaError_t e = launch_mex_doff_direct(g, false, x, w.offn, y, dy, w.part, false, s, w.flag);
+        cudaError_t e = redo_dx ? launch_mex_redo_bwd(g, x, w.offn, y, dy, redo_dx, w.part, false, s, w.flag)
+                                : launch_mex_doff_direct(g, false, x, w.offn, y, dy, w.part, false, s, w.flag);
         if (e != cudaSuccess) return e;
         const int rows = g.R * g.M;
         const bool few_rows = rows < device_sm_count() && splits >= 32;         // (one CTA per row would leave most of the GPU idle)
@@ -628,7 +689,8 @@ cudaError_t finish_doff(const MexGeo& g, const MexWs& w, int splits, const float
     count_launch();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return launch_mex_doff_direct(g, false, x, off, y, dy, doff, accumulate, s, w.flag);
+    return redo_dx ? launch_mex_redo_bwd(g, x, off, y, dy, redo_dx, doff, accumulate, s, w.flag)
+                   : launch_mex_doff_direct(g, false, x, off, y, dy, doff, accumulate, s, w.flag);
 }
 
 // Pair tiles: sibling regions alternate along the width and every tensor allows 8-byte accesses of pixel pairs.
@@ -655,19 +717,37 @@ bool use_short_bwd(const MexGeo& g, uint32_t flags, const void* a, const void* b
     return use_tc_kernels(g, flags) && !(flags & SIMNETS_FLAG_MEX_TC_ONE_TILE) && mex_short_shape(g) && !use_pair_kernels(g, flags, a, b, c, d);
 }
 
+// zero: when given, n_zero floats to be cleared as well
 cudaError_t run_prepasses(const MexGeo& g, const MexWs& w, const float* x, const float* off, cudaStream_t s, bool need_mx = true,
-                          bool pair_tiles = false, bool normalize = false) {
+                          bool pair_tiles = false, bool normalize = false, float* zero = nullptr, size_t n_zero = 0) {
     cudaError_t e = cudaMemsetAsync(w.flag, 0, 16, s);
     if (e != cudaSuccess) return e;
+    PrepArgs a = {g.M, 0, 0, w.mo, w.eo, w.eot, nullptr, nullptr, normalize ? w.offn : nullptr, w.lse, w.flag};
     if (pair_tiles) {
         // the pair-tile kernels' operand tiles (forward and input gradient) come out of the same launch
-        const int ntf = mex_pair_nt_fwd(g), ntd = mex_pair_nt_dx(g);
-        const int Mp = std::max(((g.M + ntf - 1) / ntf) * ntf, ((g.M + 15) / 16) * 16);
-        in_stream_order(mex_prep_offsets, g.R * Mp, g.K >= 2048 ? 512 : 128, 0, s)(g, Mp, off, w.mo, w.eo, w.eot, w.flag, w.tc_tiles, ntf, w.tc_tiles_dx, ntd,
-                                                                      normalize ? w.offn : nullptr, w.lse);
+        a.ntf = mex_pair_nt_fwd(g); a.ntd = mex_pair_nt_dx(g);
+        a.Mp = std::max(((g.M + a.ntf - 1) / a.ntf) * a.ntf, ((g.M + 15) / 16) * 16);
+        a.tf = w.tc_tiles; a.td = w.tc_tiles_dx;
+    }
+    const bool zero_here = g.K < 2048 && zero != nullptr && n_zero % 4 == 0 && (reinterpret_cast<uintptr_t>(zero) & 15) == 0;
+    if (zero != nullptr && !zero_here) {
+        e = cudaMemsetAsync(zero, 0, sizeof(float) * n_zero, s);
+        if (e != cudaSuccess) return e;
+    }
+    if (g.K >= 2048) {
+        in_stream_order(mex_prep_offsets, g.R * a.Mp, 512, 0, s)(g, off, a);
     } else {
-        in_stream_order(mex_prep_offsets, g.R * g.M, g.K >= 2048 ? 512 : 128, 0, s)(g, g.M, off, w.mo, w.eo, w.eot, w.flag, nullptr, 0, nullptr, 0,
-                                                                       normalize ? w.offn : nullptr, w.lse);
+        const int prep = (g.R * a.Mp + 1) / 2;
+        const bool pixels = need_mx && g.bh == 1 && g.bw == 1 && g.sh == 1 && g.sw == 1 && patches_inside_input(g) && g.H * g.W % 4 == 0 &&
+                            (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+        int slices = 1;
+        long long quads = pixels ? (long long)g.B * g.Co * (g.H * g.W / 4) : 0;
+        while (pixels && slices < 32 && quads * slices < device_sm_count() * 1024LL && g.K >= 16 * slices) slices *= 2;
+        const long long max_ctas = (quads * slices + 255) / 256, n4 = zero_here ? (long long)(n_zero / 4) : 0;
+        const long long zero_ctas = std::min<long long>((n4 + 2047) / 2048, 8LL * device_sm_count());
+        if (prep + max_ctas + zero_ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+        in_stream_order(mex_prepare, unsigned(prep + max_ctas + zero_ctas), 256, 0, s)(g, off, a, prep, x, w.mx, int(max_ctas), slices, reinterpret_cast<float4*>(zero), n4);
+        if (pixels) need_mx = false;
     }
     if (!need_mx) { count_launch(); return cudaGetLastError(); }
     // long patches over few positions are contiguous per position: reduce them with one CTA each
@@ -751,20 +831,21 @@ static cudaError_t mex_fwd_tiled_body(const MexGeo& g, const float* x, const flo
         if (e != cudaSuccess) return e;
         return launch_mex_fwd_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, s, w.flag);
     }
+    // the pair-tile kernel adds up the 2x2 sum pooling of its output, onto zeros
+    const bool pair = use_tc_kernels(g, flags) && use_pair_kernels(g, flags, x, y, y, y);
+    const bool fuse = pair && pooled != nullptr && (reinterpret_cast<uintptr_t>(pooled) & 3u) == 0;
     // (the caller may have had the layer in front leave the per-position extrema in the workspace: SIMNETS_FLAG_MEX_MAXIMA_GIVEN)
-    cudaError_t e = run_prepasses(g, w, x, off, s, !(flags & SIMNETS_FLAG_MEX_MAXIMA_GIVEN), pair_prep(g, flags), mex_norm(flags));
+    cudaError_t e = run_prepasses(g, w, x, off, s, !(flags & SIMNETS_FLAG_MEX_MAXIMA_GIVEN), pair_prep(g, flags), mex_norm(flags), fuse ? pooled : nullptr,
+                                  (size_t)g.B * g.M * (g.N >> 2));
     if (e != cudaSuccess) return e;
     if (use_tc_kernels(g, flags)) {
-        if (use_pair_kernels(g, flags, x, y, y, y)) {
-            const bool fuse = pooled != nullptr && (reinterpret_cast<uintptr_t>(pooled) & 3u) == 0;
+        if (pair) {
             e = launch_mex_fwd_pair(g, x, w.tc_tiles, w.mo, w.mx, y, fuse ? pooled : nullptr, w.flag,
                                     (flags & SIMNETS_FLAG_MEX_TEST_EXPIRE_WAIT) != 0, s);
             if (e != cudaSuccess) return e;
-            e = launch_mex_fwd_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, s, w.flag);
-            if (e != cudaSuccess || !fuse) return e;
+            if (!fuse) return launch_mex_fwd_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, s, w.flag);
             *pooled_done = true;
-            // if the exact kernel had to recompute y (a status word is set), the pooling is redone from y as well
-            return launch_sum_pool2((long long)g.B * g.M * g.Co, g.Ho, g.Wo, y, pooled, s, w.flag);
+            return launch_mex_redo_fwd_pool(g, x, mex_norm(flags) ? w.offn : off, y, pooled, s, w.flag);
         }
         e = launch_mex_tc_prep(g, false, w.eo, w.tc_tiles, s);
         if (e != cudaSuccess) return e;
@@ -831,7 +912,7 @@ int launch_mex_fwd_static(const MexGeo& g, const float* x, const float* off, flo
 }
 
 cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx,
-                                void* ws, uint32_t flags, cudaStream_t s, bool prepped) {
+                                void* ws, uint32_t flags, cudaStream_t s, bool prepped, bool redo) {
     const MexWs w = carve(g, ws);
     if (!blocks_disjoint(g))             // several positions add to one input value: gathered from their products, in a workspace part of its own
         return launch_mex_bwd_gemm(g, false, x, off, y, dy, dx, nullptr, false, w.overlap,
@@ -846,19 +927,19 @@ cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* of
     if (use_smallk_kernels(g, flags)) {
         e = launch_mex_dx_smallk(g, x, w.eo, w.mo, y, dy, dx, w.flag, s);
         if (e != cudaSuccess) return e;
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
     }
     // (the input gradient alone: the one-tile kernel pads the taps to 16 or 32 columns of its tile but fills the GPU as well with
     // many positions: 200 instances over 8x2x2 blocks at 0.4 GB of y 320 us there, 395 here; 64 over 2x2x2 176 there, 93 here)
     if (use_short_bwd(g, flags, x, y, dy, dx) && (g.K <= 12 || (long long)g.B * g.rs * g.R <= 512LL * device_sm_count())) {
         e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, dx, nullptr, w.flag, s);
         if (e != cudaSuccess) return e;
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
     }
     if (use_tc_kernels(g, flags) && use_pair_kernels(g, flags, x, y, dy, dx)) {
         e = launch_mex_dx_pair(g, x, w.tc_tiles_dx, w.mo, w.mx, y, dy, dx, w.flag, s);
         if (e != cudaSuccess) return e;
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
     }
     if (use_tc_kernels(g, flags)) {
         e = launch_mex_tc_prep(g, true, w.eot, w.tc_tiles, s);
@@ -868,7 +949,7 @@ cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* of
         e = ((flags & SIMNETS_FLAG_MEX_TC_ONE_TILE) || g.K <= 128) ? launch_mex_dx_tc(g, x, w.tc_tiles, w.mo, w.mx, y, dy, dx, w.flag, s)
                                                                    : launch_mex_dx_ws(g, x, w.tc_tiles, w.mo, w.mx, y, dy, dx, w.flag, s);
         if (e != cudaSuccess) return e;
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
     }
     if (small && smallm_shape(g) && mex_head_shape(g)) {
         if (!(prepped || forward_primes_workspace(g, flags))) {              // run_prepasses skipped the maxima for this family
@@ -877,12 +958,12 @@ cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* of
         }
         e = launch_mex_bwd_head(g, true, false, x, w.eo, w.mo, w.mx, y, dy, dx, nullptr, 1, w.flag, s);
         if (e != cudaSuccess) return e;
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
     }
     if (small) {
         e = launch_mex_dx_smallm(g, x, w.eo, w.mo, y, dy, dx, w.flag, s);
         if (e != cudaSuccess) return e;
-        return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+        return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
     }
     const long long P = (long long)g.B * g.rs;
     const bool sp1 = g.bh == 1 && g.bw == 1;
@@ -896,42 +977,42 @@ cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* of
     count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
+    return redo ? launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag) : cudaSuccess;
 }
 
 cudaError_t launch_mex_doff_tiled(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* doff,
-                                  bool accumulate, void* ws, uint32_t flags, cudaStream_t s, bool prepped) {
+                                  bool accumulate, void* ws, uint32_t flags, cudaStream_t s, bool prepped, float* redo_dx) {
     const MexWs w = carve(g, ws);
     cudaError_t e = (prepped || forward_primes_workspace(g, flags)) ? cudaSuccess : run_prepasses(g, w, x, off, s, !use_smallk_kernels(g, flags), pair_prep(g, flags), mex_norm(flags));
     if (e != cudaSuccess) return e;
     if (use_short_bwd(g, flags, x, y, dy, dy)) {
         e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, nullptr, w.part, w.flag, s);
         if (e != cudaSuccess) return e;
-        return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s, redo_dx);
     }
     if (use_tc_kernels(g, flags)) {
         int tsplits = mex_tc_doff_splits(g);
         e = use_pair_kernels(g, flags, x, y, dy, dy) ? launch_mex_doff_pair(g, x, w.mo, w.mx, y, dy, w.part, &tsplits, w.flag, s)
                                                      : launch_mex_doff_tc(g, x, w.mo, w.mx, y, dy, w.part, tsplits, w.flag, s);
         if (e != cudaSuccess) return e;
-        return finish_doff(g, w, tsplits, x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, tsplits, x, off, y, dy, doff, accumulate, flags, s, redo_dx);
     }
     const int splits = doff_splits(g);
     if (use_smallk_kernels(g, flags)) {
         e = launch_mex_doff_smallk(g, x, w.mo, y, dy, w.part, splits, w.flag, s);
         if (e != cudaSuccess) return e;
-        return finish_doff(g, w, splits, x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, splits, x, off, y, dy, doff, accumulate, flags, s, redo_dx);
     }
     if (smallm_shape(g) && mex_head_shape(g)) {
         const int hs = mex_head_splits(g);
         e = launch_mex_bwd_head(g, false, true, x, w.eo, w.mo, w.mx, y, dy, nullptr, w.part, hs, w.flag, s);
         if (e != cudaSuccess) return e;
-        return finish_doff(g, w, hs, x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, hs, x, off, y, dy, doff, accumulate, flags, s, redo_dx);
     }
     if (smallm_shape(g)) {
         e = launch_mex_doff_smallm(g, x, w.mo, w.mx, y, dy, w.part, splits, w.flag, s);
         if (e != cudaSuccess) return e;
-        return finish_doff(g, w, splits, x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, splits, x, off, y, dy, doff, accumulate, flags, s, redo_dx);
     }
     const int tile = doff_big(g) ? 128 : 64;
     const long long blocks = (long long)((g.M + tile - 1) / tile) * ((g.K + tile - 1) / tile) * g.R * splits;
@@ -943,7 +1024,7 @@ cudaError_t launch_mex_doff_tiled(const MexGeo& g, const float* x, const float* 
     count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return finish_doff(g, w, splits, x, off, y, dy, doff, accumulate, flags, s);
+    return finish_doff(g, w, splits, x, off, y, dy, doff, accumulate, flags, s, redo_dx);
 }
 
 // Both gradients of one layer in one call: the offsets prepass and the per-position maxima are computed once.
@@ -961,9 +1042,7 @@ cudaError_t launch_mex_backward_tiled(const MexGeo& g, const float* x, const flo
         }
         e = launch_mex_bwd_head(g, true, true, x, w.eo, w.mo, w.mx, y, dy, dx, w.part, hs, w.flag, s);
         if (e != cudaSuccess) return e;
-        e = launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
-        if (e != cudaSuccess) return e;
-        return finish_doff(g, w, hs, x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, hs, x, off, y, dy, doff, accumulate, flags, s, dx);
     }
     if (use_short_bwd(g, flags, x, y, dy, dx)) {
         if (!blocks_cover_input(g)) {
@@ -972,13 +1051,12 @@ cudaError_t launch_mex_backward_tiled(const MexGeo& g, const float* x, const flo
         }
         e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, dx, w.part, w.flag, s);
         if (e != cudaSuccess) return e;
-        e = launch_mex_dx_direct(g, false, x, mex_norm(flags) ? w.offn : off, y, dy, dx, s, w.flag);
-        if (e != cudaSuccess) return e;
-        return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s);
+        return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s, dx);
     }
-    e = launch_mex_dx_tiled(g, x, off, y, dy, dx, ws, flags, s, true);
+    const bool joint = blocks_disjoint(g);               // (overlapping blocks: the input gradient has its own redo)
+    e = launch_mex_dx_tiled(g, x, off, y, dy, dx, ws, flags, s, true, !joint);
     if (e != cudaSuccess) return e;
-    return launch_mex_doff_tiled(g, x, off, y, dy, doff, accumulate, ws, flags, s, true);
+    return launch_mex_doff_tiled(g, x, off, y, dy, doff, accumulate, ws, flags, s, true, joint ? dx : nullptr);
 }
 
 }  // namespace simnets
