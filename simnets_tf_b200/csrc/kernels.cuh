@@ -138,6 +138,7 @@ cudaError_t launch_mex_doff_pair(const MexGeo&, const float* x, const float* mo,
 // mex_short.cu -- both gradients of short patches from one read of y and dy; dx or part may be null
 bool mex_short_shape(const MexGeo&);
 int mex_short_splits(const MexGeo&);
+bool mex_short_doff(const MexGeo&);
 cudaError_t launch_mex_bwd_short(const MexGeo&, bool inside, const float* x, const float* eo, const float* mo, const float* mx, const float* y,
                                  const float* dy, float* dx, float* part, const int* flag, cudaStream_t);
 // mex_gemm.cu -- the factorised passes as small contractions: float64, small float32 layers, input gradients of overlapping blocks

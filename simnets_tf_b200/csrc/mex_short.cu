@@ -98,14 +98,16 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
     }
     __syncthreads();
 
-    const long long P = (long long)g.B * g.rs, tiles = (P + kShPos - 1) / kShPos;
+    // this CTA's share of the region's positions: whole runs of 32
+    const long long runs = ((long long)g.B * g.rs + 31) / 32;
+    const long long p_begin = runs * blockIdx.x / gridDim.x * 32, P = min((long long)g.B * g.rs, runs * (blockIdx.x + 1) / gridDim.x * 32);
     const float eps = float(g.eps), oob = float(g.oob), a2 = eps * 1.4426950408889634f, c2 = float(g.cst) * 1.4426950408889634f;
     constexpr int ROWS = VEC ? 16 : 4, PER = kShM / ROWS, W = VEC ? 4 : 1;      // staging: W positions, instances row0, row0 + ROWS, ...
     const int pos = VEC ? (tid & 15) * 4 : tid & (kShPos - 1), row0 = VEC ? tid >> 4 : tid >> 6;
     const int e_pos = tid & (kShPos - 1), e_row = tid >> 6;                     // Ex: one position, taps e_row, e_row + 4, ...
     float ry[PER][W], rg[PER][W], rmx[W], rx[KT / 4];
     Column col, e_col;
-    long long tile = blockIdx.x;
+    long long tile = p_begin;
     auto fetch = [&](int mc) {
         const bool live = col.base >= 0;
         const float* py = y + (live ? col.base : 0) + (long long)(mc * kShM + row0) * g.N;
@@ -125,10 +127,10 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
         }
     };
     auto open_tile = [&](long long t) {                                         // positions, their maxima and their patches
-        col = column_of(g, r, t * kShPos + pos, P, mx);
+        col = column_of(g, r, t + pos, P, mx);
         rmx[0] = col.mx;
         if (VEC) {
-            e_col = column_of(g, r, t * kShPos + e_pos, P, mx);
+            e_col = column_of(g, r, t + e_pos, P, mx);
             if (col.base >= 0) {
                 const float4 m4 = *reinterpret_cast<const float4*>(mx + col.base - (long long)col.n * (g.M - 1) * g.N);
                 rmx[0] = m4.x; rmx[W > 1 ? 1 : 0] = m4.y; rmx[W > 2 ? 2 : 0] = m4.z; rmx[W > 3 ? 3 : 0] = m4.w;
@@ -153,10 +155,10 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
     constexpr int MT = DX && DOFF ? NT : (NT + 1) / 2;                          // column tiles per warp
     const int nt0 = DX && DOFF ? 0 : (warp >> 2) * MT;
     const bool idle = nt0 >= NT;
-    if (tile < tiles) open_tile(tile);
+    if (tile < P) open_tile(tile);
     int qb = 0;
     float acc[MT][4];                                                           // input gradient: 16 positions x 8 taps
-    for (; tile < tiles; tile += gridDim.x) {
+    for (; tile < P; tile += kShPos) {
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
             }
             // request the next values before this step's products
             if (mc + 1 < MC) fetch(mc + 1);
-            else if (tile + gridDim.x < tiles) open_tile(tile + gridDim.x);
+            else if (tile + kShPos < P) open_tile(tile + kShPos);
             __syncthreads();
             if (idle) continue;
             if (does_dx) {
@@ -261,13 +263,20 @@ bool mex_short_shape(const MexGeo& g) {
     return g.K <= 32 && g.M >= 32 && g.sc >= g.bc && g.sh >= g.bh && g.sw >= g.bw && g.bh <= 256 && g.bw <= 256 && g.R <= 65535 &&
            (long long)g.C * g.H * g.W < (1LL << 31) && sh_smem_bytes(g.M, sh_taps(g)) <= 220 * 1024;
 }
-// CTAs per region: all that are resident at once, in equal shares of the position tiles
+// Positions that the one-tile kernels of mex_tc.cu sum in one accumulator.  The tensor cores truncate what they add, so a long
+// sum depends on where it is cut (18.9 K positions: 1.4e-4 of the offsets gradient's norm from the exact sum, growing with the
+// length): from 1500 positions on (1e-5) this kernel cuts where that one does, below it takes shares that fill the GPU.
+static bool sh_long_sums(const MexGeo& g) { return (long long)g.B * g.rs / mex_tc_doff_splits(g) > 1500; }
 int mex_short_splits(const MexGeo& g) {
-    const long long tiles = ((long long)g.B * g.rs + kShPos - 1) / kShPos;
+    if (sh_long_sums(g)) return mex_tc_doff_splits(g);
+    const long long runs = ((long long)g.B * g.rs + 31) / 32, tiles = (runs + 1) / 2;
     const long long ctas = std::max<long long>(1, (long long)device_sm_count() * sh_ctas_per_sm(g) / g.R);
     const long long each = (tiles + ctas - 1) / ctas;
     return int(std::max<long long>(1, (tiles + each - 1) / each));
 }
+// Whether the offsets gradient of this layer is worth it: with one CTA per SM the shares of long sums leave SMs idle (200
+// instances over 8x2x2 blocks, 0.5 M positions: both gradients 827 us, 755 in two kernels).
+bool mex_short_doff(const MexGeo& g) { return !sh_long_sums(g) || sh_ctas_per_sm(g) == 2; }
 
 cudaError_t launch_mex_bwd_short(const MexGeo& g, bool inside, const float* x, const float* eo, const float* mo, const float* mx, const float* y,
                                  const float* dy, float* dx, float* part, const int* flag, cudaStream_t s) {

@@ -985,7 +985,7 @@ cudaError_t launch_mex_doff_tiled(const MexGeo& g, const float* x, const float* 
     const MexWs w = carve(g, ws);
     cudaError_t e = (prepped || forward_primes_workspace(g, flags)) ? cudaSuccess : run_prepasses(g, w, x, off, s, !use_smallk_kernels(g, flags), pair_prep(g, flags), mex_norm(flags));
     if (e != cudaSuccess) return e;
-    if (use_short_bwd(g, flags, x, y, dy, dy)) {
+    if (mex_short_doff(g) && use_short_bwd(g, flags, x, y, dy, dy)) {
         e = launch_mex_bwd_short(g, patches_inside_input(g), x, w.eo, w.mo, w.mx, y, dy, nullptr, w.part, w.flag, s);
         if (e != cudaSuccess) return e;
         return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s, redo_dx);
@@ -1044,7 +1044,7 @@ cudaError_t launch_mex_backward_tiled(const MexGeo& g, const float* x, const flo
         if (e != cudaSuccess) return e;
         return finish_doff(g, w, hs, x, off, y, dy, doff, accumulate, flags, s, dx);
     }
-    if (use_short_bwd(g, flags, x, y, dy, dx)) {
+    if (mex_short_doff(g) && use_short_bwd(g, flags, x, y, dy, dx)) {
         if (!blocks_cover_input(g)) {
             e = cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)g.B * g.C * g.H * g.W, s);
             if (e != cudaSuccess) return e;
