@@ -1,0 +1,42 @@
+"""Both gradients of short patches under many instances from one read of y and dy: edges of the 64 x 64 tiles and of the 8, 16 and
+32 tap widths, vector and scalar staging, blocks that leave the input, gaps, and sums long enough for the fixed split."""
+import importlib
+
+import pytest
+import torch
+
+import cases
+import gpu_util
+from simnets_tf_b200 import abi
+
+mex_ops = importlib.import_module("simnets_tf_b200.ops.mex")
+pytestmark = pytest.mark.gpu
+
+SHARED = dict(unshared=False, shared_region=(-1,))
+EDGES = [
+    cases.mex_case("taps_8_rows_64", (2, 4, 16, 16), 64, (2, 2, 2), (2, 2, 2), softmax=True, eps=0.5, seed=601, **SHARED),
+    cases.mex_case("taps_9_rows_65", (3, 2, 12, 12), 65, (1, 3, 3), (1, 3, 3), softmax=True, seed=602, normalize=True, **SHARED),
+    cases.mex_case("taps_16_rows_128", (2, 8, 10, 10), 128, (4, 2, 2), (4, 2, 2), eps=-0.7, seed=603, **SHARED),
+    cases.mex_case("taps_17_odd", (3, 17, 5, 7), 50, (17, 1, 1), (17, 1, 1), softmax=True, seed=604, normalize=True, **SHARED),
+    cases.mex_case("taps_32_rows_63", (1, 8, 8, 8), 63, (8, 2, 2), (8, 2, 2), softmax=True, eps=1.5, seed=605, **SHARED),
+    cases.mex_case("regions", (2, 6, 12, 10), 70, (3, 2, 2), (3, 2, 2), softmax=True, unshared_region=(3,), seed=606, normalize=True),
+    cases.mex_case("outside", (2, 6, 9, 11), 48, (2, 3, 2), (3, 3, 3), (1, 1, 1), oob=0.4, softmax=True, seed=607, **SHARED),
+]
+
+
+@pytest.mark.parametrize("c", EDGES, ids=lambda c: c["name"])
+def test_tile_edges(port, c):
+    gpu_util.check_mex(port, c, flags=abi.FLAG_MEX_NO_SMALL_TILES, f64_tiebreak=True)
+
+
+def test_long_sums_agree_with_the_one_tile_kernels():
+    """Beyond 1500 positions per accumulator the split is the one-tile kernel's, and so are the sums."""
+    x = torch.randn(48, 2, 256, 256, device="cuda")
+    attrs = dict(blocks=[1, 2, 4], strides=[1, 2, 4], epsilon=0.5, softmax_mode=True, use_unshared_regions=False, shared_offset_region=[-1])
+    off = torch.randn(1, 64, 1, 2, 4, device="cuda")
+    y = mex_ops.mex_forward(x, off, 64, **attrs)
+    dy = torch.randn_like(y)
+    dx, doff = mex_ops.mex_backward(x, off, y, dy, 64, **attrs)
+    one_dx, one_doff = mex_ops.mex_backward(x, off, y, dy, 64, flags=abi.FLAG_MEX_TC_ONE_TILE, **attrs)
+    assert float((doff - one_doff).norm()) <= 1e-5 * float(one_doff.norm())
+    assert float((dx - one_dx).norm()) <= 1e-5 * float(one_dx.norm())

@@ -1,0 +1,39 @@
+"""The float32 Similarity kernels where they can go wrong: tap, template and channel counts around the tile sizes, strides whose
+phases have different taps and pixels, pixels that no patch covers, inputs small and large enough for every dispatch."""
+import pytest
+
+import cases
+import gpu_util
+
+pytestmark = pytest.mark.gpu
+
+NAN = cases.NAN
+MODES = [dict(fn="L2"), dict(fn="L2", norm=True), dict(fn="L2", norm=True, ignore_nan=True, nan_frac=0.2), dict(fn="L1")]
+# (batch, channels, h, w), templates, blocks, strides, padding
+SHAPES = [
+    ((1, 1, 5, 6), 1, (1, 1), (1, 1), (0, 0)),              # one tap
+    ((2, 5, 7, 9), 33, (1, 1), (1, 1), (0, 0)),             # five taps, up to eight channels
+    ((2, 3, 11, 10), 65, (3, 3), (1, 1), (1, 1)),           # 27 taps
+    ((1, 8, 9, 8), 31, (2, 2), (1, 1), (1, 1)),             # 32 taps, 8 channels
+    ((2, 9, 10, 7), 64, (2, 2), (2, 2), (1, 1)),            # 36 taps, 9 channels, four phases
+    ((1, 16, 8, 9), 32, (2, 2), (1, 2), (0, 1)),            # 64 taps
+    ((2, 13, 9, 11), 40, (5, 1), (2, 1), (2, 0)),           # 65 taps, uneven phases
+    ((1, 17, 12, 9), 20, (3, 2), (4, 3), (0, 0)),           # gaps: pixels that no patch covers
+    ((2, 33, 6, 7), 50, (2, 2), (1, 1), (1, 1)),            # 132 taps, 33 channels
+    ((1, 66, 5, 6), 129, (1, 2), (1, 1), (0, 1)),           # 66 channels, 129 templates
+    ((1, 130, 4, 5), 12, (1, 1), (1, 1), (0, 0)),           # 130 channels
+]
+
+
+@pytest.mark.parametrize("mode", MODES, ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("i", range(len(SHAPES)))
+def test_tile_edges(port, i, mode):
+    shape, M, blocks, strides, padding = SHAPES[i]
+    gpu_util.check_similarity(port, cases.sim_case("edges%d" % i, shape, M, blocks=blocks, strides=strides, padding=padding, oob=0.3, seed=700 + i, **mode),
+                              f64_tiebreak=True)
+
+
+@pytest.mark.parametrize("mode", MODES, ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("shape,M,blocks", [((160, 1, 28, 28), 40, (2, 2)), ((96, 3, 30, 33), 10, (3, 3))], ids=["resident_32", "many_pixels"])
+def test_enough_positions_for_the_streaming_kernels(port, shape, M, blocks, mode):
+    gpu_util.check_similarity(port, cases.sim_case("many", shape, M, blocks=blocks, strides=(1, 1), padding=(1, 1), seed=720, **mode), f64_tiebreak=True, tol=2e-5)
