@@ -16,6 +16,7 @@
 // CTA's partial sums are written once and added in a fixed order by the reduction.
 #include <climits>
 #include "mex_common.cuh"
+#include "mma.cuh"
 
 namespace simnets {
 namespace {
@@ -35,15 +36,6 @@ __host__ __device__ inline int sh_smem_bytes(int M, int kt) {
 // (8 rows x 4 positions, 4 rows x 8 positions) hit 32 different banks.
 __device__ __forceinline__ int sh_swizzle(int m) { return ((m & 3) << 3) | (m & 4); }
 
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// v = hi + lo exactly, hi with the bits a TF32 operand keeps
-__device__ __forceinline__ float2 split_tf32(float v) {
-    const float hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-    return make_float2(hi, v - hi);
-}
 __device__ __forceinline__ float sh_exp2(float v) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v)); return r; }
 
 // A fragment of four Q values and NT fragments of a split operand: d[nt] += Q * operand, hi lo products first
@@ -106,7 +98,7 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
     const int pos = VEC ? (tid & 15) * 4 : tid & (kShPos - 1), row0 = VEC ? tid >> 4 : tid >> 6;
     const int e_pos = tid & (kShPos - 1), e_row = tid >> 6;                     // Ex: one position, taps e_row, e_row + 4, ...
     float ry[PER][W], rg[PER][W], rmx[W], rx[KT / 4];
-    Column col, e_col;
+    Column col = {}, e_col = {};
     long long tile = p_begin;
     auto fetch = [&](int mc) {
         const bool live = col.base >= 0;
@@ -128,7 +120,8 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
     };
     auto open_tile = [&](long long t) {                                         // positions, their maxima and their patches
         col = column_of(g, r, t + pos, P, mx);
-        rmx[0] = col.mx;
+#pragma unroll
+        for (int u = 0; u < W; ++u) rmx[u] = col.mx;                            // (a dead quad: zeros, so that 0 * 2^... stays 0)
         if (VEC) {
             e_col = column_of(g, r, t + e_pos, P, mx);
             if (col.base >= 0) {

@@ -14,6 +14,7 @@
 // threads cover the tile several times over and the copies split the positions of a chunk among themselves (K = 4: sixteen
 // ways).  Partial sums of the splits are added in split order.
 #include "kernels.cuh"
+#include "mma.cuh"
 #include "tile.cuh"
 
 namespace simnets {
@@ -57,6 +58,11 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
     stream_order();
     constexpr bool MASKED = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
+    // With missing data sN is a contraction that does not involve the templates, dy times a mask of ones and zeros: on tiles of
+    // 64 taps the tensor cores take it (dy split in two TF32 parts, the mask exact, one chunk per accumulator), which leaves the
+    // FP32 pipe four operations per term instead of five.
+    constexpr bool TENSOR_N = MODE == SIM_L2N_NAN && MAXK == 64;
+    constexpr bool SUM_N = MASKED && !L1 && !TENSOR_N;
     constexpr int LD = KC + 4, TI = TM / 4;                                           // row stride, floats
     constexpr int A_PER = TM * KC / kDpThreads, B_PER = MAXK * KC / kDpThreads, ROWS = kDpThreads / KC;
     constexpr int A_FLOATS = TM * LD, B_FLOATS = MAXK * LD, STAGE = A_FLOATS + (MASKED ? 2 : 1) * B_FLOATS;
@@ -82,7 +88,9 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
     const int G = TI * tile.k2, group = threadIdx.x / G, lid = threadIdx.x - group * G;
     const bool worker = group < tile.groups;
     const int ti = lid & (TI - 1), tj = lid / TI;                        // rows ti + TI r, columns tj + k2 c
-    float2 tt[4][2], sT[4][2], sW[4][2], sN[4][MASKED ? 2 : 1];
+    float2 tt[4][2], sT[4][2], sW[4][2], sN[4][SUM_N ? 2 : 1];
+    float tN[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};       // 16 templates x 2 x 8 taps per warp
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3, n_row = (warp & 1) * 16, n_col = (warp >> 1) * 16;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -90,7 +98,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
             const int m = m0 + ti + TI * r, k = k0 + tj + tile.k2 * c;
             tt[r][c] = splat2((worker && m < g.M && k < g.K) ? -tm[(size_t)m * g.K + k] : 0.f);
             sT[r][c] = sW[r][c] = make_float2(0.f, 0.f);
-            sN[r][MASKED ? c : 0] = make_float2(0.f, 0.f);
+            sN[r][SUM_N ? c : 0] = make_float2(0.f, 0.f);
         }
 
     // staging: this thread brings position q of every chunk, rows e, e + ROWS, ...
@@ -184,12 +192,37 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
                             const float2 u = mul2(a2, d);
                             sT[r][c] = add2(sT[r][c], u);
                             sW[r][c] = fma2(u, d, sW[r][c]);
-                            if (MASKED) sN[r][MASKED ? c : 0] = fma2(a2, k2, sN[r][MASKED ? c : 0]);
+                            if (SUM_N) sN[r][SUM_N ? c : 0] = fma2(a2, k2, sN[r][SUM_N ? c : 0]);
                         }
                     }
                 }
             }
         }
+    };
+
+    auto compute_n = [&](const float* stage) {
+        const float* A = stage + (n_row + gq) * LD + tq;
+        const float* K = stage + A_FLOATS + B_FLOATS + (n_col + gq) * LD + tq;
+        float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int p = 0; p < KC; p += 8) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float2 v = split_tf32(A[(u & 1) * 8 * LD + p + (u >> 1) * 4]);
+                hi[u] = __float_as_uint(v.x); lo[u] = __float_as_uint(v.y);
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const uint32_t b0 = __float_as_uint(K[c * 8 * LD + p]), b1 = __float_as_uint(K[c * 8 * LD + p + 4]);
+                mma_tf32(s[c], lo, b0, b1);
+                mma_tf32(s[c], hi, b0, b1);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) tN[c][u] += s[c][u];
     };
 
     __syncthreads();                                                     // the tap table
@@ -203,6 +236,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
             float* next = smem + ((i + 1) & 1) * STAGE;
             const bool more = i + 1 < n_chunks;
             if (more) fetch(c_begin + i + 1);
+            if (TENSOR_N) compute_n(now);
             if (worker) compute(now);
             if (more) commit(next);
             __syncthreads();
@@ -220,11 +254,11 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     float v[3] = {sT[r][c].x + sT[r][c].y, sW[r][c].x + sW[r][c].y, 0.f};
-                    if (MASKED && !L1) v[2] = sN[r][MASKED ? c : 0].x + sN[r][MASKED ? c : 0].y;
+                    if (SUM_N) v[2] = sN[r][SUM_N ? c : 0].x + sN[r][SUM_N ? c : 0].y;
                     else if (!L1) v[2] = sN[r][0].x + sN[r][0].y;
                     const int row = ti + TI * r, col = tj + tile.k2 * c, m = m0 + row, k = k0 + col;
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) {
+                    for (int p = 0; p < (TENSOR_N ? 2 : 3); ++p) {
                         float* s = smem + (p * TM + row) * TK + col;
                         if (grp > 0) v[p] += *s;
                         if (grp < last) *s = v[p];
@@ -234,6 +268,14 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
         }
         if (grp < last) __syncthreads();
     }
+    if (TENSOR_N)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int m = m0 + n_row + gq + 8 * (u >> 1), col = n_col + 8 * c + 2 * tq + (u & 1), k = k0 + col;
+                if (m < g.M && col < TK && k < g.K) dst[2 * mk + (size_t)m * g.K + k] = tN[c][u];
+            }
 }
 
 // Sums the splits' partial sums in split order and applies the per-parameter factors of the backward functors.  512 threads =
