@@ -166,10 +166,8 @@ template <int MODE> struct ResidentPlanes {
     static constexpr int NA = MODE == SIM_L2N_NAN ? 3 : 2, NB = (MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP) ? 2 : 1;
 };
 constexpr int kResMaxK = 32, kResTN = 128;
-// (every parameter is stored twice: the packed instructions take it in both halves of a register pair, and duplicating it after
-// the load cost two moves per six packed instructions)
 template <int MODE, int TM>
-__host__ __device__ constexpr int resident_smem_floats(int K) { return (ResidentPlanes<MODE>::NA * TM * 2 + 2 * ResidentPlanes<MODE>::NB * kResTN) * K; }
+__host__ __device__ constexpr int resident_smem_floats(int K) { return (ResidentPlanes<MODE>::NA * TM + 2 * ResidentPlanes<MODE>::NB * kResTN) * K; }
 
 template <int MODE, int TM>
 __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(SimGeo g, const float* __restrict__ x, const float* __restrict__ tm,
@@ -187,14 +185,13 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     __shared__ __align__(16) float red[2][TI][kResTN];             // the extrema of each thread row, two tiles' worth
     const int K = g.K, i0 = blockIdx.y * TM;
     float* As = sm;
-    float2* As2 = reinterpret_cast<float2*>(As);
-    float* Bs = sm + NA * TM * 2 * K;
+    float* Bs = sm + NA * TM * K;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) flag[threadIdx.x] = 0;          // the workspace's status words
     for (int i = threadIdx.x; i < K * TM; i += T) {
         const int k = i / TM, m = i % TM;
         const SkParams p = sk_params<MODE>(g, tm, wt, i0 + m, k);
-        As2[i] = splat2(p.t); As2[K * TM + i] = splat2(p.scale);
-        if (NA == 3) As2[2 * K * TM + i] = splat2(p.constant);
+        As[i] = p.t; As[K * TM + i] = p.scale;
+        if (NA == 3) As[2 * K * TM + i] = p.constant;
     }
     if (threadIdx.x < TM) row_const[threadIdx.x] = MODE == SIM_L2N ? sk_row_constant(g, wt, i0 + threadIdx.x) : 0.f;
     for (int k = threadIdx.x; k < kResMaxK; k += T) tp[k] = sk_tap(g, k);
@@ -259,14 +256,15 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[r][c] = make_float2(0.f, 0.f);
         const float* B = Bs + buf * NB * K * kResTN + t.tj * 4;
-        const float* A = As + t.ti * 8;
+        const float* A = As + t.ti * 4;
 #pragma unroll 3
         for (int q = 0; q < K; ++q) {
-            float2 a[NA][4], b[NB][4];
+            float a[NA][4];
+            float2 b[NB][4];
 #pragma unroll
             for (int p = 0; p < NA; ++p) {
-                const float4 v = *reinterpret_cast<const float4*>(A + (p * K + q) * TM * 2), w = *reinterpret_cast<const float4*>(A + (p * K + q) * TM * 2 + 4);
-                a[p][0] = make_float2(v.x, v.y); a[p][1] = make_float2(v.z, v.w); a[p][2] = make_float2(w.x, w.y); a[p][3] = make_float2(w.z, w.w);
+                const float4 v = *reinterpret_cast<const float4*>(A + (p * K + q) * TM);
+                a[p][0] = v.x; a[p][1] = v.y; a[p][2] = v.z; a[p][3] = v.w;
             }
 #pragma unroll
             for (int p = 0; p < NB; ++p)
@@ -279,8 +277,8 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
             for (int r = 0; r < 4; ++r)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const float2 d = add2(a[0][r], neg2(b[0][c])), s2 = a[1][r];
-                    if (MODE == SIM_L2N_NAN) acc[r][c] = fma2(b[NB - 1][c], fma2(mul2(s2, d), d, a[NA - 1][r]), acc[r][c]);
+                    const float2 d = add2(splat2(a[0][r]), neg2(b[0][c])), s2 = splat2(a[1][r]);
+                    if (MODE == SIM_L2N_NAN) acc[r][c] = fma2(b[NB - 1][c], fma2(mul2(s2, d), d, splat2(a[NA - 1][r])), acc[r][c]);
                     else if (MODE == SIM_L1_SKIP) acc[r][c] = fma2(s2, mul2(sk_abs2(d), b[NB - 1][c]), acc[r][c]);
                     else if (L1) acc[r][c] = fma2(s2, sk_abs2(d), acc[r][c]);
                     else acc[r][c] = fma2(mul2(s2, d), d, acc[r][c]);
