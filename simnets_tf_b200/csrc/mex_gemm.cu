@@ -125,9 +125,14 @@ __device__ __forceinline__ T row_reduce(T v, T* red, bool warp) {
     return v;
 }
 
-struct GemmCol { long long base, gbase; int n, c0, h0, w0; };
+// xb: offset of the patch corner in x; inside: the whole patch lies in the input
+struct GemmCol { long long base, gbase, xb; int n, c0, h0, w0; bool inside; };
+__device__ __forceinline__ void place_patch(const MexGeo& g, GemmCol& c) {
+    c.xb = (((long long)c.n * g.C + c.c0) * g.H + c.h0) * g.W + c.w0;
+    c.inside = c.c0 >= 0 && c.c0 + g.bc <= g.C && c.h0 >= 0 && c.h0 + g.bh <= g.H && c.w0 >= 0 && c.w0 + g.bw <= g.W;
+}
 __device__ __forceinline__ GemmCol gemm_col(const MexGeo& g, int r, long long jl, long long P) {
-    GemmCol c = {-1, 0, 0, 0, 0, 0};
+    GemmCol c = {-1, 0, 0, 0, 0, 0, 0, false};
     if (jl >= P) return c;
     const int n = int(fast_div(uint32_t(jl), g.f_rs)), l = int(jl) - n * g.rs;        // (P < 2^31)
     int cc, h, w;
@@ -136,11 +141,31 @@ __device__ __forceinline__ GemmCol gemm_col(const MexGeo& g, int r, long long jl
     c.n = n; c.c0 = cc * g.sc - g.pc; c.h0 = h * g.sh - g.ph; c.w0 = w * g.sw - g.pw;
     c.base = (long long)n * g.M * g.N + pos;
     c.gbase = mex_dy_base(g, n, pos);
+    place_patch(g, c);
     return c;
+}
+// Decoded taps of a block in shared memory: {offset from the patch corner, (c << 16) | (h << 8) | w}.  Decoding a tap costs two
+// divisions and two modulos, which had been most of the instructions around a gathered value (blocks of 12 x 3 x 3).
+constexpr int kGemmTaps = 1024;
+__device__ __forceinline__ bool taps_tabled(const MexGeo& g) { return g.K <= kGemmTaps && g.bh <= 256 && g.bw <= 256; }
+__device__ __forceinline__ void table_taps(const MexGeo& g, int2* __restrict__ tab) {
+    if (taps_tabled(g))
+        for (int k = threadIdx.x; k < g.K; k += kGemmThreads) {
+            const int w = k % g.bw, q = k / g.bw, h = q % g.bh, c = q / g.bh;
+            tab[k] = make_int2((c * g.H + h) * g.W + w, (c << 16) | (h << 8) | w);
+        }
 }
 // index of the position's maximum
 __device__ __forceinline__ long long col_mx(const MexGeo& g, const GemmCol& c) { return c.base - (long long)c.n * (g.M - 1) * g.N; }
-__device__ __forceinline__ long long tap_address(const MexGeo& g, const GemmCol& c, int k) {       // offset of tap k in x, or -1 outside
+// offset of tap k in x, or -1 outside the input; tab: the table, or null
+__device__ __forceinline__ long long tap_address(const MexGeo& g, const GemmCol& c, int k, const int2* __restrict__ tab) {
+    if (g.bh * g.bw == 1 && c.inside) return c.xb + (long long)k * (g.H * g.W);
+    if (tab) {
+        const int2 t = tab[k];
+        if (c.inside) return c.xb + t.x;
+        const int cc = c.c0 + (t.y >> 16), hh = c.h0 + ((t.y >> 8) & 255), ww = c.w0 + (t.y & 255);
+        return uint32_t(cc) < uint32_t(g.C) && uint32_t(hh) < uint32_t(g.H) && uint32_t(ww) < uint32_t(g.W) ? c.xb + t.x : -1;
+    }
     int kc = k, kh = 0, kw = 0;
     if (g.bh * g.bw > 1) { kw = k % g.bw; const int q = k / g.bw; kh = q % g.bh; kc = q / g.bh; }
     const int cc = c.c0 + kc, hh = c.h0 + kh, ww = c.w0 + kw;
@@ -157,6 +182,7 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm_prep(MexGeo g, const T*
                                                               int prep_ctas, int normalize, int lanes) {
     stream_order();
     __shared__ T red[kGemmThreads];
+    __shared__ int2 tap_tab[kGemmTaps];
     const T eps = T(g.eps);
     if (int(blockIdx.x) < prep_ctas) {
         const bool warp = prep_rows(g.K) > 1;
@@ -203,22 +229,25 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm_prep(MexGeo g, const T*
     const long long total = (long long)g.B * g.N, idx = (long long)(blockIdx.x - prep_ctas) * lanes + lane;
     const bool up = g.eps > 0;
     const T oob = T(g.oob);
+    const bool pixel = g.bh * g.bw == 1;
+    const int2* tab = !pixel && taps_tabled(g) ? tap_tab : nullptr;
+    if (!pixel) { table_taps(g, tap_tab); __syncthreads(); }
     T v = -pos_inf<T>();                                      // maximum of x or of -x
     if (idx < total) {
         const int pos = int(idx % g.N);
         GemmCol c;
         c.n = int(idx / g.N);
         c.w0 = pos % g.Wo * g.sw - g.pw; c.h0 = pos / g.Wo % g.Ho * g.sh - g.ph; c.c0 = pos / (g.Wo * g.Ho) * g.sc - g.pc;
-        const bool inside = c.c0 >= 0 && c.c0 + g.bc <= g.C && c.h0 >= 0 && c.h0 + g.bh <= g.H && c.w0 >= 0 && c.w0 + g.bw <= g.W;
-        if (inside && g.bh * g.bw == 1) {
-            const T* p = x + tap_address(g, c, 0);
+        place_patch(g, c);
+        if (c.inside && pixel) {
+            const T* p = x + c.xb;
             const size_t hw = (size_t)g.H * g.W;
 #pragma unroll 8
             for (int k = slice; k < g.K; k += slices) { const T t = p[k * hw]; v = t_max(v, up ? t : -t); }
         } else {
 #pragma unroll 4
             for (int k = slice; k < g.K; k += slices) {
-                const long long a = tap_address(g, c, k);
+                const long long a = tap_address(g, c, k, tab);
                 const T t = a >= 0 ? x[a] : oob;
                 v = t_max(v, up ? t : -t);
             }
@@ -251,8 +280,13 @@ __device__ __noinline__ void exact_dx(const MexGeo& g, const T* x, const T* off,
 
 // The three contractions.  Rows i: instances (forward, offsets gradient) or taps (input gradient); columns j: positions of one
 // region (taps for the offsets gradient); reduction q: taps, instances, positions.
+// CTAs per SM that the registers are cut for (24 instances over 12 x 3 x 3 taps, 39 K positions: input gradient 82 us at four, 91
+// at three; offsets gradient 52 at three, 56 at four; forward 60 uncut, 63 at three or four)
 template <typename T, int OP, int TM>
-__global__ void __launch_bounds__(kGemmThreads) mex_gemm(const __grid_constant__ MexGeo g, GemmPlan sp, const T* __restrict__ x, const T* __restrict__ off,
+__host__ __device__ constexpr int gemm_ctas() { return sizeof(T) == 8 || TM == 64 ? 2 : (OP == kDx ? 4 : (OP == kDoff ? 3 : 1)); }
+
+template <typename T, int OP, int TM>
+__global__ void __launch_bounds__(kGemmThreads, gemm_ctas<T, OP, TM>()) mex_gemm(const __grid_constant__ MexGeo g, GemmPlan sp, const T* __restrict__ x, const T* __restrict__ off,
                                                          const T* __restrict__ eo, const T* __restrict__ mo, const T* __restrict__ mx, const T* __restrict__ y,
                                                          const T* __restrict__ dy, T* __restrict__ out, T* __restrict__ part, const int* __restrict__ verdict,
                                                          int verdicts, int to_part, int* __restrict__ flag) {
@@ -261,6 +295,9 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm(const __grid_constant__
     constexpr int NA = TM * kQ / kGemmThreads, NB = kTN * kQ / kGemmThreads;
     constexpr int RM = TM / 16, LDA = TM + 16 / int(sizeof(T)), LDB = kTN + 16 / int(sizeof(T));
     __shared__ __align__(16) T As[2][kQ][LDA], Bs[2][kQ][LDB];
+    __shared__ int2 tap_tab[OP == kDx ? 1 : kGemmTaps];
+    const int2* tab = OP != kDx && g.bh * g.bw > 1 && taps_tabled(g) ? tap_tab : nullptr;
+    if (tab) table_taps(g, tap_tab);                    // (published by the barrier of the next call)
     const bool unsafe = gemm_unsafe(verdict, verdicts);
     if (OP == kFwd && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) flag[threadIdx.x] = threadIdx.x == 0 && unsafe;
     if (unsafe) {
@@ -280,7 +317,7 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm(const __grid_constant__
     // staging, along whichever axis is contiguous in memory: element fastest or reduction step fastest
     const int ea_f = threadIdx.x % TM, qa_f = threadIdx.x / TM, eb_f = threadIdx.x % kTN, qb_f = threadIdx.x / kTN;
     const int q_s = threadIdx.x % kQ, e_s = threadIdx.x / kQ;
-    GemmCol jc = {-1, 0, 0, 0, 0, 0};
+    GemmCol jc = {-1, 0, 0, 0, 0, 0, 0, false};
     T jmx = T(0);
     if (OP != kDoff) { jc = gemm_col(g, r, j0 + eb_f, P); if (jc.base >= 0) jmx = mx[col_mx(g, jc)]; }
     T ra[NA], rb[NB];
@@ -290,7 +327,7 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm(const __grid_constant__
     };
     auto ex = [&](const GemmCol& c, T cmx, int k) {                   // Ex[k, position]
         if (c.base < 0 || k >= g.K) return T(0);
-        const long long a = tap_address(g, c, k);
+        const long long a = tap_address(g, c, k, tab);
         return Numeric<T>::exp_(eps * ((a >= 0 ? x[a] : oob) - cmx));
     };
     auto fetch = [&](int chunk) {
@@ -338,7 +375,10 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm(const __grid_constant__
             T a[RM], b[4];
             const typename Vec4<T>::type bv = *reinterpret_cast<const typename Vec4<T>::type*>(&Bs[buf][q][tj * 4]);
             b[0] = bv.x; b[1] = bv.y; b[2] = bv.z; b[3] = bv.w;
-            if (RM == 4) {
+            if (RM == 2 && sizeof(T) == 4) {
+                const float2 av = *reinterpret_cast<const float2*>(&As[buf][q][ti * 2]);
+                a[0] = av.x; a[RM > 1 ? 1 : 0] = av.y;
+            } else if (RM == 4) {
                 const typename Vec4<T>::type av = *reinterpret_cast<const typename Vec4<T>::type*>(&As[buf][q][ti * 4]);
                 a[0] = av.x; a[RM > 1 ? 1 : 0] = av.y; a[RM > 2 ? 2 : 0] = av.z; a[RM > 3 ? 3 : 0] = av.w;
             } else {
@@ -376,7 +416,7 @@ __global__ void __launch_bounds__(kGemmThreads) mex_gemm(const __grid_constant__
             if (i >= rows) continue;
             if (OP == kFwd) out[c.base + (long long)i * g.N] = cmx + mor[i] + (Numeric<T>::log_(acc[u][v]) + cst) / eps;
             else {
-                const long long a = tap_address(g, c, i);
+                const long long a = tap_address(g, c, i, nullptr);
                 if (a >= 0) out[a] = Numeric<T>::exp_(eps * (x[a] - cmx)) * acc[u][v];
             }
         }
