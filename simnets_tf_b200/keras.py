@@ -6,6 +6,7 @@ variables on first call (the counterpart of Keras' `build(input_shape)`) and run
 `perform_unsupervised_init` (k-means / GMM initialisation of Similarity layers) lives in `unsupervised.py`, built on the
 Similarity operators; the reference's PCA branch serves Keras convolution layers, which do not exist here.
 """
+import copy
 import ctypes as C
 import math
 
@@ -16,7 +17,7 @@ from . import _lib, abi
 from . import _torch_glue
 from .ops.mex import _attrs as _mex_attrs, _expand_dim_specification, _mex_dims_helper
 from .ops.mex import mex_plan as _mex_plan, mex_with_plan as _mex_with_plan
-from .ops.similarity import similarity_of_raw_weights as _similarity_of_raw_weights, _attrs as _similarity_attrs, similarity_plan as _similarity_plan
+from .ops.similarity import _attrs as _similarity_attrs, similarity_plan as _similarity_plan
 
 
 def _sinks(*params):
@@ -46,8 +47,39 @@ def _init_tensor(spec, shape, device, dtype, generator=None):
     raise ValueError("unknown initializer %r" % (spec,))
 
 
-class Similarity(torch.nn.Module):
+class _PlannedLayer(torch.nn.Module):
+    """Base of the layers: the native plans of the input shapes seen last, with the attribute values they were made for (an
+    attribute may be changed between calls, in place too)."""
+
+    _plan_attributes = ()
+
+    def __init__(self):
+        super(_PlannedLayer, self).__init__()
+        self._plans = {}
+
+    def __getstate__(self):                 # plans are native objects: copies and pickles of a layer start without
+        return dict(self.__dict__, _plans={})
+
+    def _planned(self, key, make):
+        now = [getattr(self, n) for n in self._plan_attributes]
+        hit = self._plans.get(key)
+        try:
+            if hit is not None and hit[0] == now:
+                return hit[1]
+        except ValueError:                  # (arrays do not compare to one truth value)
+            return make()
+        plan = make()
+        if len(self._plans) >= 64:
+            self._plans.clear()
+        self._plans[key] = (copy.deepcopy(now), plan)
+        return plan
+
+
+class Similarity(_PlannedLayer):
     """Similarity layer; `weights` enter the op as their absolute value, as in the reference's `call`."""
+
+    _plan_attributes = ('similarity_function', 'strides', 'blocks', 'padding', 'normalization_term', 'normalization_term_fudge',
+                        'ignore_nan_input', 'out_of_bounds_value')
 
     def __init__(self, num_instances=None, similarity_function='L2', strides=[1, 1], blocks=[3, 3], padding='SAME',
                  normalization_term=False, normalization_term_fudge=0.001, ignore_nan_input=False,
@@ -105,7 +137,11 @@ class Similarity(torch.nn.Module):
         """Shape of `forward(x)` for a channels-first tensor (the layer is built on first use, as in `forward`)."""
         if self.templates is None:
             self.build(tuple(x.shape), x.device, x.dtype)
-        return _similarity_plan(x, self.templates, self.sweights, _similarity_attrs(**self._op_attrs())).out_shape
+        return self._plan(x, self.templates, self.sweights).out_shape
+
+    def _plan(self, x, templates, weights):
+        return self._planned((x.shape, x.dtype, templates.shape, weights.shape, _torch_glue.DEFAULT_FLAGS),
+                             lambda: _similarity_plan(x, templates, weights, _similarity_attrs(**self._op_attrs())))
 
     def forward(self, x, extrema=None):
         """extrema=(max_address, min_address): also write the per-pixel maximum / minimum of the output over the
@@ -115,8 +151,10 @@ class Similarity(torch.nn.Module):
         if self.channels_last:
             x = x.permute(0, 3, 1, 2)
         # |weights| and its gradient are taken inside the op's kernels
-        y = _similarity_of_raw_weights(x, self.templates, self.sweights, extrema=extrema, grad_sinks=_sinks(self.templates, self.sweights),
-                                       **self._op_attrs())
+        templates, weights = self.templates, self.sweights
+        up, down = extrema if extrema is not None else (None, None)
+        dt, dw = _sinks(templates, weights) or (None, None)
+        y = _lib.ops().sim_apply(self._plan(x, templates, weights), x, templates, weights, abi.FLAG_SIM_ABS_WEIGHTS, up or 0, down or 0, dt, dw)
         return y.permute(0, 2, 3, 1) if self.channels_last else y
 
     def get_config(self):
@@ -177,8 +215,11 @@ class _NormalizeOffsets(torch.autograd.Function):
         return doff
 
 
-class Mex(torch.nn.Module):
+class Mex(_PlannedLayer):
     """MEX layer; `normalize_offsets` subtracts a per-(region, instance) logsumexp from the offsets variable."""
+
+    _plan_attributes = ('num_instances', 'padding', 'strides', 'blocks', 'epsilon', 'use_unshared_regions', 'shared_offset_region',
+                        'unshared_offset_region', 'softmax_mode', 'blocks_out_of_bounds_value', 'blocks_round_down')
 
     def __init__(self, num_instances=None, padding=[0, 0, 0], strides=[1, 1, 1], blocks=[1, 1, 1],
                  epsilon=1.0, use_unshared_regions=True, shared_offset_region=[-1],
@@ -257,8 +298,9 @@ class Mex(torch.nn.Module):
     def _op_flags(self, dtype, device):
         # on the GPU the op takes the raw offsets and normalises them in its own prepass (and its gradient comes back
         # with respect to the raw values); otherwise effective_offsets() does it in front of the op
-        fused = self.normalize_offsets and device.type == "cuda" and self.offsets is not None and self.offsets.dtype == dtype and \
-            self.offsets.is_cuda and (dtype == torch.float32 or (dtype == torch.float64 and math.isfinite(self.epsilon)))
+        off = self.offsets
+        fused = self.normalize_offsets and device.type == "cuda" and off is not None and off.dtype == dtype and off.is_cuda and \
+            (dtype == torch.float32 or (dtype == torch.float64 and math.isfinite(self.epsilon)))
         if _torch_glue.DEFAULT_FLAGS & (abi.FLAG_FORCE_DIRECT | abi.FLAG_MEX_EXACT):
             fused = False           # those routes run without a workspace, which the fused normalisation needs
         return abi.FLAG_MEX_NORMALIZED_OFFSETS if fused else 0
@@ -283,7 +325,8 @@ class Mex(torch.nn.Module):
         return (ws, ptr, float(self.epsilon) > 0) if ptr else None
 
     def _plan(self, shape, dtype):
-        return _mex_plan(shape, dtype, self.num_instances, _mex_attrs(**self._op_attrs()))
+        return self._planned((shape, dtype, _torch_glue.DEFAULT_FLAGS),
+                             lambda: _mex_plan(shape, dtype, self.num_instances, _mex_attrs(**self._op_attrs())))
 
     def forward(self, x, sum_pool2=False, layer_ws=None, maxima_given=False):
         """sum_pool2=True returns the 2x2 sum pooling of the layer's output (pooling gradient fused into the
@@ -295,8 +338,9 @@ class Mex(torch.nn.Module):
         op_flags = self._op_flags(x.dtype, x.device) if x.shape[0] > 0 else 0
         _torch_glue.dtype_code(x)                   # (rejects anything but float32 / float64)
         # (the raw offsets are the op's own input, and a gradient bucket its target, only when the op normalises them)
-        sink = _sinks(self.offsets) if op_flags else None
-        y = _mex_with_plan(self._plan(x.shape, x.dtype), x, self.offsets if op_flags else self.effective_offsets(), layer_ws,
+        off = self.offsets
+        sink = _sinks(off) if op_flags else None
+        y = _mex_with_plan(self._plan(x.shape, x.dtype), x, off if op_flags else self.effective_offsets(), layer_ws,
                            abi.FLAG_MEX_MAXIMA_GIVEN if maxima_given else 0, op_flags, sum_pool2, sink[0] if sink else None)
         return y.permute(0, 2, 3, 1) if self.channels_last else y
 
