@@ -159,6 +159,25 @@ __device__ __forceinline__ void pair_teardown(PairShared<STAGES>& sh, uint32_t t
     if (threadIdx.x == 0 && sh.failed) atomicExch(&flag[1], 1);
 }
 
+// ---- box copies of a tile's raw operands ---------------------------------------------------------------------------
+// The 128 pixel pairs of a tile are a run of one image row, whole rows of the pair's row class, or whole samples: ONE box of
+// the tensor seen as (w, row class, row within the class, sample, instance or channel), 16 of the last per stage, so that it
+// lands as [16][128 pairs] in tile order.  One thread asks for it.  Per-thread 8-byte copies took 64 (forward) or 128 (input
+// gradient, y and dy) warp-wide instructions per stage, and an SM issues about one in 25 cycles: 1600 cycles and more for a
+// stage whose MMAs take 768.  Plain per-CTA copies from this GPU's own tensors.  Samples past the batch and instances or
+// taps past the end lie outside the map and arrive as zeros.
+struct PairBox { int cols, rows, samples; };                     // pixel pairs along a row, rows, samples of a tile
+struct DxMaps { CUtensorMap y, dy; };
+
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3, int c4) {
+    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+
 // Stage of the forward and input-gradient kernels: [tile 0: A hi, A lo][tile 1: A hi, A lo][tile 0: B hi, B lo][tile 1: B hi, B lo]
 constexpr int kPairA = kTcPos * kTcKT * 4;                     // one plane of the position operand
 template <int NT> __host__ __device__ constexpr int pair_b_bytes() { return NT * kTcKT * 4; }
@@ -256,6 +275,44 @@ __device__ __forceinline__ void pair_mma_role(PairShared<STAGES>& sh, unsigned c
     if (!mbar_wait(&sh.drain, 0)) sh.failed = 1;
 }
 
+// Box loader role (one thread): per stage one box of `map0` (x, or y) and, for the input gradient, one of `map1` (dy, given
+// pooled or not) and the offset maxima of the stage's instances in both regions.
+template <int DEPTH, int SLOT_BYTES, int G_OFF, int MO_OFF, bool POOLED, typename Shared>
+__device__ __forceinline__ void pair_box_role(const MexGeo& g, Shared& sh, uint64_t* raw_full, uint64_t* raw_empty, unsigned char* rawbase,
+                                              const CUtensorMap* map0, const CUtensorMap* map1, const float* __restrict__ mo,
+                                              const WsPlan& plan, int my_items, int chunks, uint32_t tries) {
+    WsRing<DEPTH> slot = {0, 0u};
+    int issued = 0;
+    for (int li = 0; li < my_items && !sh.failed; ++li) {
+        const WsItem it = ws_item(plan, int(blockIdx.x) + li * int(gridDim.x));
+        const uint32_t j0 = uint32_t(it.jt) * kTcPos;                 // (fewer than 2^31 positions: pair_box_of)
+        const int n = int(fast_div(j0, g.f_rs)), l = int(j0) - n * g.rs;
+        const int lh = l / g.rw, lw = l - lh * g.rw, rh = it.r % g.oh;
+        for (int c = 0; c < chunks; ++c) {
+            if (slot.fill >= 1 && !pair_wait(sh.failed, &raw_empty[slot.stage], (slot.fill - 1) & 1u, tries)) { sh.failed = 1; break; }
+            uint64_t* bar = &raw_full[slot.stage];
+            unsigned char* dst = rawbase + slot.stage * SLOT_BYTES;
+            const int mb = MO_OFF ? min(kTcKT, g.M - c * kTcKT) * 4 : 0;
+            bulk_expect(bar, uint32_t((MO_OFF ? MO_OFF : SLOT_BYTES) + 2 * mb));
+            tma_load_5d(smem_u32(dst), map0, bar, 2 * lw, rh, lh, n, c * kTcKT);
+            if (MO_OFF) {
+                if (POOLED) tma_load_4d(smem_u32(dst + G_OFF), map1, bar, lw, lh, n, c * kTcKT);
+                else tma_load_5d(smem_u32(dst + G_OFF), map1, bar, 2 * lw, rh, lh, n, c * kTcKT);
+                bulk_copy_raw(dst + MO_OFF, mo + (2 * it.r) * g.M + c * kTcKT, uint32_t(mb), bar);
+                bulk_copy_raw(dst + MO_OFF + kTcKT * 4, mo + (2 * it.r + 1) * g.M + c * kTcKT, uint32_t(mb), bar);
+            }
+            slot.advance(1);
+            if (issued < DEPTH) ++issued;
+        }
+    }
+    // copies still in flight must land before the CTA may exit: walk back over the last `issued` slots
+    for (int d = 0; d < issued; ++d) {
+        if (slot.stage == 0) { slot.stage = DEPTH; --slot.fill; }
+        --slot.stage;
+        if (!mbar_wait(&raw_full[slot.stage], slot.fill & 1u)) sh.failed = 1;
+    }
+}
+
 // TF32 split without a conversion: the hi plane may hold v itself (the tensor core reads the sign, the exponent and the top
 // 10 mantissa bits and ignores the rest); lo = v minus that truncation, exactly.
 __device__ __forceinline__ float tf32_lo(float v) { return v - __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
@@ -281,12 +338,17 @@ struct StepCursor {
 
 // ---- forward ---------------------------------------------------------------------------------------------------
 // item = (region pair, instance tile of NT, tile of 128 pixel pairs); a stage holds 16 taps.
-template <int NT, int DEPTH>
-__global__ void __launch_bounds__(kPairThreads, 1) mex_fwd_pair(MexGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
+// BOX: raw taps come as box copies (see PairBox) through a ring of slots; else by the producers' own asynchronous copies.
+constexpr int kFwdSlots = 5, kFwdSlotBytes = kTcKT * kTcPos * 8;
+template <bool BOX> __host__ __device__ constexpr int fwd_threads() { return kPairThreads + (BOX ? 32 : 0); }
+
+template <int NT, int DEPTH, bool BOX>
+__global__ void __launch_bounds__(fwd_threads<BOX>(), 1) mex_fwd_pair(MexGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
                                                                const float* __restrict__ mo, const float* __restrict__ mx,
                                                                float* __restrict__ y, float* __restrict__ pooled, WsPlan plan,
-                                                               int* __restrict__ flag, int test_expire) {
+                                                               int* __restrict__ flag, int test_expire, const __grid_constant__ CUtensorMap xmap) {
     stream_order();
+    __shared__ uint64_t raw_full[kFwdSlots], raw_empty[kFwdSlots];
     constexpr int STAGES = pair_stages<NT>();
     constexpr int STAGE_BYTES = pair_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 4 * NT;
@@ -300,9 +362,56 @@ __global__ void __launch_bounds__(kPairThreads, 1) mex_fwd_pair(MexGeo g, const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int my_items = plan.items > int(blockIdx.x) ? (plan.items - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
     const uint32_t tries = test_expire ? 256u : kWaitTries;
-    const uint32_t tmem = pair_setup(sh, TMEM_COLS);
+    if (BOX && threadIdx.x == 0)
+        for (int d = 0; d < kFwdSlots; ++d) { mbar_init(&raw_full[d], 1); mbar_init(&raw_empty[d], kPairProducers); }
+    const uint32_t tmem = pair_setup(sh, TMEM_COLS);          // (its fence and barrier publish the two rings above as well)
 
-    if (warp < kPairProducerWarps) {
+    if (BOX && warp < kPairProducerWarps) {
+        // ---------------- producers: thread % 128 = pixel-pair row, thread / 128 = which 8 of the stage's 16 taps
+        const int prow = threadIdx.x % kTcPos, khalf = threadIdx.x / kTcPos;
+        const float a = float(g.eps) * 1.4426950408889634f;
+        auto item_column = [&](int li) {              // (read one item ahead: its maxima come from global memory)
+            const WsItem it = ws_item(plan, int(blockIdx.x) + min(li, my_items - 1) * int(gridDim.x));
+            return pair_column_of(g, it.r, (long long)it.jt * kTcPos + prow, P, mx);
+        };
+        WsRing<STAGES> ring = {0, 0u};
+        WsRing<kFwdSlots> slot = {0, 0u};
+        PairColumn next = item_column(0);
+        for (int li = 0; li < my_items && !sh.failed; ++li) {
+            const PairColumn col = next;
+            next = item_column(li + 1);
+            bool ok = true;
+            for (int c = 0; c < kchunks; ++c) {
+                const int kleft = col.base >= 0 ? g.K - c * kTcKT - khalf * 8 : 0;       // (<= 0: nothing of this thread's eight taps exists)
+                if (!pair_wait(sh.failed, &raw_full[slot.stage], slot.fill & 1u, tries)) { ok = false; break; }
+                const float2* raw = reinterpret_cast<const float2*>(dsm + STAGES * STAGE_BYTES + slot.stage * kFwdSlotBytes) + khalf * 8 * kTcPos + prow;
+                float e0[8], e1[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float2 v = raw[u * kTcPos];
+                    // x - mx first: both may be far from zero while their difference is small
+                    e0[u] = u < kleft ? ex2_ftz(a * (v.x - col.mx0)) : 0.f;
+                    e1[u] = u < kleft ? ex2_ftz(a * (v.y - col.mx1)) : 0.f;
+                }
+                mbar_arrive(&raw_empty[slot.stage]);                          // the slot may be refilled
+                slot.advance(1);
+                const int stage = ring.stage;
+                if (ring.fill >= 1 && !pair_wait(sh.failed, &sh.empty[stage], (ring.fill - 1) & 1u, tries)) { ok = false; break; }
+                unsigned char* sA = dsm + stage * STAGE_BYTES;
+                store_split8(sA, sA + kPairA, prow, khalf * 8, e0);
+                store_split8(sA + 2 * kPairA, sA + 3 * kPairA, prow, khalf * 8, e1);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_arrive(&sh.full[stage]);
+                ring.advance(1);
+            }
+            if (!ok) { sh.failed = 1; break; }
+        }
+    } else if (BOX && warp > kPairLoaderWarp) {
+        if (lane == 0)
+            pair_box_role<kFwdSlots, kFwdSlotBytes, 0, 0, false>(g, sh, raw_full, raw_empty, dsm + STAGES * STAGE_BYTES, &xmap, nullptr, nullptr, plan,
+                                                                 my_items, kchunks, tries);
+        __syncwarp();
+    } else if (warp < kPairProducerWarps) {
         // ---------------- producers: thread % 128 = pixel-pair row, thread / 128 = which 8 of the stage's 16 taps
         const int prow = threadIdx.x % kTcPos, khalf = threadIdx.x / kTcPos;
         const float a = float(g.eps) * 1.4426950408889634f;
@@ -468,12 +577,16 @@ __device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&v)[8])
 
 // WIDE: every tensor is 16-byte aligned and the map width is a multiple of 4, so two neighbouring pixel pairs of a tile are
 // 16 contiguous bytes: a raw loader then copies two rows at a time (half the copy instructions).
-template <int NT, bool POOLED, bool WIDE>
-__global__ void __launch_bounds__(kDxThreads, 1) mex_dx_pair(MexGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
+// LOAD 0: 8-byte copies; 1: those 16-byte copies; 2: box copies (see PairBox), one loader warp.
+template <int LOAD> __host__ __device__ constexpr int dx_threads() { return LOAD == 2 ? (kDxFirstRawWarp + 1) * 32 : kDxThreads; }
+template <int NT, bool POOLED, int LOAD>
+__global__ void __launch_bounds__(dx_threads<LOAD>(), 1) mex_dx_pair(MexGeo g, const float* __restrict__ x, const float* __restrict__ tiles,
                                                             const float* __restrict__ mo, const float* __restrict__ mx,
                                                             const float* __restrict__ y, const float* __restrict__ dy,
-                                                            float* __restrict__ dx, WsPlan plan, int* __restrict__ flag) {
+                                                            float* __restrict__ dx, WsPlan plan, int* __restrict__ flag,
+                                                            const __grid_constant__ DxMaps maps) {
     stream_order();
+    constexpr bool WIDE = LOAD == 1;
     constexpr int STAGES = pair_stages<NT>(), DEPTH = dx_depth<POOLED>(), kDxSlotBytes = dx_slot_bytes<POOLED>();
     constexpr int STAGE_BYTES = pair_stage_bytes<NT>();
     constexpr uint32_t TMEM_COLS = 4 * NT;
@@ -489,7 +602,7 @@ __global__ void __launch_bounds__(kDxThreads, 1) mex_dx_pair(MexGeo g, const flo
     const int total = my_items * mchunks;
     const uint32_t tries = kWaitTries;
     if (threadIdx.x == 0)
-        for (int d = 0; d < DEPTH; ++d) { mbar_init(&raw_full[d], kDxRawWarps * 32); mbar_init(&raw_empty[d], kPairProducers); }
+        for (int d = 0; d < DEPTH; ++d) { mbar_init(&raw_full[d], LOAD == 2 ? 1 : kDxRawWarps * 32); mbar_init(&raw_empty[d], kPairProducers); }
     const uint32_t tmem = pair_setup(sh, TMEM_COLS);          // (its fence and barrier publish the two rings above as well)
     const float a = float(g.eps) * 1.4426950408889634f, c2 = float(g.cst) * 1.4426950408889634f;
     unsigned char* rawbase = dsm + STAGES * STAGE_BYTES;
@@ -500,9 +613,14 @@ __global__ void __launch_bounds__(kDxThreads, 1) mex_dx_pair(MexGeo g, const flo
         const int M = g.M;
         WsRing<STAGES> ring = {0, 0u};
         WsRing<DEPTH> slot = {0, 0u};
+        auto item_column = [&](int li) {              // (read one item ahead: its maxima come from global memory)
+            const WsItem it = ws_item(plan, int(blockIdx.x) + min(li, my_items - 1) * int(gridDim.x));
+            return pair_column_of(g, it.r, (long long)it.jt * kTcPos + prow, P, mx);
+        };
+        PairColumn next = item_column(0);
         for (int li = 0; li < my_items && !sh.failed; ++li) {
-            const WsItem it = ws_item(plan, int(blockIdx.x) + li * int(gridDim.x));
-            const PairColumn col = pair_column_of(g, it.r, (long long)it.jt * kTcPos + prow, P, mx);
+            const PairColumn col = next;
+            next = item_column(li + 1);
             bool ok = true;
             for (int c = 0; c < mchunks; ++c) {
                 const int mleft = col.base >= 0 ? M - c * kTcKT - mhalf * 8 : 0;     // a dead row contributes nothing
@@ -543,6 +661,11 @@ __global__ void __launch_bounds__(kDxThreads, 1) mex_dx_pair(MexGeo g, const flo
         pair_loader_role<NT, STAGES>(sh, dsm, tiles, plan, my_items, ktiles, mchunks, tries);
     } else if (warp == kPairMmaWarp) {
         pair_mma_role<NT, STAGES>(sh, dsm, tmem, my_items, mchunks, tries, -1);
+    } else if (LOAD == 2 && warp >= kDxFirstRawWarp) {
+        if (lane == 0)
+            pair_box_role<DEPTH, kDxSlotBytes, kTcKT * kTcPos * 8, dx_mo_off<POOLED>(), POOLED>(g, sh, raw_full, raw_empty, rawbase, &maps.y, &maps.dy, mo,
+                                                                                              plan, my_items, mchunks, tries);
+        __syncwarp();
     } else if (warp >= kDxFirstRawWarp) {
         // ---------------- raw loaders.  8-byte copies: thread = pixel-pair row, all 16 instances of a stage.  WIDE: thread =
         // (two neighbouring rows, half of the instances), 16-byte copies.
@@ -707,15 +830,6 @@ struct DoPairPlan { int units, mgroups, ktiles, splits; };
 // of one image row, or a few whole rows, of the region pair's rows -- times all instances are ONE box.  Plain per-CTA
 // tiled copies from this GPU's own tensors; each CTA fetches its own boxes, nothing is shared between CTAs.
 struct DoMaps { CUtensorMap y, dy, x, mx; };
-
-__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3, int c4) {
-    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
 
 // LOAD: how the raw loaders fetch a chunk.  0: 8-byte asynchronous copies, one pixel pair per thread; 1: 16-byte copies,
 // two neighbouring pairs per thread; 2: four tensor-map box copies per chunk issued by one thread (see DoMaps).
@@ -1021,6 +1135,59 @@ inline bool mex_pair_wide(const MexGeo& g, const void* a, const void* b, const v
 
 inline int pair_nt(int n) { return n > 64 ? 128 : 64; }
 
+// cuTensorMapEncodeTiled of the driver, looked up once (the library links no driver stub); nullptr if unavailable
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline EncodeTiledFn encode_tiled_fn() {
+    static EncodeTiledFn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) p = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
+    return fn;
+}
+
+// A float32 tensor seen as rank-4 or rank-5 (dims fastest first, strides in floats for dims 1..), one box per copy
+inline bool encode_f32_map(CUtensorMap* map, const float* base, int rank, const long long* dims, const long long* strides, const int* box) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    cuuint64_t gd[5], gs[4];
+    cuuint32_t bd[5], es[5];
+    for (int i = 0; i < rank; ++i) { gd[i] = cuuint64_t(dims[i]); bd[i] = cuuint32_t(box[i]); es[i] = 1; }
+    for (int i = 0; i + 1 < rank; ++i) gs[i] = cuuint64_t(strides[i]) * 4;
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, cuuint32_t(rank), const_cast<float*>(base), gd, gs, bd, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The box of a tile (see PairBox): one channel block and one region along the channels, rows of the region pair a fixed number
+// apart with the height a multiple of it, and tiles that are a run of one row, whole rows or whole samples; every stride a
+// multiple of 16 bytes.
+inline bool pair_box_of(const MexGeo& g, PairBox* b) {
+    if (g.Co != 1 || g.oc != 1 || g.rc != 1 || g.H % g.oh != 0 || g.rh * g.oh != g.H || g.W % 4 != 0) return false;
+    if ((long long)g.B * g.rs + kTcPos > 0x7fffffffLL) return false;
+    if (g.rw % kTcPos == 0) *b = {kTcPos, 1, 1};
+    else if (kTcPos % g.rw == 0 && g.rs % kTcPos == 0) *b = {g.rw, kTcPos / g.rw, 1};
+    else if (kTcPos % g.rs == 0) *b = {g.rw, g.rh, kTcPos / g.rs};
+    else return false;
+    return true;
+}
+// [B][n][H][W] (samples `per_sample` floats apart) in boxes of 16 planes x one tile
+inline bool pair_box_map(const MexGeo& g, const PairBox& b, const float* t, int n, long long per_sample, CUtensorMap* map) {
+    const long long dims[5] = {g.W, g.oh, g.H / g.oh, g.B, n}, strides[4] = {g.W, (long long)g.W * g.oh, per_sample, (long long)g.H * g.W};
+    const int box[5] = {2 * b.cols, 1, b.rows, b.samples, kTcKT};
+    return (reinterpret_cast<uintptr_t>(t) & 15u) == 0 && encode_f32_map(map, t, 5, dims, strides, box);
+}
+inline bool dx_box_maps(const MexGeo& g, const float* mo, const float* y, const float* dy, DxMaps* maps) {
+    PairBox b;
+    if (g.M % 4 != 0 || (reinterpret_cast<uintptr_t>(mo) & 15u) != 0 || !pair_box_of(g, &b) || !pair_box_map(g, b, y, g.M, (long long)g.M * g.N, &maps->y)) return false;      // (M: 16-byte rows of offset maxima)
+    if (g.gp != 2) return pair_box_map(g, b, dy, g.M, (long long)g.M * g.N, &maps->dy);
+    if (g.oh != 2 || g.W % 8 != 0 || (reinterpret_cast<uintptr_t>(dy) & 15u) != 0) return false;
+    const long long dims[4] = {g.W / 2, g.H / 2, g.B, g.M}, strides[3] = {g.W / 2, (long long)g.M * g.Ng, g.Ng};      // one value per pixel pair and row pair
+    const int box[4] = {b.cols, b.rows, b.samples, kTcKT};
+    return encode_f32_map(&maps->dy, dy, 4, dims, strides, box);
+}
+
 template <int NT>
 cudaError_t launch_fwd_pair_nt(const MexGeo& g, const float* x, const float* tiles, const float* mo, const float* mx, float* y, float* pooled,
                                int* flag, int test_expire, cudaStream_t s) {
@@ -1030,8 +1197,14 @@ cudaError_t launch_fwd_pair_nt(const MexGeo& g, const float* x, const float* til
     if (items >= 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const WsPlan plan = {int(items), make_fastdiv(pairs), make_fastdiv(mtiles)};
     const int grid = int(std::min<long long>(items, ws_sm_count()));
-    constexpr int smem = pair_stages<NT>() * pair_stage_bytes<NT>() + pair_raw_bytes<3, 8>();
-    PAIR_RUN((mex_fwd_pair<NT, 3>), kPairThreads, smem, grid, g, x, tiles, mo, mx, y, pooled, plan, flag, test_expire);
+    constexpr int stages = pair_stages<NT>() * pair_stage_bytes<NT>(), smem = stages + pair_raw_bytes<3, 8>(), smem_box = stages + kFwdSlots * kFwdSlotBytes;
+    static_assert(smem <= 227 * 1024 && smem_box <= 227 * 1024, "stages and slot ring must fit the shared memory of one CTA");
+    CUtensorMap xmap;
+    memset(&xmap, 0, sizeof(xmap));
+    PairBox b;
+    if (pair_box_of(g, &b) && pair_box_map(g, b, x, g.K, (long long)g.C * g.H * g.W, &xmap))
+        PAIR_RUN((mex_fwd_pair<NT, 3, true>), fwd_threads<true>(), smem_box, grid, g, x, tiles, mo, mx, y, pooled, plan, flag, test_expire, xmap);
+    else PAIR_RUN((mex_fwd_pair<NT, 3, false>), fwd_threads<false>(), smem, grid, g, x, tiles, mo, mx, y, pooled, plan, flag, test_expire, xmap);
     count_launch();
     return cudaGetLastError();
 }
@@ -1047,8 +1220,11 @@ cudaError_t launch_dx_pair_nt(const MexGeo& g, const float* x, const float* tile
     const int grid = int(std::min<long long>(items, ws_sm_count()));
     constexpr int smem = pair_stages<NT>() * pair_stage_bytes<NT>() + dx_depth<POOLED>() * dx_slot_bytes<POOLED>();
     static_assert(smem <= 227 * 1024, "stages and slot ring must fit the shared memory of one CTA");
-    if (mex_pair_wide(g, x, y, dy, dx)) PAIR_RUN((mex_dx_pair<NT, POOLED, true>), kDxThreads, smem, grid, g, x, tiles, mo, mx, y, dy, dx, plan, flag);
-    else PAIR_RUN((mex_dx_pair<NT, POOLED, false>), kDxThreads, smem, grid, g, x, tiles, mo, mx, y, dy, dx, plan, flag);
+    DxMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    if (dx_box_maps(g, mo, y, dy, &maps)) PAIR_RUN((mex_dx_pair<NT, POOLED, 2>), dx_threads<2>(), smem, grid, g, x, tiles, mo, mx, y, dy, dx, plan, flag, maps);
+    else if (mex_pair_wide(g, x, y, dy, dx)) PAIR_RUN((mex_dx_pair<NT, POOLED, 1>), kDxThreads, smem, grid, g, x, tiles, mo, mx, y, dy, dx, plan, flag, maps);
+    else PAIR_RUN((mex_dx_pair<NT, POOLED, 0>), kDxThreads, smem, grid, g, x, tiles, mo, mx, y, dy, dx, plan, flag, maps);
     count_launch();
     return cudaGetLastError();
 }
@@ -1073,31 +1249,6 @@ inline DoPairPlan dopair_plan(const MexGeo& g) {
     if (s < 1) s = 1;
     p.splits = int(s);
     return p;
-}
-
-// cuTensorMapEncodeTiled of the driver, looked up once (the library links no driver stub); nullptr if unavailable
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult st;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) p = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
-// A float32 tensor seen as rank-4 or rank-5 (dims fastest first, strides in floats for dims 1..), one box per copy
-inline bool encode_f32_map(CUtensorMap* map, const float* base, int rank, const long long* dims, const long long* strides, const int* box) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return false;
-    cuuint64_t gd[5], gs[4];
-    cuuint32_t bd[5], es[5];
-    for (int i = 0; i < rank; ++i) { gd[i] = cuuint64_t(dims[i]); bd[i] = cuuint32_t(box[i]); es[i] = 1; }
-    for (int i = 0; i + 1 < rank; ++i) gs[i] = cuuint64_t(strides[i]) * 4;
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, cuuint32_t(rank), const_cast<float*>(base), gd, gs, bd, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // The box copies need: one channel block and one region along the channels; rows of the region pair a fixed number of rows
