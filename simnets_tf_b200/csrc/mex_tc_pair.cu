@@ -482,12 +482,14 @@ __global__ void __launch_bounds__(fwd_threads<BOX>(), 1) mex_fwd_pair(MexGeo g, 
     } else if (warp == kPairMmaWarp) {
         pair_mma_role<NT, STAGES>(sh, dsm, tmem, my_items, kchunks, tries, test_expire ? 0 : -1);
     } else {
-        // ---------------- epilogue: lane = pixel pair, registers = instances of both tiles
+        // ---------------- epilogue: lane = pixel pair, registers = instances of both tiles.  Sixteen logarithms at a time, then
+        // their stores: with a guard around every instance a warp waited out the chain of shared load, logarithm and store
+        // 64 times per item, and the kernel waited for its epilogue (256 x 16 x 16: 17,000 of 19,000 cycles per item).
         const int ew = warp - kPairProducerWarps, quarter = warp & 3, half = ew >> 2;
         float* mow0 = mo_w[ew][0];
         float* mow1 = mo_w[ew][1];
         const float inv_eps = 1.f / float(g.eps), k_log = 0.69314718056f * inv_eps, c_add = float(g.cst) * inv_eps;
-        const unsigned Nu = unsigned(g.N);
+        const unsigned Nu = unsigned(g.N), Nq = Nu >> 2;
         for (int li = 0; li < my_items; ++li) {
             const int buf = li & 1;
             if (__any_sync(0xffffffffu, sh.failed)) break;
@@ -499,20 +501,19 @@ __global__ void __launch_bounds__(fwd_threads<BOX>(), 1) mex_fwd_pair(MexGeo g, 
                 mow1[i] = in ? __ldg(mo + (2 * it.r + 1) * g.M + m0 + i) : 0.f;
             }
             __syncwarp();
-            const PairColumn col = pair_column_of(g, it.r, (long long)it.jt * kTcPos + quarter * 32 + lane, P, mx);
-            const float cadd0 = col.mx0 + c_add, cadd1 = col.mx1 + c_add;
-            float* yb = y + (col.base >= 0 ? col.base : 0) + (long long)m0 * g.N;
+            const Column col = column_of(g, 2 * it.r, (long long)it.jt * kTcPos + quarter * 32 + lane, P, nullptr);
+            const bool live = col.base >= 0;
+            const int pos = live ? int(col.base - (long long)col.n * g.M * g.N) : 0;
+            const float2 mxv = live ? ldg2(mx + (long long)col.n * g.N + pos) : make_float2(0.f, 0.f);
+            const float cadd0 = mxv.x + c_add, cadd1 = mxv.y + c_add;
+            float* yb = y + (live ? col.base : 0) + (long long)m0 * g.N;
             // 2x2 sum pooling of the output, fused: a pixel pair is the upper or the lower half of a pooling window, and the
             // other half belongs to the sibling region pair (another work item).  Each half is added to a zeroed tensor by
             // one reduction: 0 + a + b with two addends is the same number in either order, so the sum is deterministic.
             float* pb = nullptr;
-            if (pooled != nullptr && col.base >= 0) {
-                const long long mn = (long long)g.M * g.N;
-                const int n = int(col.base / mn), pos = int(col.base - (long long)n * mn);
-                const int w = pos % g.Wo, hc = pos / g.Wo, h = hc % g.Ho, cc = hc / g.Ho;
-                const int Ng = g.N >> 2;
-                pb = pooled + (long long)n * g.M * Ng + (cc * (g.Ho >> 1) + (h >> 1)) * (g.Wo >> 1) + (w >> 1) + (long long)m0 * Ng;
-            }
+            if (pooled != nullptr && live)                  // (the patch corner is the position: stride 1, no padding)
+                pb = pooled + ((long long)col.n * g.M + m0) * Nq + ((pos - col.h0 * g.Wo - col.w0) >> 2) + (col.h0 >> 1) * (g.Wo >> 1) + (col.w0 >> 1);
+            const int left = live ? g.M - m0 : 0;           // instances of this half that exist
             if (!pair_wait_warp(sh.failed, &sh.acc_full[buf], (uint32_t(li) >> 1) & 1u, tries, 1024)) { sh.failed = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
@@ -521,17 +522,31 @@ __global__ void __launch_bounds__(fwd_threads<BOX>(), 1) mex_fwd_pair(MexGeo g, 
                 const uint32_t taddr = tmem + uint32_t(buf * 2 * NT + half * (NT / 2) + c0) + (uint32_t(quarter * 32) << 16);
                 tmem_ld16_issue(taddr, v0);
                 tmem_ld16_issue(taddr + NT, v1);
+                float4 b0[4], b1[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) { b0[q] = reinterpret_cast<const float4*>(mow0 + c0)[q]; b1[q] = reinterpret_cast<const float4*>(mow1 + c0)[q]; }
                 tmem_ld_wait();
-                if (col.base >= 0) {
-                    float* yp = yb + (size_t)c0 * Nu;
+                float2 o[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    o[i].x = fmaf(lg2_ftz(__uint_as_float(v0[i])), k_log, cadd0 + (&b0[i / 4].x)[i % 4]);
+                    o[i].y = fmaf(lg2_ftz(__uint_as_float(v1[i])), k_log, cadd1 + (&b1[i / 4].x)[i % 4]);
+                }
+                float* yp = yb + (size_t)c0 * Nu;
+                float* pp = pb + (size_t)c0 * Nq;
+                if (left >= c0 + 16) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) __stcs(reinterpret_cast<float2*>(yp + i * Nu), o[i]);
+                    if (pb != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) atomicAdd(pp + i * Nq, o[i].x + o[i].y);
+                    }
+                } else {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        if (m0 + c0 + i < g.M) {
-                            float2 o;
-                            o.x = fmaf(lg2_ftz(__uint_as_float(v0[i])), k_log, cadd0 + mow0[c0 + i]);
-                            o.y = fmaf(lg2_ftz(__uint_as_float(v1[i])), k_log, cadd1 + mow1[c0 + i]);
-                            __stcs(reinterpret_cast<float2*>(yp + i * Nu), o);
-                            if (pb != nullptr) atomicAdd(pb + (size_t)(c0 + i) * (Nu >> 2), o.x + o.y);
+                        if (c0 + i < left) {
+                            __stcs(reinterpret_cast<float2*>(yp + i * Nu), o[i]);
+                            if (pb != nullptr) atomicAdd(pp + i * Nq, o[i].x + o[i].y);
                         }
                     }
                 }
