@@ -490,22 +490,40 @@ __global__ void __launch_bounds__(fwd_threads<BOX>(), 1) mex_fwd_pair(MexGeo g, 
         float* mow1 = mo_w[ew][1];
         const float inv_eps = 1.f / float(g.eps), k_log = 0.69314718056f * inv_eps, c_add = float(g.cst) * inv_eps;
         const unsigned Nu = unsigned(g.N), Nq = Nu >> 2;
+        // The position of an item, its maxima among it, is requested one item ahead; the offset maxima stay while they are the same.
+        struct Place { Column col; float2 mx; int pos; };
+        auto place_of = [&](const WsItem& it) {
+            Place p;
+            p.col = column_of(g, 2 * it.r, (long long)it.jt * kTcPos + quarter * 32 + lane, P, nullptr);
+            p.pos = p.col.base >= 0 ? int(p.col.base - (long long)p.col.n * g.M * g.N) : 0;
+            p.mx = p.col.base >= 0 ? ldg2(mx + (long long)p.col.n * g.N + p.pos) : make_float2(0.f, 0.f);
+            return p;
+        };
+        WsItem next_it = ws_item(plan, int(blockIdx.x));
+        Place next = place_of(next_it);
+        int held_r = -1, held_mt = -1;
         for (int li = 0; li < my_items; ++li) {
             const int buf = li & 1;
             if (__any_sync(0xffffffffu, sh.failed)) break;
-            const WsItem it = ws_item(plan, int(blockIdx.x) + li * int(gridDim.x));
-            const int m0 = it.mt * NT + half * (NT / 2);
-            for (int i = lane; i < NT / 2; i += 32) {
-                const bool in = m0 + i < g.M;
-                mow0[i] = in ? __ldg(mo + (2 * it.r) * g.M + m0 + i) : 0.f;
-                mow1[i] = in ? __ldg(mo + (2 * it.r + 1) * g.M + m0 + i) : 0.f;
-            }
-            __syncwarp();
-            const Column col = column_of(g, 2 * it.r, (long long)it.jt * kTcPos + quarter * 32 + lane, P, nullptr);
+            const WsItem it = next_it;
+            const Column col = next.col;
+            const int pos = next.pos, m0 = it.mt * NT + half * (NT / 2);
             const bool live = col.base >= 0;
-            const int pos = live ? int(col.base - (long long)col.n * g.M * g.N) : 0;
-            const float2 mxv = live ? ldg2(mx + (long long)col.n * g.N + pos) : make_float2(0.f, 0.f);
-            const float cadd0 = mxv.x + c_add, cadd1 = mxv.y + c_add;
+            const float cadd0 = next.mx.x + c_add, cadd1 = next.mx.y + c_add;
+            if (it.r != held_r || it.mt != held_mt) {
+                __syncwarp();                                   // every lane is done with the previous contents
+                for (int i = lane; i < NT / 2; i += 32) {
+                    const bool in = m0 + i < g.M;
+                    mow0[i] = in ? __ldg(mo + (2 * it.r) * g.M + m0 + i) : 0.f;
+                    mow1[i] = in ? __ldg(mo + (2 * it.r + 1) * g.M + m0 + i) : 0.f;
+                }
+                __syncwarp();
+                held_r = it.r; held_mt = it.mt;
+            }
+            if (li + 1 < my_items) {
+                next_it = ws_item(plan, int(blockIdx.x) + (li + 1) * int(gridDim.x));
+                next = place_of(next_it);
+            }
             float* yb = y + (live ? col.base : 0) + (long long)m0 * g.N;
             // 2x2 sum pooling of the output, fused: a pixel pair is the upper or the lower half of a pooling window, and the
             // other half belongs to the sibling region pair (another work item).  Each half is added to a zeroed tensor by
@@ -774,13 +792,17 @@ __global__ void __launch_bounds__(dx_threads<LOAD>(), 1) mex_dx_pair(MexGeo g, c
                 }
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (i < kleft) {
-                        float2 o;
-                        o.x = ex2_ftz(a * (xr[i].x - col.mx0)) * __uint_as_float(v0[i]);
-                        o.y = ex2_ftz(a * (xr[i].y - col.mx1)) * __uint_as_float(v1[i]);
-                        *reinterpret_cast<float2*>(db + (size_t)(c0 + i) * hw) = o;
-                    }
+                for (int i = 0; i < 8; ++i) {                   // (all eight before the first store: a guard around each would make a chain of them)
+                    xr[i].x = ex2_ftz(a * (xr[i].x - col.mx0)) * __uint_as_float(v0[i]);
+                    xr[i].y = ex2_ftz(a * (xr[i].y - col.mx1)) * __uint_as_float(v1[i]);
+                }
+                float* dp = db + (size_t)c0 * hw;
+                if (kleft >= 8) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) *reinterpret_cast<float2*>(dp + i * hw) = xr[i];
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) if (i < kleft) *reinterpret_cast<float2*>(dp + i * hw) = xr[i];
                 }
                 kleft -= 8;
 #pragma unroll
