@@ -122,11 +122,12 @@ __global__ void __launch_bounds__(kThreads) sim_dx_direct(SimGeo g, const T* __r
     }
 }
 
-// One block per (instance m, tap k): reduces over batch and output positions.
+// One block per (instance m, tap k): reduces over batch and output positions.  Positions are decoded by multiply and shift
+// (f_N, f_ow; totals of 2^31 and more by division): a 64-bit division and modulo per term had been most of the instructions.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T* __restrict__ x, const T* __restrict__ tm,
                                                                const T* __restrict__ wt, const T* __restrict__ dy,
-                                                               T* __restrict__ dt, T* __restrict__ dw, int accumulate) {
+                                                               T* __restrict__ dt, T* __restrict__ dw, int accumulate, FastDiv f_N, FastDiv f_ow) {
     stream_order();
     __shared__ T smem[kThreads];
     const int mk = blockIdx.x;
@@ -137,8 +138,8 @@ __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T
     T st = T(0), sw_ = T(0);
     const long long total = (long long)g.B * g.N;
     for (long long i = threadIdx.x; i < total; i += kThreads) {
-        const int j = int(i % g.N), n = int(i / g.N);
-        const int ho = j / g.ow, wo = j % g.ow;
+        const int n = total <= 0x7fffffffLL ? int(fast_div(uint32_t(i), f_N)) : int(i / g.N), j = int(i - (long long)n * g.N);
+        const int ho = int(fast_div(uint32_t(j), f_ow)), wo = j - ho * g.ow;
         const int hh = ho * g.sh - g.ph + kh, ww = wo * g.sw - g.pw + kw;
         const T v = (hh >= 0 && hh < g.H && ww >= 0 && ww < g.W) ? x[(((size_t)n * g.C + c) * g.H + hh) * g.W + ww] : oob;
         const T err = dy[((size_t)n * g.M + m) * g.N + j];
@@ -284,8 +285,8 @@ cudaError_t launch_sim_dparams_direct(const SimGeo& g, bool f64, const void* x, 
                                       void* dt, void* dw, bool accumulate, cudaStream_t s) {
     const int blocks = g.M * g.K;
     SIMNETS_DTYPE_SWITCH(f64,
-        (in_stream_order(sim_dparams_direct<float>, blocks, kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dt, (float*)dw, accumulate)),
-        (in_stream_order(sim_dparams_direct<double>, blocks, kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dt, (double*)dw, accumulate)));
+        (in_stream_order(sim_dparams_direct<float>, blocks, kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dt, (float*)dw, accumulate, make_fastdiv(g.N), make_fastdiv(g.ow))),
+        (in_stream_order(sim_dparams_direct<double>, blocks, kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dt, (double*)dw, accumulate, make_fastdiv(g.N), make_fastdiv(g.ow))));
     count_launch();
     return cudaGetLastError();
 }
