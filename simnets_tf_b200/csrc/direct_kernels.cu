@@ -281,6 +281,20 @@ cudaError_t launch_sim_dx_direct(const SimGeo& g, bool f64, const void* x, const
     return cudaGetLastError();
 }
 
+namespace {
+__global__ void __launch_bounds__(kThreads) zero_words(int* __restrict__ p, int n) {
+    stream_order();
+    for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) p[i] = 0;
+}
+}  // namespace
+
+cudaError_t launch_zero_words(int* p, int n, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    in_stream_order(zero_words, std::min((n + kThreads - 1) / kThreads, 64), kThreads, 0, s)(p, n);
+    count_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_sim_dparams_direct(const SimGeo& g, bool f64, const void* x, const void* t, const void* w, const void* dy,
                                       void* dt, void* dw, bool accumulate, cudaStream_t s) {
     const int blocks = g.M * g.K;

@@ -27,6 +27,8 @@ cudaError_t launch_sum_pool2(long long planes, int H, int W, const float* x, flo
 cudaError_t launch_sim_fwd_direct(const SimGeo&, bool f64, const void* x, const void* t, const void* w, void* y, cudaStream_t,
                                   const int* gate = nullptr);
 cudaError_t launch_sim_dx_direct(const SimGeo&, bool f64, const void* x, const void* t, const void* w, const void* dy, void* dx, cudaStream_t);
+// n ints cleared by a launch that overlaps like the kernels around it (a memset between two of them costs 3 us of idle GPU)
+cudaError_t launch_zero_words(int* p, int n, cudaStream_t s);
 cudaError_t launch_sim_dparams_direct(const SimGeo&, bool f64, const void* x, const void* t, const void* w, const void* dy,
                                       void* dt, void* dw, bool accumulate, cudaStream_t);
 // MEX launchers take an optional device flag: with `gate` non-null the kernel runs only if *gate != 0

@@ -79,7 +79,7 @@ cudaError_t launch_softmax_xent(int batch, int classes, float scale, const float
                                 float* dlogits, void* ws, cudaStream_t s) {
     unsigned* ticket = static_cast<unsigned*>(ws);
     float* partial = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
-    const cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(unsigned), s);
+    const cudaError_t e = launch_zero_words(static_cast<int*>(ws), 1, s);
     if (e != cudaSuccess) return e;
     in_stream_order(softmax_xent, loss_grid(batch), kLossThreads, 0, s)(batch, classes, scale, logits, labels, loss, dlogits, partial, ticket);
     count_launch();

@@ -650,7 +650,7 @@ cudaError_t launch_mex_fwd_head(const MexGeo& g, const float* x, const float* eo
         if (groups * slices > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
         float* partial = scratch;
         int* tickets = reinterpret_cast<int*>(scratch + size_t(P + kWidePB) * head_slices_max(g) * (pad4(g.M) + 1));
-        cudaError_t e = cudaMemsetAsync(tickets, 0, sizeof(int) * size_t(groups), s);
+        cudaError_t e = launch_zero_words(tickets, int(groups), s);
         if (e != cudaSuccess) return e;
         const int blocks = int(groups * slices);
 #define HEAD_WIDE(MP)                                                                                                   \
@@ -683,7 +683,7 @@ cudaError_t launch_mex_fwd_head(const MexGeo& g, const float* x, const float* eo
     if (groups * slices > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     float* partial = scratch;
     int* tickets = reinterpret_cast<int*>(scratch + size_t(P + kWidePB) * head_slices_max(g) * (pad4(g.M) + 1));
-    cudaError_t e = cudaMemsetAsync(tickets, 0, sizeof(int) * size_t(groups), s);
+    cudaError_t e = launch_zero_words(tickets, int(groups), s);
     if (e != cudaSuccess) return e;
     const int blocks = int(groups * slices);
     switch (pad4(g.M)) {

@@ -720,7 +720,7 @@ bool use_short_bwd(const MexGeo& g, uint32_t flags, const void* a, const void* b
 // zero: when given, n_zero floats to be cleared as well
 cudaError_t run_prepasses(const MexGeo& g, const MexWs& w, const float* x, const float* off, cudaStream_t s, bool need_mx = true,
                           bool pair_tiles = false, bool normalize = false, float* zero = nullptr, size_t n_zero = 0) {
-    cudaError_t e = cudaMemsetAsync(w.flag, 0, 16, s);
+    cudaError_t e = launch_zero_words(w.flag, 4, s);
     if (e != cudaSuccess) return e;
     PrepArgs a = {g.M, 0, 0, w.mo, w.eo, w.eot, nullptr, nullptr, normalize ? w.offn : nullptr, w.lse, w.flag};
     if (pair_tiles) {
