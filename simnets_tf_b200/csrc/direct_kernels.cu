@@ -40,16 +40,17 @@ __device__ __forceinline__ T block_sum(T v, T* smem) {
 // ------------------------------------------------------------------ Similarity
 template <typename T>
 __global__ void __launch_bounds__(kThreads) sim_fwd_direct(SimGeo g, const T* __restrict__ x, const T* __restrict__ tm,
-                                                           const T* __restrict__ wt, T* __restrict__ y, const int* __restrict__ gate) {
+                                                           const T* __restrict__ wt, T* __restrict__ y, const int* __restrict__ gate,
+                                                           FastDiv f_N, FastDiv f_M, FastDiv f_ow) {
     stream_order();
     if (gate && gate[1] == 0) return;
     const long long total = (long long)g.B * g.M * g.N;
     const T oob = T(g.oob), fudge = T(g.fudge);
     for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads) {
-        const int j = int(idx % g.N);
-        const long long q = idx / g.N;
-        const int m = int(q % g.M), n = int(q / g.M);
-        const int ho = j / g.ow, wo = j % g.ow;
+        const long long q = total <= 0x7fffffffLL ? (long long)fast_div(uint32_t(idx), f_N) : idx / g.N;
+        const int n = total <= 0x7fffffffLL ? int(fast_div(uint32_t(q), f_M)) : int(q / g.M);
+        const int j = int(idx - q * g.N), m = int(q - (long long)n * g.M);
+        const int ho = int(fast_div(uint32_t(j), f_ow)), wo = j - ho * g.ow;
         const T* xs = x + (size_t)n * g.C * g.H * g.W;
         const T* tp = tm + (size_t)m * g.K;
         const T* wp = wt + (size_t)m * g.K;
@@ -265,8 +266,8 @@ cudaError_t launch_sim_fwd_direct(const SimGeo& g, bool f64, const void* x, cons
     const long long total = (long long)g.B * g.M * g.N;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (in_stream_order(sim_fwd_direct<float>, grid_for(total), kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (float*)y, gate)),
-        (in_stream_order(sim_fwd_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (double*)y, gate)));
+        (in_stream_order(sim_fwd_direct<float>, grid_for(total), kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (float*)y, gate, make_fastdiv(g.N), make_fastdiv(g.M), make_fastdiv(g.ow))),
+        (in_stream_order(sim_fwd_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (double*)y, gate, make_fastdiv(g.N), make_fastdiv(g.M), make_fastdiv(g.ow))));
     count_launch();
     return cudaGetLastError();
 }

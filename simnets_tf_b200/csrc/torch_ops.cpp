@@ -308,7 +308,7 @@ Tensor mex_apply(const MexPlanPtr& p, const Tensor& x, const Tensor& off, OptTen
             std::tie(y, out) = mex_forward_impl(*p, x, off, fwd_flags | op_flags, ws, true);
         } else {
             y = out = mex_forward_impl(*p, x, off, fwd_flags | op_flags, ws, false).first;
-            if (pooled) out = at::avg_pool2d(y, {2, 2}).mul_(4.0);
+            if (pooled) out = at::avg_pool2d(y, {2, 2}, {2, 2}, 0, false, true, 1);        // (the sum of each window)
         }
     }
     if (!track) return out;
