@@ -39,6 +39,30 @@ def sequence_key(v):
     return tuple(v) if isinstance(v, (list, tuple)) else v
 
 
+class _Recorded(torch.autograd.Function):
+    """An operator call as one node of the graph that torch.jit.trace records.  The tracer sees torch's own operators only: it
+    would keep the result of a native call as a constant.  As a node, the call is made again (plan, checks and gradient
+    included) whenever the recorded graph runs."""
+
+    @staticmethod
+    def forward(ctx, call, *tensors):
+        with torch.enable_grad():
+            ctx.inputs = [t.detach().requires_grad_(wanted) for t, wanted in zip(tensors, ctx.needs_input_grad[1:])]
+            ctx.output = call(*ctx.inputs)
+        return ctx.output.detach()
+
+    @staticmethod
+    def backward(ctx, grad):
+        wanted = [t for t in ctx.inputs if t.requires_grad]
+        got = iter(torch.autograd.grad(ctx.output, wanted, grad, retain_graph=True, create_graph=torch.is_grad_enabled()))
+        return (None,) + tuple(next(got) if t.requires_grad else None for t in ctx.inputs)
+
+
+def recorded(call, *tensors):
+    """call(*tensors) while torch.jit.trace is recording (see `_Recorded`)."""
+    return _Recorded.apply(call, *tensors)
+
+
 class PlanCache(object):
     """The native plans (descriptor, geometry) of the calls seen last, by everything that determines them.  Bounded: a
     program that keeps changing shapes starts over after `limit` of them."""
