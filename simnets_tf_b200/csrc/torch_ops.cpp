@@ -102,6 +102,15 @@ std::string shape_text(at::IntArrayRef s) {
 Tensor scratch(const Tensor& like, size_t bytes) {
     return at::empty({int64_t(bytes)}, at::TensorOptions().dtype(at::kByte).device(like.device()));
 }
+// The operators have no forward-mode derivative: a tangent is refused, as a torch.autograd.Function without a jvp refuses it,
+// instead of being dropped (the kernels see values only).
+void refuse_tangents(std::initializer_list<const Tensor*> inputs) {
+    for (const Tensor* t : inputs)
+        if (t->_fw_grad(0).defined()) {
+            PyErr_SetString(PyExc_NotImplementedError, "simnets_b200 operators have no forward-mode derivative (jvp)");
+            throw py::error_already_set();
+        }
+}
 inline cudaStream_t stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 inline void* ptr(const Tensor& t) { return t.data_ptr(); }
 
@@ -299,6 +308,7 @@ struct MexNode : torch::autograd::Node {
 
 // The differentiable op; `pooled` returns the 2x2 sum pooling of the output.  See ops/mex.py for the extras.
 Tensor mex_apply(const MexPlanPtr& p, const Tensor& x, const Tensor& off, OptTensor ws, uint32_t fwd_flags, uint32_t op_flags, bool pooled, const OptTensor& sink) {
+    refuse_tangents({&x, &off});
     const bool track = at::GradMode::is_enabled() && (x.requires_grad() || off.requires_grad());
     Tensor y, out;
     {
@@ -406,6 +416,7 @@ struct SimNode : torch::autograd::Node {
 
 Tensor sim_apply(const SimPlanPtr& p, const Tensor& x, const Tensor& t, const Tensor& w, uint32_t flags, uint64_t ch_max, uint64_t ch_min,
                  const OptTensor& dt_sink, const OptTensor& dw_sink) {
+    refuse_tangents({&x, &t, &w});
     const bool track = at::GradMode::is_enabled() && (x.requires_grad() || t.requires_grad() || w.requires_grad());
     Tensor y;
     {
@@ -483,6 +494,7 @@ struct XentNode : torch::autograd::Node {
 };
 
 Tensor xent_apply(const Tensor& logits, const Tensor& labels, double scale) {
+    refuse_tangents({&logits});
     const bool track = at::GradMode::is_enabled() && logits.requires_grad();
     Tensor loss, dlogits;
     {

@@ -1,8 +1,9 @@
-"""What surrounds the native gradient nodes: torch.jit.trace records the calls."""
+"""What surrounds the native gradient nodes: forward-mode differentiation is refused, torch.jit.trace records the calls."""
 import importlib
 
 import pytest
 import torch
+import torch.autograd.forward_ad as forward_ad
 
 from simnets_tf_b200 import keras
 from simnets_tf_b200.ops.loss import softmax_cross_entropy
@@ -45,6 +46,16 @@ def _operators():
 
 
 OPERATORS = ["similarity", "mex", "mex_pooled", "mex_pooled_f64", "cross_entropy"]
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_tangents_are_refused(name):
+    op, x = _operators()[name]
+    for wanted in (False, True):
+        with forward_ad.dual_level():
+            dual = forward_ad.make_dual(x.clone().requires_grad_(wanted), torch.ones_like(x))
+            with pytest.raises(NotImplementedError):
+                op(dual)
 
 
 def _gradients(op, x):
