@@ -278,8 +278,7 @@ std::pair<Tensor, Tensor> mex_backward(const MexPlanPtr& p, const Tensor& x, con
 // node keeps and finds primed (per-position extrema, offset tables, operand tiles).
 struct MexNode : torch::autograd::Node {
     MexPlanPtr plan;
-    SavedVariable x, off, y_saved;
-    Tensor y_plain;             // the unpooled output of a pooled layer: not an output of the node
+    SavedVariable x, off, y;    // (y of a pooled layer is not an output of the node)
     OptTensor ws, sink;
     uint32_t flags = 0;
     bool pooled = false;
@@ -290,8 +289,7 @@ struct MexNode : torch::autograd::Node {
         if (!grads[0].defined()) return out;
         const bool want_dx = task_should_compute_output(0), want_doff = task_should_compute_output(1);
         if (!want_dx && !want_doff) return out;
-        const Tensor xv = x.unpack(), ov = off.unpack(), yv = pooled ? y_plain : y_saved.unpack(shared_from_this());
-        TORCH_CHECK(yv.defined(), "Trying to backward through the graph a second time, but its saved tensors have already been freed");
+        const Tensor xv = x.unpack(), ov = off.unpack(), yv = y.unpack(pooled ? nullptr : shared_from_this());
         // (with a sink the offsets gradient is added straight into the caller's tensor, a gradient bucket; nothing is left to accumulate)
         const auto g = mex_grads(*plan, xv, ov, yv, grads[0], flags | (sink ? SIMNETS_FLAG_ACCUMULATE : 0u), ws, pooled, want_dx, want_doff, sink);
         if (want_dx) out[0] = g.first;
@@ -300,8 +298,7 @@ struct MexNode : torch::autograd::Node {
     }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
-        x.reset_data(); off.reset_data(); y_saved.reset_data();
-        y_plain.reset();
+        x.reset_data(); off.reset_data(); y.reset_data();
         ws.reset();
     }
 };
@@ -332,7 +329,7 @@ Tensor mex_apply(const MexPlanPtr& p, const Tensor& x, const Tensor& off, OptTen
     node->flags = op_flags;
     node->pooled = pooled;
     torch::autograd::set_history(out, node);
-    if (pooled) node->y_plain = y; else node->y_saved = SavedVariable(out, true);
+    node->y = pooled ? SavedVariable(y, false) : SavedVariable(out, true);
     return out;
 }
 
@@ -479,17 +476,16 @@ std::pair<Tensor, Tensor> xent_with_grad(const Tensor& logits_in, const Tensor& 
 }
 
 struct XentNode : torch::autograd::Node {
-    Tensor dlogits;
+    SavedVariable dlogits;
     std::string name() const override { return "SoftmaxCrossEntropyBackward"; }
     variable_list apply(variable_list&& grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
         if (!grads[0].defined()) return variable_list(1);
-        TORCH_CHECK(dlogits.defined(), "Trying to backward through the graph a second time, but its saved tensors have already been freed");
-        return {dlogits * grads[0]};
+        return {dlogits.unpack() * grads[0]};
     }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
-        dlogits.reset();
+        dlogits.reset_data();
     }
 };
 
@@ -504,7 +500,7 @@ Tensor xent_apply(const Tensor& logits, const Tensor& labels, double scale) {
     if (!track) return loss;
     auto node = std::shared_ptr<XentNode>(new XentNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(logits));
-    node->dlogits = dlogits;
+    node->dlogits = SavedVariable(dlogits, false);
     torch::autograd::set_history(loss, node);
     return loss;
 }

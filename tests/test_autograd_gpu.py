@@ -1,4 +1,5 @@
-"""What surrounds the native gradient nodes: forward-mode differentiation is refused, torch.jit.trace records the calls."""
+"""What surrounds the native gradient nodes: forward-mode differentiation is refused, torch.jit.trace records the calls, hooks
+on saved tensors see everything a node keeps."""
 import importlib
 
 import pytest
@@ -81,6 +82,20 @@ def test_a_recorded_network_runs_again_on_other_inputs():
     traced = torch.jit.trace(net, (x,), check_trace=False)
     for v in (x, x * 0.5, torch.rand(5, 1, 28, 28, device="cuda") - 0.5):
         assert torch.allclose(traced(v), net(v), rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("name", OPERATORS)
+def test_hooks_see_every_saved_tensor(name):
+    op, x = _operators()[name]
+    seen = []
+    x = x.clone().requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.shape) or t.cpu(), lambda t: t.cuda()):
+        y = op(x)
+    g = torch.autograd.grad(y.sum(), [x] + list(op.parameters()))
+    want = {"similarity": [x.shape] + [p.shape for p in op.params], "cross_entropy": [x.shape]}.get(name, [x.shape, op.params[0].shape if len(op.params) else None, (6, 8, 8, 8)])
+    assert seen == want
+    for ours, ref in zip(g, torch.autograd.grad(op(x).sum(), [x] + list(op.parameters()))):
+        assert torch.equal(ours, ref)
 
 
 def test_a_layer_of_a_recorded_graph_takes_its_bucket_gradient_through_autograd():
