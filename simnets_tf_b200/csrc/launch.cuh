@@ -8,6 +8,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <utility>
+#include "smem_limit.hpp"
 
 namespace simnets {
 

@@ -655,13 +655,10 @@ cudaError_t launch_mex_fwd_head(const MexGeo& g, const float* x, const float* eo
         const int blocks = int(groups * slices);
 #define HEAD_WIDE(MP)                                                                                                   \
         do {                                                                                                            \
-            static bool attr_done = false;                                                                              \
+            static SmemLimit limit;                                                                                     \
             constexpr int smem = MP * kWideSlice * 4;                                                                   \
-            if (!attr_done) {                                                                                           \
-                e = cudaFuncSetAttribute(mex_fwd_head_wide<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);     \
-                if (e != cudaSuccess) return e;                                                                         \
-                attr_done = true;                                                                                       \
-            }                                                                                                           \
+            e = limit.raise(mex_fwd_head_wide<MP>, smem);                                                               \
+            if (e != cudaSuccess) return e;                                                                             \
             in_stream_order(mex_fwd_head_wide<MP>, blocks, kT, smem, s)(g, slices, x, eo, mo, mx, y, partial, tickets, flag);        \
         } while (0)
         switch (pad4(g.M)) {

@@ -397,18 +397,10 @@ __global__ void __launch_bounds__(kTcThreads, NT == 64 ? 3 : 2) mex_doff_tc(MexG
     tc_end(tmem_d, NT);
 }
 
-template <class Kernel>
-cudaError_t set_smem_once(Kernel kernel, int smem, bool& done) {
-    if (done) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) done = true;
-    return e;
-}
-
 #define TC_RUN(KERNEL, SMEM, GRID, ...)                                        \
     do {                                                                       \
-        static bool attr_done = false;                                         \
-        const cudaError_t e_ = set_smem_once(KERNEL, SMEM, attr_done);          \
+        static SmemLimit limit;                                                \
+        const cudaError_t e_ = limit.raise(KERNEL, SMEM);                      \
         if (e_ != cudaSuccess) return e_;                                      \
         in_stream_order(KERNEL, GRID, kTcThreads, SMEM, s)(__VA_ARGS__);                     \
     } while (0)
@@ -442,8 +434,8 @@ cudaError_t launch_dx_nt(const MexGeo& g, const float* x, const float* tiles, co
     const int smem = tc_smem_bytes<NT, kTcKT, 128, 2>() + ((g.M + kTcKT - 1) / kTcKT) * kTcKT * 4;
 #define DX_RUN(KERNEL)                                                                              \
     do {                                                                                            \
-        static bool attr_done = false;                                                              \
-        const cudaError_t e_ = set_smem_once(KERNEL, smem_max, attr_done);                          \
+        static SmemLimit limit;                                                                     \
+        const cudaError_t e_ = limit.raise(KERNEL, smem_max);                                       \
         if (e_ != cudaSuccess) return e_;                                                           \
         in_stream_order(KERNEL, int(blocks), kTcThreads, smem, s)(g, x, tiles, mo, mx, y, dy, dx, flag);         \
     } while (0)

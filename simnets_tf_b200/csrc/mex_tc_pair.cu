@@ -1158,8 +1158,8 @@ __global__ void __launch_bounds__(do_pair_threads(LOAD), 1) mex_doff_pair(MexGeo
 
 #define PAIR_RUN(KERNEL, THREADS, SMEM, GRID, ...)                               \
     do {                                                                        \
-        static bool attr_done = false;                                          \
-        const cudaError_t e_ = ws_set_smem(KERNEL, SMEM, attr_done);            \
+        static SmemLimit limit;                                                 \
+        const cudaError_t e_ = limit.raise(KERNEL, SMEM);                       \
         if (e_ != cudaSuccess) return e_;                                       \
         in_stream_order(KERNEL, GRID, THREADS, SMEM, s)(__VA_ARGS__);                         \
     } while (0)

@@ -15,7 +15,6 @@
 // warp at 12 to 16 warps per SM do not cover the latency of difference -> product -> sum (2048 x 3 x 32 x 32 input, 64
 // templates of 3x3: 610 to 636 us).  All five modes of the forward functor (include/utils/similarity_utils.hpp:17-60 of the
 // reference) are covered.
-#include <atomic>
 #include "kernels.cuh"
 #include "tile.cuh"
 
@@ -360,16 +359,10 @@ cudaError_t launch_sk(const SimGeo& g, int slice, const float* x, const float* t
 
 template <int MODE, int TM>
 cudaError_t launch_resident(const SimGeo& g, const float* x, const float* t, const float* w, float* y, float* ch_max, float* ch_min, int* flag, cudaStream_t s) {
-    static std::atomic<uint64_t> opted{0};                  // devices on which the kernel may use more than 48 KB
+    static SmemLimit limit;
     const int smem = int(sizeof(float)) * resident_smem_floats<MODE, TM>(g.K);
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = limit.raise(sim_fwd_resident<MODE, TM>, int(sizeof(float)) * resident_smem_floats<MODE, TM>(kResMaxK));
     if (e != cudaSuccess) return e;
-    if (!(opted.load(std::memory_order_relaxed) >> (dev & 63) & 1u)) {
-        e = cudaFuncSetAttribute(sim_fwd_resident<MODE, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(float)) * resident_smem_floats<MODE, TM>(kResMaxK));
-        if (e != cudaSuccess) return e;
-        opted.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
-    }
     const long long tiles = ((long long)g.B * g.N + kResTN - 1) / kResTN;
     const int mtiles = (g.M + TM - 1) / TM, per_sm = std::min(TM == 64 ? 2 : 4, 220 * 1024 / (smem + 2 * (TM / 4) * kResTN * int(sizeof(float)) + 4096));
     const int resident = std::max(1, device_sm_count() * per_sm / mtiles);

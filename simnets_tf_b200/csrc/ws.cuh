@@ -170,18 +170,10 @@ __device__ __forceinline__ void ws_mma_role(WsShared<STAGES>& sh, unsigned char*
 
 inline int ws_sm_count() { return device_sm_count(); }
 
-template <class Kernel>
-cudaError_t ws_set_smem(Kernel kernel, int smem, bool& done) {
-    if (done) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) done = true;
-    return e;
-}
-
 #define WS_RUN(KERNEL, SMEM, GRID, ...)                                         \
     do {                                                                        \
-        static bool attr_done = false;                                          \
-        const cudaError_t e_ = ws_set_smem(KERNEL, SMEM, attr_done);            \
+        static SmemLimit limit;                                                 \
+        const cudaError_t e_ = limit.raise(KERNEL, SMEM);                       \
         if (e_ != cudaSuccess) return e_;                                       \
         in_stream_order(KERNEL, GRID, kWsThreads, SMEM, s)(__VA_ARGS__);                      \
     } while (0)
