@@ -251,7 +251,14 @@ SIMNETS_API int get_mex_offsets_nregions(int n_input_dim, const int* input_dim,
                                          int n_shared_offset_region, const int* shared_offset_region,
                                          int n_unshared_offset_region, const int* unshared_offset_region);
 
+/* Scratch of a MEX layer.  simnets_mex_workspace_bytes: enough for every entry point below.
+ * simnets_mex_forward_workspace_bytes: what simnets_mex_forward, simnets_mex_offsets_grad and a workspace that is kept
+ * for primed gradients need.  simnets_mex_products_bytes: what only the input gradient of overlapping blocks needs
+ * beside that (the products of all taps and positions, up to 256 MB or one sample's; 0 for layers whose blocks do not
+ * overlap), which simnets_mex_gradients takes separately. */
 SIMNETS_API size_t simnets_mex_workspace_bytes(const simnets_mex_desc* d);
+SIMNETS_API size_t simnets_mex_forward_workspace_bytes(const simnets_mex_desc* d);
+SIMNETS_API size_t simnets_mex_products_bytes(const simnets_mex_desc* d);
 
 /* MEX forward: y[batch, num_instances * channels_out, height_out, width_out].
  * Replaces MEXKernelGPU<T>::Compute (src/kernels/mex_kernel_gpu.cu:60-159),
@@ -341,6 +348,15 @@ SIMNETS_API int simnets_mex_offsets_grad(const simnets_mex_desc* d,
 SIMNETS_API int simnets_mex_backward(const simnets_mex_desc* d,
                                      const void* x, const void* offsets, const void* y, const void* dy,
                                      void* dx, void* doffsets, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Either or both MEX gradients (a NULL dx or doffsets is not computed; same results as the calls above), with the
+ * products of overlapping blocks in scratch of their own instead of at the end of the workspace: a caller that keeps a
+ * layer's workspace between the passes keeps simnets_mex_forward_workspace_bytes and lends simnets_mex_products_bytes to
+ * this call (NULL and 0 where that is 0 or dx is not wanted). */
+SIMNETS_API int simnets_mex_gradients(const simnets_mex_desc* d,
+                                      const void* x, const void* offsets, const void* y, const void* dy,
+                                      void* dx, void* doffsets, void* workspace, size_t workspace_bytes,
+                                      void* products, size_t products_bytes, void* stream);
 
 /* ---- measurement probe ---------------------------------------------------- */
 /* Launches a register-only kernel of independent FP32 fused multiply-adds on every SM (packed != 0: the packed

@@ -29,6 +29,38 @@ using namespace simnets;
 namespace {
 inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 inline int from_cuda(cudaError_t e) { return e == cudaSuccess ? SIMNETS_OK : int(e); }
+
+// The MEX gradients that have a place to go (an empty batch may come without tensors of its size).
+int mex_gradients(const MexGeo& g, const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff,
+                  void* ws, size_t ws_bytes, void* products, size_t products_bytes, cudaStream_t s) {
+    const bool f64 = d->dtype == SIMNETS_F64, acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
+    const bool gemm = mex_use_gemm(g, f64, d->flags), tiled = !gemm && mex_use_tiled(g, f64, d->flags);
+    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !gemm && !tiled) return SIMNETS_E_UNSUPPORTED;
+    if (gemm || tiled) {
+        if (!ws || ws_bytes < (gemm ? mex_gemm_workspace_bytes(g, f64) : mex_workspace_bytes(g, f64, d->flags))) return SIMNETS_E_WORKSPACE;
+        const size_t need = dx ? mex_products_bytes(g, f64, d->flags) : 0;
+        if (need > 0 && (!products || products_bytes < need)) return SIMNETS_E_WORKSPACE;
+    }
+    if (gemm) return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, doff, acc, ws, products, d->flags, s));
+    if (tiled) {
+        const float *xf = (const float*)x, *of = (const float*)off, *yf = (const float*)y, *dyf = (const float*)dy;
+        if (dx && doff) return from_cuda(launch_mex_backward_tiled(g, xf, of, yf, dyf, (float*)dx, (float*)doff, acc, ws, products, d->flags, s));
+        return from_cuda(dx ? launch_mex_dx_tiled(g, xf, of, yf, dyf, (float*)dx, ws, products, d->flags, s)
+                            : launch_mex_doff_tiled(g, xf, of, yf, dyf, (float*)doff, acc, ws, d->flags, s));
+    }
+    cudaError_t e = dx ? launch_mex_dx_direct(g, f64, x, off, y, dy, dx, s) : cudaSuccess;
+    if (e == cudaSuccess && doff) e = launch_mex_doff_direct(g, f64, x, off, y, dy, doff, acc, s);
+    return from_cuda(e);
+}
+
+// the same with the products at the end of one workspace
+int mex_gradients_in(const MexGeo& g, const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff,
+                     void* ws, size_t ws_bytes, cudaStream_t s) {
+    const bool f64 = d->dtype == SIMNETS_F64;
+    const size_t kept = mex_use_gemm(g, f64, d->flags) ? mex_gemm_workspace_bytes(g, f64) : mex_workspace_bytes(g, f64, d->flags);
+    const bool more = ws && ws_bytes > kept;
+    return mex_gradients(g, d, x, off, y, dy, dx, doff, ws, ws_bytes, more ? static_cast<char*>(ws) + kept : nullptr, more ? ws_bytes - kept : 0, s);
+}
 }  // namespace
 
 extern "C" {
@@ -179,12 +211,25 @@ int get_mex_offsets_nregions(int n_input_dim, const int* input_dim, int n_paddin
     return g.num_regions;
 }
 
-size_t simnets_mex_workspace_bytes(const simnets_mex_desc* d) {
+size_t simnets_mex_forward_workspace_bytes(const simnets_mex_desc* d) {
     MexGeo g;
     if (mex_geometry(d, nullptr, &g)) return 0;
     const bool f64 = d->dtype == SIMNETS_F64;
     // (room for either family: a caller may size a workspace once and pass other flags later)
     return std::max(mex_workspace_bytes(g, f64, d->flags), mex_use_gemm(g, f64, d->flags) ? mex_gemm_workspace_bytes(g, f64) : size_t(256));
+}
+
+size_t simnets_mex_products_bytes(const simnets_mex_desc* d) {
+    MexGeo g;
+    return mex_geometry(d, nullptr, &g) ? 0 : mex_products_bytes(g, d->dtype == SIMNETS_F64, d->flags);
+}
+
+size_t simnets_mex_workspace_bytes(const simnets_mex_desc* d) {
+    MexGeo g;
+    if (mex_geometry(d, nullptr, &g)) return 0;
+    const bool f64 = d->dtype == SIMNETS_F64;
+    return simnets_mex_forward_workspace_bytes(d) +
+           std::max(mex_products_bytes(g, f64, d->flags), mex_products_bytes(g, f64, d->flags | SIMNETS_FLAG_MEX_NO_SMALL_TILES));
 }
 
 int simnets_mex_forward(const simnets_mex_desc* d, const void* x, const void* off, void* y, void* ws, size_t ws_bytes, void* stream) {
@@ -262,24 +307,22 @@ int simnets_mex_forward_static_scratch(const simnets_mex_desc* d, const void* x,
     return launch_mex_fwd_static(g, (const float*)x, (const float*)off, (float*)y, d->flags, as_stream(stream));
 }
 
+int simnets_mex_gradients(const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff,
+                          void* ws, size_t ws_bytes, void* products, size_t products_bytes, void* stream) {
+    MexGeo g;
+    const int rc = mex_geometry(d, nullptr, &g);
+    if (rc) return rc;
+    if (!off || (g.B > 0 && (!x || !y || !dy || (!dx && !doff)))) return SIMNETS_E_NULL;
+    return mex_gradients(g, d, x, off, y, dy, dx, doff, ws, ws_bytes, products, products_bytes, as_stream(stream));
+}
+
 int simnets_mex_input_grad(const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy, void* dx,
                            void* ws, size_t ws_bytes, void* stream) {
     MexGeo g;
     const int rc = mex_geometry(d, nullptr, &g);
     if (rc) return rc;
     if (!off || (g.B > 0 && (!x || !y || !dy || !dx))) return SIMNETS_E_NULL;
-    const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
-    if (mex_use_gemm(g, f64, d->flags)) {
-        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, nullptr, false, ws, d->flags, as_stream(stream)));
-    }
-    if (mex_use_tiled(g, f64, d->flags)) {
-        if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_dx_tiled(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx,
-                                             ws, d->flags, as_stream(stream)));
-    }
-    return from_cuda(launch_mex_dx_direct(g, f64, x, off, y, dy, dx, as_stream(stream)));
+    return mex_gradients_in(g, d, x, off, y, dy, dx, nullptr, ws, ws_bytes, as_stream(stream));
 }
 
 int simnets_mex_offsets_grad(const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy,
@@ -288,19 +331,7 @@ int simnets_mex_offsets_grad(const simnets_mex_desc* d, const void* x, const voi
     const int rc = mex_geometry(d, nullptr, &g);
     if (rc) return rc;
     if (!off || !doff || (g.B > 0 && (!x || !y || !dy))) return SIMNETS_E_NULL;
-    const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
-    const bool acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
-    if (mex_use_gemm(g, f64, d->flags)) {
-        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, nullptr, doff, acc, ws, d->flags, as_stream(stream)));
-    }
-    if (mex_use_tiled(g, f64, d->flags)) {
-        if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_doff_tiled(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy,
-                                               (float*)doff, acc, ws, d->flags, as_stream(stream)));
-    }
-    return from_cuda(launch_mex_doff_direct(g, f64, x, off, y, dy, doff, acc, as_stream(stream)));
+    return mex_gradients_in(g, d, x, off, y, dy, nullptr, doff, ws, ws_bytes, as_stream(stream));
 }
 
 int simnets_mex_backward(const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy,
@@ -309,21 +340,7 @@ int simnets_mex_backward(const simnets_mex_desc* d, const void* x, const void* o
     const int rc = mex_geometry(d, nullptr, &g);
     if (rc) return rc;
     if (!off || !doff || (g.B > 0 && (!x || !y || !dy || !dx))) return SIMNETS_E_NULL;
-    const bool f64 = d->dtype == SIMNETS_F64;
-    if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !mex_use_gemm(g, f64, d->flags) && !mex_use_tiled(g, f64, d->flags)) return SIMNETS_E_UNSUPPORTED;
-    const bool acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
-    if (mex_use_gemm(g, f64, d->flags)) {
-        if (!ws || ws_bytes < mex_gemm_workspace_bytes(g, f64)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, doff, acc, ws, d->flags, as_stream(stream)));
-    }
-    if (mex_use_tiled(g, f64, d->flags)) {
-        if (!ws || ws_bytes < mex_workspace_bytes(g, f64, d->flags)) return SIMNETS_E_WORKSPACE;
-        return from_cuda(launch_mex_backward_tiled(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy,
-                                                   (float*)dx, (float*)doff, acc, ws, d->flags, as_stream(stream)));
-    }
-    const int r1 = from_cuda(launch_mex_dx_direct(g, f64, x, off, y, dy, dx, as_stream(stream)));
-    if (r1) return r1;
-    return from_cuda(launch_mex_doff_direct(g, f64, x, off, y, dy, doff, acc, as_stream(stream)));
+    return mex_gradients_in(g, d, x, off, y, dy, dx, doff, ws, ws_bytes, as_stream(stream));
 }
 
 int simnets_normalize_offsets_forward(int64_t rows, int32_t k, const void* off, void* out, void* stream) {

@@ -80,6 +80,8 @@ cudaError_t launch_sim_fwd_smallk(const SimGeo&, const float* x, const float* t,
                                   bool* extrema_done, int* flag, cudaStream_t);
 bool mex_use_tiled(const MexGeo&, bool f64, uint32_t flags);
 size_t mex_workspace_bytes(const MexGeo&, bool f64, uint32_t flags);
+// what the input gradient of overlapping blocks needs beside the workspace (`products` of the launchers below), 0 for other layers
+size_t mex_products_bytes(const MexGeo&, bool f64, uint32_t flags);
 // pooled: when given, the 2x2 sum pooling of y is produced as well (fused into the pair-tile kernel, a pooling launch behind the others)
 cudaError_t launch_mex_fwd_tiled(const MexGeo&, const float* x, const float* off, float* y, void* ws, uint32_t flags, cudaStream_t,
                                  float* pooled = nullptr);
@@ -146,11 +148,12 @@ cudaError_t launch_mex_bwd_short(const MexGeo&, bool inside, const float* x, con
 // mex_gemm.cu -- the factorised passes as small contractions: float64, small float32 layers, input gradients of overlapping blocks
 bool mex_use_gemm(const MexGeo&, bool f64, uint32_t flags);
 size_t mex_gemm_workspace_bytes(const MexGeo&, bool f64);
+size_t mex_gemm_products_bytes(const MexGeo&, bool f64);
 void* mex_gemm_maxima(const MexGeo&, bool f64, void* ws);
 cudaError_t launch_mex_fwd_gemm(const MexGeo&, bool f64, const void* x, const void* off, void* y, void* ws, uint32_t flags, cudaStream_t);
 // dx or doff may be null
 cudaError_t launch_mex_bwd_gemm(const MexGeo&, bool f64, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff,
-                                bool accumulate, void* ws, uint32_t flags, cudaStream_t);
+                                bool accumulate, void* ws, void* products, uint32_t flags, cudaStream_t);
 // number of multiprocessors of the current device (148 when no device answers)
 int device_sm_count();
 
@@ -160,9 +163,9 @@ cudaError_t launch_softmax_xent(int batch, int classes, float scale, const float
 // forward on the library's fixed device scratch; returns a status code of simnets_b200.h
 int launch_mex_fwd_static(const MexGeo&, const float* x, const float* off, float* y, uint32_t flags, cudaStream_t);
 cudaError_t launch_mex_dx_tiled(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* dx,
-                                void* ws, uint32_t flags, cudaStream_t, bool prepped = false, bool redo = true);
+                                void* ws, void* products, uint32_t flags, cudaStream_t, bool prepped = false, bool redo = true);
 cudaError_t launch_mex_backward_tiled(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* dx,
-                                      float* doff, bool accumulate, void* ws, uint32_t flags, cudaStream_t);
+                                      float* doff, bool accumulate, void* ws, void* products, uint32_t flags, cudaStream_t);
 cudaError_t launch_mex_doff_tiled(const MexGeo&, const float* x, const float* off, const float* y, const float* dy, float* doff,
                                   bool accumulate, void* ws, uint32_t flags, cudaStream_t, bool prepped = false, float* redo_dx = nullptr);
 }  // namespace simnets

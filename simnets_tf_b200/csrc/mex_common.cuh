@@ -21,7 +21,6 @@ struct MexWs {           // workspace carve-up, every part 256-byte aligned
     float* offn;         // [R][M][K] offsets minus their row's log-sum-exp, when the caller passes raw offsets
     float* lse;          // [R][M] that log-sum-exp
     float* dtmp;         // [R][M][K] offsets gradient with respect to the normalised rows
-    void* overlap;       // workspace of the input gradient of overlapping blocks (mex_gemm.cu)
     size_t bytes;
     size_t fwd_bytes;    // bytes the forward pass touches (everything before `part`)
 };
@@ -139,7 +138,6 @@ __host__ inline MexWs carve(const MexGeo& g_in, void* base) {
     w.offn = reinterpret_cast<float*>(take(sizeof(float) * (size_t)g.R * g.M * g.K));
     w.lse = reinterpret_cast<float*>(take(sizeof(float) * g.R * g.M));
     w.dtmp = reinterpret_cast<float*>(take(sizeof(float) * (size_t)g.R * g.M * g.K));
-    w.overlap = take(g.sc < g.bc || g.sh < g.bh || g.sw < g.bw ? mex_gemm_workspace_bytes(g, false) : 0);
     w.bytes = off;
     return w;
 }

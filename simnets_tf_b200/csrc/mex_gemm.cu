@@ -103,7 +103,8 @@ __host__ GemmWs<T> carve_gemm(const MexGeo& g, void* base) {
     w.eo = vals((size_t)g.R * g.M * g.K);
     w.offn = vals((size_t)g.R * g.M * g.K);
     w.mx = vals((size_t)g.B * g.N);
-    w.part = vals(std::max(part_elements(g, kFwd, sizeof(T)), std::max(part_elements(g, kDx, sizeof(T)), part_elements(g, kDoff, sizeof(T)))));
+    // (the products of overlapping blocks are scratch of the input gradient alone: mex_gemm_products_bytes)
+    w.part = vals(std::max(part_elements(g, kFwd, sizeof(T)), std::max(overlapping(g) ? 0 : part_elements(g, kDx, sizeof(T)), part_elements(g, kDoff, sizeof(T)))));
     w.bytes = off;
     return w;
 }
@@ -544,8 +545,10 @@ cudaError_t gemm_run(const MexGeo& g, const GemmWs<T>& w, const T* x, const T* o
 }
 
 template <typename T>
-cudaError_t gemm_dx(const MexGeo& g, const GemmWs<T>& w, const T* x, const T* off, const T* y, const T* dy, T* dx, cudaStream_t s) {
-    if (!overlapping(g)) {
+cudaError_t gemm_dx(const MexGeo& g, GemmWs<T> w, T* products, const T* x, const T* off, const T* y, const T* dy, T* dx, cudaStream_t s) {
+    if (overlapping(g)) {
+        w.part = products;
+    } else {
         const GemmPlan sp = plan_of(g, kDx, Numeric<T>::kQ);
         if (sp.splits == 1) {
             const bool covers = g.pc == 0 && g.ph == 0 && g.pw == 0 && g.sc == g.bc && g.sh == g.bh && g.sw == g.bw && g.C % g.bc == 0 && g.H % g.bh == 0 && g.W % g.bw == 0;
@@ -556,7 +559,7 @@ cudaError_t gemm_dx(const MexGeo& g, const GemmWs<T>& w, const T* x, const T* of
             return gemm_run<T, kDx>(g, w, x, off, w.mx, y, dy, dx, sp, 0, s);
         }
     }
-    // T goes through the workspace, as many samples at a time as it has room for
+    // T goes through scratch, as many samples at a time as that has room for
     const int step = overlapping(g) ? overlap_samples(g, sizeof(T)) : g.B;
     for (int n = 0; n < g.B; n += step) {
         const MexGeo q = with_samples(g, std::min(step, g.B - n));
@@ -589,14 +592,15 @@ cudaError_t gemm_forward(const MexGeo& g, const T* x, const T* off, T* y, void* 
 }
 
 template <typename T>
-cudaError_t gemm_backward(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* dx, T* doff, bool accumulate, void* ws, uint32_t flags, cudaStream_t s) {
+cudaError_t gemm_backward(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* dx, T* doff, bool accumulate, void* ws, void* products, uint32_t flags,
+                          cudaStream_t s) {
     const GemmWs<T> w = carve_gemm<T>(g, ws);
     // (a primed workspace holds what the forward pass prepared for the same input and offsets)
     cudaError_t e = flags & SIMNETS_FLAG_MEX_WORKSPACE_PRIMED ? cudaSuccess : gemm_prepare(g, w, x, off, flags & ~uint32_t(SIMNETS_FLAG_MEX_MAXIMA_GIVEN), s);
     if (e != cudaSuccess) return e;
     const T* rows = gemm_norm(flags) ? w.offn : off;
     if (dx != nullptr) {
-        e = gemm_dx(g, w, x, rows, y, dy, dx, s);
+        e = gemm_dx(g, w, static_cast<T*>(products), x, rows, y, dy, dx, s);
         if (e != cudaSuccess) return e;
     }
     if (doff == nullptr) return cudaSuccess;
@@ -632,15 +636,19 @@ bool mex_use_gemm(const MexGeo& g, bool f64, uint32_t flags) {
     return mex_small_layer(g);
 }
 size_t mex_gemm_workspace_bytes(const MexGeo& g, bool f64) { return f64 ? carve_gemm<double>(g, nullptr).bytes : carve_gemm<float>(g, nullptr).bytes; }
+size_t mex_gemm_products_bytes(const MexGeo& g, bool f64) {
+    const size_t size = f64 ? sizeof(double) : sizeof(float);
+    return overlapping(g) ? (part_elements(g, kDx, size) * size + 255) & ~size_t(255) : 0;
+}
 void* mex_gemm_maxima(const MexGeo& g, bool f64, void* ws) { return f64 ? static_cast<void*>(carve_gemm<double>(g, ws).mx) : carve_gemm<float>(g, ws).mx; }
 
 cudaError_t launch_mex_fwd_gemm(const MexGeo& g, bool f64, const void* x, const void* off, void* y, void* ws, uint32_t flags, cudaStream_t s) {
     return f64 ? gemm_forward<double>(g, (const double*)x, (const double*)off, (double*)y, ws, flags, s) : gemm_forward<float>(g, (const float*)x, (const float*)off, (float*)y, ws, flags, s);
 }
 cudaError_t launch_mex_bwd_gemm(const MexGeo& g, bool f64, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff, bool accumulate,
-                                void* ws, uint32_t flags, cudaStream_t s) {
-    return f64 ? gemm_backward<double>(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, (double*)doff, accumulate, ws, flags, s)
-               : gemm_backward<float>(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx, (float*)doff, accumulate, ws, flags, s);
+                                void* ws, void* products, uint32_t flags, cudaStream_t s) {
+    return f64 ? gemm_backward<double>(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, (double*)doff, accumulate, ws, products, flags, s)
+               : gemm_backward<float>(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx, (float*)doff, accumulate, ws, products, flags, s);
 }
 
 }  // namespace simnets

@@ -802,6 +802,14 @@ size_t mex_workspace_bytes(const MexGeo& g, bool f64, uint32_t flags) {
     return carve(g, nullptr).bytes;
 }
 
+size_t mex_products_bytes(const MexGeo& g, bool f64, uint32_t flags) {
+    if (blocks_disjoint(g)) return 0;
+    const bool gemm = mex_use_gemm(g, f64, flags);
+    if (!gemm && !mex_use_tiled(g, f64, flags)) return 0;
+    // (the other families hand the call to the small contractions, with a workspace of those inside `products`)
+    return mex_gemm_products_bytes(g, f64) + (gemm ? 0 : mex_gemm_workspace_bytes(g, false));
+}
+
 static cudaError_t mex_fwd_tiled_body(const MexGeo& g, const float* x, const float* off, float* y, void* ws, uint32_t flags, cudaStream_t s,
                                       float* pooled, bool* pooled_done);
 
@@ -912,10 +920,10 @@ int launch_mex_fwd_static(const MexGeo& g, const float* x, const float* off, flo
 }
 
 cudaError_t launch_mex_dx_tiled(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx,
-                                void* ws, uint32_t flags, cudaStream_t s, bool prepped, bool redo) {
+                                void* ws, void* products, uint32_t flags, cudaStream_t s, bool prepped, bool redo) {
     const MexWs w = carve(g, ws);
-    if (!blocks_disjoint(g))             // several positions add to one input value: gathered from their products, in a workspace part of its own
-        return launch_mex_bwd_gemm(g, false, x, off, y, dy, dx, nullptr, false, w.overlap,
+    if (!blocks_disjoint(g))             // several positions add to one input value: gathered from their products
+        return launch_mex_bwd_gemm(g, false, x, off, y, dy, dx, nullptr, false, products, static_cast<char*>(products) + mex_gemm_workspace_bytes(g, false),
                                    flags & ~uint32_t(SIMNETS_FLAG_MEX_WORKSPACE_PRIMED | SIMNETS_FLAG_MEX_MAXIMA_GIVEN), s);
     const bool small = smallm_shape(g) || use_smallk_kernels(g, flags);
     cudaError_t e = (prepped || forward_primes_workspace(g, flags)) ? cudaSuccess : run_prepasses(g, w, x, off, s, !small, pair_prep(g, flags), mex_norm(flags));
@@ -1029,7 +1037,7 @@ cudaError_t launch_mex_doff_tiled(const MexGeo& g, const float* x, const float* 
 
 // Both gradients of one layer in one call: the offsets prepass and the per-position maxima are computed once.
 cudaError_t launch_mex_backward_tiled(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx,
-                                      float* doff, bool accumulate, void* ws, uint32_t flags, cudaStream_t s) {
+                                      float* doff, bool accumulate, void* ws, void* products, uint32_t flags, cudaStream_t s) {
     const MexWs w = carve(g, ws);
     cudaError_t e = forward_primes_workspace(g, flags) ? cudaSuccess : run_prepasses(g, w, x, off, s, !use_smallk_kernels(g, flags), pair_prep(g, flags), mex_norm(flags));
     if (e != cudaSuccess) return e;
@@ -1054,7 +1062,7 @@ cudaError_t launch_mex_backward_tiled(const MexGeo& g, const float* x, const flo
         return finish_doff(g, w, mex_short_splits(g), x, off, y, dy, doff, accumulate, flags, s, dx);
     }
     const bool joint = blocks_disjoint(g);               // (overlapping blocks: the input gradient has its own redo)
-    e = launch_mex_dx_tiled(g, x, off, y, dy, dx, ws, flags, s, true, !joint);
+    e = launch_mex_dx_tiled(g, x, off, y, dy, dx, ws, products, flags, s, true, !joint);
     if (e != cudaSuccess) return e;
     return launch_mex_doff_tiled(g, x, off, y, dy, doff, accumulate, ws, flags, s, true, joint ? dx : nullptr);
 }

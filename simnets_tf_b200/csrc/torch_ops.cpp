@@ -125,7 +125,7 @@ struct MexPlan {
         check(simnets_mex_dims(&d, &g));
     }
     simnets_mex_desc with(uint32_t flags) const { simnets_mex_desc q = d; q.flags |= flags; return q; }
-    size_t workspace_bytes(uint32_t flags) const { const simnets_mex_desc q = with(flags); return simnets_mex_workspace_bytes(&q); }
+    size_t workspace_bytes(uint32_t flags) const { const simnets_mex_desc q = with(flags); return simnets_mex_forward_workspace_bytes(&q); }
     // room for the forward call and, if wanted, the gradient calls with a pooled dy
     size_t layer_bytes(uint32_t flags, bool pooled) const {
         return std::max<size_t>(256, std::max(workspace_bytes(flags), pooled ? workspace_bytes(flags | SIMNETS_FLAG_MEX_DY_POOLED2) : size_t(0)));
@@ -254,12 +254,13 @@ std::pair<Tensor, Tensor> mex_grads(const MexPlan& p, const Tensor& x_in, const 
     if (want_dx) dx = at::empty(x.sizes(), x.options());
     if (want_doff) doff = grad_target(off, out);
     const Tensor ws = mex_workspace(p, x, flags, primed);
+    Tensor products;            // (overlapping blocks: not part of a workspace that a layer keeps between its passes)
+    if (const size_t n = want_dx ? simnets_mex_products_bytes(&d) : 0) products = scratch(x, n);
     const char* op = want_dx && want_doff ? "mex_backward" : want_dx ? "mex_input_grad" : "mex_offsets_grad";
     const char* kind = want_dx && want_doff ? "bwd" : want_dx ? "dx" : "doff";
     Timed<MexPlan> timed(p, op, kind, s, pooled && want_dx && want_doff ? 3.0 * dy.numel() * dy.element_size() : 0.0);
-    if (want_dx && want_doff) check(simnets_mex_backward(&d, ptr(x), ptr(off), ptr(y), ptr(dy), ptr(dx), ptr(doff), ptr(ws), ws.numel(), s));
-    else if (want_dx) check(simnets_mex_input_grad(&d, ptr(x), ptr(off), ptr(y), ptr(dy), ptr(dx), ptr(ws), ws.numel(), s));
-    else if (want_doff) check(simnets_mex_offsets_grad(&d, ptr(x), ptr(off), ptr(y), ptr(dy), ptr(doff), ptr(ws), ws.numel(), s));
+    check(simnets_mex_gradients(&d, ptr(x), ptr(off), ptr(y), ptr(dy), want_dx ? ptr(dx) : nullptr, want_doff ? ptr(doff) : nullptr, ptr(ws), ws.numel(),
+                                products.defined() ? ptr(products) : nullptr, products.defined() ? products.numel() : 0, s));
     timed.done();
     return {dx, doff};
 }

@@ -65,8 +65,9 @@ protected:
                t.dim_size(3) == g.width_out;
     }
 
-    static Status Workspace(OpKernelContext* ctx, const simnets_mex_desc& d, Tensor* ws, size_t* bytes) {
-        *bytes = simnets_mex_workspace_bytes(&d);
+    // input_grad: with room for the products of overlapping blocks, which the other two ops do not need
+    static Status Workspace(OpKernelContext* ctx, const simnets_mex_desc& d, bool input_grad, Tensor* ws, size_t* bytes) {
+        *bytes = input_grad ? simnets_mex_workspace_bytes(&d) : simnets_mex_forward_workspace_bytes(&d);
         return ctx->allocate_temp(DT_UINT8, TensorShape({int64(*bytes ? *bytes : 1)}), ws);
     }
 };
@@ -86,7 +87,7 @@ public:
         Tensor* y = nullptr;
         OP_REQUIRES_OK(ctx, ctx->allocate_output(0, TensorShape({int64(d.batch), int64(g.channels_out_total), int64(g.height_out), int64(g.width_out)}), &y));
         Tensor ws; size_t n = 0;
-        OP_REQUIRES_OK(ctx, Workspace(ctx, d, &ws, &n));
+        OP_REQUIRES_OK(ctx, Workspace(ctx, d, false, &ws, &n));
         void* stream = (void*)ctx->template eigen_device<Eigen::GpuDevice>().stream();
         B200_REQUIRES_OK(ctx, simnets_mex_forward(&d, x.flat<T>().data(), offsets.flat<T>().data(), y->flat<T>().data(),
                                                   ws.flat<uint8>().data(), n, stream));
@@ -110,7 +111,7 @@ public:
         Tensor* dx = nullptr;
         OP_REQUIRES_OK(ctx, ctx->allocate_output(0, x.shape(), &dx));
         Tensor ws; size_t n = 0;
-        OP_REQUIRES_OK(ctx, Workspace(ctx, d, &ws, &n));
+        OP_REQUIRES_OK(ctx, Workspace(ctx, d, true, &ws, &n));
         void* stream = (void*)ctx->template eigen_device<Eigen::GpuDevice>().stream();
         B200_REQUIRES_OK(ctx, simnets_mex_input_grad(&d, x.flat<T>().data(), offsets.flat<T>().data(), y.flat<T>().data(), dy.flat<T>().data(),
                                                      dx->flat<T>().data(), ws.flat<uint8>().data(), n, stream));
@@ -134,7 +135,7 @@ public:
         Tensor* doff = nullptr;
         OP_REQUIRES_OK(ctx, ctx->allocate_output(0, offsets.shape(), &doff));
         Tensor ws; size_t n = 0;
-        OP_REQUIRES_OK(ctx, Workspace(ctx, d, &ws, &n));
+        OP_REQUIRES_OK(ctx, Workspace(ctx, d, false, &ws, &n));
         void* stream = (void*)ctx->template eigen_device<Eigen::GpuDevice>().stream();
         B200_REQUIRES_OK(ctx, simnets_mex_offsets_grad(&d, x.flat<T>().data(), offsets.flat<T>().data(), y.flat<T>().data(), dy.flat<T>().data(),
                                                        doff->flat<T>().data(), ws.flat<uint8>().data(), n, stream));

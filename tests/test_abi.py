@@ -105,6 +105,23 @@ def test_mex_validation(cuda_lib):
         abi.make_mex_desc((1, 4, 8, 8), 3, blocks=(1, 1, 1), epsilon=float("nan"))
 
 
+def test_products_of_overlapping_blocks_are_not_part_of_a_kept_workspace(cuda_lib):
+    """The input gradient of overlapping blocks has a quarter of a gigabyte of products; forward calls and workspaces that a
+    layer keeps until its backward pass must not."""
+    def sizes(block, dtype, flags=0, batch=12):
+        d = abi.make_mex_desc((batch, 16, 128, 128), 4, blocks=(16, block, block), strides=(16, 1, 1), padding=(0, block // 2, block // 2),
+                              use_unshared_regions=False, dtype=dtype, flags=flags)
+        return [f(C.byref(d)) for f in (cuda_lib.simnets_mex_workspace_bytes, cuda_lib.simnets_mex_forward_workspace_bytes, cuda_lib.simnets_mex_products_bytes)]
+
+    for dtype in (abi.F32, abi.F64):
+        for flags in (0, abi.FLAG_MEX_NO_SMALL_TILES):
+            total, kept, products = sizes(5, dtype, flags)
+            assert total >= kept + products and products > 100 << 20 and kept < 16 << 20 and kept % 256 == 0
+            total, kept, products = sizes(1, dtype, flags)
+            assert total == kept and products == 0
+    assert sizes(5, abi.F32, abi.FLAG_MEX_EXACT)[1:] == [256, 0]
+
+
 def test_legacy_region_count_helper():
     """get_mex_offsets_nregions keeps the reference's symbol and argument order (src/kernels/mex_dims_helper.cpp:8-44)."""
     assert _mex_dims_helper([32, 16, 16], 64, [32, 1, 1], [0, 0, 0], [32, 1, 1], unshared_offset_region=[2]) == 4

@@ -1,5 +1,6 @@
 """The small-contraction MEX kernels (float64 layers, small float32 layers, input gradients of overlapping blocks) at the
 edges of their tiles, and the tensor-core kernels at the small sizes that would otherwise run on them."""
+import ctypes as C
 import importlib
 
 import numpy as np
@@ -52,6 +53,62 @@ def test_overlapping_input_gradient_in_parts(flags):
     for n in (0, 9, 10, 11):
         one = mex_ops.mex_input_grad(x[n:n + 1], off, y[n:n + 1], dy[n:n + 1], 4, flags=flags, **attrs)
         assert torch.allclose(dx[n:n + 1], one, rtol=1e-5, atol=1e-5 * float(one.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
+def test_products_of_overlapping_blocks_live_for_one_call(dtype):
+    """Neither a forward call nor the workspace that a differentiated layer keeps has room for the products (189 or 252 MB here)."""
+    x, off = torch.randn(12, 16, 128, 128, device="cuda", dtype=dtype), torch.randn(1, 4, 16, 3, 5, device="cuda", dtype=dtype, requires_grad=True)
+    attrs = dict(blocks=[16, 3, 5], strides=[16, 1, 1], padding=[0, 1, 2], softmax_mode=True, use_unshared_regions=False, shared_offset_region=[-1])
+    out = 4 * 12 * 128 * 128 * x.element_size()
+    torch.cuda.synchronize()
+    for x in (x, x.requires_grad_()):
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        y = mex_ops.mex(x, off, 4, **attrs)
+        assert torch.cuda.max_memory_allocated() - before < out + (16 << 20)
+    torch.autograd.grad(y.sum(), (x, off))
+    assert torch.cuda.max_memory_allocated() - before > 170 << 20
+
+
+@pytest.mark.parametrize("dtype", [abi.F32, abi.F64], ids=["f32", "f64"])
+@pytest.mark.parametrize("flags", [0, abi.FLAG_MEX_NO_SMALL_TILES], ids=["small", "large"])
+@pytest.mark.parametrize("c", [c for c in EDGES if c["name"].startswith("overlap")], ids=lambda c: c["name"])
+def test_scratch_of_exactly_the_stated_sizes(cuda_lib, c, flags, dtype):
+    """Workspace and products fenced on both sides: nothing outside is written, and results do not depend on what was inside."""
+    def fenced(n, fill):
+        t = torch.full((n + 512,), fill, dtype=torch.uint8, device="cuda")
+        t[:256], t[256 + n:] = 0x5A, 0x5A
+        return t, t.data_ptr() + 256
+
+    np_t, t_t = (np.float32, torch.float32) if dtype == abi.F32 else (np.float64, torch.float64)
+    d = cases.mex_desc(c, dtype=dtype)
+    d.flags |= flags
+    g = abi.MexGeometry()
+    assert cuda_lib.simnets_mex_dims(C.byref(d), C.byref(g)) == 0
+    oshape = (c["shape"][0], g.channels_out_total, g.height_out, g.width_out)
+    x, off, dy = (gpu_util.dev(a, t_t) for a in cases.mex_inputs(c, (g.num_regions, g.M, g.block_c, g.block_h, g.block_w), oshape, np_t))
+    kept, products = cuda_lib.simnets_mex_forward_workspace_bytes(C.byref(d)), cuda_lib.simnets_mex_products_bytes(C.byref(d))
+    assert products > 0
+    stream, got = torch.cuda.current_stream().cuda_stream, []
+    for fill in (0, 0xFF):
+        (ws, wp), (pr, pp) = fenced(kept, fill), fenced(products, fill)
+        y, dx, doff = torch.empty(oshape, dtype=t_t, device="cuda"), torch.empty_like(x), torch.empty_like(off)
+        assert cuda_lib.simnets_mex_forward(C.byref(d), x.data_ptr(), off.data_ptr(), y.data_ptr(), wp, kept, stream) == 0
+        args = [C.byref(d), x.data_ptr(), off.data_ptr(), y.data_ptr(), dy.data_ptr(), dx.data_ptr(), doff.data_ptr(), wp]
+        assert cuda_lib.simnets_mex_gradients(*args, kept, pp, products - 256, stream) == abi.E_WORKSPACE
+        assert cuda_lib.simnets_mex_gradients(*args, 256, pp, products, stream) == abi.E_WORKSPACE
+        assert cuda_lib.simnets_mex_gradients(*args, kept, pp, products, stream) == 0
+        for t, n in ((ws, kept), (pr, products)):
+            assert bool((t[:256] == 0x5A).all()) and bool((t[256 + n:] == 0x5A).all())
+        got.append((y, dx, doff))
+        one = torch.empty(kept + products, dtype=torch.uint8, device="cuda")
+        dx2, doff2 = torch.empty_like(dx), torch.empty_like(doff)
+        args = [C.byref(d), x.data_ptr(), off.data_ptr(), y.data_ptr(), dy.data_ptr(), dx2.data_ptr(), doff2.data_ptr(), one.data_ptr()]
+        assert cuda_lib.simnets_mex_backward(*args, kept + products, stream) == 0
+        got.append((y, dx2, doff2))
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
