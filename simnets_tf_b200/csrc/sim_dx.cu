@@ -12,10 +12,12 @@
 // reduction index by M for each staged value had taken as many instructions as the terms themselves (256 x 64 x 32 x 32 input,
 // 256 templates of 3x3: 10.2 ms).
 //
-// NaN pixels give 0 in the ignore_nan_input modes, and so does a pixel that no patch covers in every mode.
-// Known deviation: a pixel holding +-inf whose coverage is partial (taps cut off by padding) yields NaN where the reference
-// yields +-inf, because a cut-off tap contributes 0 * (t - inf).
+// NaN pixels give 0 in the ignore_nan_input modes, and so does a pixel that no patch covers in every mode.  A tap that the
+// padding cuts off, or a step past the last one, contributes 0 * (t - x), which is NaN for an infinite x (or an infinite
+// parameter): a sum that came out NaN over a number is added up again over the taps that are there (dx_redo; the test costs 1.5 %
+// where 64 rows of channels share a tile: 128 x 64 x 32 x 32 input, 128 templates of 3x3, 1231 -> 1251 us).
 #include "kernels.cuh"
+#include "sim_exact.cuh"
 #include "tile.cuh"
 
 namespace simnets {
@@ -70,6 +72,12 @@ struct DxPixel {
     }
 };
 
+// The value at dx[at] again, term by term, if it is NaN and x[at] is not.
+__device__ __noinline__ void dx_redo(const SimGeo& g, const float* __restrict__ x, const float* __restrict__ tm, const float* __restrict__ wt,
+                                     const float* __restrict__ dy, float* dx, long long at) {
+    if (is_nan(dx[at]) && !is_nan(x[at])) dx[at] = sim_exact_dx(g, x, tm, wt, dy, at);
+}
+
 // (t, s w)[tap][m][Cp], channel-contiguous, for the tile kernel
 __global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, const float* __restrict__ tm, const float* __restrict__ wt, float* __restrict__ dxp) {
     stream_order();
@@ -94,7 +102,8 @@ template <int TM> struct DxCfg {
 
 template <int TM, int MODE>
 __global__ void __launch_bounds__(DxCfg<TM>::Cfg::THREADS, DxCfg<TM>::Cfg::THREADS == 256 ? (TM == 128 ? 1 : 2) : 3)
-sim_dx_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ dxp, const float* __restrict__ dy, float* __restrict__ dx) {
+sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, const float* __restrict__ dxp, const float* __restrict__ tm, const float* __restrict__ wt,
+             const float* __restrict__ dy, float* __restrict__ dx) {
     stream_order();
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     constexpr bool SKIP_NAN = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
@@ -196,6 +205,7 @@ sim_dx_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ dx
     };
     tile_mainloop<Cfg, false, false>(smem, (Q + Cfg::KC - 1) / Cfg::KC, t, fetchA, fetchB, commitA, commitB, comb);
 
+    bool redo = false;
 #pragma unroll
     for (int c_ = 0; c_ < Cfg::RN; ++c_) {
         const long long cb = col_base[t.col(c_)];
@@ -208,9 +218,17 @@ sim_dx_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ dx
             float v = (c_ & 1) ? acc[r_][c_ >> 1].y : acc[r_][c_ >> 1].x;
             const float xv = (c_ & 1) ? xx[r_][c_ >> 1].y : xx[r_][c_ >> 1].x;
             if (!covered || (SKIP_NAN && xv != xv)) v = 0.f;
+            redo |= is_nan(v);
             dx[cb + (size_t)c * chw] = v;
         }
     }
+    if (redo)
+#pragma unroll 1
+        for (int i = 0; i < Cfg::RM * Cfg::RN; ++i) {
+            const int c = i0 + t.row(i / Cfg::RN);
+            const long long cb = col_base[t.col(i % Cfg::RN)];
+            if (c < g.C && cb >= 0) dx_redo(g, x, tm, wt, dy, dx, cb + (long long)(c * chw));
+        }
 }
 
 // Few channels (an image's): a thread owns PP pixels with all CT >= C channels of each, so that a dy value is read once per
@@ -219,7 +237,7 @@ sim_dx_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ dx
 constexpr int kNarrowThreads = 128, kNarrowQ = 64;
 
 template <int CT, int PP, int MODE>
-__global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(SimGeo g, const float* __restrict__ x, const float* __restrict__ tm,
+__global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_constant__ SimGeo g, const float* __restrict__ x, const float* __restrict__ tm,
                                                                 const float* __restrict__ wt, const float* __restrict__ dy, float* __restrict__ dx) {
     stream_order();
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
@@ -277,9 +295,17 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(SimGeo g, const 
     for (int p = 0; p < PP; ++p) {
         if (px[p].base < 0) continue;
         const bool covered = px[p].covered(g, ph);
+        bool redo = false;
 #pragma unroll
         for (int c = 0; c < CT; ++c)
-            if (c < g.C) dx[px[p].base + c * chw] = (!covered || (SKIP_NAN && xv[p][c] != xv[p][c])) ? 0.f : acc[p][c];
+            if (c < g.C) {
+                const float v = (!covered || (SKIP_NAN && is_nan(xv[p][c]))) ? 0.f : acc[p][c];
+                redo |= is_nan(v);
+                dx[px[p].base + c * chw] = v;
+            }
+        if (redo)
+#pragma unroll 1
+            for (int c = 0; c < g.C; ++c) dx_redo(g, x, tm, wt, dy, dx, px[p].base + (long long)(c * chw));
     }
 }
 
@@ -330,7 +356,7 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
     const long long blocks = ((pixels + tn - 1) / tn) * ((g.C + tm - 1) / tm);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const dim3 grid{unsigned(blocks), unsigned(phases)};
-#define DX(TM, MODE) in_stream_order(sim_dx_tiled<TM, MODE>, grid, DxCfg<TM>::Cfg::THREADS, 0, s)(g, x, dxp, dy, dx)
+#define DX(TM, MODE) in_stream_order(sim_dx_tiled<TM, MODE>, grid, DxCfg<TM>::Cfg::THREADS, 0, s)(g, x, dxp, t, w, dy, dx)
 #define DX_16(MODE) DX(16, MODE)
 #define DX_32(MODE) DX(32, MODE)
 #define DX_64(MODE) DX(64, MODE)

@@ -1,5 +1,6 @@
 """The float32 Similarity kernels where they can go wrong: tap, template and channel counts around the tile sizes, strides whose
 phases have different taps and pixels, pixels that no patch covers, inputs small and large enough for every dispatch."""
+import numpy as np
 import pytest
 
 import cases
@@ -37,3 +38,22 @@ def test_tile_edges(port, i, mode):
 @pytest.mark.parametrize("shape,M,blocks", [((160, 1, 28, 28), 40, (2, 2)), ((96, 3, 30, 33), 10, (3, 3))], ids=["resident_32", "many_pixels"])
 def test_enough_positions_for_the_streaming_kernels(port, shape, M, blocks, mode):
     gpu_util.check_similarity(port, cases.sim_case("many", shape, M, blocks=blocks, strides=(1, 1), padding=(1, 1), seed=720, **mode), f64_tiebreak=True, tol=2e-5)
+
+
+@pytest.mark.parametrize("mode", MODES, ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("i", range(len(SHAPES)))
+def test_infinite_pixels_meet_only_the_taps_that_are_there(port, i, mode):
+    """With dy >= 0 an infinite pixel has an infinite gradient; a tap cut off by the padding, or a step past the last one, must
+    not turn it into NaN."""
+    shape, M, blocks, strides, padding = SHAPES[i]
+    c = cases.sim_case("inf%d" % i, shape, M, blocks=blocks, strides=strides, padding=padding, oob=0.3, seed=740 + i, **mode)
+    d = cases.sim_desc(c)
+    x, t, w, dy = cases.sim_inputs(c, port.sim_out_shape(d))
+    rng = np.random.default_rng(i)
+    x[rng.random(x.shape) < 0.2] = np.inf
+    x[rng.random(x.shape) < 0.1] = -np.inf
+    dy = np.abs(dy)
+    dx = gpu_util.sim_ops.similarity_input_grad(*(gpu_util.dev(a) for a in (x, t, w, dy)), **cases.sim_attrs(c)).cpu().numpy()
+    ref = port.similarity_input_grad(d, x, t, w, dy)
+    assert np.isinf(ref).any() or mode["fn"] == "L1"
+    cases.assert_parity(dx, ref, what=c["name"])
