@@ -70,6 +70,8 @@ __global__ void __launch_bounds__(kMixThreads) mixture_responsibilities(long lon
             }
             continue;
         }
+        // (the running maximum may still be -inf, components so far away that their distance overflowed: exp(-inf - 0) adds nothing)
+        const auto above = [](float top) { return top > -CUDART_INF_F ? top : 0.f; };
         int c = 0;
         for (; c + 8 <= k; c += 8) {
             float v[8], top = hi;
@@ -77,15 +79,16 @@ __global__ void __launch_bounds__(kMixThreads) mixture_responsibilities(long lon
             for (int u = 0; u < 8; ++u) v[u] = 0.5f * (p[(long long)(c + u) * N] - ld[c + u]);
 #pragma unroll
             for (int u = 0; u < 8; ++u) top = fmaxf(top, v[u]);
+            const float ref = above(top);
             float add = 0.f;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) add += expf(v[u] - top);
-            sum = sum * expf(hi - top) + add;
+            for (int u = 0; u < 8; ++u) add += expf(v[u] - ref);
+            sum = sum * expf(hi - ref) + add;
             hi = top;
         }
         for (; c < k; ++c) {
-            const float v = 0.5f * (p[(long long)c * N] - ld[c]), top = fmaxf(hi, v);
-            sum = sum * expf(hi - top) + expf(v - top);
+            const float v = 0.5f * (p[(long long)c * N] - ld[c]), top = fmaxf(hi, v), ref = above(top);
+            sum = sum * expf(hi - ref) + expf(v - ref);
             hi = top;
         }
         const float inv = 1.f / sum;

@@ -140,3 +140,18 @@ def test_sequence_of_layers_and_channels_last():
     _close(b.templates.detach(), centres, 2e-4, "second layer's templates")
     with pytest.raises(ValueError, match="defined for Similarity layers"):
         layers.perform_unsupervised_init([a, b], layers=[torch.nn.Identity()], data=data, batch_size=4)
+
+
+def test_components_at_an_infinite_distance_claim_nothing():
+    """More components than a thread keeps in registers, the first eight of them so far away that their distances overflow."""
+    x = torch.rand(6, 3, 11, 12, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda")
+    near = un.DiagonalGMM([2, 2], [1, 1], 62)
+    near.init(x)
+    far = un.DiagonalGMM([2, 2], [1, 1], 70)
+    far.init(x)
+    far.means = torch.cat([torch.full_like(near.means[:8], 1e20), near.means]).contiguous()
+    far.covs = torch.cat([torch.ones_like(near.covs[:8]), near.covs]).contiguous()
+    near.update(x)
+    far.update(x)
+    assert bool((far.means[:8] == 1e20).all()) and torch.allclose(far.covs[:8], torch.full_like(far.covs[:8], near.min_var))
+    assert torch.allclose(far.means[8:], near.means, rtol=1e-5, atol=1e-6) and torch.allclose(far.covs[8:], near.covs, rtol=1e-4, atol=1e-6)
