@@ -9,10 +9,14 @@ import torch
 
 import cases
 import gpu_util
-from simnets_tf_b200 import abi
+from simnets_tf_b200 import _torch_glue, abi
 mex_ops = importlib.import_module("simnets_tf_b200.ops.mex")
 
 pytestmark = pytest.mark.gpu
+
+# Small layers run on the small-contraction kernels; what a test names is then only reached with the flag that keeps them on the
+# kernels of large layers.
+EITHER_FAMILY = pytest.mark.parametrize("family", [0, abi.FLAG_MEX_NO_SMALL_TILES], ids=["as_sized", "large_layer_kernels"])
 
 
 @pytest.mark.parametrize("c", cases.MEX_SMALL, ids=lambda c: c["name"])
@@ -66,13 +70,14 @@ def test_head_shapes(port, c):
     gpu_util.check_mex(port, c, f64_tiebreak=True)
 
 
+@EITHER_FAMILY
 @pytest.mark.parametrize("c", cases.MEX_HEAD + [c for c in cases.MEX_CONFIGS if c["name"] == "cfg5_head_sub"], ids=lambda c: c["name"])
-def test_head_gradients_from_the_forward_pass_workspace(port, c):
+def test_head_gradients_from_the_forward_pass_workspace(port, c, family):
     """The head's forward kernel leaves the per-position maxima in the workspace; primed gradients must not change."""
     d = cases.mex_desc(c)
     x, off, dy = cases.mex_inputs(c, port.mex_offsets_shape(d), port.mex_out_shape(d))
     xd, od, dyd = (gpu_util.dev(a) for a in (x, off, dy))
-    attrs = cases.mex_attrs(c)
+    attrs = dict(cases.mex_attrs(c), flags=family)
     ws = mex_ops.mex_layer_workspace(xd, c["M"], **attrs)
     yd = mex_ops.mex_forward(xd, od, c["M"], workspace=ws, **attrs)
     ry = port.mex_forward(d, x, off)
@@ -88,7 +93,8 @@ def test_head_gradients_from_the_forward_pass_workspace(port, c):
                         port.mex_offsets_grad(d, x, off, ry, dy), tol=2e-5, what="doff alone")
 
 
-def test_pair_tiles_need_8_byte_alignment(port):
+@EITHER_FAMILY
+def test_pair_tiles_need_8_byte_alignment(port, family):
     """Tensors that start on an odd float cannot be read as pixel pairs: the library takes the one-region kernels."""
     c = cases.MEX_PAIR[0]
     d = cases.mex_desc(c)
@@ -103,7 +109,7 @@ def test_pair_tiles_need_8_byte_alignment(port):
         return v
     xd, dyd, ryd = odd(x), odd(dy), odd(ry)
     od = gpu_util.dev(off)
-    attrs = cases.mex_attrs(c)
+    attrs = dict(cases.mex_attrs(c), flags=family)
     cases.assert_parity(mex_ops.mex_forward(xd, od, c["M"], **attrs).cpu().numpy(), ry, what="y")
     dx, doff = mex_ops.mex_backward(xd, od, ryd, dyd, c["M"], **attrs)
     cases.assert_parity(dx.cpu().numpy(), port.mex_input_grad(d, x, off, ry, dy), what="dx")
@@ -170,29 +176,31 @@ def test_autograd_wiring_matches_grad_ops(port):
     cases.assert_parity(od.grad.cpu().numpy(), port.mex_offsets_grad(d, x, off, ry, dy), tol=2e-5, what="doff")
 
 
+@EITHER_FAMILY
 @pytest.mark.parametrize("name", ["blocks_bug", "eps_half", "tiled_regions", "head_disjoint", "wide_M_K", "eps_pinf"])
-def test_fused_backward_equals_the_two_gradient_ops(port, name):
+def test_fused_backward_equals_the_two_gradient_ops(port, name, family):
     """simnets_mex_backward shares the prepasses between the two gradients; results must not change."""
     c = next(c for c in cases.MEX_SMALL if c["name"] == name)
     d = cases.mex_desc(c)
     x, off, dy = cases.mex_inputs(c, port.mex_offsets_shape(d), port.mex_out_shape(d))
     xd, od, dyd = (gpu_util.dev(a) for a in (x, off, dy))
     yd = gpu_util.dev(port.mex_forward(d, x, off))
-    attrs = cases.mex_attrs(c)
+    attrs = dict(cases.mex_attrs(c), flags=family)
     dx, doff = mex_ops.mex_backward(xd, od, yd, dyd, c["M"], **attrs)
     assert torch.equal(dx, mex_ops.mex_input_grad(xd, od, yd, dyd, c["M"], **attrs))
     assert torch.equal(doff, mex_ops.mex_offsets_grad(xd, od, yd, dyd, c["M"], **attrs))
 
 
+@EITHER_FAMILY
 @pytest.mark.parametrize("c", cases.MEX_SMALL + cases.MEX_CONFIGS, ids=lambda c: c["name"])
-def test_gradients_from_the_forward_pass_workspace(port, c):
+def test_gradients_from_the_forward_pass_workspace(port, c, family):
     """SIMNETS_FLAG_MEX_WORKSPACE_PRIMED: gradients that reuse what the forward pass left in the layer's own
     workspace are the gradients computed from scratch (full and pooled dy, all three entry points)."""
     d = cases.mex_desc(c)
     oshape = port.mex_out_shape(d)
     x, off, dy = cases.mex_inputs(c, port.mex_offsets_shape(d), oshape)
     xd, od, dyd = (gpu_util.dev(a) for a in (x, off, dy))
-    attrs, fl = cases.mex_attrs(c), c["flags"]
+    attrs, fl = cases.mex_attrs(c), c["flags"] | family
     pooled_ok = oshape[0] > 0 and oshape[2] % 2 == 0 and oshape[3] % 2 == 0
     for pooled in ([False, True] if pooled_ok else [False]):
         g = dyd[:, :, ::2, ::2].contiguous() if pooled else dyd
@@ -274,8 +282,10 @@ def test_normalize_offsets_kernels(shape):
         assert torch.allclose(a.grad.double(), b.grad, rtol=1e-5, atol=1e-6)
 
 
-def test_mex_sum_pool2_equals_mex_then_pooling():
+@EITHER_FAMILY
+def test_mex_sum_pool2_equals_mex_then_pooling(monkeypatch, family):
     """The fused MEX + 2x2 sum pooling op: same forward bits, same gradients as the two ops chained."""
+    monkeypatch.setattr(_torch_glue, "DEFAULT_FLAGS", family)
     torch.manual_seed(3)
     x = torch.randn(6, 64, 8, 8, device="cuda")
     off = (0.3 * torch.randn(4, 96, 64, 1, 1, device="cuda"))
@@ -312,7 +322,7 @@ def test_rows_past_the_last_position_do_not_leak(port):
     x64, o64, dy64 = (a.astype(np.float64) for a in (x, off, dy))
     y64 = port.mex_forward(d64, x64, o64)
     dx64, doff64 = port.mex_input_grad(d64, x64, o64, y64, dy64), port.mex_offsets_grad(d64, x64, o64, y64, dy64)
-    for flags in (0, abi.FLAG_MEX_TC_ONE_TILE):
+    for flags in (0, abi.FLAG_MEX_NO_SMALL_TILES, abi.FLAG_MEX_TC_ONE_TILE):
         dx, doff = mex_ops.mex_backward(xd, od, ryd, dyd, c["M"], flags=flags, **attrs)
         cases.assert_parity(dx.cpu().numpy(), port.mex_input_grad(d, x, off, ry, dy), dx64, tol=2e-5, what="dx")
         cases.assert_parity(doff.cpu().numpy(), port.mex_offsets_grad(d, x, off, ry, dy), doff64, tol=2e-5, what="doff")
@@ -394,7 +404,7 @@ def test_forward_with_pooled_output(port, c):
         with pytest.raises(RuntimeError):
             mex_ops.mex_forward_pool2(gpu_util.dev(x), gpu_util.dev(off), c["M"], **cases.mex_attrs(c))
         return
-    for flags in (0, abi.FLAG_MEX_NO_PAIR_TILES):
+    for flags in (0, abi.FLAG_MEX_NO_SMALL_TILES, abi.FLAG_MEX_NO_PAIR_TILES):
         y, yp = mex_ops.mex_forward_pool2(gpu_util.dev(x), gpu_util.dev(off), c["M"], flags=c["flags"] | flags, **cases.mex_attrs(c))
         cases.assert_parity(y.cpu().numpy(), ry, what="y")
         cases.assert_parity(yp.cpu().numpy(), _pool2(ry).astype(np.float32), tol=1e-5, what="pooled y (flags %d)" % flags)
@@ -412,7 +422,8 @@ def test_pooled_output_on_the_recomputing_routes(port, cuda_lib):
     status = (C.c_int32 * 2)(7, 7)
     wide = off.copy()
     wide[0, 0, 0] = 300.0
-    for o, flags, want in ((off, abi.FLAG_MEX_TEST_EXPIRE_WAIT, (0, 1)), (wide, 0, (1, 0)), (off, 0, (0, 0))):
+    for o, flags, want in ((off, abi.FLAG_MEX_TEST_EXPIRE_WAIT, (0, 1)), (wide, 0, (1, 0)), (wide, abi.FLAG_MEX_NO_SMALL_TILES, (1, 0)),
+                           (off, 0, (0, 0)), (off, abi.FLAG_MEX_NO_SMALL_TILES, (0, 0))):
         ry = port.mex_forward(d, x, o)
         xd, od = gpu_util.dev(x), gpu_util.dev(o)
         ws = mex_ops.mex_layer_workspace(xd, c["M"], flags=flags, **attrs)
@@ -433,11 +444,15 @@ def _normalise(off):
     return (flat - lse).reshape(o.shape), np.exp(flat - lse)          # normalised offsets, softmax of every row
 
 
-_RAW = cases.MEX_PAIR[::2] + cases.MEX_HEAD[::2] + [c for c in cases.MEX_CONFIGS if not c["name"].startswith("cfg4")] + cases.MEX_SMALL[::5]
+# (row lengths at the edges of the reduction's register blocks: 128 taps per block, 1, 2, 4 or 8 of them)
+_ROWS = [cases.mex_case("row_%d" % k, (2, k, 4, 4), 50 + i, (k, 1, 1), (k, 1, 1), softmax=True, unshared_region=(2,) if i % 2 else (1,), seed=420 + i)
+         for i, k in enumerate((128, 129, 256, 257, 512, 513, 1024))]
+_RAW = cases.MEX_PAIR[::2] + cases.MEX_HEAD[::2] + [c for c in cases.MEX_CONFIGS if not c["name"].startswith("cfg4")] + cases.MEX_SMALL[::5] + _ROWS
 
 
+@EITHER_FAMILY
 @pytest.mark.parametrize("c", _RAW, ids=lambda c: c["name"])
-def test_raw_offsets_are_normalised_inside_the_op(port, c):
+def test_raw_offsets_are_normalised_inside_the_op(port, c, family):
     """Forward and input gradient as with offsets - logsumexp(row) in front of the op; the offsets gradient comes back with
     respect to the raw values: d - softmax(row) * sum(d) of the oracle's gradient d."""
     d = cases.mex_desc(c)
@@ -451,8 +466,11 @@ def test_raw_offsets_are_normalised_inside_the_op(port, c):
     rdoff = (flat - soft * flat.sum(axis=1, keepdims=True)).reshape(off.shape)
     xd, od, dyd, ryd = (gpu_util.dev(a) for a in (x, off, dy, ry))
     attrs = cases.mex_attrs(c)
-    fl = c["flags"] | abi.FLAG_MEX_NORMALIZED_OFFSETS
-    cases.assert_parity(mex_ops.mex_forward(xd, od, c["M"], flags=fl, **attrs).cpu().numpy(), ry, what="y")
+    fl = c["flags"] | abi.FLAG_MEX_NORMALIZED_OFFSETS | family
+    # (the tensor cores truncate what they add: up to 2^-23 of the sum for each of three additions per eight taps, and the output is
+    # its logarithm)
+    tol = max(1e-5, 3 * (off[0, 0].size / 8) * 2.0 ** -23 / (abs(c["eps"]) * float(np.abs(ry).max()))) if c in _ROWS else 1e-5
+    cases.assert_parity(mex_ops.mex_forward(xd, od, c["M"], flags=fl, **attrs).cpu().numpy(), ry, tol=tol, what="y")
     cases.assert_parity(mex_ops.mex_input_grad(xd, od, ryd, dyd, c["M"], flags=fl, **attrs).cpu().numpy(), rdx, tol=2e-5, what="dx")
     cases.assert_parity(mex_ops.mex_offsets_grad(xd, od, ryd, dyd, c["M"], flags=fl, **attrs).cpu().numpy(), rdoff.astype(np.float32), tol=3e-5,
                         what="doff (raw)")
@@ -465,7 +483,8 @@ def test_raw_offsets_are_normalised_inside_the_op(port, c):
     cases.assert_parity(acc.cpu().numpy() - 2.0, rdoff.astype(np.float32), tol=1e-4, what="doff accumulated")
 
 
-def test_raw_offsets_on_the_exact_route(port):
+@EITHER_FAMILY
+def test_raw_offsets_on_the_exact_route(port, family):
     """A row spread that makes the factorisation unsafe: the exact kernels work on the normalised rows kept in the workspace."""
     c = next(c for c in cases.MEX_CONFIGS if c["name"] == "cfg5_mex1_sub")
     d = cases.mex_desc(c)
@@ -480,7 +499,7 @@ def test_raw_offsets_on_the_exact_route(port):
     rdoff = (flat - soft * flat.sum(axis=1, keepdims=True)).reshape(off.shape)
     xd, od, dyd, ryd = (gpu_util.dev(a) for a in (x, off, dy, ry))
     attrs = cases.mex_attrs(c)
-    fl = abi.FLAG_MEX_NORMALIZED_OFFSETS
+    fl = abi.FLAG_MEX_NORMALIZED_OFFSETS | family
     cases.assert_parity(mex_ops.mex_forward(xd, od, c["M"], flags=fl, **attrs).cpu().numpy(), ry, what="y")
     dx, doff = mex_ops.mex_backward(xd, od, ryd, dyd, c["M"], flags=fl, **attrs)
     cases.assert_parity(dx.cpu().numpy(), port.mex_input_grad(d, x, offn, ry, dy), tol=2e-5, what="dx")
@@ -489,8 +508,10 @@ def test_raw_offsets_on_the_exact_route(port):
         mex_ops.mex_forward(xd, od, c["M"], flags=fl | abi.FLAG_FORCE_DIRECT, **attrs)
 
 
-def test_layer_with_fused_and_separate_normalisation():
+@EITHER_FAMILY
+def test_layer_with_fused_and_separate_normalisation(monkeypatch, family):
     from simnets_tf_b200 import keras as layers
+    monkeypatch.setattr(_torch_glue, "DEFAULT_FLAGS", family)
     torch.manual_seed(0)
     x = torch.randn(4, 64, 8, 8, device="cuda")
     kw = dict(num_instances=96, blocks=[64, 1, 1], strides=[64, 1, 1], softmax_mode=True, unshared_offset_region=[2], normalize_offsets=True)
@@ -509,9 +530,10 @@ def test_layer_with_fused_and_separate_normalisation():
     assert torch.allclose(a.offsets.grad, b.offsets.grad, rtol=1e-4, atol=3e-5 * float(b.offsets.grad.abs().max()))
 
 
+@EITHER_FAMILY
 @pytest.mark.parametrize("shape,M", [((6, 32, 16, 16), 64), ((4, 64, 32, 32), 128), ((5, 40, 8, 16), 70)], ids=["K32", "cfg5_mex1", "ragged"])
 @pytest.mark.parametrize("norm", [0, abi.FLAG_MEX_NORMALIZED_OFFSETS], ids=["plain", "raw_offsets"])
-def test_results_do_not_depend_on_what_the_workspace_held(shape, M, norm):
+def test_results_do_not_depend_on_what_the_workspace_held(shape, M, norm, family):
     """A forward call and the gradient calls that reuse its workspace (pooled dy) read nothing they did not write: a
     workspace poisoned with NaN bytes or with large values gives the bits of a zeroed one.  (A layout that depended on
     the pooled flag once made the gradient call look for the forward pass's tables in the wrong place.)"""
@@ -523,10 +545,10 @@ def test_results_do_not_depend_on_what_the_workspace_held(shape, M, norm):
     dyp = torch.randn(B, M, H // 2, W // 2, device="cuda")
 
     def run(fill):
-        ws = mex_ops.mex_layer_workspace(x, M, pooled=True, flags=norm, **attrs)
+        ws = mex_ops.mex_layer_workspace(x, M, pooled=True, flags=norm | family, **attrs)
         ws.fill_(fill)
-        y, yp = mex_ops.mex_forward_pool2(x, off, M, flags=norm, workspace=ws, **attrs)
-        dx, doff = mex_ops.mex_backward(x, off, y, dyp, M, flags=norm, primed_workspace=ws, pooled=True, **attrs)
+        y, yp = mex_ops.mex_forward_pool2(x, off, M, flags=norm | family, workspace=ws, **attrs)
+        dx, doff = mex_ops.mex_backward(x, off, y, dyp, M, flags=norm | family, primed_workspace=ws, pooled=True, **attrs)
         return y, yp, dx, doff
     ref = run(0)
     for fill in (255, 127):

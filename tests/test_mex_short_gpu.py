@@ -40,3 +40,26 @@ def test_long_sums_agree_with_the_one_tile_kernels():
     one_dx, one_doff = mex_ops.mex_backward(x, off, y, dy, 64, flags=abi.FLAG_MEX_TC_ONE_TILE, **attrs)
     assert float((doff - one_doff).norm()) <= 1e-5 * float(one_doff.norm())
     assert float((dx - one_dx).norm()) <= 1e-5 * float(one_dx.norm())
+
+
+def test_long_sums_against_float64():
+    """The tensor cores truncate what they add to an accumulator: each of its additions loses up to 2^-23 of it, and there are three
+    (hi lo, lo hi, hi hi) for every eight positions of a share.  Shares are at least as many as multiprocessors."""
+    x = torch.randn(48, 2, 256, 256, device="cuda")
+    attrs = dict(blocks=[1, 2, 4], strides=[1, 2, 4], epsilon=0.5, softmax_mode=True, use_unshared_regions=False, shared_offset_region=[-1])
+    off = torch.randn(1, 64, 1, 2, 4, device="cuda")
+    y = mex_ops.mex_forward(x, off, 64, **attrs)
+    dy = torch.randn_like(y)
+    doff = mex_ops.mex_offsets_grad(x, off, y, dy, 64, **attrs)
+    eo, want, positions = torch.exp(0.5 * off.double()).reshape(64, 8), 0, 0
+    for n in range(48):                                     # disjoint blocks: sum over positions of dy * softmax weights
+        patches = x[n].double().reshape(2, 128, 2, 64, 4).permute(0, 1, 3, 2, 4).reshape(-1, 8)
+        ex = torch.exp(0.5 * (patches - patches.amax(1, keepdim=True)))
+        q = dy[n].double().reshape(64, -1).t() / (ex @ eo.t())
+        want = want + eo * (q.t() @ ex)
+        positions += patches.shape[0]
+    share = positions / torch.cuda.get_device_properties(0).multi_processor_count
+    bound = 3 * (share / 8) * 2.0 ** -23 + 1e-6
+    err = float((doff.reshape(64, 8).double() - want).norm() / want.norm())
+    print("offsets gradient over %d positions: %.2e of its norm from float64 (bound %.2e)" % (positions, err, bound))
+    assert err <= bound
