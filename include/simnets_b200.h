@@ -75,9 +75,9 @@ enum { SIMNETS_SIM_L1 = 0, SIMNETS_SIM_L2 = 1 };
  * otherwise run on kernels that read and write pixel pairs); same results, kept for comparison measurements. */
 #define SIMNETS_FLAG_MEX_NO_PAIR_TILES (1u << 9)
 
-/* MEX only, float32: never run small layers on the small-contraction kernels (three launches per call instead of the
- * tensor-core kernels' seven); same results, for comparison measurements and so that tests reach the tensor-core
- * kernels at small sizes. */
+/* MEX only, float32: never run small layers on the small-contraction kernels (two or three launches per forward call
+ * and FP32 sums, instead of the tensor-core kernels' four); same results within the library's bounds, for comparison
+ * measurements and so that tests reach the tensor-core kernels at small sizes. */
 #define SIMNETS_FLAG_MEX_NO_SMALL_TILES (1u << 15)
 
 /* Test hook, simnets_mex_forward on a pair-tile shape only: the kernel's MMA role withholds the completion signal of

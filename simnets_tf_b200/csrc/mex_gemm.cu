@@ -9,10 +9,10 @@
 // per (m, k, j) term.  The factorised form is safe while |eps| * spread(offsets) stays bounded; the prepass leaves a verdict per
 // group of offset rows, and where one of them says no the kernels evaluate term by term instead (mex_exact.cuh).
 //
-// Why a family of its own for small layers: a call is three launches (parameters and maxima, contraction, a finishing step when
-// the reduction is split), and a CTA's tile is small enough that a few hundred positions fill the GPU.  The tensor-core kernels
-// need seven launches and walk one tile per SM pair: 512 instances over 256 channels of 2x2 pixels at batch 256 took 51 us
-// forward and 144 us for the input gradient, because that layer has eight of their tiles.
+// Why a family of its own for small layers: a forward call is two or three launches (parameters and maxima, contraction, a
+// finishing step when the reduction is split), both gradients are three to five, and a CTA's tile is small enough that a few
+// hundred positions fill the GPU.  The tensor-core kernels take four and six and walk the chunks of one tile after another on few
+// SMs: 512 instances over 256 channels of 2x2 pixels at batch 128, forward and both gradients: 90 us here, 236 there.
 //
 // Tile: TM rows (16, 32 or 64, whichever pads least) x 64 columns, TM/16 x 4 outputs per thread, 32 (float64: 16) steps of the
 // reduction per chunk, double buffered.  The reduction is split over CTAs until two per SM are busy; partial sums are added in split order.
@@ -615,12 +615,21 @@ cudaError_t gemm_backward(const MexGeo& g, const T* x, const T* off, const T* y,
 
 }  // namespace
 
-// float32 layers whose contractions are so small that launches, and the one tile after another that a CTA of the tensor-core
-// kernels walks, would dominate.  Measured forward + both gradients, us, here / there: 64 instances over 32 channels at 17 M
-// multiply-adds per pass 47 / 54, at 67 M 88 / 73; 128 over 64 at 17 M 54 / 57, at 67 M 77 / 62; 256 over 128 at 67 M 79 / 88;
-// 512 over 256 at 67 M 101 / 230: the line grows with the layer's M K, whose chunks the tensor-core kernels walk serially.
-// Overlapping blocks: 24 instances over 12x3x3 taps at 139 M 283 / 313.  Classifier heads (M <= 16) up to 1024 taps: 512 taps
-// at 0.7 M 39 / 122; longer patches are read better by their own kernels.
+// float32 layers small enough for this family.  Forward with pooling + both gradients on the kept workspace, captured, us, here /
+// there (pixel layers with 2 x 2 regions; "there" = the tensor-core kernels):
+//     64 over 32, 16x16 pixels     4 M multiply-adds per pass 48 / 37,   17 M  51 / 42,   67 M  88 / 49
+//     128 over 64, 8x8             4 M  53 / 45,   17 M  60 / 47,   67 M  78 / 51
+//     256 over 128, 8x8            4 M  49 / 62,   25 M  62 / 64,   67 M  74 / 68,  101 M  92 / 70
+//     512 over 256, 4x4           17 M  57 / 99,   67 M  78 / 114, 134 M 111 / 119, 200 M 151 / 119
+//     1024 over 512, 2x2         200 M 210 / 328
+// The line grows with the layer's M K, whose chunks the tensor-core kernels walk serially.  Below M K = 10^4 it lies higher than
+// the times alone would have it, by 10 us a layer: sums are FP32 here, truncated after every eight taps there (distance of y from
+// float64, here / there: 64 over 32 3e-7 / 9e-7, 128 over 64 4e-7 / 2e-6, 512 over 256 4e-7 / 8e-6), a forward call and its
+// gradients are 6 or 7 launches here and 10 there, which is what such a layer costs a host, and networks of a few images stay on
+// one family whatever their batch.
+// Overlapping blocks: 24 instances over 12x3x3 taps at 105 M 210 / 248, at 209 M 384 / 428; 8 over 8x5x5 at 41 M 236 / 302.
+// Classifier heads (M <= 16) up to 1024 taps: the same reasons; 512 taps at 0.3 M 39 / 31, 1024 at 5 M 59 / 41.  Longer patches
+// are read better by their own kernels.
 static bool mex_small_layer(const MexGeo& g) {
     const double macs = double(g.R) * g.M * g.K * (double(g.B) * g.rs);
     if (g.M <= 16 && g.K >= 256) return g.K <= 1024 && macs <= 8e6;
