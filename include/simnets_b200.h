@@ -311,11 +311,11 @@ SIMNETS_API int simnets_mex_workspace_status(const void* workspace, void* stream
  * process exits.  It calls no device allocator and no allocating library routine.
  *
  *  - Route and tolerance: the call honours d->flags and adds SIMNETS_FLAG_MEX_NO_TENSORCORE, i.e. it
- *    always runs the CUDA-core kernels (the fixed array has no room for tensor-core operand tiles).
- *    float64 and the float32 shapes that need no scratch give the bits simnets_mex_forward gives; for
- *    the float32 shapes that simnets_mex_forward sends to the tensor cores the two results agree to
- *    the library's float32 bound, |a - b| <= 1e-5 * max(1, |b|), and each is within that bound of the
- *    reference's float64 result.
+ *    always runs the CUDA-core kernels (the fixed array has no room for tensor-core operand tiles),
+ *    float64 term by term.  Where simnets_mex_forward runs other kernels (float64, small layers and the
+ *    shapes of the tensor cores in float32) the two results agree to the library's bounds,
+ *    |a - b| <= 1e-5 * max(1, |b|) in float32 and 1e-12 in float64, and each is within that bound of
+ *    the reference's float64 result; infinite epsilon gives the same bits.
  *  - Problems whose forward scratch exceeds the array are rejected with SIMNETS_E_TOO_LARGE before
  *    anything is launched (scratch need = 4 bytes * (batch*N + 2*num_regions*M*K) plus a few hundred
  *    bytes of padding; use simnets_mex_forward with a caller workspace for those).

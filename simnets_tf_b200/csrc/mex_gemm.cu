@@ -623,10 +623,9 @@ cudaError_t gemm_backward(const MexGeo& g, const T* x, const T* off, const T* y,
 //     512 over 256, 4x4           17 M  57 / 99,   67 M  78 / 114, 134 M 111 / 119, 200 M 151 / 119
 //     1024 over 512, 2x2         200 M 210 / 328
 // The line grows with the layer's M K, whose chunks the tensor-core kernels walk serially.  Below M K = 10^4 it lies higher than
-// the times alone would have it, by 10 us a layer: sums are FP32 here, truncated after every eight taps there (distance of y from
-// float64, here / there: 64 over 32 3e-7 / 9e-7, 128 over 64 4e-7 / 2e-6, 512 over 256 4e-7 / 8e-6), a forward call and its
-// gradients are 6 or 7 launches here and 10 there, which is what such a layer costs a host, and networks of a few images stay on
-// one family whatever their batch.
+// these times alone would have it, by 10 us a layer: sums are FP32 here, truncated after every eight taps there (distance of y from
+// float64, here / there: 64 over 32 3e-7 / 9e-7, 128 over 64 4e-7 / 2e-6, 512 over 256 4e-7 / 8e-6), and a forward call with its
+// gradients is 6 or 7 launches here and 10 there, which is what such a layer costs a host.
 // Overlapping blocks: 24 instances over 12x3x3 taps at 105 M 210 / 248, at 209 M 384 / 428; 8 over 8x5x5 at 41 M 236 / 302.
 // Classifier heads (M <= 16) up to 1024 taps: the same reasons; 512 taps at 0.3 M 39 / 31, 1024 at 5 M 59 / 41.  Longer patches
 // are read better by their own kernels.

@@ -754,8 +754,12 @@ cudaError_t run_prepasses(const MexGeo& g, const MexWs& w, const float* x, const
     if (g.K >= 256 && g.N <= 16) { count_launch(); return launch_mex_colmax_wide(g, x, w.mx, w.flag, s); }
     const long long total = (long long)g.B * g.N;
     const int inside = patches_inside_input(g) ? 1 : 0;
-    // (measured on 32x32x64, 16x16x128 and 8x8x256 maps at batches 256 and 2048: eight threads per position win for
-    // long patches while one thread per position would not fill the GPU's thread slots: 2048 per multiprocessor)
+    // Maps that mex_prepare does not cover (blocks of several pixels, padding, pixel counts that no quad divides).  Eight threads
+    // per position win for long patches while one thread per position would not fill the GPU's thread slots, 2048 per
+    // multiprocessor.  The pass alone, us, one / eight: 256 channels of 7x7 pixels at 3 K positions 13 / 3, at 100 K 42 / 38;
+    // 128 channels of 7x7 or 15x15 at 58 K 12 / 12, at 230 K 43 / 45, at 401 K 48 / 69; 16 channels in 3x3 blocks at 16 K 31 / 10,
+    // at 131 K 70 / 55, at 524 K 210 / 206.  (Blocks of two or four columns read whole block rows below, which would win here as
+    // well: 64 channels in 2x2 blocks at 66 K 21 / 53.)
     if (g.K >= 128 && total < (long long)device_sm_count() * 2048) {
         const int grid = int(std::min<long long>((total + 31) / 32, (long long)device_sm_count() * 32));
         if (g.bh == 1 && g.bw == 1) in_stream_order(mex_colmax_sliced<true>, grid, 256, 0, s)(g, x, w.mx, w.flag, inside);

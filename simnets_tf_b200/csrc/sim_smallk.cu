@@ -42,9 +42,6 @@ __device__ __forceinline__ SkColumn sk_column(const SimGeo& g, long long j, long
     return c;
 }
 
-// KT >= K: the patch length at compile time (the tap loops are fully unrolled, the patches are register arrays); taps past K
-// have zero parameters.  A CTA works on templates [blockIdx.y * slice, ...): all of them unless the parameters would not fit
-// shared memory or the positions alone would not fill the GPU.
 struct SkParams {                               // how the parameters of one (template, tap) enter the arithmetic
     float t, scale, constant;
 };

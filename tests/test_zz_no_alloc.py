@@ -63,6 +63,22 @@ def test_static_scratch_keeps_the_callers_flags_and_matches_the_oracle_on_a_tens
     cases.assert_parity(b, a, tol=1e-5, what="static scratch vs workspace, caller flag kept")
 
 
+def test_static_scratch_in_float64(cuda_lib):
+    """float64 goes term by term there and in factorised form in a workspace."""
+    c = cases.mex_case("static_f64", (3, 12, 9, 10), 5, (4, 2, 3), (4, 2, 1), (0, 1, 1), eps=0.5, unshared=False, shared_region=(2,))
+    d = cases.mex_desc(c, dtype=abi.F64)
+    g = abi.MexGeometry()
+    assert cuda_lib.simnets_mex_dims(C.byref(d), C.byref(g)) == 0
+    x = torch.randn(c["shape"], dtype=torch.float64, device="cuda")
+    off = torch.randn(g.num_regions, c["M"], g.block_c, g.block_h, g.block_w, dtype=torch.float64, device="cuda")
+    a, b = (torch.empty((3, g.channels_out_total, g.height_out, g.width_out), dtype=torch.float64, device="cuda") for _ in range(2))
+    n = cuda_lib.simnets_mex_workspace_bytes(C.byref(d))
+    ws, stream = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.cuda.current_stream().cuda_stream
+    assert cuda_lib.simnets_mex_forward(C.byref(d), x.data_ptr(), off.data_ptr(), a.data_ptr(), ws.data_ptr(), n, stream) == 0
+    assert cuda_lib.simnets_mex_forward_static_scratch(C.byref(d), x.data_ptr(), off.data_ptr(), b.data_ptr(), stream) == 0
+    assert torch.allclose(a, b, rtol=1e-12, atol=1e-12)
+
+
 def test_static_scratch_rejects_problems_beyond_its_capacity(cuda_lib):
     big = cases.mex_case("static_big", (256, 256, 32, 32), 256, (4, 2, 2), (4, 2, 2), eps=0.5, softmax=True, unshared=False)
     d = cases.mex_desc(big)
