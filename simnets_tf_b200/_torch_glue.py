@@ -58,6 +58,9 @@ class _Recorded(torch.autograd.Function):
         return (None,) + tuple(next(got) if t.requires_grad else None for t in ctx.inputs)
 
 
+is_tracing = torch._C._is_tracing           # (torch.jit.is_tracing without its Python frame: every operator call asks)
+
+
 def recorded(call, *tensors):
     """call(*tensors) while torch.jit.trace is recording (see `_Recorded`)."""
     return _Recorded.apply(call, *tensors)

@@ -125,6 +125,7 @@ struct MexPlan {
         check(simnets_mex_dims(&d, &g));
     }
     simnets_mex_desc with(uint32_t flags) const { simnets_mex_desc q = d; q.flags |= flags; return q; }
+    bool overlapping() const { return g.stride_c < g.block_c || g.stride_h < g.block_h || g.stride_w < g.block_w; }
     size_t workspace_bytes(uint32_t flags) const { const simnets_mex_desc q = with(flags); return simnets_mex_forward_workspace_bytes(&q); }
     // room for the forward call and, if wanted, the gradient calls with a pooled dy
     size_t layer_bytes(uint32_t flags, bool pooled) const {
@@ -255,7 +256,7 @@ std::pair<Tensor, Tensor> mex_grads(const MexPlan& p, const Tensor& x_in, const 
     if (want_doff) doff = grad_target(off, out);
     const Tensor ws = mex_workspace(p, x, flags, primed);
     Tensor products;            // (overlapping blocks: not part of a workspace that a layer keeps between its passes)
-    if (const size_t n = want_dx ? simnets_mex_products_bytes(&d) : 0) products = scratch(x, n);
+    if (const size_t n = want_dx && p.overlapping() ? simnets_mex_products_bytes(&d) : 0) products = scratch(x, n);
     const char* op = want_dx && want_doff ? "mex_backward" : want_dx ? "mex_input_grad" : "mex_offsets_grad";
     const char* kind = want_dx && want_doff ? "bwd" : want_dx ? "dx" : "doff";
     Timed<MexPlan> timed(p, op, kind, s, pooled && want_dx && want_doff ? 3.0 * dy.numel() * dy.element_size() : 0.0);

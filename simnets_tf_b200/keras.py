@@ -16,8 +16,8 @@ import torch
 from . import _lib, abi
 from . import _torch_glue
 from .ops.mex import _attrs as _mex_attrs, _expand_dim_specification, _mex_dims_helper
-from .ops.mex import mex_plan as _mex_plan, mex_with_plan as _mex_with_plan
-from .ops.similarity import _attrs as _similarity_attrs, similarity_plan as _similarity_plan, similarity_with_plan as _similarity_with_plan
+from .ops.mex import mex_plan as _mex_plan, mex_recorded as _mex_recorded, mex_with_plan as _mex_with_plan
+from .ops.similarity import _attrs as _similarity_attrs, similarity_plan as _similarity_plan, similarity_recorded as _similarity_recorded
 
 
 def _sinks(*params):
@@ -152,7 +152,12 @@ class Similarity(_PlannedLayer):
             x = x.permute(0, 3, 1, 2)
         # |weights| and its gradient are taken inside the op's kernels
         templates, weights = self.templates, self.sweights
-        y = _similarity_with_plan(self._plan, x, templates, weights, abi.FLAG_SIM_ABS_WEIGHTS, extrema, _sinks(templates, weights))
+        if _torch_glue.is_tracing():
+            y = _similarity_recorded(self._plan, x, templates, weights, abi.FLAG_SIM_ABS_WEIGHTS, extrema)
+        else:
+            up, down = extrema if extrema is not None else (None, None)
+            dt, dw = _sinks(templates, weights) or (None, None)
+            y = _lib.ops().sim_apply(self._plan(x, templates, weights), x, templates, weights, abi.FLAG_SIM_ABS_WEIGHTS, up or 0, down or 0, dt, dw)
         return y.permute(0, 2, 3, 1) if self.channels_last else y
 
     def get_config(self):
@@ -338,8 +343,13 @@ class Mex(_PlannedLayer):
         # (the raw offsets are the op's own input, and a gradient bucket its target, only when the op normalises them)
         off = self.offsets
         sink = _sinks(off) if op_flags else None
-        y = _mex_with_plan(lambda x: self._plan(x.shape, x.dtype), x, off if op_flags else self.effective_offsets(), layer_ws,
-                           abi.FLAG_MEX_MAXIMA_GIVEN if maxima_given else 0, op_flags, sum_pool2, sink[0] if sink else None)
+        fwd_flags = abi.FLAG_MEX_MAXIMA_GIVEN if maxima_given else 0
+        if _torch_glue.is_tracing():
+            y = _mex_recorded(lambda x: self._plan(x.shape, x.dtype), x, off if op_flags else self.effective_offsets(), layer_ws, fwd_flags, op_flags,
+                              sum_pool2)
+        else:
+            y = _mex_with_plan(self._plan(x.shape, x.dtype), x, off if op_flags else self.effective_offsets(), layer_ws, fwd_flags, op_flags,
+                               sum_pool2, sink[0] if sink else None)
         return y.permute(0, 2, 3, 1) if self.channels_last else y
 
     def get_config(self):

@@ -1,7 +1,5 @@
 """Softmax cross-entropy over logit rows as one library kernel (loss and gradient in the same launch): the loss the
 reference's example networks train with (HUJI-Deep/simnets-tf README.md:108-111)."""
-import torch
-
 from .. import _lib
 from .. import _torch_glue
 
@@ -14,6 +12,6 @@ def softmax_cross_entropy_with_grad(logits, labels, scale=1.0):
 
 def softmax_cross_entropy(logits, labels, scale=1.0):
     """Differentiable (w.r.t. the logits) form of softmax_cross_entropy_with_grad."""
-    if torch.jit.is_tracing():
+    if _torch_glue.is_tracing():
         return _torch_glue.recorded(lambda l, k: _lib.ops().xent_apply(l, k, float(scale)), logits, labels)
     return _lib.ops().xent_apply(logits, labels, float(scale))

@@ -158,14 +158,14 @@ def sum_pool2x2(y):
     return out
 
 
-def mex_with_plan(plan_of, input, offsets, layer_ws=None, fwd_flags=0, op_flags=0, sum_pool2=False, grad_sink=None):
-    """`mex_in_workspace` on the plan that `plan_of(input)` holds (`mex_plan`)."""
-    if torch.jit.is_tracing():              # (the gradient of a recorded call goes through autograd, which adds it to the sink's `.grad`)
-        return _torch_glue.recorded(lambda x, o: _mex_with_plan(plan_of(x), x, o, layer_ws, fwd_flags, op_flags, sum_pool2, None), input, offsets)
-    return _mex_with_plan(plan_of(input), input, offsets, layer_ws, fwd_flags, op_flags, sum_pool2, grad_sink)
+def mex_recorded(plan_of, input, offsets, layer_ws=None, fwd_flags=0, op_flags=0, sum_pool2=False):
+    """`mex_with_plan` while torch.jit.trace records, on the plan of whatever input the recorded graph gets: `plan_of(input)`.  Its
+    gradients go through autograd, also to the `.grad` that a sink stands for."""
+    return _torch_glue.recorded(lambda x, o: mex_with_plan(plan_of(x), x, o, layer_ws, fwd_flags, op_flags, sum_pool2), input, offsets)
 
 
-def _mex_with_plan(plan, input, offsets, layer_ws, fwd_flags, op_flags, sum_pool2, grad_sink):
+def mex_with_plan(plan, input, offsets, layer_ws=None, fwd_flags=0, op_flags=0, sum_pool2=False, grad_sink=None):
+    """`mex_in_workspace` on a plan the caller holds (`mex_plan`)."""
     apply = _lib.ops().mex_apply
     if sum_pool2 and (plan.height_out % 2 or plan.width_out % 2):
         return torch.nn.functional.avg_pool2d(apply(plan, input, offsets, layer_ws, fwd_flags, op_flags, False, grad_sink), 2) * 4.0
@@ -185,7 +185,13 @@ def mex(input, offsets, num_instances, softmax_mode=None, padding=None, strides=
                    blocks_out_of_bounds_value=blocks_out_of_bounds_value, blocks_round_down=blocks_round_down,
                    use_unshared_regions=use_unshared_regions, shared_offset_region=shared_offset_region,
                    unshared_offset_region=unshared_offset_region)
-    return mex_with_plan(lambda x: _plan_of(x, num_instances, attrs), input, offsets)
+    return _mex(input, offsets, num_instances, attrs)
+
+
+def _mex(input, offsets, num_instances, attrs, layer_ws=None, fwd_flags=0, op_flags=0, sum_pool2=False, grad_sink=None):
+    if _torch_glue.is_tracing():
+        return mex_recorded(lambda x: _plan_of(x, num_instances, attrs), input, offsets, layer_ws, fwd_flags, op_flags, sum_pool2)
+    return mex_with_plan(_plan_of(input, num_instances, attrs), input, offsets, layer_ws, fwd_flags, op_flags, sum_pool2, grad_sink)
 
 
 def mex_sum_pool2(input, offsets, num_instances, layer_ws=None, fwd_flags=0, op_flags=0, grad_sink=None, **kwargs):
@@ -204,4 +210,4 @@ def mex_in_workspace(input, offsets, num_instances, layer_ws=None, fwd_flags=0, 
     and the gradient comes back with respect to them), a tensor that the offsets gradient is ADDED to instead of being
     handed to autograd (`grad_sink`: the offsets' slice of a data-parallel gradient bucket)."""
     attrs = _attrs(**{k: v for k, v in kwargs.items() if k != "name"})
-    return mex_with_plan(lambda x: _plan_of(x, num_instances, attrs), input, offsets, layer_ws, fwd_flags, op_flags, sum_pool2, grad_sink)
+    return _mex(input, offsets, num_instances, attrs, layer_ws, fwd_flags, op_flags, sum_pool2, grad_sink)

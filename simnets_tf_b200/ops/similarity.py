@@ -3,8 +3,6 @@
 `_similarity_grad` (same file, :18-45).  Tensors are torch CUDA tensors; the work is done by the
 CUDA library through the C ABI.
 """
-import torch
-
 from .. import _lib, abi
 from .. import _torch_glue
 from .._torch_glue import dtype_code, sequence_key
@@ -67,18 +65,20 @@ def similarity_parameters_grad(input, templates, weights, output_grad, flags=0, 
     return _lib.ops().sim_params_grad(similarity_plan(input, templates, weights, _attrs(**attrs)), input, templates, weights, output_grad, flags, dt, dw)
 
 
-def similarity_with_plan(plan_of, input, templates, weights, flags=0, extrema=None, grad_sinks=None):
-    """The differentiable op on the plan that `plan_of(input, templates, weights)` holds (`similarity_plan`)."""
+def similarity_recorded(plan_of, input, templates, weights, flags=0, extrema=None):
+    """The differentiable op while torch.jit.trace records, on the plan of whatever input the recorded graph gets: `plan_of(input,
+    templates, weights)`.  Its gradients go through autograd, also to the `.grad` that a sink stands for."""
     up, down = extrema if extrema is not None else (None, None)
-    dt, dw = grad_sinks if grad_sinks is not None else (None, None)
-    apply = _lib.ops().sim_apply
-    if torch.jit.is_tracing():              # (the gradients of a recorded call go through autograd, which adds them to the sinks' `.grad`)
-        return _torch_glue.recorded(lambda x, t, w: apply(plan_of(x, t, w), x, t, w, flags, up or 0, down or 0, None, None), input, templates, weights)
-    return apply(plan_of(input, templates, weights), input, templates, weights, flags, up or 0, down or 0, dt, dw)
+    return _torch_glue.recorded(lambda x, t, w: _lib.ops().sim_apply(plan_of(x, t, w), x, t, w, flags, up or 0, down or 0, None, None),
+                                input, templates, weights)
 
 
 def _apply(input, templates, weights, attrs, flags=0, extrema=None, grad_sinks=None):
-    return similarity_with_plan(lambda x, t, w: similarity_plan(x, t, w, attrs), input, templates, weights, flags, extrema, grad_sinks)
+    if _torch_glue.is_tracing():
+        return similarity_recorded(lambda x, t, w: similarity_plan(x, t, w, attrs), input, templates, weights, flags, extrema)
+    up, down = extrema if extrema is not None else (None, None)
+    dt, dw = grad_sinks if grad_sinks is not None else (None, None)
+    return _lib.ops().sim_apply(similarity_plan(input, templates, weights, attrs), input, templates, weights, flags, up or 0, down or 0, dt, dw)
 
 
 def similarity(input, templates, weights, similarity_function=None, blocks=None, strides=None, padding=None,

@@ -16,6 +16,7 @@ import torch
 import torch.nn.functional as F
 
 from . import keras as layers
+from ._torch_glue import is_tracing
 from .ops.loss import softmax_cross_entropy
 
 
@@ -105,7 +106,7 @@ class SimNet(torch.nn.Module):
             entry, mod = plan[i]
             pooled_next = lambda j: self.fuse_pooling and j + 1 < len(plan) and plan[j + 1][0] == ("sumpool", 2)
             # (a recorded graph outlives the workspace whose address the extrema go to)
-            if entry[0] == "similarity" and self.fuse_extrema and i + 1 < end and plan[i + 1][0][0] == "mex" and not torch.jit.is_tracing():
+            if entry[0] == "similarity" and self.fuse_extrema and i + 1 < end and plan[i + 1][0][0] == "mex" and not is_tracing():
                 # Similarity -> MEX over the channels of each pixel: the Similarity kernel leaves the per-pixel extrema of its
                 # output in the MEX layer's workspace, and the MEX forward pass skips its pass over that tensor
                 nxt = plan[i + 1][1]
