@@ -15,7 +15,7 @@
 // NaN pixels give 0 in the ignore_nan_input modes, and so does a pixel that no patch covers in every mode.  A tap that the
 // padding cuts off, or a step past the last one, contributes 0 * (t - x), which is NaN for an infinite x (or an infinite
 // parameter): a sum that came out NaN over a number is added up again over the taps that are there (dx_redo; the test costs 1.5 %
-// where 64 rows of channels share a tile: 128 x 64 x 32 x 32 input, 128 templates of 3x3, 1231 -> 1251 us).
+// where 64 rows of channels share a tile: 128 x 64 x 32 x 32 input, 128 templates of 3x3, 1231 -> 1243 us, with kDxFold).
 #include "kernels.cuh"
 #include "sim_exact.cuh"
 #include "tile.cuh"
@@ -95,9 +95,15 @@ __global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, const float* __rest
     }
 }
 
+// Steps after which a sum is set aside (a private slot in shared memory) and begins again: a sum of M bh bw terms in one register
+// is several times farther from the exact one than the reference's, which adds the taps' sums over m (256 templates of 5x5: 1.4e-6
+// of the gradient's norm against 3e-7).
+constexpr int kDxFold = 256;
+
 template <int TM> struct DxCfg {
     static constexpr int RM = TM == 128 ? 8 : 4, TN = TM == 16 ? 256 : 128;
     using Cfg = TileCfg<TM, TN, 8, RM, 8, 2, 1>;
+    static constexpr int SLOT_BYTES = 4 * RM * 8 * Cfg::THREADS;
 };
 
 template <int TM, int MODE>
@@ -111,6 +117,7 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
     constexpr int T = Cfg::THREADS, COLS = Cfg::TN > T ? Cfg::TN / T : 1, QSTEP = T > Cfg::TN ? T / Cfg::TN : 1, QPER = Cfg::KC / QSTEP;
     constexpr int VEC = TM / 4, APER = (2 * Cfg::KC * VEC + T - 1) / T;
     __shared__ __align__(16) float smem[Cfg::SMEM_FLOATS];
+    extern __shared__ __align__(16) float2 slots[];                     // [RM x RN / 2][THREADS], if the launch has sums of more than kDxFold steps
     __shared__ long long col_base[Cfg::TN];
     __shared__ unsigned char col_covered[Cfg::TN];
     const DxPhase ph(g, blockIdx.y);
@@ -203,7 +210,23 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
         const float2 e = mul2(a[1], b[0]);
         acc[r_][cp] = fma2(e, L1 ? make_float2(dx_sign(d.x), dx_sign(d.y)) : d, acc[r_][cp]);
     };
-    tile_mainloop<Cfg, false, false>(smem, (Q + Cfg::KC - 1) / Cfg::KC, t, fetchA, fetchB, commitA, commitB, comb);
+    const int chunks = (Q + Cfg::KC - 1) / Cfg::KC;
+    auto fold = [&](int c) {
+        const bool first = c == kDxFold / Cfg::KC;
+#pragma unroll
+        for (int i = 0; i < Cfg::RM * Cfg::RN / 2; ++i) {
+            float2& a = acc[i / (Cfg::RN / 2)][i % (Cfg::RN / 2)];
+            slots[i * T + threadIdx.x] = first ? a : add2(slots[i * T + threadIdx.x], a);
+            a = make_float2(0.f, 0.f);
+        }
+    };
+    tile_mainloop<Cfg, false, false, kDxFold / Cfg::KC>(smem, chunks, t, fetchA, fetchB, commitA, commitB, comb, fold);
+    if (Q > kDxFold)
+#pragma unroll
+        for (int i = 0; i < Cfg::RM * Cfg::RN / 2; ++i) {
+            float2& a = acc[i / (Cfg::RN / 2)][i % (Cfg::RN / 2)];
+            a = add2(slots[i * T + threadIdx.x], a);
+        }
 
     bool redo = false;
 #pragma unroll
@@ -243,6 +266,7 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_con
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     constexpr bool SKIP_NAN = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
     __shared__ __align__(16) float s_t[kNarrowQ * CT], s_w[kNarrowQ * CT];
+    __shared__ float slots[PP * CT][kNarrowThreads];                    // sums set aside, see kDxFold
     const DxPhase ph(g, blockIdx.y);
     const long long j0 = (long long)blockIdx.x * (kNarrowThreads * PP);
     if (j0 >= (long long)g.B * ph.h.n * ph.w.n) return;
@@ -257,6 +281,8 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_con
 #pragma unroll
         for (int c = 0; c < CT; ++c) { xv[p][c] = (px[p].base >= 0 && c < g.C) ? __ldg(x + px[p].base + c * chw) : 0.f; acc[p][c] = 0.f; }
     }
+    int steps = 0;
+    bool aside = false;
     for (int a = 0; a < ph.h.taps; ++a)
         for (int b = 0; b < ph.w.taps; ++b) {
             const int tap = (ph.rh + a * g.sh) * g.bw + ph.rw + b * g.sw;
@@ -265,6 +291,18 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_con
             for (int p = 0; p < PP; ++p) at[p] = px[p].at(g, a, b);
             for (int m0 = 0; m0 < g.M; m0 += kNarrowQ) {
                 const int nm = min(kNarrowQ, g.M - m0);
+                if ((steps += nm) > kDxFold) {
+#pragma unroll
+                    for (int p = 0; p < PP; ++p)
+#pragma unroll
+                        for (int c = 0; c < CT; ++c) {
+                            float& s = slots[p * CT + c][threadIdx.x];
+                            s = aside ? s + acc[p][c] : acc[p][c];
+                            acc[p][c] = 0.f;
+                        }
+                    steps = nm;
+                    aside = true;
+                }
                 __syncthreads();
                 for (int i = threadIdx.x; i < nm * CT; i += kNarrowThreads) {
                     const int c = i % CT, m = m0 + i / CT;
@@ -291,6 +329,11 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_con
                 }
             }
         }
+    if (aside)
+#pragma unroll
+        for (int p = 0; p < PP; ++p)
+#pragma unroll
+            for (int c = 0; c < CT; ++c) acc[p][c] += slots[p * CT + c][threadIdx.x];
 #pragma unroll
     for (int p = 0; p < PP; ++p) {
         if (px[p].base < 0) continue;
@@ -356,7 +399,14 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
     const long long blocks = ((pixels + tn - 1) / tn) * ((g.C + tm - 1) / tm);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const dim3 grid{unsigned(blocks), unsigned(phases)};
-#define DX(TM, MODE) in_stream_order(sim_dx_tiled<TM, MODE>, grid, DxCfg<TM>::Cfg::THREADS, 0, s)(g, x, dxp, t, w, dy, dx)
+    const bool folds = (long long)((g.bh + g.sh - 1) / g.sh) * ((g.bw + g.sw - 1) / g.sw) * g.M > kDxFold;         // (the most taps of a phase)
+#define DX(TM, MODE)                                                                                                                          \
+    do {                                                                                                                                      \
+        static SmemLimit limit;                                                                                                               \
+        const cudaError_t e = limit.raise(sim_dx_tiled<TM, MODE>, DxCfg<TM>::SLOT_BYTES);                                                     \
+        if (e != cudaSuccess) return e;                                                                                                       \
+        in_stream_order(sim_dx_tiled<TM, MODE>, grid, DxCfg<TM>::Cfg::THREADS, folds ? DxCfg<TM>::SLOT_BYTES : 0, s)(g, x, dxp, t, w, dy, dx); \
+    } while (0)
 #define DX_16(MODE) DX(16, MODE)
 #define DX_32(MODE) DX(32, MODE)
 #define DX_64(MODE) DX(64, MODE)

@@ -119,10 +119,12 @@ __device__ __forceinline__ void tile_compute(const float* __restrict__ As, const
 
 // Double-buffered main loop over `nchunks` chunks of the reduction index.  fetchX(chunk, dst) may either
 // load into registers (to be transformed and stored by commitX(dst)) or start asynchronous copies straight
-// into the destination stage (commitX then only waits for them).
-template <class Cfg, bool ASWZ, bool BSWZ, class FetchA, class FetchB, class CommitA, class CommitB, class Comb>
+// into the destination stage (commitX then only waits for them).  after(c): called when the first c chunks are done, for every
+// multiple c of SEGMENT but the last chunk's.
+struct TileNothing { __device__ __forceinline__ void operator()(int) const {} };
+template <class Cfg, bool ASWZ, bool BSWZ, int SEGMENT = 0, class FetchA, class FetchB, class CommitA, class CommitB, class Comb, class After = TileNothing>
 __device__ __forceinline__ void tile_mainloop(float* smem, int nchunks, const TileThread<Cfg>& t, FetchA fetchA, FetchB fetchB,
-                                              CommitA commitA, CommitB commitB, Comb comb) {
+                                              CommitA commitA, CommitB commitB, Comb comb, After after = After()) {
     float* As0 = smem;
     float* As1 = smem + Cfg::A_STAGE;
     float* Bs0 = smem + 2 * Cfg::A_STAGE;
@@ -131,14 +133,19 @@ __device__ __forceinline__ void tile_mainloop(float* smem, int nchunks, const Ti
     fetchA(0, As0); fetchB(0, Bs0);
     commitA(As0); commitB(Bs0);
     __syncthreads();
-    for (int c = 0; c < nchunks; ++c) {
-        const bool more = c + 1 < nchunks;
-        float* An = (c & 1) ? As0 : As1;
-        float* Bn = (c & 1) ? Bs0 : Bs1;
-        if (more) { fetchA(c + 1, An); fetchB(c + 1, Bn); }
-        tile_compute<Cfg, ASWZ, BSWZ>((c & 1) ? As1 : As0, (c & 1) ? Bs1 : Bs0, t, comb);
-        if (more) { commitA(An); commitB(Bn); }
-        __syncthreads();
+    for (int c = 0;;) {
+        const int stop = SEGMENT > 0 ? min(nchunks, c + SEGMENT) : nchunks;
+        for (; c < stop; ++c) {
+            const bool more = c + 1 < nchunks;
+            float* An = (c & 1) ? As0 : As1;
+            float* Bn = (c & 1) ? Bs0 : Bs1;
+            if (more) { fetchA(c + 1, An); fetchB(c + 1, Bn); }
+            tile_compute<Cfg, ASWZ, BSWZ>((c & 1) ? As1 : As0, (c & 1) ? Bs1 : Bs0, t, comb);
+            if (more) { commitA(An); commitB(Bn); }
+            __syncthreads();
+        }
+        if (c == nchunks) return;
+        after(c);
     }
 }
 
