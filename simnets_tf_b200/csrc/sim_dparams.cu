@@ -22,6 +22,13 @@ namespace {
 
 constexpr int kDpThreads = 256, kDpMaxK2 = 32, kDpCtasPerSm = 2;
 
+// Positions after which a thread sets its sums aside (private slots in shared memory) and begins again: one wave of splits leaves a
+// split up to all positions, and a sum of that many terms in one register is farther from the exact one the longer it is
+// (256 x 64 x 32 x 32 input, 256 templates of 3x3, 65536 positions a split: 2.9e-6 of the gradient's norm; set aside: 5.3e-7).  It costs 1-2 % (L1, the least work per term: 4 %);
+// shorter splits instead would write and read their partial sums.
+constexpr int kDpFold = 2048;
+__host__ __device__ constexpr int dp_slots(int mode) { return mode == SIM_L1 || mode == SIM_L1_SKIP || mode == SIM_L2 ? 16 : 24; }
+
 struct DpTile { int k2, groups, tm, kc; };       // tap columns / 2, copies of the tile per CTA, templates per tile, positions per chunk
 
 // Tile of a patch of K taps: the patch in n equal tiles of at most 64 taps, n the smallest that keeps nearly as many threads
@@ -68,6 +75,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
     constexpr int A_FLOATS = TM * LD, B_FLOATS = MAXK * LD, STAGE = A_FLOATS + (MASKED ? 2 : 1) * B_FLOATS;
     static_assert(2 * STAGE >= 3 * TM * MAXK || MAXK == 64, "the copies' sums are added up in the stages");
     __shared__ __align__(16) float smem[2 * STAGE];
+    extern __shared__ float slots[];                                     // [dp_slots][threads], if a split has more than kDpFold positions
     __shared__ int2 taps[MAXK];                                          // {byte offset inside a sample, kh << 16 | kw}
 
     const long long P = (long long)g.B * g.N;
@@ -231,15 +239,47 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
         fetch(c_begin);
         commit(smem);
         __syncthreads();
-        for (int i = 0; i < n_chunks; ++i) {
-            float* now = smem + (i & 1) * STAGE;
-            float* next = smem + ((i + 1) & 1) * STAGE;
-            const bool more = i + 1 < n_chunks;
-            if (more) fetch(c_begin + i + 1);
-            if (TENSOR_N) compute_n(now);
-            if (worker) compute(now);
-            if (more) commit(next);
-            __syncthreads();
+        for (int i = 0;;) {
+            const int stop = min(n_chunks, i + kDpFold / KC);
+            for (; i < stop; ++i) {
+                float* now = smem + (i & 1) * STAGE;
+                float* next = smem + ((i + 1) & 1) * STAGE;
+                const bool more = i + 1 < n_chunks;
+                if (more) fetch(c_begin + i + 1);
+                if (TENSOR_N) compute_n(now);
+                if (worker) compute(now);
+                if (more) commit(next);
+                __syncthreads();
+            }
+            if (i == n_chunks) break;
+            const bool first = i == kDpFold / KC;
+            float* s = slots + threadIdx.x;
+            auto aside = [&](float2& v) {
+                const float now = v.x + v.y;
+                *s = first ? now : *s + now;
+                s += kDpThreads;
+                v = make_float2(0.f, 0.f);
+            };
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    aside(sT[r][c]);
+                    aside(sW[r][c]);
+                    if (SUM_N || (c == 0 && MODE == SIM_L2N)) aside(sN[r][SUM_N ? c : 0]);
+                }
+        }
+        if (n_chunks > kDpFold / KC) {
+            const float* s = slots + threadIdx.x;
+            auto join = [&](float2& v) { v.x += *s; s += kDpThreads; };
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    join(sT[r][c]);
+                    join(sW[r][c]);
+                    if (SUM_N || (c == 0 && MODE == SIM_L2N)) join(sN[r][SUM_N ? c : 0]);
+                }
         }
     }
 
@@ -341,7 +381,15 @@ cudaError_t launch_sim_dparams(const SimGeo& g, const float* x, const float* t, 
     const long long blocks = (long long)dp_tiles(g, tile) * splits;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const FastDiv f_N = make_fastdiv(g.N), f_ow = make_fastdiv(g.ow);
-#define DP_TILE(MODE, KC, MAXK, TM) in_stream_order(sim_dparams<MODE, KC, MAXK, TM>, int(blocks), kDpThreads, 0, s)(g, f_N, f_ow, tile, x, t, dy, part, splits)
+    const bool folds = ((long long)g.B * g.N + splits - 1) / splits > kDpFold - tile.kc;          // (a split may have one chunk more than another)
+#define DP_TILE(MODE, KC, MAXK, TM)                                                                                                                  \
+    do {                                                                                                                                             \
+        constexpr int bytes = 4 * kDpThreads * dp_slots(MODE);                                                                                       \
+        static SmemLimit limit;                                                                                                                      \
+        const cudaError_t e = limit.raise(sim_dparams<MODE, KC, MAXK, TM>, bytes);                                                                   \
+        if (e != cudaSuccess) return e;                                                                                                              \
+        in_stream_order(sim_dparams<MODE, KC, MAXK, TM>, int(blocks), kDpThreads, folds ? bytes : 0, s)(g, f_N, f_ow, tile, x, t, dy, part, splits); \
+    } while (0)
 #define DP(MODE)                                            \
     do {                                                    \
         if (tile.tm == 64) DP_TILE(MODE, 32, 32, 64);       \

@@ -80,3 +80,22 @@ def test_input_gradients_of_long_sums_are_folded(channels, strides, m, attrs):
     want = gpu_util.sim_ops.similarity_input_grad(x.double(), t.double(), w.double(), dy.double(), **kw)
     got = gpu_util.sim_ops.similarity_input_grad(x, t, w, dy, **kw).double()
     assert float((got - want).norm() / want.norm()) <= _of_folded(256, 25)
+
+
+@pytest.mark.parametrize("attrs", [dict(), dict(normalization_term=True), dict(normalization_term=True, ignore_nan_input=True), dict(similarity_function="L1")],
+                         ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("m,channels,block,batch", [(256, 32, 3, 128), (64, 3, 3, 2048), (32, 1, 2, 8192), (64, 64, 3, 72), (64, 64, 3, 74)],
+                         ids=["wide", "image", "copies", "few_aside", "one_more"])
+def test_parameter_gradients_of_long_sums_are_folded(m, channels, block, batch, attrs):
+    """Up to 60000 positions of a split, set aside every 2048 of them."""
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    x, t = torch.randn(batch, channels, 32, 32, generator=gen, device="cuda"), 0.1 * torch.randn(m, channels, block, block, generator=gen, device="cuda")
+    w = 1 + 0.1 * torch.rand(t.shape, generator=gen, device="cuda")
+    kw = dict(blocks=[block, block], strides=[1, 1], padding=[0, 0], **attrs)
+    dy = torch.randn(batch, m, 33 - block, 33 - block, generator=gen, device="cuda")
+    want = [0, 0]
+    for i in range(0, batch, 512):
+        for k, g in enumerate(gpu_util.sim_ops.similarity_parameters_grad(x[i:i + 512].double(), t.double(), w.double(), dy[i:i + 512].double(), **kw)):
+            want[k] = want[k] + g
+    for g, e in zip(gpu_util.sim_ops.similarity_parameters_grad(x, t, w, dy, **kw), want):
+        assert float((g.double() - e).norm() / e.norm()) <= _of_folded(2048, 32)
