@@ -60,7 +60,7 @@ template <int NT, bool DX, bool DOFF, bool VEC>
 __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int inside, const float* __restrict__ x, const float* __restrict__ eo,
                                                                const float* __restrict__ mo, const float* __restrict__ mx, const float* __restrict__ y,
                                                                const float* __restrict__ dy, float* __restrict__ dx, float* __restrict__ part,
-                                                               const int* __restrict__ flag) {
+                                                               int fold, const int* __restrict__ flag) {
     stream_order();
     if (*flag) return;
     constexpr int KT = NT * 8, LD = sh_ld(KT);
@@ -187,17 +187,29 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
                 const int p0 = (rt * 16 + gq) ^ (tq << 3);
                 const float* q0 = Q + tq * kShPos;
                 const float2* b = Eos + (mc * kShM + tq) * LD + nt0 * 8 + gq;
+                float s[MT][4];                                                 // (64 instances on the tensor cores, these sums in FP32)
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) s[i][u] = 0.f;
 #pragma unroll
                 for (int m = 0; m < kShM; m += 8) {
                     const float *lo = q0 + m * kShPos, *hi = lo + 4 * kShPos;
-                    sh_step<MT>(acc, lo[p0], lo[p0 ^ 8], hi[p0 ^ 4], hi[p0 ^ 12], b + m * LD, 4 * LD);
+                    sh_step<MT>(s, lo[p0], lo[p0 ^ 8], hi[p0 ^ 4], hi[p0 ^ 12], b + m * LD, 4 * LD);
                 }
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc[i][u] += s[i][u];
             } else if (DOFF) {
                 // rows = instances 16 rt.., columns = taps, reduction = positions
                 float4* own = reinterpret_cast<float4*>(Ds) + (mc * NT + nt0) * 128 + (warp & 3) * 32 + lane;
                 float s[MT][4];
 #pragma unroll
-                for (int i = 0; i < MT; ++i) { const float4 v = own[i * 128]; s[i][0] = v.x; s[i][1] = v.y; s[i][2] = v.z; s[i][3] = v.w; }
+                for (int i = 0; i < MT; ++i) {
+                    const float4 v = fold ? make_float4(0.f, 0.f, 0.f, 0.f) : own[i * 128];
+                    s[i][0] = v.x; s[i][1] = v.y; s[i][2] = v.z; s[i][3] = v.w;
+                }
                 const float* q0 = Q + (rt * 16 + gq) * kShPos;
                 const int sw = sh_swizzle(gq);
                 const float2* b = E + tq * LD + nt0 * 8 + gq;
@@ -207,7 +219,10 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
                     sh_step<MT>(s, q0[c0], q0[8 * kShPos + c0], q0[c1], q0[8 * kShPos + c1], b + p * LD, 4 * LD);
                 }
 #pragma unroll
-                for (int i = 0; i < MT; ++i) own[i * 128] = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+                for (int i = 0; i < MT; ++i) {
+                    const float4 v = fold ? own[i * 128] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    own[i * 128] = make_float4(v.x + s[i][0], v.y + s[i][1], v.z + s[i][2], v.w + s[i][3]);
+                }
             }
         }
         if (does_dx && !idle) {
@@ -258,7 +273,9 @@ bool mex_short_shape(const MexGeo& g) {
 }
 // Positions that the one-tile kernels of mex_tc.cu sum in one accumulator.  The tensor cores truncate what they add, so a long
 // sum depends on where it is cut (18.9 K positions: 1.4e-4 of the offsets gradient's norm from the exact sum, growing with the
-// length): from 1500 positions on (1e-5) this kernel cuts where that one does, below it takes shares that fill the GPU.
+// length): from 1500 positions on (1e-5) this kernel cuts where that one does and accumulates as that one does; below it takes
+// shares that fill the GPU and adds the products of 64 positions in FP32 (64 instances over 2x2x2 blocks, 885 positions a share:
+// 6.4e-6 of the norm otherwise, the one-tile kernel 4.5e-6; 7.4e-7 so).
 static bool sh_long_sums(const MexGeo& g) { return (long long)g.B * g.rs / mex_tc_doff_splits(g) > 1500; }
 int mex_short_splits(const MexGeo& g) {
     if (sh_long_sums(g)) return mex_tc_doff_splits(g);
@@ -274,13 +291,14 @@ bool mex_short_doff(const MexGeo& g) { return !sh_long_sums(g) || sh_ctas_per_sm
 cudaError_t launch_mex_bwd_short(const MexGeo& g, bool inside, const float* x, const float* eo, const float* mo, const float* mx, const float* y,
                                  const float* dy, float* dx, float* part, const int* flag, cudaStream_t s) {
     const int kt = sh_taps(g), smem = sh_smem_bytes(g.M, kt);
+    const int fold = !sh_long_sums(g);
     const dim3 grid(unsigned(mex_short_splits(g)), unsigned(g.R));
     const bool vec = g.R == 1 && g.gp == 1 && g.N % 4 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(dy)) & 15) == 0;
-#define SH(NT, DX, DOFF, VEC)                                                                                                                  \
-    do {                                                                                                                                       \
-        const cudaError_t e = cudaFuncSetAttribute(mex_bwd_short<NT, DX, DOFF, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);  \
-        if (e != cudaSuccess) return e;                                                                                                        \
-        in_stream_order(mex_bwd_short<NT, DX, DOFF, VEC>, grid, kShThreads, smem, s)(g, int(inside), x, eo, mo, mx, y, dy, dx, part, flag);     \
+#define SH(NT, DX, DOFF, VEC)                                                                                                                     \
+    do {                                                                                                                                          \
+        const cudaError_t e = cudaFuncSetAttribute(mex_bwd_short<NT, DX, DOFF, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);    \
+        if (e != cudaSuccess) return e;                                                                                                           \
+        in_stream_order(mex_bwd_short<NT, DX, DOFF, VEC>, grid, kShThreads, smem, s)(g, int(inside), x, eo, mo, mx, y, dy, dx, part, fold, flag); \
     } while (0)
 #define SH_VEC(NT, DX, DOFF) do { if (vec) SH(NT, DX, DOFF, true); else SH(NT, DX, DOFF, false); } while (0)
 #define SH_WANTS(NT)                                                                                     \

@@ -63,3 +63,20 @@ def test_long_sums_against_float64():
     err = float((doff.reshape(64, 8).double() - want).norm() / want.norm())
     print("offsets gradient over %d positions: %.2e of its norm from float64 (bound %.2e)" % (positions, err, bound))
     assert err <= bound
+
+
+@pytest.mark.parametrize("m,block", [(64, (2, 2, 2)), (100, (4, 2, 2)), (256, (8, 2, 2))], ids=["taps_8", "taps_16", "taps_32"])
+def test_products_of_64_are_added_in_fp32(m, block):
+    """Up to 1500 positions per accumulator of the one-tile kernels: what 64 positions (offsets gradient) or 64 instances (input
+    gradient) contribute is added in FP32, so that neither gradient is farther from float64 than FP32 sums are (1e-6 of its norm; truncated
+    additions would be at 3 / 8 x 2^-23 per position, 4e-5 at a thousand)."""
+    attrs = dict(blocks=list(block), strides=list(block), epsilon=0.5, softmax_mode=True, use_unshared_regions=False, shared_offset_region=[-1])
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x, off = torch.randn(64, 16, 32, 32, generator=gen, device="cuda"), torch.randn((1, m) + block, generator=gen, device="cuda")
+    y = mex_ops.mex_forward(x, off, m, flags=abi.FLAG_MEX_NO_SMALL_TILES, **attrs)
+    dy = torch.randn(y.shape, generator=gen, device="cuda")
+    got = mex_ops.mex_backward(x, off, y, dy, m, flags=abi.FLAG_MEX_NO_SMALL_TILES, **attrs)
+    y64 = mex_ops.mex_forward(x.double(), off.double(), m, **attrs)
+    want = mex_ops.mex_backward(x.double(), off.double(), y64, dy.double(), m, **attrs)
+    for g, w in zip(got, want):
+        assert float((g.double() - w).norm() / w.norm()) <= 1e-6
