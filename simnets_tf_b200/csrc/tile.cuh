@@ -133,19 +133,23 @@ __device__ __forceinline__ void tile_mainloop(float* smem, int nchunks, const Ti
     fetchA(0, As0); fetchB(0, Bs0);
     commitA(As0); commitB(Bs0);
     __syncthreads();
-    for (int c = 0;;) {
-        const int stop = SEGMENT > 0 ? min(nchunks, c + SEGMENT) : nchunks;
-        for (; c < stop; ++c) {
-            const bool more = c + 1 < nchunks;
-            float* An = (c & 1) ? As0 : As1;
-            float* Bn = (c & 1) ? Bs0 : Bs1;
-            if (more) { fetchA(c + 1, An); fetchB(c + 1, Bn); }
-            tile_compute<Cfg, ASWZ, BSWZ>((c & 1) ? As1 : As0, (c & 1) ? Bs1 : Bs0, t, comb);
-            if (more) { commitA(An); commitB(Bn); }
-            __syncthreads();
+    auto step = [&](int c) {
+        const bool more = c + 1 < nchunks;
+        float* An = (c & 1) ? As0 : As1;
+        float* Bn = (c & 1) ? Bs0 : Bs1;
+        if (more) { fetchA(c + 1, An); fetchB(c + 1, Bn); }
+        tile_compute<Cfg, ASWZ, BSWZ>((c & 1) ? As1 : As0, (c & 1) ? Bs1 : Bs0, t, comb);
+        if (more) { commitA(An); commitB(Bn); }
+        __syncthreads();
+    };
+    if constexpr (SEGMENT == 0) {
+        for (int c = 0; c < nchunks; ++c) step(c);
+    } else {
+        for (int c = 0;;) {
+            for (const int stop = min(nchunks, c + SEGMENT); c < stop; ++c) step(c);
+            if (c == nchunks) return;
+            after(c);
         }
-        if (c == nchunks) return;
-        after(c);
     }
 }
 
