@@ -120,7 +120,7 @@ __device__ __forceinline__ float2 abs2(float2 v) { return make_float2(fabsf(v.x)
 // chunk costs a round trip to L2).
 template <int TM, int TN> struct FwdTile {
     static constexpr int RM = TM == 128 ? 8 : 4, RN = TN == 128 ? 8 : 4, KC = TM * TN <= 2048 ? 16 : 8, THREADS = (TM / RM) * (TN / RN);
-    static constexpr int PER_SM = TM == 128 ? 2 : (TN == 128 ? 1 : 512 / THREADS);
+    static constexpr int PER_SM = TN == 128 ? 2 : 512 / THREADS;
 };
 
 template <int TM, int TN, int MODE>
@@ -165,11 +165,27 @@ __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER
         for (int p = 0; p < NA; ++p)
             stage_copy_async<Cfg, TM>(As + p * Cfg::KC * TM, planes + p * plane, ldm, chunk * Cfg::KC, g.K, i0, g.M);
     };
+    // A gathered value hangs on its tap's entry: the entries of the next chunk are read while this one is multiplied, so that a
+    // chunk waits for one read and not for two in a row (8 x 16 x 20 x 20 input, 48 templates of 3x3: 24.1 -> 19.0 us; 128 x 16 x
+    // 24 x 24, 33 of 5x5 with stride 2: 98.7 -> 78.6).  8 x 8 blocking, or 4 x 8 with masks, has no registers left for them
+    // (256 x 64 x 32 x 32, 256 of 3x3: 4134 -> 4245).
+    constexpr bool AHEAD = Cfg::RM * Cfg::RN <= (NB == 2 ? 16 : 32);
+    int2 tap[AHEAD ? Cfg::B_PER : 1];
+    if (AHEAD) {
+#pragma unroll
+        for (int s = 0; s < Cfg::B_PER; ++s) tap[AHEAD ? s : 0] = __ldg(taps + min(s_k + s * QSTEP, g.K - 1));
+    }
     auto fetchB = [&](int chunk, float*) {
 #pragma unroll
         for (int s = 0; s < Cfg::B_PER; ++s) {
             const int k = chunk * Cfg::KC + s_k + s * QSTEP;
             // rows past K pair a zero scale / zero constant with a finite value: the term is exactly 0
+            if (AHEAD) {
+                rb[s] = 0.f;
+                if (k < g.K && live) rb[s] = inside ? __ldg(xc + tap[AHEAD ? s : 0].x) : sim_tap_value(g, xs, sc, tap[AHEAD ? s : 0], oob);
+                tap[AHEAD ? s : 0] = __ldg(taps + min(k + Cfg::KC, g.K - 1));
+                continue;
+            }
             if (k >= g.K || !live) rb[s] = 0.f;
             else if (inside) rb[s] = __ldg(xc + __ldg(taps + k).x);
             else rb[s] = sim_tap_value(g, xs, sc, __ldg(taps + k), oob);
@@ -267,13 +283,16 @@ static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const flo
     // The tile with the least estimated time: tiles per SM (rounded up) x outputs per tile x the relative cost of a term at
     // that tile's register blocking, stretched where too few warps are resident to keep the FP32 pipe fed (the larger tiles on
     // small inputs: 16 x 20 x 20 inputs under 48 templates fill 56 tiles of 64 x 128 on 148 SMs).
-    struct { int tm, tn, threads; double cost; } const tiles[] = {{128, 128, 256, 1.0}, {64, 128, 256, 1.05}, {32, 64, 128, 1.6}, {16, 32, 32, 2.0}};
+    // With masks the 8 x 8 blocking spills at 128 registers, 4 x 8 does not (terms from registers and shared memory alone: 6.5
+    // and 7.7 T/s).  Under 16 warps per SM, one CTA of the large tiles, nothing covers a CTA's barriers (16 x 64 x 32 x 32 input,
+    // 128 templates of 3x3: 206 us in 128 tiles of 128 x 128, 191 in 256 of 64 x 128; with masks 309 and 239).
+    struct { int tm, tn, threads; double cost; } const tiles[] = {{128, 128, 256, 1.0}, {64, 128, 256, g.mode == SIM_L2N_NAN ? 0.98 : 1.05}, {32, 64, 128, 1.6}, {16, 32, 32, 2.0}};
     int pick = 0;
     double best = 0;
     for (int i = 0; i < 4; ++i) {
         const double ctas = double((P + tiles[i].tn - 1) / tiles[i].tn) * ((g.M + tiles[i].tm - 1) / tiles[i].tm);
         const double per_sm = std::ceil(ctas / device_sm_count()), warps = per_sm * tiles[i].threads / 32;
-        const double t = per_sm * tiles[i].tm * tiles[i].tn * tiles[i].cost * (warps < 8 ? 8 / warps : 1.0);
+        const double t = per_sm * tiles[i].tm * tiles[i].tn * tiles[i].cost * (warps < 8 ? 8 / warps : 1.0) * (warps < 16 ? 1.15 : 1.0);
         if (i == 0 || t < best) { best = t; pick = i; }
     }
     const long long blocks = ((P + tiles[pick].tn - 1) / tiles[pick].tn) * ((g.M + tiles[pick].tm - 1) / tiles[pick].tm);
