@@ -99,3 +99,37 @@ def test_parameter_gradients_of_long_sums_are_folded(m, channels, block, batch, 
             want[k] = want[k] + g
     for g, e in zip(gpu_util.sim_ops.similarity_parameters_grad(x, t, w, dy, **kw), want):
         assert float((g.double() - e).norm() / e.norm()) <= _of_folded(2048, 32)
+
+
+# parameter gradients on 64 templates x 32 or 64 taps: (batch, channels, h, w), templates, blocks, strides, padding
+PARAM_TILES = [
+    ((1, 17, 6, 5), 33, (1, 1), (1, 1), (0, 0)),            # 17 taps, one chunk
+    ((2, 8, 9, 7), 64, (2, 2), (1, 1), (1, 1)),             # 32 taps
+    ((2, 11, 8, 9), 65, (3, 1), (1, 2), (1, 0)),            # 33 taps, a second row tile of one template
+    ((3, 16, 7, 8), 100, (2, 2), (2, 1), (0, 1)),           # 64 taps
+    ((2, 13, 9, 6), 70, (1, 5), (1, 1), (0, 2)),            # 65 taps: three tiles of 22
+    ((2, 43, 5, 6), 130, (3, 1), (1, 1), (1, 0)),           # 129 taps: five tiles of 26
+    ((2, 2, 17, 12), 40, (16, 1), (1, 1), (8, 0)),          # blocks of sixteen rows
+    ((2, 2, 18, 9), 40, (17, 1), (1, 1), (8, 0)),           # and of seventeen, which take the smaller tiles
+    ((40, 3, 13, 11), 64, (3, 3), (1, 1), (1, 1)),          # several chunks set aside
+]
+
+
+@pytest.mark.parametrize("mode", MODES, ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("special", [False, True], ids=["plain", "special"])
+@pytest.mark.parametrize("i", range(len(PARAM_TILES)))
+def test_parameter_gradients_at_the_edges_of_their_tiles(port, i, special, mode):
+    """special: values that equal a template's (the sign of a difference of 0 is 0), with L1 also infinities and NaN."""
+    shape, M, blocks, strides, padding = PARAM_TILES[i]
+    c = cases.sim_case("params%d" % i, shape, M, blocks=blocks, strides=strides, padding=padding, oob=0.0 if special else 0.3, seed=760 + i, **mode)
+    d = cases.sim_desc(c)
+    x, t, w, dy = cases.sim_inputs(c, port.sim_out_shape(d))
+    if special:
+        rng = np.random.default_rng(i)
+        x = np.where(rng.random(x.shape) < 0.1, rng.choice(t.reshape(-1), x.shape), x).astype(np.float32)
+        if mode["fn"] == "L1":
+            x[0, 0, 0, 0], x[0, 0, 1, 1], x[0, 0, 2, 2], t[1, 0, 0, 0] = np.inf, NAN, -np.inf, np.inf
+    got = gpu_util.sim_ops.similarity_parameters_grad(*(gpu_util.dev(a) for a in (x, t, w, dy)), **cases.sim_attrs(c))
+    d64 = cases.sim_desc(c, dtype=gpu_util.abi.F64)
+    for g, ref, ref64 in zip(got, port.similarity_params_grad(d, x, t, w, dy), port.similarity_params_grad(d64, *(a.astype(np.float64) for a in (x, t, w, dy)))):
+        cases.assert_parity(g.cpu().numpy(), ref, ref64, what=c["name"])
