@@ -2,17 +2,16 @@
 // current means and covariances, and the new parameters from them.  The distances are the L2 Similarity forward kernel and the
 // moments its parameter-gradient kernel; what lies between and around them is here.
 //
-// Bound: HBM.  The log-likelihoods of 64 components over 512 x 30 x 30 patches are 118 MB; the element-wise passes, the softmax
-// over a strided axis and the sum over positions as separate tensor operations took 435 us of a 935 us step.  Here a thread owns
-// a position with its k values in registers (up to 64 components: one read, one exponential each, one write in place; more are
-// read twice) and adds each responsibility to a sum of its own in shared memory.  The whole step: 935 -> 423 us.
+// Bound: HBM, 36 us for the log-likelihoods of 64 components over 512 x 30 x 30 patches (118 MB read and written in place).  G lanes share
+// a position, each with every G-th component in registers: a maximum and a sum over G lanes, and since a lane always has the same
+// components, their masses stay in its registers over all positions.  A thread with all 64 components of a position (251 registers,
+// eight warps per SM, masses in shared memory) took 101 us; this takes 57 (24 warps per SM; with 126 registers, 16 warps, 67).
 #include "kernels.cuh"
 
 namespace simnets {
 namespace {
 
-constexpr int kMixThreads = 128;
-constexpr size_t kMixSmem = 100 * 1024;
+constexpr int kMixThreads = 128, kMixMost = 198;          // (198: what the first form of this had room for)
 
 // 1 / covariance and log-determinant of every component
 __global__ void __launch_bounds__(128) mixture_prep(int taps, const float* __restrict__ covs, float* __restrict__ scales, float* __restrict__ logdet) {
@@ -35,78 +34,61 @@ __global__ void __launch_bounds__(128) mixture_prep(int taps, const float* __res
 }
 
 // score[b][c][p] = -sum scale (patch - mean)^2 becomes the responsibility softmax_c(score / 2 - logdet / 2); part[cta][c] = sum
-// over the CTA's positions.
-template <int KT>
-__global__ void __launch_bounds__(kMixThreads) mixture_responsibilities(long long P, int k, int N, float* __restrict__ score, const float* __restrict__ logdet,
+// over the CTA's positions.  Lane l of a warp: position l mod (32 / G) of its run, components l / (32 / G) + G i, KT of them.
+template <int G, int KT>
+__global__ void __launch_bounds__(kMixThreads, 6) mixture_responsibilities(long long P, int k, FastDiv f_N, float* __restrict__ score, const float* __restrict__ logdet,
                                                                         float* __restrict__ part) {
     stream_order();
-    extern __shared__ float sm[];                       // [k][128] sums, [k] log-determinants
-    float* ld = sm + k * kMixThreads;
-    for (int i = threadIdx.x; i < k * kMixThreads; i += kMixThreads) sm[i] = 0.f;
-    for (int c = threadIdx.x; c < k; c += kMixThreads) ld[c] = logdet[c];
+    constexpr int RUN = 32 / G, WARPS = kMixThreads / 32;
+    __shared__ float red[WARPS][G * KT], ld[G * KT];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, first = lane / RUN;
+    const long long N = f_N.d, step = G * N;
+    for (int i = threadIdx.x; i < G * KT; i += kMixThreads) ld[i] = i < k ? logdet[i] : 0.f;
     __syncthreads();
-    for (long long j = (long long)blockIdx.x * kMixThreads + threadIdx.x; j < P; j += (long long)gridDim.x * kMixThreads) {
-        const long long n = j / N;
-        float* p = score + n * k * N + (j - n * N);
-        float hi = -CUDART_INF_F, sum = 0.f;
-        if (KT > 0) {                                   // KT >= k
-            float v[KT > 0 ? KT : 1];
+    float mass[KT];
 #pragma unroll
-            for (int c = 0; c < KT; ++c) v[c] = c < k ? p[(long long)c * N] : -CUDART_INF_F;
+    for (int i = 0; i < KT; ++i) mass[i] = 0.f;
+    for (long long j0 = ((long long)blockIdx.x * WARPS + warp) * RUN; j0 < P; j0 += (long long)gridDim.x * WARPS * RUN) {
+        const long long j = j0 + lane % RUN;
+        const bool live = j < P;
+        const long long n = !live ? 0 : P <= 0x7fffffffLL ? (long long)fast_div(uint32_t(j), f_N) : j / N;
+        float* p = score + n * k * N + (live ? j - n * N : 0) + first * N;
+        const float* q = p;
+        float v[KT], hi = -CUDART_INF_F, sum = 0.f;
 #pragma unroll
-            for (int c = 0; c < KT; ++c) {
-                if (c < k) v[c] = 0.5f * (v[c] - ld[c]);
-                hi = fmaxf(hi, v[c]);
-            }
+        for (int i = 0; i < KT; ++i, q += step) v[i] = live && first + G * i < k ? *q : -CUDART_INF_F;
 #pragma unroll
-            for (int c = 0; c < KT; ++c) { v[c] = c < k ? expf(v[c] - hi) : 0.f; sum += v[c]; }
-            const float inv = 1.f / sum;
+        for (int i = 0; i < KT; ++i) { v[i] = 0.5f * (v[i] - ld[first + G * i]); hi = fmaxf(hi, v[i]); }
 #pragma unroll
-            for (int c = 0; c < KT; ++c) {
-                if (c >= k) break;
-                const float r = v[c] * inv;
-                p[(long long)c * N] = r;
-                sm[c * kMixThreads + threadIdx.x] += r;
-            }
-            continue;
-        }
-        // (the running maximum may still be -inf, components so far away that their distance overflowed: exp(-inf - 0) adds nothing)
-        const auto above = [](float top) { return top > -CUDART_INF_F ? top : 0.f; };
-        int c = 0;
-        for (; c + 8 <= k; c += 8) {
-            float v[8], top = hi;
+        for (int d = RUN; d < 32; d <<= 1) hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = 0.5f * (p[(long long)(c + u) * N] - ld[c + u]);
+        for (int i = 0; i < KT; ++i) { v[i] = first + G * i < k ? expf(v[i] - hi) : 0.f; sum += v[i]; }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) top = fmaxf(top, v[u]);
-            const float ref = above(top);
-            float add = 0.f;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) add += expf(v[u] - ref);
-            sum = sum * expf(hi - ref) + add;
-            hi = top;
-        }
-        for (; c < k; ++c) {
-            const float v = 0.5f * (p[(long long)c * N] - ld[c]), top = fmaxf(hi, v), ref = above(top);
-            sum = sum * expf(hi - ref) + expf(v - ref);
-            hi = top;
-        }
+        for (int d = RUN; d < 32; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (!live) continue;
         const float inv = 1.f / sum;
-#pragma unroll 8
-        for (c = 0; c < k; ++c) {
-            const float r = expf(0.5f * (p[(long long)c * N] - ld[c]) - hi) * inv;
-            p[(long long)c * N] = r;
-            sm[c * kMixThreads + threadIdx.x] += r;
-        }
+        asm volatile("" : "+l"(p));                     // (sixteen addresses kept from the reads: 126 registers instead of 80)
+#pragma unroll
+        for (int i = 0; i < KT; ++i, p += step)
+            if (first + G * i < k) {
+                const float r = v[i] * inv;
+                *p = r;
+                mass[i] += r;
+            }
+    }
+#pragma unroll
+    for (int i = 0; i < KT; ++i) {
+        float s = mass[i];
+#pragma unroll
+        for (int d = RUN / 2; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (lane % RUN == 0) red[warp][first + G * i] = s;
     }
     __syncthreads();
-    // one warp per component, a quarter of them each
-    for (int c = threadIdx.x >> 5; c < k; c += kMixThreads / 32) {
+    for (int c = threadIdx.x; c < k; c += kMixThreads) {
         float s = 0.f;
-        for (int i = threadIdx.x & 31; i < kMixThreads; i += 32) s += sm[c * kMixThreads + i];
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-        if ((threadIdx.x & 31) == 0) part[(size_t)blockIdx.x * k + c] = s;
+        for (int w = 0; w < WARPS; ++w) s += red[w][c];
+        part[(size_t)blockIdx.x * k + c] = s;
     }
 }
 
@@ -135,10 +117,10 @@ __global__ void __launch_bounds__(256) mixture_parameters(int n, int taps, float
     new_means[i] = means[i] + step;
 }
 
-size_t mix_smem(int k) { return sizeof(float) * (size_t)k * (kMixThreads + 1); }
+// lanes per position: at most sixteen components each
+int mix_lanes(int k) { return k <= 64 ? 4 : (k <= 128 ? 8 : 16); }
 int mix_ctas(const SimGeo& g) {
-    const long long P = (long long)g.B * g.N, tiles = (P + kMixThreads - 1) / kMixThreads;
-    const long long resident = (long long)device_sm_count() * std::max<long long>(1, std::min<long long>(12, (200 * 1024) / (long long)(mix_smem(g.M) + 1024)));
+    const long long P = (long long)g.B * g.N, per = kMixThreads / mix_lanes(g.M), tiles = (P + per - 1) / per, resident = (long long)device_sm_count() * 6;
     const long long rounds = (tiles + resident - 1) / resident;
     return int((tiles + rounds - 1) / rounds);
 }
@@ -161,7 +143,7 @@ MixWs mix_carve(const SimGeo& g, void* base) {
 }  // namespace
 
 bool mixture_shape(const SimGeo& g, bool f64, uint32_t flags) {
-    return sim_use_tiled(g, f64, flags) && flags == 0 && g.mode == SIM_L2 && (long long)g.C * g.H * g.W < (1LL << 29) && mix_smem(g.M) <= kMixSmem;
+    return sim_use_tiled(g, f64, flags) && flags == 0 && g.mode == SIM_L2 && (long long)g.C * g.H * g.W < (1LL << 29) && g.M <= kMixMost;
 }
 size_t mixture_workspace_bytes(const SimGeo& g) { return mix_carve(g, nullptr).bytes; }
 
@@ -172,13 +154,10 @@ cudaError_t launch_mixture_statistics(const SimGeo& g, const float* x, const flo
     cudaError_t e = launch_sim_fwd_tiled(g, x, means, w.scales, w.score, w.sim, 0, s);
     if (e != cudaSuccess) return e;
     const int ctas = mix_ctas(g);
-#define MIX(KT) in_stream_order(mixture_responsibilities<KT>, ctas, kMixThreads, mix_smem(g.M), s)((long long)g.B * g.N, g.M, g.N, w.score, w.logdet, w.part)
-    if (g.M <= 16) MIX(16); else if (g.M <= 32) MIX(32); else if (g.M <= 48) MIX(48); else if (g.M <= 64) MIX(64);
-    else {
-        e = cudaFuncSetAttribute(mixture_responsibilities<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMixSmem));
-        if (e != cudaSuccess) return e;
-        MIX(0);
-    }
+    const FastDiv f_N = make_fastdiv(g.N);
+#define MIX(G, KT) in_stream_order(mixture_responsibilities<G, KT>, ctas, kMixThreads, 0, s)((long long)g.B * g.N, g.M, f_N, w.score, w.logdet, w.part)
+    if (g.M <= 16) MIX(4, 4); else if (g.M <= 32) MIX(4, 8); else if (g.M <= 48) MIX(4, 12); else if (g.M <= 64) MIX(4, 16);
+    else if (g.M <= 96) MIX(8, 12); else if (g.M <= 128) MIX(8, 16); else MIX(16, 13);
 #undef MIX
     in_stream_order(mixture_mass, g.M, 128, 0, s)(ctas, g.M, w.part, stats + 2 * n);
     count_launch(3);

@@ -155,3 +155,19 @@ def test_components_at_an_infinite_distance_claim_nothing():
     far.update(x)
     assert bool((far.means[:8] == 1e20).all()) and torch.allclose(far.covs[:8], torch.full_like(far.covs[:8], near.min_var))
     assert torch.allclose(far.means[8:], near.means, rtol=1e-5, atol=1e-6) and torch.allclose(far.covs[8:], near.covs, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("k", [1, 3, 16, 17, 33, 49, 64, 65, 97, 128, 129, 198])
+@pytest.mark.parametrize("shape", [(1, 2, 5, 7), (5, 1, 13, 12), (40, 3, 24, 23)], ids=["few", "odd", "many"])
+def test_responsibilities_at_the_edges_of_their_lanes(shape, k):
+    """Component counts around what 4, 8 and 16 lanes of a position hold, position counts that divide nothing: float32 statistics
+    against the float64 step from the same parameters (tensor operations, softmax over all components)."""
+    x = torch.rand(shape, generator=torch.Generator(device="cuda").manual_seed(k), device="cuda")
+    one, two = un.DiagonalGMM([2, 2], [1, 1], k), un.DiagonalGMM([2, 2], [1, 1], k)
+    one.init(x)
+    one.covs = (one.covs * 4).contiguous()                    # (wide components: every one of them holds a visible share)
+    two.means, two.covs = one.means.double(), one.covs.double()
+    one.update(x)
+    two.update(x.double())
+    _close(one.means, two.means.cpu().numpy().reshape(k, -1), TOL[torch.float32], "means")
+    _close(one.covs, two.covs.cpu().numpy().reshape(k, -1), TOL[torch.float32], "covariances")
