@@ -8,9 +8,15 @@
 //
 // With strides a pixel only meets the taps of its own phase, (h + pad) mod stride = kh mod stride: the grid's y index is the
 // phase, and a CTA walks the taps of that phase only (a 5x3 block at stride 2x1 would otherwise spend half its terms on dy
-// values that are zero by construction).  The (tap, m) cursor of every staging thread advances by additions; dividing the
-// reduction index by M for each staged value had taken as many instructions as the terms themselves (256 x 64 x 32 x 32 input,
-// 256 templates of 3x3: 10.2 ms).
+// values that are zero by construction).
+//
+// Bound: the FP32 pipe, 3 packed operations per term, which every other instruction holds up.  A thread of 4, 5 or 6 channels x 8
+// pixels takes 10 T terms/s from registers and shared memory, so the tile's rows follow the channels (16, 20, 24, 32, 40, 48 or 64 of
+// them; 19 channels in 32 rows had spent 41 % on padding), and a chunk is instances of ONE tap: its operands advance by one addition
+// each, where a cursor per staged value had cost several instructions.  256 x 64 x 32 x 32 input, 256 templates of 3x3: 4981 -> 4237 us
+// (62 -> 74 % of the pipe); 37 x 19 x 45 x 37, 100 of 5x3 at stride 2 and 1, L1:
+// 490 -> 277; 64 x 24 x 30 x 31, 90 of 3x3: 308 -> 203.  L1 adds e with the sign of d put on it, 0 selected where d is 0 or NaN: one
+// instruction per term less than multiplying by a sign (from registers 5.0 -> 5.9 T terms/s).
 //
 // NaN pixels give 0 in the ignore_nan_input modes, and so does a pixel that no patch covers in every mode.  A tap that the
 // padding cuts off, or a step past the last one, contributes 0 * (t - x), which is NaN for an infinite x (or an infinite
@@ -23,9 +29,11 @@
 namespace simnets {
 namespace {
 
-__host__ __device__ inline int dx_pad4(int v) { return (v + 3) & ~3; }
 // sign of d, 0 for 0 and NaN as in the reference
 __device__ __forceinline__ float dx_sign(float d) { return fabsf(d) > 0.f ? __uint_as_float(0x3f800000u | (__float_as_uint(d) & 0x80000000u)) : 0.f; }
+
+// e sign(d)
+__device__ __forceinline__ float dx_signed(float e, float d) { return fabsf(d) > 0.f ? __uint_as_float(__float_as_uint(e) ^ (__float_as_uint(d) & 0x80000000u)) : 0.f; }
 
 // The pixels and taps of one phase along one axis: pixels first, first + stride, ... (n of them), taps r, r + stride, ... (taps
 // of them); pixel i meets tap a at output i + shift - a.
@@ -78,15 +86,25 @@ __device__ __noinline__ void dx_redo(const SimGeo& g, const float* __restrict__ 
     if (is_nan(dx[at]) && !is_nan(x[at])) dx[at] = sim_exact_dx(g, x, tm, wt, dy, at);
 }
 
-// (t, s w)[tap][m][Cp], channel-contiguous, for the tile kernel
-__global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, const float* __restrict__ tm, const float* __restrict__ wt, float* __restrict__ dxp) {
+// The tile: 4 WI x 16 threads of RM channels x 8 pixels each, KC steps per chunk.  A thread's channels are one or two 16-byte vectors
+// of a row of parameters, so rows of five or six channels per thread are stored in slots of eight.  Sixteen steps per chunk where a
+// thread then stages eight values of dy; the narrower tiles would hold sixteen or thirty-two (96 channels of 48-row tiles: 15 % slower).
+template <int RM, int WI> struct DxTile {
+    static constexpr int SLOT = RM == 4 ? 4 : 8, TM = 4 * WI * RM, ROW = 4 * WI * SLOT, TN = 128, T = 64 * WI, KC = WI == 4 ? 16 : 8;
+    static constexpr int COLS = T < TN ? TN / T : 1, QSTEP = T > TN ? T / TN : 1, QPER = KC / QSTEP, A_COPIES = 2 * KC * ROW / 4;
+    static constexpr int STAGE = 2 * KC * ROW + KC * TN, SLOT_BYTES = 4 * RM * 8 * T, PER_SM = WI == 4 ? 2 : (WI == 2 ? (RM == 4 ? 4 : 3) : (RM == 6 ? 5 : 6));
+};
+
+// (t, s w)[tap][m][channel tile][slots], for the tile kernel
+__global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, int rm, int slot, int rows, int tiles, const float* __restrict__ tm, const float* __restrict__ wt,
+                                                   float* __restrict__ dxp) {
     stream_order();
-    const int taps = g.bh * g.bw, cp = dx_pad4(g.C);
-    const long long total = (long long)taps * g.M * cp;
+    const int taps = g.bh * g.bw, row = tiles * rows * slot;             // (rows: of threads per tile)
+    const long long total = (long long)taps * g.M * row;
     const float s = g.mode == SIM_L2 ? 2.f : 1.f;
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
-        const int c = int(i % cp);
-        const long long q = i / cp;
+        const long long q = i / row;
+        const int e = int(i - q * row), r = e % slot, c = r < rm ? e / slot * rm + r : g.C;
         const int m = int(q % g.M), tap = int(q / g.M);
         const size_t src = ((size_t)m * g.C + c) * taps + tap;
         const float w = c < g.C ? wt[src] : 0.f;
@@ -100,42 +118,39 @@ __global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, const float* __rest
 // of the gradient's norm against 3e-7).
 constexpr int kDxFold = 256;
 
-template <int TM> struct DxCfg {
-    static constexpr int RM = TM == 128 ? 8 : 4, TN = TM == 16 ? 256 : 128;
-    using Cfg = TileCfg<TM, TN, 8, RM, 8, 2, 1>;
-    static constexpr int SLOT_BYTES = 4 * RM * 8 * Cfg::THREADS;
-};
-
-template <int TM, int MODE>
-__global__ void __launch_bounds__(DxCfg<TM>::Cfg::THREADS, DxCfg<TM>::Cfg::THREADS == 256 ? (TM == 128 ? 1 : 2) : 3)
+template <int RM, int WI, int MODE>
+__global__ void __launch_bounds__(DxTile<RM, WI>::T, DxTile<RM, WI>::PER_SM)
 sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, const float* __restrict__ dxp, const float* __restrict__ tm, const float* __restrict__ wt,
              const float* __restrict__ dy, float* __restrict__ dx) {
     stream_order();
     constexpr bool L1 = MODE == SIM_L1 || MODE == SIM_L1_SKIP;
     constexpr bool SKIP_NAN = MODE == SIM_L2N_NAN || MODE == SIM_L1_SKIP;
-    using Cfg = typename DxCfg<TM>::Cfg;
-    constexpr int T = Cfg::THREADS, COLS = Cfg::TN > T ? Cfg::TN / T : 1, QSTEP = T > Cfg::TN ? T / Cfg::TN : 1, QPER = Cfg::KC / QSTEP;
-    constexpr int VEC = TM / 4, APER = (2 * Cfg::KC * VEC + T - 1) / T;
-    __shared__ __align__(16) float smem[Cfg::SMEM_FLOATS];
-    extern __shared__ __align__(16) float2 slots[];                     // [RM x RN / 2][THREADS], if the launch has sums of more than kDxFold steps
-    __shared__ long long col_base[Cfg::TN];
-    __shared__ unsigned char col_covered[Cfg::TN];
+    using Tile = DxTile<RM, WI>;
+    constexpr int T = Tile::T, TN = Tile::TN, TM = Tile::TM, ROW = Tile::ROW, SLOT = Tile::SLOT, KC = Tile::KC, COLS = Tile::COLS, QSTEP = Tile::QSTEP, QPER = Tile::QPER;
+    constexpr int PLANE = KC * ROW, A_PER = (Tile::A_COPIES + T - 1) / T;
+    __shared__ __align__(16) float smem[2 * Tile::STAGE];
+    extern __shared__ __align__(16) float2 slots[];                     // [4 RM][T], if the launch has sums of more than kDxFold steps
+    __shared__ long long col_base[TN];
+    __shared__ unsigned char col_covered[TN];
     const DxPhase ph(g, blockIdx.y);
     const int ctiles = (g.C + TM - 1) / TM;
     const int ct = blockIdx.x % ctiles;
-    const long long j0 = (long long)(blockIdx.x / ctiles) * Cfg::TN;
+    const long long j0 = (long long)(blockIdx.x / ctiles) * TN;
     if (j0 >= (long long)g.B * ph.h.n * ph.w.n) return;
     const int i0 = ct * TM;
-    const int Q = ph.h.taps * ph.w.taps * g.M, ldc = dx_pad4(g.C);
-    const size_t plane = (size_t)g.bh * g.bw * g.M * ldc;
-    const TileThread<Cfg> t;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // 4 x 8 threads per warp, rows interleaved in pairs as in tile.cuh; columns tj * 4 .. + 3 of either half of the tile
+    const int ti = (warp % WI) * 4 + (((lane >> 4) << 1) | (lane & 1)), tj = (warp / WI) * 8 + ((lane & 15) >> 1);
+    const auto col = [&](int c) { return (c >> 2) * (TN / 2) + tj * 4 + (c & 3); };
 
-    // dy staging: columns s_lane (+ T), steps s_k, s_k + QSTEP, ... of every chunk; the cursor (tap a, b and m) moves along
-    const int s_lane = threadIdx.x % Cfg::TN, s_k = threadIdx.x / Cfg::TN;
+    // A chunk is KC instances of one tap (fewer at the end of a tap).  The next chunk to be staged: tap (a, b) of the phase, instances
+    // from m_next on.  This thread brings dy of columns s_lane (+ T), instances s_k, s_k + QSTEP, ...
+    const int s_lane = threadIdx.x % TN, s_k = threadIdx.x / TN, chunks_per_tap = (g.M + KC - 1) / KC;
+    const int chunks = ph.h.taps * ph.w.taps * chunks_per_tap;
+    int a = 0, b = 0, m_next = 0, row_next = 0;                          // row_next: first row of the chunk in dxp
     DxPixel px[COLS];
-    long long at[COLS];
-    int ca = 0, cb_ = 0, cm = s_k;
-    float rb[COLS][QPER];
+    const float* at[COLS];
+    bool ok[COLS];
 #pragma unroll
     for (int u = 0; u < COLS; ++u) {
         px[u] = DxPixel(g, ph, j0 + s_lane + u * T);
@@ -143,100 +158,143 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
         col_covered[s_lane + u * T] = px[u].covered(g, ph);
     }
     auto locate = [&]() {
-        while (cm >= g.M) { cm -= g.M; if (++cb_ == ph.w.taps) { cb_ = 0; ++ca; } }
 #pragma unroll
         for (int u = 0; u < COLS; ++u) {
-            const long long o = ca < ph.h.taps ? px[u].at(g, ca, cb_) : -1;
-            at[u] = o < 0 ? -1 : o + (long long)cm * g.N;
+            const long long o = a < ph.h.taps ? px[u].at(g, a, b) : -1;
+            ok[u] = o >= 0;
+            at[u] = dy + (ok[u] ? o + (long long)s_k * g.N : 0);
         }
+        row_next = ((ph.rh + a * g.sh) * g.bw + ph.rw + b * g.sw) * g.M;
     };
-    if (Q > 0) locate();
-    const size_t step = (size_t)QSTEP * g.N;
-    auto fetchB = [&](int, float*) {
+    if (chunks > 0) locate();
+    // parameter staging: A_PER copies of 16 bytes per thread; their places inside a chunk do not change
+    const size_t row_floats = (size_t)ctiles * ROW, plane = (size_t)g.bh * g.bw * g.M * row_floats;
+    float rb[COLS][QPER];
+    auto fetch = [&](float* stage) {
 #pragma unroll
-        for (int s = 0; s < QPER; ++s) {
+        for (int v = 0; v < A_PER; ++v) {
+            const int i = threadIdx.x + v * T, p = i / (PLANE / 4), r = i % (PLANE / 4) / (ROW / 4), e = i % (ROW / 4) * 4;
+            const bool there = m_next + r < g.M;
+            if (Tile::A_COPIES % T == 0 || i < Tile::A_COPIES)
+                cp_async16(stage + p * PLANE + r * ROW + e, there ? dxp + p * plane + (row_next + r) * row_floats + ct * ROW + e : dxp, there ? 16 : 0);
+        }
+        const bool whole = m_next + KC <= g.M;
 #pragma unroll
-            for (int u = 0; u < COLS; ++u) {
+        for (int u = 0; u < COLS; ++u)
+#pragma unroll
+            for (int s = 0; s < QPER; ++s) {
                 rb[u][s] = 0.f;
-                if (at[u] >= 0) { rb[u][s] = __ldg(dy + at[u]); at[u] += step; }
+                if (ok[u] && (whole || m_next + s_k + s * QSTEP < g.M)) rb[u][s] = __ldg(at[u] + (size_t)(s * QSTEP) * g.N);
             }
-            cm += QSTEP;
-            if (cm >= g.M) locate();
+        m_next += KC; row_next += KC;
+#pragma unroll
+        for (int u = 0; u < COLS; ++u) at[u] += (size_t)KC * g.N;
+        if (m_next >= g.M) {
+            m_next = 0;
+            if (++b == ph.w.taps) { b = 0; ++a; }
+            locate();
         }
     };
-    auto commitB = [&](float* Bs) {
+    auto commit = [&](float* stage) {
+        float* B = stage + 2 * PLANE + s_k * TN + s_lane;
 #pragma unroll
         for (int s = 0; s < QPER; ++s)
 #pragma unroll
-            for (int u = 0; u < COLS; ++u) Bs[(s_k + s * QSTEP) * Cfg::TN + s_lane + u * T] = rb[u][s];
+            for (int u = 0; u < COLS; ++u) B[s * QSTEP * TN + u * T] = rb[u][s];
+        cp_async_wait_all();
     };
-    // parameter staging: APER 16-byte copies per thread and chunk, each with a cursor of its own
-    int aa[APER], ab[APER], am[APER];
-#pragma unroll
-    for (int v = 0; v < APER; ++v) { aa[v] = ab[v] = 0; am[v] = ((threadIdx.x + v * T) % (Cfg::KC * VEC)) / VEC; }
-    auto fetchA = [&](int, float* As) {
-#pragma unroll
-        for (int v = 0; v < APER; ++v) {
-            const int idx = threadIdx.x + v * T;
-            if (idx < 2 * Cfg::KC * VEC) {
-                const int p = idx / (Cfg::KC * VEC), row = (idx % (Cfg::KC * VEC)) / VEC, e = (idx % VEC) * 4;
-                while (am[v] >= g.M) { am[v] -= g.M; if (++ab[v] == ph.w.taps) { ab[v] = 0; ++aa[v]; } }
-                const int left = aa[v] < ph.h.taps ? g.C - (i0 + e) : 0;          // (rows of dxp are padded to a multiple of four channels)
-                const int tap = (ph.rh + aa[v] * g.sh) * g.bw + ph.rw + ab[v] * g.sw;
-                cp_async16(As + (p * Cfg::KC + row) * TM + e, left > 0 ? dxp + p * plane + ((size_t)tap * g.M + am[v]) * ldc + i0 + e : dxp, left > 0 ? 16 : 0);
-                am[v] += Cfg::KC;
-            }
-        }
-    };
-    auto commitA = [&](float*) { cp_async_wait_all(); };
 
     // this thread's own x values (one per output)
     __syncthreads();
-    float2 xx[Cfg::RM][Cfg::RN / 2], acc[Cfg::RM][Cfg::RN / 2];
+    float2 xx[RM][4], acc[RM][4];
     const size_t chw = (size_t)g.H * g.W;
 #pragma unroll
-    for (int r_ = 0; r_ < Cfg::RM; ++r_) {
-        const int c = i0 + t.row(r_);
+    for (int r_ = 0; r_ < RM; ++r_) {
+        const int c = i0 + ti * RM + r_;
 #pragma unroll
-        for (int c_ = 0; c_ < Cfg::RN; ++c_) {
-            const long long cb = col_base[t.col(c_)];
+        for (int c_ = 0; c_ < 8; ++c_) {
+            const long long cb = col_base[col(c_)];
             const float v = (c < g.C && cb >= 0) ? __ldg(x + cb + (size_t)c * chw) : 0.f;
             if (c_ & 1) xx[r_][c_ >> 1].y = -v; else xx[r_][c_ >> 1].x = -v;
             acc[r_][c_ >> 1] = make_float2(0.f, 0.f);
         }
     }
-    auto comb = [&](int r_, int cp, const float2 (&a)[2], const float2 (&b)[1]) {
-        const float2 d = add2(a[0], xx[r_][cp]);
-        const float2 e = mul2(a[1], b[0]);
-        acc[r_][cp] = fma2(e, L1 ? make_float2(dx_sign(d.x), dx_sign(d.y)) : d, acc[r_][cp]);
-    };
-    const int chunks = (Q + Cfg::KC - 1) / Cfg::KC;
-    auto fold = [&](int c) {
-        const bool first = c == kDxFold / Cfg::KC;
+    auto step = [&](const float* stage, int q) {
+        float t[SLOT], w[SLOT];
+        const float* A = stage + q * ROW + ti * SLOT;
+        const float4 t4 = *reinterpret_cast<const float4*>(A), w4 = *reinterpret_cast<const float4*>(A + PLANE);
+        t[0] = t4.x; t[1] = t4.y; t[2] = t4.z; t[3] = t4.w;
+        w[0] = w4.x; w[1] = w4.y; w[2] = w4.z; w[3] = w4.w;
+        if (RM == 5) { t[SLOT > 4 ? 4 : 0] = A[4]; w[SLOT > 4 ? 4 : 0] = A[PLANE + 4]; }
+        if (RM == 6) {
+            const float2 t2 = *reinterpret_cast<const float2*>(A + 4), w2 = *reinterpret_cast<const float2*>(A + PLANE + 4);
+            t[SLOT > 4 ? 4 : 0] = t2.x; t[SLOT > 4 ? 5 : 0] = t2.y;
+            w[SLOT > 4 ? 4 : 0] = w2.x; w[SLOT > 4 ? 5 : 0] = w2.y;
+        }
+        float2 g2[4];
 #pragma unroll
-        for (int i = 0; i < Cfg::RM * Cfg::RN / 2; ++i) {
-            float2& a = acc[i / (Cfg::RN / 2)][i % (Cfg::RN / 2)];
-            slots[i * T + threadIdx.x] = first ? a : add2(slots[i * T + threadIdx.x], a);
-            a = make_float2(0.f, 0.f);
+        for (int h = 0; h < 2; ++h) {
+            const float4 v = *reinterpret_cast<const float4*>(stage + 2 * PLANE + q * TN + h * (TN / 2) + tj * 4);
+            g2[2 * h] = make_float2(v.x, v.y); g2[2 * h + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int r = 0; r < RM; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float2 d = add2(splat2(t[r]), xx[r][c]), e = mul2(splat2(w[r]), g2[c]);
+                acc[r][c] = L1 ? add2(acc[r][c], make_float2(dx_signed(e.x, d.x), dx_signed(e.y, d.y))) : fma2(e, d, acc[r][c]);
+            }
+    };
+    auto compute = [&](const float* stage, int steps) {
+        // (one branch in the middle and no more: a branch every four steps costs 15 %, and a second copy of the steps for partial
+        // chunks as much again where the code grows with it, L1 above all)
+#pragma unroll
+        for (int q = 0; q < KC; ++q) {
+            if (q == KC / 2 && steps <= KC / 2) break;
+            step(stage, q);
         }
     };
-    tile_mainloop<Cfg, false, false, kDxFold / Cfg::KC>(smem, chunks, t, fetchA, fetchB, commitA, commitB, comb, fold);
-    if (Q > kDxFold)
+    if (chunks > 0) {
+        fetch(smem);
+        commit(smem);
+        __syncthreads();
+        int m_now = 0, since = 0;
+        bool aside = false;
+        for (int i = 0; i < chunks; ++i) {
+            float* now = smem + (i & 1) * Tile::STAGE;
+            float* next = smem + ((i + 1) & 1) * Tile::STAGE;
+            const bool more = i + 1 < chunks;
+            const int steps = min(KC, g.M - m_now);
+            if ((since += steps) > kDxFold) {
 #pragma unroll
-        for (int i = 0; i < Cfg::RM * Cfg::RN / 2; ++i) {
-            float2& a = acc[i / (Cfg::RN / 2)][i % (Cfg::RN / 2)];
-            a = add2(slots[i * T + threadIdx.x], a);
+                for (int k = 0; k < RM * 4; ++k) {
+                    float2& v = acc[k >> 2][k & 3];
+                    slots[k * T + threadIdx.x] = aside ? add2(slots[k * T + threadIdx.x], v) : v;
+                    v = make_float2(0.f, 0.f);
+                }
+                aside = true;
+                since = steps;
+            }
+            if (more) fetch(next);
+            compute(now, steps);
+            if (more) commit(next);
+            __syncthreads();
+            if ((m_now += KC) >= g.M) m_now = 0;
         }
+        if (aside)
+#pragma unroll
+            for (int k = 0; k < RM * 4; ++k) acc[k >> 2][k & 3] = add2(slots[k * T + threadIdx.x], acc[k >> 2][k & 3]);
+    }
 
     bool redo = false;
 #pragma unroll
-    for (int c_ = 0; c_ < Cfg::RN; ++c_) {
-        const long long cb = col_base[t.col(c_)];
+    for (int c_ = 0; c_ < 8; ++c_) {
+        const long long cb = col_base[col(c_)];
         if (cb < 0) continue;
-        const bool covered = col_covered[t.col(c_)];
+        const bool covered = col_covered[col(c_)];
 #pragma unroll
-        for (int r_ = 0; r_ < Cfg::RM; ++r_) {
-            const int c = i0 + t.row(r_);
+        for (int r_ = 0; r_ < RM; ++r_) {
+            const int c = i0 + ti * RM + r_;
             if (c >= g.C) continue;
             float v = (c_ & 1) ? acc[r_][c_ >> 1].y : acc[r_][c_ >> 1].x;
             const float xv = (c_ & 1) ? xx[r_][c_ >> 1].y : xx[r_][c_ >> 1].x;
@@ -247,9 +305,9 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
     }
     if (redo)
 #pragma unroll 1
-        for (int i = 0; i < Cfg::RM * Cfg::RN; ++i) {
-            const int c = i0 + t.row(i / Cfg::RN);
-            const long long cb = col_base[t.col(i % Cfg::RN)];
+        for (int i = 0; i < RM * 8; ++i) {
+            const int c = i0 + ti * RM + i / 8;
+            const long long cb = col_base[col(i % 8)];
             if (c < g.C && cb >= 0) dx_redo(g, x, tm, wt, dy, dx, cb + (long long)(c * chw));
         }
 }
@@ -354,7 +412,25 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_con
 
 }  // namespace
 
-size_t sim_dx_scratch_floats(const SimGeo& g) { return g.C <= 8 ? 0 : 2 * (size_t)g.bh * g.bw * g.M * dx_pad4(g.C); }
+// The tile of a number of channels: the least padding, a tile of few rows counting for more (every row of it shares the dy values it
+// stages).
+struct DxPick { int rm, wi, slot, tiles; };
+static DxPick dx_pick(int channels) {
+    static const struct { int rm, wi; } all[] = {{4, 4}, {6, 2}, {5, 2}, {4, 2}, {6, 1}, {5, 1}, {4, 1}};
+    DxPick best = {4, 4, 4, 1};
+    double least = 0;
+    for (const auto& t : all) {
+        const int rows = 4 * t.rm * t.wi, tiles = (channels + rows - 1) / rows;
+        const double cost = double(tiles) * rows * (1 + 3.0 / rows);
+        if (least == 0 || cost < least) { least = cost; best = {t.rm, t.wi, t.rm == 4 ? 4 : 8, tiles}; }
+    }
+    return best;
+}
+size_t sim_dx_scratch_floats(const SimGeo& g) {
+    if (g.C <= 8) return 0;
+    const DxPick t = dx_pick(g.C);
+    return 2 * (size_t)g.bh * g.bw * g.M * t.tiles * 4 * t.wi * t.slot;
+}
 
 cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const float* w, const float* dy, float* dx, float* dxp, cudaStream_t s) {
     const int phases = g.sh * g.sw;
@@ -388,30 +464,37 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
         count_launch();
         return cudaGetLastError();
     }
-    const long long total = (long long)g.bh * g.bw * g.M * dx_pad4(g.C);
-    in_stream_order(sim_dx_prep, int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(g, t, w, dxp);
-    // the tile height that pads the channels least; of two equal ones the taller (its dy values serve more rows)
-    const auto padded = [&](int tm) { return (g.C + tm - 1) / tm * tm; };
-    int tm = 128;
-    for (int c : {64, 32, 16}) if (padded(c) < padded(tm)) tm = c;
-    if (tm == 128 && g.C <= 64) tm = 64;
-    const int tn = tm == 16 ? 256 : 128;
-    const long long blocks = ((pixels + tn - 1) / tn) * ((g.C + tm - 1) / tm);
+    const DxPick pick = dx_pick(g.C);
+    const long long total = (long long)g.bh * g.bw * g.M * pick.tiles * 4 * pick.wi * pick.slot;
+    in_stream_order(sim_dx_prep, int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(g, pick.rm, pick.slot, 4 * pick.wi, pick.tiles, t, w, dxp);
+    const long long blocks = (pixels + 127) / 128 * pick.tiles;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const dim3 grid{unsigned(blocks), unsigned(phases)};
     const bool folds = (long long)((g.bh + g.sh - 1) / g.sh) * ((g.bw + g.sw - 1) / g.sw) * g.M > kDxFold;         // (the most taps of a phase)
-#define DX(TM, MODE)                                                                                                                          \
+#define DX(RM, WI, MODE)                                                                                                                      \
     do {                                                                                                                                      \
+        using Tile = DxTile<RM, WI>;                                                                                                          \
         static SmemLimit limit;                                                                                                               \
-        const cudaError_t e = limit.raise(sim_dx_tiled<TM, MODE>, DxCfg<TM>::SLOT_BYTES);                                                     \
+        const cudaError_t e = limit.raise(sim_dx_tiled<RM, WI, MODE>, Tile::SLOT_BYTES);                                                      \
         if (e != cudaSuccess) return e;                                                                                                       \
-        in_stream_order(sim_dx_tiled<TM, MODE>, grid, DxCfg<TM>::Cfg::THREADS, folds ? DxCfg<TM>::SLOT_BYTES : 0, s)(g, x, dxp, t, w, dy, dx); \
+        in_stream_order(sim_dx_tiled<RM, WI, MODE>, grid, Tile::T, folds ? Tile::SLOT_BYTES : 0, s)(g, x, dxp, t, w, dy, dx);                 \
     } while (0)
-#define DX_16(MODE) DX(16, MODE)
-#define DX_32(MODE) DX(32, MODE)
-#define DX_64(MODE) DX(64, MODE)
-#define DX_128(MODE) DX(128, MODE)
-    if (tm == 16) { DX_MODES(DX_16) } else if (tm == 32) { DX_MODES(DX_32) } else if (tm == 64) { DX_MODES(DX_64) } else { DX_MODES(DX_128) }
+#define DX_41(MODE) DX(4, 1, MODE)
+#define DX_51(MODE) DX(5, 1, MODE)
+#define DX_61(MODE) DX(6, 1, MODE)
+#define DX_42(MODE) DX(4, 2, MODE)
+#define DX_52(MODE) DX(5, 2, MODE)
+#define DX_62(MODE) DX(6, 2, MODE)
+#define DX_44(MODE) DX(4, 4, MODE)
+    switch (pick.wi * 8 + pick.rm) {
+    case 12: DX_MODES(DX_41) break;
+    case 13: DX_MODES(DX_51) break;
+    case 14: DX_MODES(DX_61) break;
+    case 20: DX_MODES(DX_42) break;
+    case 21: DX_MODES(DX_52) break;
+    case 22: DX_MODES(DX_62) break;
+    default: DX_MODES(DX_44) break;
+    }
     count_launch(2);
     return cudaGetLastError();
 #undef DX

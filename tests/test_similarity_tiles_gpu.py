@@ -60,6 +60,20 @@ def test_infinite_pixels_meet_only_the_taps_that_are_there(port, i, mode):
     cases.assert_parity(dx, ref, what=c["name"])
 
 
+# rows of channels per tile: 16, 20, 24, 32, 40, 48, 64; instances per chunk: 8, and 16 for 64 rows, four steps at a time
+@pytest.mark.parametrize("mode", MODES, ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("channels,m", [(16, 9), (17, 1), (20, 8), (21, 4), (24, 5), (25, 12), (32, 7), (33, 17), (40, 16), (41, 3), (48, 10), (49, 15), (64, 16), (65, 20),
+                                        (63, 33), (80, 4), (97, 13), (128, 31), (129, 5)])
+def test_input_gradients_at_the_edges_of_their_tiles(port, channels, m, mode):
+    c = cases.sim_case("rows%d" % channels, (2, channels, 9, 8), m, blocks=(3, 2), strides=(2, 1), padding=(1, 0), oob=0.3, seed=800 + channels, **mode)
+    d = cases.sim_desc(c)
+    x, t, w, dy = cases.sim_inputs(c, port.sim_out_shape(d))
+    x[0, :, 2, 3] = t[0, :, 1, 1]                          # (differences of exactly 0)
+    dx = gpu_util.sim_ops.similarity_input_grad(*(gpu_util.dev(a) for a in (x, t, w, dy)), **cases.sim_attrs(c)).cpu().numpy()
+    a64 = [a.astype(np.float64) for a in (x, t, w, dy)]
+    cases.assert_parity(dx, port.similarity_input_grad(d, x, t, w, dy), port.similarity_input_grad(cases.sim_desc(c, dtype=gpu_util.abi.F64), *a64), what=c["name"])
+
+
 # One FP32 register is about 0.3 x 2^-24 x sqrt(n) of a sum of n such terms away from it (measured: n = 252: 2.8e-7, n = 6400: 1.4e-6).
 def _of_folded(steps, folds):
     return 0.3 * 2.0 ** -24 * (steps ** 0.5 + folds ** 0.5)
