@@ -27,23 +27,29 @@ struct DependentLaunch {
     dim3 grid, block;
     size_t smem;
     cudaStream_t stream;
+    int cluster;                                        // CTAs per cluster along the grid's y (which it divides)
     template <class... Args>
     void operator()(Args&&... args) const {
-        cudaLaunchAttribute attr = {};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = attr[1].val.clusterDim.z = 1;
+        attr[1].val.clusterDim.y = unsigned(cluster);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
         cfg.blockDim = block;
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = cluster > 1 ? 2 : 1;
         cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);         // (a failure is what cudaGetLastError returns next)
     }
 };
 
 template <class Kernel>
-DependentLaunch<Kernel> in_stream_order(Kernel* kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream) { return {kernel, grid, block, smem, stream}; }
+DependentLaunch<Kernel> in_stream_order(Kernel* kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster = 1) {
+    return {kernel, grid, block, smem, stream, cluster};
+}
 
 }  // namespace simnets

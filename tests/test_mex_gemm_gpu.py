@@ -26,6 +26,18 @@ EDGES = [
     cases.mex_case("overlap_padded", (3, 5, 7, 8), 9, (3, 3, 2), (2, 1, 1), (1, 1, 1), oob=0.4, softmax=True, unshared_region=(2,), seed=507, normalize=True),
     cases.mex_case("overlap_strided", (2, 4, 11, 10), 18, (4, 5, 3), (4, 2, 2), (0, 2, 1), eps=1.5, unshared=False, shared_region=(2,), seed=508),
     cases.mex_case("gaps", (2, 6, 9, 9), 5, (2, 2, 2), (3, 3, 4), softmax=True, seed=509),
+    # maps of a few pixels (lanes along instances), reductions split over clusters of two to eight CTAs and over more than a cluster holds
+    cases.mex_case("map_2x2_split", (5, 150, 2, 2), 70, (150, 1, 1), (150, 1, 1), softmax=True, unshared_region=(2,), seed=510, normalize=True),
+    cases.mex_case("map_2x2_many", (70, 33, 2, 2), 33, (33, 1, 1), (33, 1, 1), softmax=True, unshared_region=(2,), seed=511),
+    cases.mex_case("map_1x1_cluster_of_8", (3, 500, 1, 1), 20, (500, 1, 1), (500, 1, 1), softmax=True, seed=512, normalize=True),
+    cases.mex_case("map_1x1_11_splits", (3, 700, 1, 1), 129, (700, 1, 1), (700, 1, 1), eps=0.7, softmax=True, seed=513),
+    cases.mex_case("map_3x3", (4, 40, 3, 3), 33, (40, 1, 1), (40, 1, 1), softmax=True, unshared=False, shared_region=(-1,), seed=514),
+    cases.mex_case("whole_planes", (2, 90, 4, 4), 20, (90, 4, 4), (90, 4, 4), softmax=True, seed=515, normalize=True),
+    # windows that overlap: also along channels, off the input on every side, in maps wider than the prepass holds and just not so
+    cases.mex_case("overlap_channels", (2, 6, 9, 8), 11, (3, 2, 3), (2, 1, 2), (1, 1, 1), oob=0.7, eps=-1.2, unshared=False, shared_region=(2,), seed=516),
+    cases.mex_case("overlap_wide_1", (1, 2, 5, 600), 3, (2, 3, 3), (2, 1, 1), (0, 1, 1), oob=-5.0, softmax=True, seed=517),
+    cases.mex_case("overlap_wide_2", (1, 2, 4, 900), 3, (2, 3, 3), (2, 1, 1), (0, 1, 1), oob=5.0, softmax=True, seed=518),
+    cases.mex_case("overlap_72_rows", (2, 8, 9, 9), 6, (8, 3, 3), (8, 1, 1), (0, 1, 1), softmax=True, unshared_region=(2,), seed=519),
 ]
 
 
@@ -111,13 +123,14 @@ def test_scratch_of_exactly_the_stated_sizes(cuda_lib, c, flags, dtype):
         assert all(torch.equal(a, b) for a, b in zip(got[0], other))
 
 
+@pytest.mark.parametrize("shape,m", [((3, 12, 6, 6), 10), ((3, 200, 2, 2), 20), ((2, 700, 1, 1), 18)], ids=["one", "cluster", "splits"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64], ids=["f32", "f64"])
-def test_offsets_beyond_the_safe_spread_are_evaluated_term_by_term(port, dtype):
-    c = cases.mex_case("spread", (3, 12, 6, 6), 10, (12, 1, 1), (12, 1, 1), softmax=True, unshared_region=(2,), seed=520)
+def test_offsets_beyond_the_safe_spread_are_evaluated_term_by_term(port, dtype, shape, m):
+    c = cases.mex_case("spread", shape, m, (shape[1], 1, 1), (shape[1], 1, 1), softmax=True, unshared_region=(2 if shape[2] > 1 else 1,), seed=520)
     code = abi.F32 if dtype == torch.float32 else abi.F64
     d = cases.mex_desc(c, dtype=code)
     x, off, dy = cases.mex_inputs(c, port.mex_offsets_shape(d), port.mex_out_shape(d), np.float32 if code == abi.F32 else np.float64)
-    off[2, 3, 5] = -500.0
+    off[off.shape[0] // 2, 3, 5] = -500.0
     xd, od, dyd = (gpu_util.dev(a, dtype) for a in (x, off, dy))
     attrs = cases.mex_attrs(c)
     ry = port.mex_forward(d, x, off)
