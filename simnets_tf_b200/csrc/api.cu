@@ -34,14 +34,15 @@ inline int from_cuda(cudaError_t e) { return e == cudaSuccess ? SIMNETS_OK : int
 int mex_gradients(const MexGeo& g, const simnets_mex_desc* d, const void* x, const void* off, const void* y, const void* dy, void* dx, void* doff,
                   void* ws, size_t ws_bytes, void* products, size_t products_bytes, cudaStream_t s) {
     const bool f64 = d->dtype == SIMNETS_F64, acc = (d->flags & SIMNETS_FLAG_ACCUMULATE) != 0;
-    const bool gemm = mex_use_gemm(g, f64, d->flags), tiled = !gemm && mex_use_tiled(g, f64, d->flags);
+    const bool alone = mex_gradients_by_gemm(g, f64, d->flags), gemm = alone || mex_use_gemm(g, f64, d->flags), tiled = !gemm && mex_use_tiled(g, f64, d->flags);
     if ((d->flags & SIMNETS_FLAG_MEX_NORMALIZED_OFFSETS) && g.B > 0 && !gemm && !tiled) return SIMNETS_E_UNSUPPORTED;
     if (gemm || tiled) {
         if (!ws || ws_bytes < (gemm ? mex_gemm_workspace_bytes(g, f64) : mex_workspace_bytes(g, f64, d->flags))) return SIMNETS_E_WORKSPACE;
         const size_t need = dx ? mex_products_bytes(g, f64, d->flags) : 0;
         if (need > 0 && (!products || products_bytes < need)) return SIMNETS_E_WORKSPACE;
     }
-    if (gemm) return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, doff, acc, ws, products, d->flags, s));
+    const uint32_t unprimed = ~uint32_t(alone ? SIMNETS_FLAG_MEX_WORKSPACE_PRIMED | SIMNETS_FLAG_MEX_MAXIMA_GIVEN : 0);
+    if (gemm) return from_cuda(launch_mex_bwd_gemm(g, f64, x, off, y, dy, dx, doff, acc, ws, products, d->flags & unprimed, s));
     if (tiled) {
         const float *xf = (const float*)x, *of = (const float*)off, *yf = (const float*)y, *dyf = (const float*)dy;
         if (dx && doff) return from_cuda(launch_mex_backward_tiled(g, xf, of, yf, dyf, (float*)dx, (float*)doff, acc, ws, products, d->flags, s));
@@ -216,7 +217,8 @@ size_t simnets_mex_forward_workspace_bytes(const simnets_mex_desc* d) {
     if (mex_geometry(d, nullptr, &g)) return 0;
     const bool f64 = d->dtype == SIMNETS_F64;
     // (room for either family: a caller may size a workspace once and pass other flags later)
-    return std::max(mex_workspace_bytes(g, f64, d->flags), mex_use_gemm(g, f64, d->flags) ? mex_gemm_workspace_bytes(g, f64) : size_t(256));
+    const bool gemm = mex_use_gemm(g, f64, d->flags) || mex_gradients_by_gemm(g, f64, d->flags);
+    return std::max(mex_workspace_bytes(g, f64, d->flags), gemm ? mex_gemm_workspace_bytes(g, f64) : size_t(256));
 }
 
 size_t simnets_mex_products_bytes(const simnets_mex_desc* d) {

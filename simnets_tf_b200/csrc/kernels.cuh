@@ -147,6 +147,9 @@ cudaError_t launch_mex_bwd_short(const MexGeo&, bool inside, const float* x, con
                                  const float* dy, float* dx, float* part, const int* flag, cudaStream_t);
 // mex_gemm.cu -- the factorised passes as small contractions: float64, small float32 layers, input gradients of overlapping blocks
 bool mex_use_gemm(const MexGeo&, bool f64, uint32_t flags);
+// layers whose forward pass another family does: their gradients run here, on a workspace of this family at the same place (nothing of
+// the forward pass's is used, so they take no primed one)
+bool mex_gradients_by_gemm(const MexGeo&, bool f64, uint32_t flags);
 size_t mex_gemm_workspace_bytes(const MexGeo&, bool f64);
 size_t mex_gemm_products_bytes(const MexGeo&, bool f64);
 void* mex_gemm_maxima(const MexGeo&, bool f64, void* ws);

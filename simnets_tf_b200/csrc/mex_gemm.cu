@@ -959,32 +959,41 @@ cudaError_t gemm_backward(const MexGeo& g, const T* x, const T* off, const T* y,
 }  // namespace
 
 // float32 layers small enough for this family.  Forward with pooling + both gradients on the kept workspace, captured, us, here /
-// there (pixel layers with 2 x 2 regions; "there" = the tensor-core kernels):
-//     64 over 32, 16x16 pixels     4 M multiply-adds per pass 48 / 37,   17 M  51 / 42,   67 M  88 / 49
-//     128 over 64, 8x8             4 M  53 / 45,   17 M  60 / 47,   67 M  78 / 51
-//     256 over 128, 8x8            4 M  49 / 62,   25 M  62 / 64,   67 M  74 / 68,  101 M  92 / 70
-//     512 over 256, 4x4           17 M  57 / 99,   67 M  78 / 114, 134 M 111 / 119, 200 M 151 / 119
-//     1024 over 512, 2x2         200 M 210 / 328
-// The line grows with the layer's M K, whose chunks the tensor-core kernels walk serially.  Below M K = 10^4 it lies higher than
-// these times alone would have it, by 10 us a layer: sums are FP32 here, truncated after every eight taps there (distance of y from
-// float64, here / there: 64 over 32 3e-7 / 9e-7, 128 over 64 4e-7 / 2e-6, 512 over 256 4e-7 / 8e-6), and a forward call with its
-// gradients is 6 or 7 launches here and 10 there, which is what such a layer costs a host.
-// Overlapping blocks: 24 instances over 12x3x3 taps at 105 M 210 / 248, at 209 M 384 / 428; 8 over 8x5x5 at 41 M 236 / 302.
-// Classifier heads (M <= 16) up to 1024 taps: the same reasons; 512 taps at 0.3 M 39 / 31, 1024 at 5 M 59 / 41.  Longer patches
-// are read better by their own kernels.
+// there (pixel layers with 2 x 2 regions; "there" = the tensor-core kernels), around where the two meet:
+//     64 over 32, 16x16 pixels    17 M multiply-adds per pass 35 / 39,   34 M  43 / 43,   50 M  51 / 45
+//     128 over 64, 8x8            50 M  47 / 49,   67 M  47 / 49,  100 M  62 / 51
+//     256 over 128, 8x8          101 M  69 / 70,  134 M  68 / 68,  199 M  92 / 72
+//     512 over 256, 4x4          199 M 109 / 117,  268 M 119 / 120,  401 M 171 / 125;   2x2   536 M 219 / 260
+//     1024 over 512, 4x4         403 M 189 / 216,  537 M 217 / 219;                     2x2   799 M 351 / 470
+// The line grows with the root of the layer's M K, whose chunks the tensor-core kernels walk serially, and lies twice as high on maps of
+// up to four pixels, which those read a sector at a time.  Sums are FP32 here, truncated after every eight taps there (distance of y
+// from float64, here / there: 64 over 32 4e-8 / 9e-7, 512 over 256 4e-8 / 6e-7 of normal data).
+// Overlapping blocks, 24 instances over 12x3x3 taps: 105 M 124 / 192, 837 M 785 / 1121; 64 over 32x3x3: 472 M 246 / 317, 944 M 454 / 527;
+// 128 over 32x3x3: 944 M 403 / 409.
+// Classifier heads (M <= 16) up to 1024 taps are slower here by 4 to 10 us (512 taps, 0.3 M: 37 / 31) and take half of the launches, which
+// is what such a layer costs a host.  Longer patches are read better by their own kernels.
 static bool mex_small_layer(const MexGeo& g) {
     const double macs = double(g.R) * g.M * g.K * (double(g.B) * g.rs);
     if (g.M <= 16 && g.K >= 256) return g.K <= 1024 && macs <= 8e6;
-    if (overlapping(g)) return macs <= 200e6;
-    return macs <= std::min(200e6, std::max(12e6, 25e6 * std::pow(double(g.M) * g.K / 8192.0, 0.75)));
+    if (overlapping(g)) return g.M < 48 || macs <= 900e6 * 64 / g.M;
+    return macs <= 68e6 * std::sqrt(double(g.M) * g.K / 8192.0) * (g.N <= 4 ? 2 : 1);
+}
+// what every float32 call of this family needs: finite epsilon, positions that 31 bits count, no flag that asks for other kernels
+static bool gemm_serves(const MexGeo& g, uint32_t flags) {
+    return g.finite && g.B > 0 && (long long)g.B * g.rs < 0x7fffffffLL &&
+           !(flags & (SIMNETS_FLAG_FORCE_DIRECT | SIMNETS_FLAG_MEX_EXACT | SIMNETS_FLAG_MEX_NO_TENSORCORE | SIMNETS_FLAG_MEX_TC_ONE_TILE | SIMNETS_FLAG_MEX_NO_PAIR_TILES |
+                      SIMNETS_FLAG_MEX_TEST_EXPIRE_WAIT | SIMNETS_FLAG_MEX_NO_SMALL_TILES));
 }
 
-// Finite epsilon, and positions that 31 bits count.
 bool mex_use_gemm(const MexGeo& g, bool f64, uint32_t flags) {
-    if (!g.finite || g.B == 0 || (flags & (SIMNETS_FLAG_FORCE_DIRECT | SIMNETS_FLAG_MEX_EXACT)) || (long long)g.B * g.rs >= 0x7fffffffLL) return false;
-    if (f64) return true;
-    if (flags & (SIMNETS_FLAG_MEX_NO_TENSORCORE | SIMNETS_FLAG_MEX_TC_ONE_TILE | SIMNETS_FLAG_MEX_NO_PAIR_TILES | SIMNETS_FLAG_MEX_TEST_EXPIRE_WAIT | SIMNETS_FLAG_MEX_NO_SMALL_TILES)) return false;
-    return mex_small_layer(g);
+    if (f64) return g.finite && g.B > 0 && !(flags & (SIMNETS_FLAG_FORCE_DIRECT | SIMNETS_FLAG_MEX_EXACT)) && (long long)g.B * g.rs < 0x7fffffffLL;
+    return gemm_serves(g, flags) && mex_small_layer(g);
+}
+// Gradients of larger layers with too few instances for the tensor cores, whose forward pass other kernels do as well: both gradients, us,
+// here / there: 16 instances over 32 taps, 60 M multiply-adds 58 / 221; 8 over 4x2x2, 60 M 193 / 495; 30 over 8x2x2, 601 M 400 / 1586;
+// 40 over 64, 600 M 228 / 275; 47 over 200, 600 M 244 / 381.  They prepare their own workspace, in place of the forward pass's.
+bool mex_gradients_by_gemm(const MexGeo& g, bool f64, uint32_t flags) {
+    return !f64 && g.M < 48 && !(g.M <= 16 && g.K >= 256) && !overlapping(g) && gemm_serves(g, flags) && !mex_small_layer(g);
 }
 size_t mex_gemm_workspace_bytes(const MexGeo& g, bool f64) { return f64 ? carve_gemm<double>(g, nullptr).bytes : carve_gemm<float>(g, nullptr).bytes; }
 size_t mex_gemm_products_bytes(const MexGeo& g, bool f64) {
