@@ -13,8 +13,9 @@
 // same operations as everywhere else, so results equal the tile kernel's up to summation order.  Patches in registers with 2
 // or 4 positions per thread had left that pipe half idle whichever way the packed instructions were paired: 8 to 12 chains per
 // warp at 12 to 16 warps per SM do not cover the latency of difference -> product -> sum (2048 x 3 x 32 x 32 input, 64
-// templates of 3x3: 610 to 636 us).  All five modes of the forward functor (include/utils/similarity_utils.hpp:17-60 of the
-// reference) are covered.
+// templates of 3x3: 610 to 636 us).  What the resident kernel spends beside the arithmetic adds to its time: 612 us there with two
+// range tests per gathered value, 493 with one test of two bits (332 from registers and shared memory alone).  All five modes of the
+// forward functor (include/utils/similarity_utils.hpp:17-60 of the reference) are covered.
 #include "kernels.cuh"
 #include "tile.cuh"
 
@@ -156,6 +157,12 @@ __global__ void __launch_bounds__(kSkThreads, 4) sim_fwd_smallk(SimGeo g, int sl
     }
 }
 
+// the taps first .. of a block axis that leave the image, as bits (block <= 16)
+__device__ __forceinline__ uint32_t sk_missing(int first, int size) {
+    const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
+    return 0xffffu & ~(((1u << hi) - 1u) & ~((1u << lo) - 1u));
+}
+
 // Parameters resident in shared memory, tiles of 128 positions streamed past them: rows = templates (TM per CTA, blockIdx.y
 // picks them), columns = positions.
 template <int MODE> struct ResidentPlanes {
@@ -177,7 +184,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     extern __shared__ __align__(16) float sm[];
     __shared__ long long col_base[2][kResTN];
     __shared__ float row_const[TM];
-    __shared__ int2 tp[kResMaxK];
+    __shared__ int2 tp[kResMaxK];                                  // {byte offset inside a sample, bit kh | bit 16 + kw (blocks of up to 16 x 16, else kh << 16 | kw)}
     __shared__ __align__(16) float red[2][TI][kResTN];             // the extrema of each thread row, two tiles' worth
     const int K = g.K, i0 = blockIdx.y * TM;
     float* As = sm;
@@ -190,7 +197,11 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
         if (NA == 3) As[2 * K * TM + i] = p.constant;
     }
     if (threadIdx.x < TM) row_const[threadIdx.x] = MODE == SIM_L2N ? sk_row_constant(g, wt, i0 + threadIdx.x) : 0.f;
-    for (int k = threadIdx.x; k < kResMaxK; k += T) tp[k] = sk_tap(g, k);
+    const bool bits = g.bh <= 16 && g.bw <= 16;
+    for (int k = threadIdx.x; k < kResMaxK; k += T) {
+        const int2 at = sk_tap(g, k);
+        tp[k] = make_int2(4 * at.x, bits ? (1 << (at.y >> 16)) | (0x10000 << (at.y & 0xffff)) : at.y);
+    }
     __syncthreads();
 
     const TileThread<Cfg> t;
@@ -203,12 +214,30 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     long long rbase = -1;
     auto fetch = [&](long long tile) {
         const SkColumn c = sk_column(g, tile * kResTN + s_lane, P);
-        const float* xs = x + (size_t)c.n * g.C * g.H * g.W + c.h0 * g.W + c.w0;
+        const char* xs = reinterpret_cast<const char*>(x + (size_t)c.n * g.C * g.H * g.W + c.h0 * g.W + c.w0);
         rbase = c.base;
+        const float outside = c.base >= 0 ? oob : 0.f;
+        if (bits) {
+            // one test per tap, of its two bits against what the patch misses
+            const int missing = c.base >= 0 ? int(sk_missing(c.h0, g.H) | (sk_missing(c.w0, g.W) << 16)) : -1;
 #pragma unroll
-        for (int s = 0; s < PER; ++s) {
-            const int k = s_k + s * QSTEP;
-            if (k < K) rb[s] = c.base >= 0 ? sk_load(g, xs, c, tp[k], oob) : 0.f;
+            for (int s = 0; s < PER; ++s) {
+                const int k = s_k + s * QSTEP;
+                if (k >= K) break;
+                const int2 t = tp[k];
+                rb[s] = outside;
+                if ((t.y & missing) == 0) rb[s] = __ldg(reinterpret_cast<const float*>(xs + t.x));
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < PER; ++s) {
+                const int k = s_k + s * QSTEP;
+                if (k >= K) break;
+                const int2 t = tp[k];
+                rb[s] = outside;
+                if (c.base >= 0 && uint32_t(c.h0 + (t.y >> 16)) < uint32_t(g.H) && uint32_t(c.w0 + (t.y & 0xffff)) < uint32_t(g.W))
+                    rb[s] = __ldg(reinterpret_cast<const float*>(xs + t.x));
+            }
         }
     };
     auto commit = [&](int buf) {
@@ -253,7 +282,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
             for (int c = 0; c < 4; ++c) acc[r][c] = make_float2(0.f, 0.f);
         const float* B = Bs + buf * NB * K * kResTN + t.tj * 4;
         const float* A = As + t.ti * 4;
-#pragma unroll 3
+#pragma unroll 9
         for (int q = 0; q < K; ++q) {
             float a[NA][4];
             float2 b[NB][4];

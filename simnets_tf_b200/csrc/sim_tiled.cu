@@ -25,6 +25,7 @@ struct SimWs {
     float* planes;   // [3][K][Mp]: t, scale (-w or -0.5w), per-term constant; Mp = M rounded up to 4 floats
     float* cm;       // [M] per-instance constant added once per output
     int2* taps;      // [K]: {offset of tap inside a sample, (kh << 16) | kw}
+    int2* tests;     // [K]: {byte offset, bit kh | bit 16 + kw}, blocks of up to 16 x 16
     float* part;     // [S][3][M][K] split partial sums of the parameter gradients
     float* dxp;      // [2][bh*bw*M][Cp]: t and s*w (s = 2 for plain L2, else 1), channel-contiguous, for the input gradient
     float* tc_tiles; // pre-split parameter tiles of the tensor-core forward kernel
@@ -44,6 +45,7 @@ __host__ SimWs carve(const SimGeo& g, void* base) {
     w.planes = reinterpret_cast<float*>(take(sizeof(float) * 3 * (size_t)g.K * pad4(g.M)));
     w.cm = reinterpret_cast<float*>(take(sizeof(float) * g.M));
     w.taps = reinterpret_cast<int2*>(take(sizeof(int2) * g.K));
+    w.tests = reinterpret_cast<int2*>(take(sizeof(int2) * g.K));
     w.part = reinterpret_cast<float*>(take(sizeof(float) * 3 * (size_t)sim_dparams_splits(g) * g.M * g.K));
     w.dxp = reinterpret_cast<float*>(take(sizeof(float) * sim_dx_scratch_floats(g)));
     w.tc_tiles = reinterpret_cast<float*>(take(sizeof(float) * sim_tc_tile_floats(g)));
@@ -52,10 +54,20 @@ __host__ SimWs carve(const SimGeo& g, void* base) {
     return w;
 }
 
+// The test of a tap against the image as one AND of two bits with what the position's patch misses: blocks of up to 16 x 16, 32-bit byte
+// offsets.  (Two range tests per gathered value, although a patch inside the image skipped them: 256 x 64 x 32 x 32 input, 256 templates
+// of 3x3 4134 -> 3913 us, with masks 6046 -> 5557, L1 3119 -> 2838.)
+__host__ __device__ inline bool sim_tap_bits(const SimGeo& g) { return g.bh <= 16 && g.bw <= 16 && (long long)g.C * g.H * g.W < (1LL << 29); }
+// the taps of a block axis that leave the image, as bits
+__device__ __forceinline__ uint32_t sim_missing(int first, int size) {
+    const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
+    return 0xffffu & ~(((1u << hi) - 1u) & ~((1u << lo) - 1u));
+}
+
 // One block per instance m: tap-major parameter planes, the per-instance constant, and (block 0) the tap table.
 __global__ void __launch_bounds__(128) sim_prep(SimGeo g, const float* __restrict__ tm, const float* __restrict__ wt,
                                                 float* __restrict__ planes, float* __restrict__ cm, int2* __restrict__ taps,
-                                                int* __restrict__ flag) {
+                                                int2* __restrict__ tests, int* __restrict__ flag) {
     stream_order();
     __shared__ float red[128];
     const int m = blockIdx.x;
@@ -73,7 +85,10 @@ __global__ void __launch_bounds__(128) sim_prep(SimGeo g, const float* __restric
         planes[plane + (size_t)k * ldm + m] = scale;
         planes[2 * plane + (size_t)k * ldm + m] = c;
         const int kw = k % g.bw, kh = (k / g.bw) % g.bh, c_ = k / (g.bw * g.bh);
-        if (m == 0) taps[k] = make_int2((c_ * g.H + kh) * g.W + kw, (kh << 16) | kw);
+        if (m == 0) {
+            taps[k] = make_int2((c_ * g.H + kh) * g.W + kw, (kh << 16) | kw);
+            if (sim_tap_bits(g)) tests[k] = make_int2(4 * ((c_ * g.H + kh) * g.W + kw), (1 << kh) | (0x10000 << kw));
+        }
     }
     red[threadIdx.x] = csum;
     __syncthreads();
@@ -125,7 +140,7 @@ template <int TM, int TN> struct FwdTile {
 
 template <int TM, int TN, int MODE>
 __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER_SM) sim_fwd_tiled(SimGeo g, const float* __restrict__ x, const float* __restrict__ planes,
-                                                     const float* __restrict__ cm, const int2* __restrict__ taps, float* __restrict__ y) {
+                                                     const float* __restrict__ cm, const int2* __restrict__ taps, int bits, float* __restrict__ y) {
     stream_order();
     constexpr int NA = FwdPlanes<MODE>::NA, NB = FwdPlanes<MODE>::NB;
     using Cfg = TileCfg<TM, TN, FwdTile<TM, TN>::KC, FwdTile<TM, TN>::RM, FwdTile<TM, TN>::RN, NA, NB>;
@@ -148,10 +163,10 @@ __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER
     const SimColumn sc = sim_column(g, j0 + s_lane, P);
     if (s_k == 0) col_base[s_lane] = sc.base;
     const bool live = sc.base >= 0;
-    // a patch that lies entirely inside the image needs no per-tap bounds test
-    const bool inside = live && sc.h0 >= 0 && sc.w0 >= 0 && sc.h0 + g.bh <= g.H && sc.w0 + g.bw <= g.W;
+    const int missing = live ? int(sim_missing(sc.h0, g.H) | (sim_missing(sc.w0, g.W) << 16)) : -1;
+    const float outside = live ? oob : 0.f;
     const float* xs = x + (size_t)sc.n * g.C * g.H * g.W;
-    const float* xc = xs + sc.h0 * g.W + sc.w0;
+    const char* xc = reinterpret_cast<const char*>(xs + sc.h0 * g.W + sc.w0);
     float rb[Cfg::B_PER];
 
     float2 acc[Cfg::RM][Cfg::RN / 2];
@@ -175,20 +190,26 @@ __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER
 #pragma unroll
         for (int s = 0; s < Cfg::B_PER; ++s) tap[AHEAD ? s : 0] = __ldg(taps + min(s_k + s * QSTEP, g.K - 1));
     }
+    // (rows past K pair a zero scale / zero constant with a finite value: the term is exactly 0)
     auto fetchB = [&](int chunk, float*) {
+        if (bits) {
 #pragma unroll
-        for (int s = 0; s < Cfg::B_PER; ++s) {
-            const int k = chunk * Cfg::KC + s_k + s * QSTEP;
-            // rows past K pair a zero scale / zero constant with a finite value: the term is exactly 0
-            if (AHEAD) {
+            for (int s = 0; s < Cfg::B_PER; ++s) {
+                const int k = chunk * Cfg::KC + s_k + s * QSTEP;
                 rb[s] = 0.f;
-                if (k < g.K && live) rb[s] = inside ? __ldg(xc + tap[AHEAD ? s : 0].x) : sim_tap_value(g, xs, sc, tap[AHEAD ? s : 0], oob);
-                tap[AHEAD ? s : 0] = __ldg(taps + min(k + Cfg::KC, g.K - 1));
-                continue;
+                if (k < g.K) {
+                    const int2 t = AHEAD ? tap[AHEAD ? s : 0] : __ldg(taps + k);
+                    rb[s] = outside;
+                    if ((t.y & missing) == 0) rb[s] = __ldg(reinterpret_cast<const float*>(xc + t.x));
+                }
+                if (AHEAD) tap[AHEAD ? s : 0] = __ldg(taps + min(k + Cfg::KC, g.K - 1));
             }
-            if (k >= g.K || !live) rb[s] = 0.f;
-            else if (inside) rb[s] = __ldg(xc + __ldg(taps + k).x);
-            else rb[s] = sim_tap_value(g, xs, sc, __ldg(taps + k), oob);
+        } else {
+#pragma unroll
+            for (int s = 0; s < Cfg::B_PER; ++s) {
+                const int k = chunk * Cfg::KC + s_k + s * QSTEP;
+                rb[s] = k < g.K && live ? sim_tap_value(g, xs, sc, __ldg(taps + k), oob) : 0.f;
+            }
         }
     };
     auto commitA = [&](float*) { cp_async_wait_all(); };
@@ -238,7 +259,7 @@ __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER
 }
 
 void launch_prep(const SimGeo& g, const SimWs& w, const float* t, const float* wt, cudaStream_t s) {
-    in_stream_order(sim_prep, g.M, 128, 0, s)(g, t, wt, w.planes, w.cm, w.taps, w.flag);
+    in_stream_order(sim_prep, g.M, 128, 0, s)(g, t, wt, w.planes, w.cm, w.taps, w.tests, w.flag);
     count_launch();
 }
 
@@ -285,7 +306,7 @@ static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const flo
     // small inputs: 16 x 20 x 20 inputs under 48 templates fill 56 tiles of 64 x 128 on 148 SMs).
     // With masks the 8 x 8 blocking spills at 128 registers, 4 x 8 does not (terms from registers and shared memory alone: 6.5
     // and 7.7 T/s).  Under 16 warps per SM, one CTA of the large tiles, nothing covers a CTA's barriers (16 x 64 x 32 x 32 input,
-    // 128 templates of 3x3: 206 us in 128 tiles of 128 x 128, 191 in 256 of 64 x 128; with masks 309 and 239).
+    // 128 templates of 3x3: 206 us in 128 tiles of 128 x 128, 191 in 256 of 64 x 128; with masks 309 and 239, before both staged less).
     struct { int tm, tn, threads; double cost; } const tiles[] = {{128, 128, 256, 1.0}, {64, 128, 256, g.mode == SIM_L2N_NAN ? 0.98 : 1.05}, {32, 64, 128, 1.6}, {16, 32, 32, 2.0}};
     int pick = 0;
     double best = 0;
@@ -297,7 +318,9 @@ static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const flo
     }
     const long long blocks = ((P + tiles[pick].tn - 1) / tiles[pick].tn) * ((g.M + tiles[pick].tm - 1) / tiles[pick].tm);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-#define FWD(TM, TN, MODE) in_stream_order(sim_fwd_tiled<TM, TN, MODE>, int(blocks), FwdTile<TM, TN>::THREADS, 0, s)(g, x, W.planes, W.cm, W.taps, y)
+    const int bits = sim_tap_bits(g);
+    const int2* taps = bits ? W.tests : W.taps;
+#define FWD(TM, TN, MODE) in_stream_order(sim_fwd_tiled<TM, TN, MODE>, int(blocks), FwdTile<TM, TN>::THREADS, 0, s)(g, x, W.planes, W.cm, taps, bits, y)
 #define FWD_MODES(TM, TN)                                        \
     switch (g.mode) {                                            \
     case SIM_L1: FWD(TM, TN, SIM_L1); break;                     \

@@ -147,3 +147,19 @@ def test_parameter_gradients_at_the_edges_of_their_tiles(port, i, special, mode)
     d64 = cases.sim_desc(c, dtype=gpu_util.abi.F64)
     for g, ref, ref64 in zip(got, port.similarity_params_grad(d, x, t, w, dy), port.similarity_params_grad(d64, *(a.astype(np.float64) for a in (x, t, w, dy)))):
         cases.assert_parity(g.cpu().numpy(), ref, ref64, what=c["name"])
+
+
+@pytest.mark.parametrize("mode", MODES, ids=["l2", "l2n", "l2nan", "l1"])
+@pytest.mark.parametrize("blocks,padding,stride", [((16, 1), (15, 0), 1), ((1, 16), (0, 15), 2), ((17, 1), (16, 0), 1), ((1, 18), (0, 9), 1), ((16, 16), (8, 8), 3)],
+                         ids=["rows16", "columns16", "rows17", "columns18", "square16"])
+@pytest.mark.parametrize("batch,m", [(2, 7), (120, 33)], ids=["few", "many"])
+def test_patches_that_leave_the_image_on_every_side(port, batch, m, blocks, padding, stride, mode):
+    """Blocks up to and beyond sixteen rows or columns (how a tap is tested against the image changes there), patches almost entirely
+    outside, on the kernels for few and for many positions."""
+    size = (batch, 1, 21, 20) if blocks[0] * blocks[1] < 100 else (max(1, batch // 40), 1, 21, 20)
+    c = cases.sim_case("leaves", size, m, blocks=blocks, strides=(stride, stride), padding=padding, oob=0.3, seed=850, **mode)
+    d = cases.sim_desc(c)
+    x, t, w, _ = cases.sim_inputs(c, port.sim_out_shape(d))
+    y = gpu_util.sim_ops.similarity_forward(*(gpu_util.dev(a) for a in (x, t, w)), **cases.sim_attrs(c)).cpu().numpy()
+    cases.assert_parity(y, port.similarity_forward(d, x, t, w), port.similarity_forward(cases.sim_desc(c, dtype=gpu_util.abi.F64), *(a.astype(np.float64) for a in (x, t, w))),
+                        what=c["name"])
