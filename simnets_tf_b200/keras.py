@@ -146,12 +146,14 @@ class Similarity(_PlannedLayer):
     def forward(self, x, extrema=None):
         """extrema=(max_address, min_address): also write the per-pixel maximum / minimum of the output over the
         templates to those device addresses (see Mex.extrema_slot)."""
-        if self.templates is None:
+        templates = self.templates
+        if templates is None:
             self.build(tuple(x.shape), x.device, x.dtype)
+            templates = self.templates
         if self.channels_last:
             x = x.permute(0, 3, 1, 2)
         # |weights| and its gradient are taken inside the op's kernels
-        templates, weights = self.templates, self.sweights
+        weights = self.sweights
         if _torch_glue.is_tracing():
             y = _similarity_recorded(self._plan, x, templates, weights, abi.FLAG_SIM_ABS_WEIGHTS, extrema)
         else:
@@ -334,14 +336,15 @@ class Mex(_PlannedLayer):
     def forward(self, x, sum_pool2=False, layer_ws=None, maxima_given=False):
         """sum_pool2=True returns the 2x2 sum pooling of the layer's output (pooling gradient fused into the
         MEX gradient kernels).  layer_ws / maxima_given: see extrema_slot."""
-        if self.offsets is None:
+        off = self.offsets
+        if off is None:
             self.build(tuple(x.shape), x.device, x.dtype)
+            off = self.offsets
         if self.channels_last:
             x = x.permute(0, 3, 1, 2)
         op_flags = self._op_flags(x.dtype, x.device) if x.shape[0] > 0 else 0
         _torch_glue.dtype_code(x)                   # (rejects anything but float32 / float64)
         # (the raw offsets are the op's own input, and a gradient bucket its target, only when the op normalises them)
-        off = self.offsets
         sink = _sinks(off) if op_flags else None
         fwd_flags = abi.FLAG_MEX_MAXIMA_GIVEN if maxima_given else 0
         if _torch_glue.is_tracing():

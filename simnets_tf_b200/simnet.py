@@ -11,9 +11,12 @@ cfg5: the deeper 3x32x32 network of the data-parallel configuration (last layer 
       test/basic_net_mnist_tf_ll.py:149-154).
 Sum pooling is a 2x2 average pool times 4, as the reference's README builds it.
 """
+import math
+
 import numpy as np
 import torch
 import torch.nn.functional as F
+from torch.nn.modules import module as _module
 
 from . import keras as layers
 from ._torch_glue import is_tracing
@@ -54,6 +57,19 @@ def sum_pool(x, k):
     if x.shape[2] % k or x.shape[3] % k:
         return F.avg_pool2d(x, k) * float(k * k)
     return _SumPool.apply(x, k)
+
+
+def _caller():
+    """How a network calls its layers: by their own forward() where nothing hangs on the call of the module (1.5 us of host time
+    each), else as modules (hooks of the layer or of all modules, a subclass with a call of its own, a compiled or recorded one)."""
+    hooked = getattr(_module, "_has_any_global_hook", lambda: True)() or is_tracing()
+
+    def call(m):
+        if hooked or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or \
+                type(m).__call__ is not torch.nn.Module.__call__ or getattr(m, "_compiled_call_impl", None) is not None:
+            return m
+        return m.forward
+    return call
 
 
 class SimNet(torch.nn.Module):
@@ -102,27 +118,30 @@ class SimNet(torch.nn.Module):
     def forward_range(self, x, begin, end):
         """Layers plan[begin:end] (a MEX + sum-pool pair is never split: `begin` and `end` are layer starts)."""
         plan, i = self._plan, begin
+        call = _caller()
         while i < end:
             entry, mod = plan[i]
             pooled_next = lambda j: self.fuse_pooling and j + 1 < len(plan) and plan[j + 1][0] == ("sumpool", 2)
             # (a recorded graph outlives the workspace whose address the extrema go to)
             if entry[0] == "similarity" and self.fuse_extrema and i + 1 < end and plan[i + 1][0][0] == "mex" and not is_tracing():
                 # Similarity -> MEX over the channels of each pixel: the Similarity kernel leaves the per-pixel extrema of its
-                # output in the MEX layer's workspace, and the MEX forward pass skips its pass over that tensor
-                nxt = plan[i + 1][1]
-                slot = None if mod.channels_last else nxt.extrema_slot(mod.output_shape_for(x), x.dtype, x.device, sum_pool2=pooled_next(i + 1))
+                # output in the MEX layer's workspace, and the MEX forward pass skips its pass over that tensor.  (Making the
+                # place for them takes the host 9 us; a tensor of 4 MB is read again in one.)
+                nxt, slot = plan[i + 1][1], None
+                if not mod.channels_last and math.prod(shape := mod.output_shape_for(x)) >= 1 << 20:
+                    slot = nxt.extrema_slot(shape, x.dtype, x.device, sum_pool2=pooled_next(i + 1))
                 if slot is not None:
                     ws, ptr, up = slot
-                    x = mod(x, extrema=(ptr, None) if up else (None, ptr))
-                    x = nxt(x, sum_pool2=pooled_next(i + 1), layer_ws=ws, maxima_given=True)
+                    x = call(mod)(x, extrema=(ptr, None) if up else (None, ptr))
+                    x = call(nxt)(x, sum_pool2=pooled_next(i + 1), layer_ws=ws, maxima_given=True)
                     i += 3 if pooled_next(i + 1) else 2
                     continue
             if entry[0] == "mex" and pooled_next(i):
-                x = mod(x, sum_pool2=True)          # MEX + 2x2 sum pooling, pooling gradient inside the MEX gradient kernels
+                x = call(mod)(x, sum_pool2=True)    # MEX + 2x2 sum pooling, pooling gradient inside the MEX gradient kernels
                 i += 2
                 continue
             if mod is not None:
-                x = mod(x)
+                x = call(mod)(x)
             elif entry[0] == "sumpool":
                 x = sum_pool(x, entry[1])
             elif entry[0] == "flatten":

@@ -9,6 +9,7 @@ import torch
 import cases
 import gpu_util
 from simnets_tf_b200 import abi
+from simnets_tf_b200.simnet import SPECS, SimNet
 
 sim_ops = importlib.import_module("simnets_tf_b200.ops.similarity")
 loss_ops = importlib.import_module("simnets_tf_b200.ops.loss")
@@ -147,3 +148,38 @@ def test_network_with_and_without_the_extrema_hand_over():
         outs.append([loss.detach()] + [p.grad.clone() for p in net.parameters()])
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+def test_layers_of_a_network_are_called_as_modules_where_something_hangs_on_that():
+    """Hooks of a layer, hooks of all modules and a subclass's own call see every layer; without any the results are the same."""
+    net = SimNet(SPECS["cfg3"], seed=4)
+    x = torch.rand(3, 1, 28, 28, device="cuda") - 0.5
+    plain = net(x)
+    seen = []
+    handles = [m.register_forward_hook(lambda m, i, o: seen.append(m)) for m in net.stages]
+    assert torch.equal(net(x), plain) and seen == list(net.stages)
+    for h in handles:
+        h.remove()
+    seen.clear()
+    handle = torch.nn.modules.module.register_module_forward_pre_hook(lambda m, i: seen.append(m) if m in set(net.stages) else None)
+    assert torch.equal(net(x), plain)
+    handle.remove()
+    assert seen == list(net.stages)
+
+    class Counted(type(net.stages[1])):
+        def __call__(self, *args, **kwargs):
+            seen.append(self)
+            return super().__call__(*args, **kwargs)
+    seen.clear()
+    net.stages[1].__class__ = Counted
+    assert torch.equal(net(x), plain) and seen == [net.stages[1]]
+
+
+@pytest.mark.parametrize("batch", [2, 40])
+def test_pooled_outputs_without_a_gradient(batch):
+    """A pooled layer whose unpooled output nobody keeps, on both kernel families: the values of a differentiated call."""
+    net = SimNet(SPECS["cfg5"], seed=5)
+    x = torch.rand(batch, 3, 32, 32, device="cuda") - 0.5
+    with torch.no_grad():
+        free = net(x)
+    assert torch.equal(free, net(x).detach())
