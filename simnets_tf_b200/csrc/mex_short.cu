@@ -12,7 +12,9 @@
 // four warps 16 positions each against Eo over the instances.  The products are slivers of K columns, which is why these are
 // warp instructions: a tcgen05 tile would be 16 columns wide and its operand staging would cost more than the product.
 // Operands are split into two TF32 parts, three products each, as everywhere in this library; Ex and Eo lie split in shared
-// memory, Q is split once per row tile.  The offsets sums of the CTA live in shared memory, each value private to one thread; a
+// memory, Q is split once per row tile.  The values' own loads run one step ahead, as far as registers go, and leave the kernel waiting
+// for memory (3.1 TB/s with the products switched off): their lines are prefetched into L2 three steps ahead, one line per thread and
+// step (256 instances over 4x2x2 blocks, batch 256: 3833 -> 3554 us; two or six steps 3578, 3662, twelve 3969).  The offsets sums of the CTA live in shared memory, each value private to one thread; a
 // CTA's partial sums are written once and added in a fixed order by the reduction.
 #include <climits>
 #include "mex_common.cuh"
@@ -21,7 +23,7 @@
 namespace simnets {
 namespace {
 
-constexpr int kShThreads = 256, kShPos = 64, kShM = 64;
+constexpr int kShThreads = 256, kShPos = 64, kShM = 64, kShAhead = 3;
 
 struct ShCol { long long sample; int c0, h0, w0, corner; };         // offset of the sample in x, patch corner; corner = its offset inside the sample
 
@@ -142,6 +144,21 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
         }
         fetch(0);
     };
+    // the L2 lines of a later step: one per thread, 64 rows x 2 lines of y and of dy (positions and instances that exist only)
+    const float* const pf_of = (tid >> 7 ? dy : y);
+    const int pf_row = (tid >> 1) & (kShM - 1), pf_half = (tid & 1) * 32;
+    long long pf_tile = p_begin, pf_base = -1;
+    int pf_mc = 0;
+    auto pf_place = [&]() {
+        const Column c = column_of(g, r, pf_tile + pf_half, P, nullptr);
+        pf_base = c.base;
+    };
+    auto prefetch = [&]() {
+        if (!VEC) return;
+        if (pf_base >= 0 && pf_mc * kShM + pf_row < g.M) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_of + pf_base + (long long)(pf_mc * kShM + pf_row) * g.N));
+        if (++pf_mc == MC) { pf_mc = 0; pf_tile += kShPos; pf_place(); }
+    };
+    if (VEC) { pf_place(); for (int i = 0; i < kShAhead; ++i) prefetch(); }
     // who multiplies what: both products, four warps each; one product alone, two warps per row tile
     const int rt = warp & 3;
     const bool does_dx = DX && (!DOFF || warp < 4);
@@ -166,6 +183,7 @@ __global__ void __launch_bounds__(kShThreads, 2) mex_bwd_short(MexGeo g, int ins
             cols[tid] = ShCol{(long long)e_col.n * g.C * g.H * g.W, e_col.c0, e_col.h0, e_col.w0, e_col.base >= 0 ? (e_col.c0 * g.H + e_col.h0) * g.W + e_col.w0 : INT_MIN};
         for (int mc = 0; mc < MC; ++mc, qb ^= 1) {
             float* Q = Qs + qb * kShM * kShPos;
+            prefetch();
 #pragma unroll
             for (int i = 0; i < PER; ++i) {
                 const int m = row0 + ROWS * i;
