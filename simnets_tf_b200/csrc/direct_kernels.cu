@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kThreads) mex_redo_bwd(MexGeo g, const float* 
 // just fills the GPU keeps the usual case (every CTA reads the flag and returns) at a few microseconds
 inline int grid_for(long long total, bool gated = false) {
     const long long blocks = (total + kThreads - 1) / kThreads;
-    const long long cap = (long long)device_sm_count() * (gated ? 8 : 32);
+    const long long cap = (long long)device_sm_count() * (gated ? 2 : 32);          // (a gated grid is there to find that nothing is to be done)
     return int(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
 }
 
@@ -377,7 +377,7 @@ cudaError_t launch_mex_redo_fwd_pool(const MexGeo& g, const float* x, const floa
 
 cudaError_t launch_mex_redo_bwd(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx, float* doff, bool accumulate,
                                 cudaStream_t s, const int* gate) {
-    in_stream_order(mex_redo_bwd, device_sm_count() * 8, kThreads, 0, s)(g, x, off, y, dy, dx, doff, int(accumulate), gate);
+    in_stream_order(mex_redo_bwd, device_sm_count() * 2, kThreads, 0, s)(g, x, off, y, dy, dx, doff, int(accumulate), gate);
     count_launch();
     return cudaGetLastError();
 }
