@@ -21,6 +21,13 @@ struct SimGeo {
     double fudge, oob;
 };
 
+// Whether every offset that a tap or the corner of a patch can have inside a sample is below `limit` elements (in a corner, above -limit):
+// what kernels ask that keep such offsets in 32 bits, in bytes (2^29) or in elements (2^31).
+__host__ __device__ inline bool sim_offsets_below(const SimGeo& g, long long limit) {
+    const long long tap = ((g.C - 1LL) * g.H + g.bh - 1) * g.W + g.bw - 1, corner = ((long long)g.H + g.ph) * g.W + g.W + g.pw;
+    return tap < limit && corner < limit;
+}
+
 // Division of 0 <= n < 2^31 by a positive constant known on the host: n / d = (n * mul) >> shift, exactly
 // (mul = ceil(2^shift / d), shift = 31 + ceil(log2 d)).  One wide multiply and a shift instead of a division loop.
 struct FastDiv { uint32_t d, mul, shift; };

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     extern __shared__ __align__(16) float sm[];
     __shared__ long long col_base[2][kResTN];
     __shared__ float row_const[TM];
-    __shared__ int2 tp[kResMaxK];                                  // {byte offset inside a sample, bit kh | bit 16 + kw (blocks of up to 16 x 16, else kh << 16 | kw)}
+    __shared__ int2 tp[kResMaxK];                                  // {byte offset inside a sample, bit kh | bit 16 + kw}, or as sk_tap has it
     __shared__ __align__(16) float red[2][TI][kResTN];             // the extrema of each thread row, two tiles' worth
     const int K = g.K, i0 = blockIdx.y * TM;
     float* As = sm;
@@ -197,10 +197,12 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
         if (NA == 3) As[2 * K * TM + i] = p.constant;
     }
     if (threadIdx.x < TM) row_const[threadIdx.x] = MODE == SIM_L2N ? sk_row_constant(g, wt, i0 + threadIdx.x) : 0.f;
-    const bool bits = g.bh <= 16 && g.bw <= 16;
+    // one test of two bits per tap, and an offset that is added as it is (2 % less time than one that is scaled): blocks of up to
+    // 16 x 16 and offsets whose bytes 32 bits count.  Else two range tests and offsets in elements.
+    const bool bits = g.bh <= 16 && g.bw <= 16 && sim_offsets_below(g, 1LL << 29);
     for (int k = threadIdx.x; k < kResMaxK; k += T) {
         const int2 at = sk_tap(g, k);
-        tp[k] = make_int2(4 * at.x, bits ? (1 << (at.y >> 16)) | (0x10000 << (at.y & 0xffff)) : at.y);
+        tp[k] = bits ? make_int2(4 * at.x, (1 << (at.y >> 16)) | (0x10000 << (at.y & 0xffff))) : at;
     }
     __syncthreads();
 
@@ -214,11 +216,10 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
     long long rbase = -1;
     auto fetch = [&](long long tile) {
         const SkColumn c = sk_column(g, tile * kResTN + s_lane, P);
-        const char* xs = reinterpret_cast<const char*>(x + (size_t)c.n * g.C * g.H * g.W + c.h0 * g.W + c.w0);
+        const float* xs = x + (size_t)c.n * g.C * g.H * g.W + c.h0 * g.W + c.w0;
         rbase = c.base;
         const float outside = c.base >= 0 ? oob : 0.f;
         if (bits) {
-            // one test per tap, of its two bits against what the patch misses
             const int missing = c.base >= 0 ? int(sk_missing(c.h0, g.H) | (sk_missing(c.w0, g.W) << 16)) : -1;
 #pragma unroll
             for (int s = 0; s < PER; ++s) {
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
                 if (k >= K) break;
                 const int2 t = tp[k];
                 rb[s] = outside;
-                if ((t.y & missing) == 0) rb[s] = __ldg(reinterpret_cast<const float*>(xs + t.x));
+                if ((t.y & missing) == 0) rb[s] = __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(xs) + t.x));
             }
         } else {
 #pragma unroll
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
                 const int2 t = tp[k];
                 rb[s] = outside;
                 if (c.base >= 0 && uint32_t(c.h0 + (t.y >> 16)) < uint32_t(g.H) && uint32_t(c.w0 + (t.y & 0xffff)) < uint32_t(g.W))
-                    rb[s] = __ldg(reinterpret_cast<const float*>(xs + t.x));
+                    rb[s] = __ldg(xs + t.x);
             }
         }
     };

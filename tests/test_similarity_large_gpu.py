@@ -1,0 +1,36 @@
+"""Samples whose values outnumber 32-bit offsets.  A stride picks few positions out of such a sample; the same positions gathered
+into a small sample have the same patches, and a kernel that is the same for both gives the same values bit for bit."""
+import pytest
+import torch
+
+import gpu_util
+
+pytestmark = pytest.mark.gpu
+
+
+def _parameters(m, c, bh, bw):
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    t = torch.rand(m, c, bh, bw, generator=gen, device="cuda") - 0.5
+    return t, 0.5 + torch.rand(m, c, bh, bw, generator=gen, device="cuda")
+
+
+def _sample(*shape):
+    return torch.rand(shape, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+
+
+@pytest.mark.parametrize("attrs", [dict(), dict(normalization_term=True, ignore_nan_input=True), dict(similarity_function="L1")], ids=["l2", "l2nan", "l1"])
+@pytest.mark.parametrize("m", [64, 20], ids=["rows64", "rows32"])
+def test_offsets_of_channels_beyond_31_bits_of_bytes(m, attrs):
+    """Three channels of 2^28 pixels: the third begins 2^31 bytes into the sample."""
+    x, (t, w) = _sample(1, 3, 1 << 14, 1 << 14), _parameters(m, 3, 1, 1)
+    y = gpu_util.sim_ops.similarity_forward(x, t, w, blocks=[1, 1], strides=[56, 56], padding=[0, 0], **attrs)
+    few = x[:, :, ::56, ::56].contiguous()
+    assert torch.equal(y, gpu_util.sim_ops.similarity_forward(few, t, w, blocks=[1, 1], strides=[1, 1], padding=[0, 0], **attrs))
+
+
+def test_offsets_of_rows_beyond_31_bits_of_bytes():
+    """Blocks of seventeen rows (tested against the image by ranges, not bits), 2^27 bytes apart."""
+    x, (t, w) = _sample(1, 1, 17, 1 << 25), _parameters(64, 1, 17, 1)
+    y = gpu_util.sim_ops.similarity_forward(x, t, w, blocks=[17, 1], strides=[1, 512], padding=[0, 0])
+    few = x[:, :, :, ::512].contiguous()
+    assert torch.equal(y, gpu_util.sim_ops.similarity_forward(few, t, w, blocks=[17, 1], strides=[1, 1], padding=[0, 0]))
