@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kThreads) sim_fwd_direct_rows(SimGeo g, const 
 // Positions are decoded by multiply and shift (f_N, f_ow; totals of 2^31 and more by division).  The sums are those of the other kernels
 // (sim_dparams.cu), the factors of an instance and tap applied at the end.  64 templates of 3x3 over 12 x 3 x 32 x 32 in float64: 92 us
 // with one tap per block, 42 so.
-template <typename T, int TK>
+template <typename T, int TK, typename Offset>
 __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T* __restrict__ x, const T* __restrict__ tm,
                                                                const T* __restrict__ wt, const T* __restrict__ dy,
                                                                T* __restrict__ dt, T* __restrict__ dw, int accumulate, FastDiv f_N, FastDiv f_ow) {
@@ -147,12 +147,13 @@ __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T
     const T oob = T(g.oob);
     const bool l1 = g.mode == SIM_L1 || g.mode == SIM_L1_SKIP, skips = g.mode == SIM_L1_SKIP || g.mode == SIM_L2N_NAN;
     T t[TK], sT[TK], sW[TK], sN[TK];
-    int at[TK], hk[TK], wk[TK];                          // (a tap's offset inside a sample: below 2^31, as every index of the geometry)
+    Offset at[TK];                                       // a tap's offset inside a sample
+    int hk[TK], wk[TK];
 #pragma unroll
     for (int u = 0; u < TK; ++u) {
         const int k = min(k0 + u, g.K - 1), c = k / (g.bw * g.bh);
         wk[u] = k % g.bw; hk[u] = k / g.bw % g.bh;
-        at[u] = (c * g.H + hk[u]) * g.W + wk[u];
+        at[u] = (Offset(c) * g.H + hk[u]) * g.W + wk[u];
         t[u] = tm[(size_t)m * g.K + k];
         sT[u] = sW[u] = sN[u] = T(0);
     }
@@ -347,13 +348,14 @@ cudaError_t launch_zero_words(int* p, int n, cudaStream_t s) {
 
 cudaError_t launch_sim_dparams_direct(const SimGeo& g, bool f64, const void* x, const void* t, const void* w, const void* dy,
                                       void* dt, void* dw, bool accumulate, cudaStream_t s) {
-    // as many taps per block as leave every SM one
-#define DP(TK)                                                                                                                                          \
+    // as many taps per block as leave every SM one; one where their offsets need 64 bits
+#define DP(TK, Offset)                                                                                                                                  \
     SIMNETS_DTYPE_SWITCH(f64,                                                                                                                           \
-        (in_stream_order(sim_dparams_direct<float, TK>, g.M * ((g.K + TK - 1) / TK), kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dt, (float*)dw, accumulate, make_fastdiv(g.N), make_fastdiv(g.ow))), \
-        (in_stream_order(sim_dparams_direct<double, TK>, g.M * ((g.K + TK - 1) / TK), kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dt, (double*)dw, accumulate, make_fastdiv(g.N), make_fastdiv(g.ow))))
-    const auto fills = [&](int taps) { return (long long)g.M * ((g.K + taps - 1) / taps) >= device_sm_count(); };
-    if (fills(8)) { DP(8); } else if (fills(4)) { DP(4); } else if (fills(2)) { DP(2); } else { DP(1); }
+        (in_stream_order(sim_dparams_direct<float, TK, Offset>, g.M * ((g.K + TK - 1) / TK), kThreads, 0, s)(g, (const float*)x, (const float*)t, (const float*)w, (const float*)dy, (float*)dt, (float*)dw, accumulate, make_fastdiv(g.N), make_fastdiv(g.ow))), \
+        (in_stream_order(sim_dparams_direct<double, TK, Offset>, g.M * ((g.K + TK - 1) / TK), kThreads, 0, s)(g, (const double*)x, (const double*)t, (const double*)w, (const double*)dy, (double*)dt, (double*)dw, accumulate, make_fastdiv(g.N), make_fastdiv(g.ow))))
+    const bool near = sim_offsets_below(g, 1LL << 31);
+    const auto fills = [&](int taps) { return near && (long long)g.M * ((g.K + taps - 1) / taps) >= device_sm_count(); };
+    if (fills(8)) { DP(8, int); } else if (fills(4)) { DP(4, int); } else if (fills(2)) { DP(2, int); } else { DP(1, long long); }
 #undef DP
     count_launch();
     return cudaGetLastError();

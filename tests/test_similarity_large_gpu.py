@@ -34,3 +34,16 @@ def test_offsets_of_rows_beyond_31_bits_of_bytes():
     y = gpu_util.sim_ops.similarity_forward(x, t, w, blocks=[17, 1], strides=[1, 512], padding=[0, 0])
     few = x[:, :, :, ::512].contiguous()
     assert torch.equal(y, gpu_util.sim_ops.similarity_forward(few, t, w, blocks=[17, 1], strides=[1, 1], padding=[0, 0]))
+
+
+@pytest.mark.parametrize("attrs", [dict(), dict(normalization_term=True, ignore_nan_input=True), dict(similarity_function="L1")], ids=["l2", "l2nan", "l1"])
+def test_parameter_gradients_of_offsets_beyond_31_bits(attrs):
+    """33 channels of 8200 x 8200 pixels: the last one begins 2^31 values into the sample.  Such samples go to the shape-agnostic kernel, which
+    takes eight taps per block of the small one."""
+    x, (t, w) = _sample(1, 33, 8200, 8200), _parameters(32, 33, 1, 1)
+    few = x[:, :, ::64, ::64].contiguous()
+    dy = torch.randn(1, 32, 129, 129, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    got = gpu_util.sim_ops.similarity_parameters_grad(x, t, w, dy, blocks=[1, 1], strides=[64, 64], padding=[0, 0], **attrs)
+    want = gpu_util.sim_ops.similarity_parameters_grad(few, t, w, dy, blocks=[1, 1], strides=[1, 1], padding=[0, 0], flags=gpu_util.abi.FLAG_FORCE_DIRECT, **attrs)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
