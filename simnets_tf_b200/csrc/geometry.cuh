@@ -21,11 +21,12 @@ struct SimGeo {
     double fudge, oob;
 };
 
-// Whether every offset that a tap or the corner of a patch can have inside a sample is below `limit` elements (in a corner, above -limit):
-// what kernels ask that keep such offsets in 32 bits, in bytes (2^29) or in elements (2^31).
+// Whether the offset of every tap from the corner of its patch is below `limit` elements, and that of every corner inside its sample fits 32
+// bits: what kernels ask that keep tap offsets in 32 bits, in bytes (2^29) or in elements (2^31).  (A block may reach beyond the image.)
 __host__ __device__ inline bool sim_offsets_below(const SimGeo& g, long long limit) {
-    const long long tap = ((g.C - 1LL) * g.H + g.bh - 1) * g.W + g.bw - 1, corner = ((long long)g.H + g.ph) * g.W + g.W + g.pw;
-    return tap < limit && corner < limit;
+    const long long tap = ((g.C - 1LL) * g.H + g.bh - 1) * g.W + g.bw - 1;
+    const long long first = (long long)g.ph * g.W + g.pw, last = ((g.oh - 1LL) * g.sh - g.ph) * g.W + (g.ow - 1LL) * g.sw - g.pw;
+    return tap < limit && first < (1LL << 31) && last < (1LL << 31);
 }
 
 // Division of 0 <= n < 2^31 by a positive constant known on the host: n / d = (n * mul) >> shift, exactly

@@ -143,7 +143,7 @@ MixWs mix_carve(const SimGeo& g, void* base) {
 }  // namespace
 
 bool mixture_shape(const SimGeo& g, bool f64, uint32_t flags) {
-    return sim_use_tiled(g, f64, flags) && flags == 0 && g.mode == SIM_L2 && (long long)g.C * g.H * g.W < (1LL << 29) && g.M <= kMixMost;
+    return sim_use_tiled(g, f64, flags) && flags == 0 && g.mode == SIM_L2 && sim_offsets_below(g, 1LL << 29) && g.M <= kMixMost;
 }
 size_t mixture_workspace_bytes(const SimGeo& g) { return mix_carve(g, nullptr).bytes; }
 

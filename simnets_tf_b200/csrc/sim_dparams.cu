@@ -679,7 +679,7 @@ int sim_dparams_splits(const SimGeo& g) {
 
 cudaError_t launch_sim_dparams(const SimGeo& g, const float* x, const float* t, const float* w, const float* dy, float* dt, float* dw,
                                bool accumulate, float* part, cudaStream_t s) {
-    if ((long long)g.C * g.H * g.W >= (1LL << 29)) return launch_sim_dparams_direct(g, false, x, t, w, dy, dt, dw, accumulate, s);    // (32-bit byte offsets)
+    if (!sim_offsets_below(g, 1LL << 29)) return launch_sim_dparams_direct(g, false, x, t, w, dy, dt, dw, accumulate, s);    // (32-bit byte offsets)
     const DpTile tile = dp_tile(g);
     const int splits = sim_dparams_splits(g), wide = dw_taps(g);
     const long long blocks = (long long)(wide > 0 ? dw_tiles(g, wide) : dp_tiles(g, tile)) * splits;

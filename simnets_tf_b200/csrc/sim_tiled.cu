@@ -57,7 +57,7 @@ __host__ SimWs carve(const SimGeo& g, void* base) {
 // The test of a tap against the image as one AND of two bits with what the position's patch misses: blocks of up to 16 x 16, 32-bit byte
 // offsets.  (Two range tests per gathered value, although a patch inside the image skipped them: 256 x 64 x 32 x 32 input, 256 templates
 // of 3x3 4134 -> 3913 us, with masks 6046 -> 5557, L1 3119 -> 2838.)
-__host__ __device__ inline bool sim_tap_bits(const SimGeo& g) { return g.bh <= 16 && g.bw <= 16 && (long long)g.C * g.H * g.W < (1LL << 29); }
+__host__ __device__ inline bool sim_tap_bits(const SimGeo& g) { return g.bh <= 16 && g.bw <= 16 && sim_offsets_below(g, 1LL << 29); }
 // the taps of a block axis that leave the image, as bits
 __device__ __forceinline__ uint32_t sim_missing(int first, int size) {
     const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
@@ -291,6 +291,10 @@ cudaError_t launch_sim_fwd_tiled(const SimGeo& g, const float* x, const float* t
 static cudaError_t sim_fwd_tiled_body(const SimGeo& g, const float* x, const float* t, const float* w, float* y, void* ws, uint32_t flags,
                                       cudaStream_t s, float* ch_max, float* ch_min, bool* extrema_done) {
     const SimWs W = carve(g, ws);
+    if (!sim_offsets_below(g, 1LL << 31)) {                 // (the tap tables hold 32 bits)
+        const cudaError_t e = launch_zero_words(W.flag, 2, s);
+        return e != cudaSuccess ? e : launch_sim_fwd_direct(g, false, x, t, w, y, s);
+    }
     if (!sim_tc_shape(g, flags) && sim_smallk_shape(g)) return launch_sim_fwd_smallk(g, x, t, w, y, ch_max, ch_min, extrema_done, W.flag, s);
     launch_prep(g, W, t, w, s);
     if (sim_tc_shape(g, flags)) {

@@ -28,23 +28,25 @@ int main() {
         const int bh = 1 + std::rand() % 6, bw = 1 + std::rand() % 6, ph = std::rand() % 6, pw = std::rand() % 6;
         const SimGeo g = shape(1 + std::rand() % 4, std::max(1, bh - 2 * ph) + std::rand() % 6, std::max(1, bw - 2 * pw) + std::rand() % 9, bh, bw, 1 + std::rand() % 3,
                                1 + std::rand() % 3, ph, pw);
-        long long most = 0, last = 0;
+        long long tap = 0;
         for (int c = 0; c < g.C; ++c)
             for (int kh = 0; kh < g.bh; ++kh)
-                for (int kw = 0; kw < g.bw; ++kw) last = std::max(last, (long long)(c * g.H + kh) * g.W + kw);
-        for (int h = 0; h < g.oh; ++h)
-            for (int w = 0; w < g.ow; ++w) most = std::max(most, std::llabs((long long)(h * g.sh - g.ph) * g.W + w * g.sw - g.pw));
-        most = std::max(most, last);
-        EXPECT(!simnets::sim_offsets_below(g, most));                       // (whatever is too small is refused)
-        EXPECT(simnets::sim_offsets_below(g, (long long)g.C * g.H * g.W + (g.bh + g.ph + 1LL) * g.W + g.bw + g.pw + 1));          // (and not much more is asked for)
+                for (int kw = 0; kw < g.bw; ++kw) tap = std::max(tap, (long long)(c * g.H + kh) * g.W + kw);
+        EXPECT(!simnets::sim_offsets_below(g, tap) && simnets::sim_offsets_below(g, tap + 1));
     }
     // the line between 31 and 32 bits of a byte offset, and of an element's
     EXPECT(simnets::sim_offsets_below(shape(1, 1 << 14, (1 << 15) - 3, 1, 1, 1, 1, 0, 0), 1LL << 29));
     EXPECT(!simnets::sim_offsets_below(shape(3, 1 << 14, 1 << 14, 1, 1, 56, 56, 0, 0), 1LL << 29));
     EXPECT(!simnets::sim_offsets_below(shape(1, 17, 1 << 25, 17, 1, 1, 512, 0, 0), 1LL << 29));
-    EXPECT(!simnets::sim_offsets_below(shape(1, 1, 1 << 25, 16, 1, 1, 512, 15, 0), 1LL << 29));          // rows of the block beyond the image
+    EXPECT(!simnets::sim_offsets_below(shape(1, 1, 1 << 25, 18, 1, 1, 512, 17, 0), 1LL << 29));          // rows of the block beyond the image
     EXPECT(simnets::sim_offsets_below(shape(3, 1 << 14, 1 << 14, 1, 1, 56, 56, 0, 0), 1LL << 31));
     EXPECT(!simnets::sim_offsets_below(shape(33, 8200, 8200, 1, 1, 64, 64, 0, 0), 1LL << 31));
+    EXPECT(!simnets::sim_offsets_below(shape(1, 46342, 46342, 1, 1, 1, 1, 0, 0), 1LL << 31));          // corners beyond 32 bits, on either side
+    EXPECT(simnets::sim_offsets_below(shape(1, 46342, 46338, 3, 1, 1, 1, 0, 0), 1LL << 31));
+    EXPECT(!simnets::sim_offsets_below(shape(1, 1, 1 << 27, 16, 1, 1, 512, 16, 0), 1LL << 31));
+    // nothing that lies in a sample of fewer than 2^29 values, blocks inside the image, is refused
+    EXPECT(simnets::sim_offsets_below(shape(1, 16384, 32767, 1, 1, 1, 1, 0, 0), 1LL << 29));
+    EXPECT(simnets::sim_offsets_below(shape(8, 64, (1 << 20) - 1, 64, 5, 1, 1, 63, 4), 1LL << 29));
     return 0;
 }
 """

@@ -47,3 +47,28 @@ def test_parameter_gradients_of_offsets_beyond_31_bits(attrs):
     want = gpu_util.sim_ops.similarity_parameters_grad(few, t, w, dy, blocks=[1, 1], strides=[1, 1], padding=[0, 0], flags=gpu_util.abi.FLAG_FORCE_DIRECT, **attrs)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def test_blocks_of_rows_beyond_a_wide_image():
+    """Sixteen rows of 2^26 pixels around an image of two: most of the block lies outside, where its offsets need 32 bits and more."""
+    x, dy = _sample(1, 1, 2, 1 << 26), None
+    few = x[:, :, :, ::4096].contiguous()
+    for m, attrs in ((64, dict()), (64, dict(normalization_term=True, ignore_nan_input=True)), (12, dict(similarity_function="L1"))):
+        t, w = _parameters(m, 1, 16, 1)
+        y = gpu_util.sim_ops.similarity_forward(x, t, w, blocks=[16, 1], strides=[1, 4096], padding=[14, 0], **attrs)
+        want = gpu_util.sim_ops.similarity_forward(few, t, w, blocks=[16, 1], strides=[1, 1], padding=[14, 0], **attrs)
+        assert float((y - want).abs().max()) <= 1e-5 * float(want.abs().max())
+        dy = torch.randn(y.shape, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+        got = gpu_util.sim_ops.similarity_parameters_grad(x, t, w, dy, blocks=[16, 1], strides=[1, 4096], padding=[14, 0], **attrs)
+        want = gpu_util.sim_ops.similarity_parameters_grad(few, t, w, dy, blocks=[16, 1], strides=[1, 1], padding=[14, 0], **attrs)
+        for a, b in zip(got, want):
+            assert float((a - b).norm()) <= 1e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("m,attrs", [(32, dict()), (5, dict(normalization_term=True)), (32, dict(similarity_function="L1"))], ids=["l2", "l2n", "l1"])
+def test_forward_of_offsets_beyond_31_bits(m, attrs):
+    """The sample of the parameter gradients' test, through the default dispatch of the forward pass."""
+    x, (t, w) = _sample(1, 33, 8200, 8200), _parameters(m, 33, 1, 1)
+    y = gpu_util.sim_ops.similarity_forward(x, t, w, blocks=[1, 1], strides=[64, 64], padding=[0, 0], **attrs)
+    want = gpu_util.sim_ops.similarity_forward(x[:, :, ::64, ::64].contiguous(), t, w, blocks=[1, 1], strides=[1, 1], padding=[0, 0], **attrs)
+    assert float((y - want).abs().max()) <= 1e-5 * float(want.abs().max())
