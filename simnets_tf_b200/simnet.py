@@ -59,14 +59,21 @@ def sum_pool(x, k):
     return _SumPool.apply(x, k)
 
 
+# What a call of a module runs, as torch defines it; replaced functions (instrumentation, symbolic tracers) are found by comparing with these,
+# and by where they come from if that happened before this file was imported.
+_CALL = (torch.nn.Module.__call__, torch.nn.Module._call_impl)
+_CALL_IS_TORCHS = all(getattr(getattr(f, "__code__", None), "co_filename", None) == _module.__file__ for f in _CALL)
+
+
 def _caller():
     """How a network calls its layers: by their own forward() where nothing hangs on the call of the module (1.5 us of host time
-    each), else as modules (hooks of the layer or of all modules, a subclass with a call of its own, a compiled or recorded one)."""
-    hooked = getattr(_module, "_has_any_global_hook", lambda: True)() or is_tracing()
+    each), else as modules (hooks of the layer or of all modules, a call that the layer's class or anybody else has replaced, a compiled or
+    recorded one)."""
+    hooked = not _CALL_IS_TORCHS or getattr(_module, "_has_any_global_hook", lambda: True)() or is_tracing()
 
     def call(m):
         if hooked or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or \
-                type(m).__call__ is not torch.nn.Module.__call__ or getattr(m, "_compiled_call_impl", None) is not None:
+                type(m).__call__ is not _CALL[0] or type(m)._call_impl is not _CALL[1] or getattr(m, "_compiled_call_impl", None) is not None:
             return m
         return m.forward
     return call
