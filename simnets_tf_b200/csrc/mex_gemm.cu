@@ -342,6 +342,31 @@ __device__ __noinline__ void exact_dx(const MexGeo& g, const T* x, const T* off,
     for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kGemmThreads + threadIdx.x; i < total; i += step) dx[i] = mex_exact_dx(g, x, off, y, dy, i);
 }
 
+// The sums of the offsets gradient term by term, into sums[r][m][k]: the threads of a CTA share the positions of one of them at a time, so
+// that a register adds up 1 / 256 of its B rs terms.  One thread per sum, 459 K positions under 8 instances of 4x2x2 taps: 306 ms and 1e-5
+// of the gradient's norm from float64; so 1.6 ms and 6e-7.
+template <typename T>
+__device__ __noinline__ void exact_doff(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* sums, T* red) {
+    const long long total = (long long)g.R * g.M * g.K, P = (long long)g.B * g.rs, ctas = (long long)gridDim.x * gridDim.y;
+    const T eps = T(g.eps), cst = T(g.cst), oob = T(g.oob);
+    for (long long i = (long long)blockIdx.y * gridDim.x + blockIdx.x; i < total; i += ctas) {
+        const int k = int(i % g.K), m = int(i / g.K % g.M), r = int(i / g.K / g.M), kw = k % g.bw, kh = k / g.bw % g.bh, kc = k / (g.bw * g.bh);
+        const long long tap = ((long long)kc * g.H + kh) * g.W + kw;
+        const T o = off[i];
+        T v = T(0);
+#pragma unroll 2
+        for (long long j = threadIdx.x; j < P; j += kGemmThreads) {
+            const GemmCol c = gemm_col(g, r, j, P);
+            if (c.base < 0) continue;
+            const int cc = c.c0 + kc, h = c.h0 + kh, w = c.w0 + kw;
+            const bool in = c.inside || (cc >= 0 && cc < g.C && h >= 0 && h < g.H && w >= 0 && w < g.W);
+            v += mex_weight(g, eps, cst, in ? x[c.xb + tap] : oob, o, y[c.base + (long long)m * g.N], dy[c.gbase + (long long)m * g.Ng]);
+        }
+        v = row_reduce<T, true>(v, red, false);
+        if (threadIdx.x == 0) sums[i] = v;
+    }
+}
+
 // What a CTA multiplies, in shared memory: As[2][kQ][LDA], Bs[2][kQ][LDB], step by step.  A thread's reads of them are the bound (32
 // lanes x 16 bytes take four cycles however few different addresses they have):
 //  * float32: TM/8 x 4 outputs per thread in packed arithmetic, half of the threads cover the tile and the two halves share the steps
@@ -611,7 +636,8 @@ __global__ void __launch_bounds__(kGemmThreads, gemm_ctas<T, OP, TM>()) mex_gemm
             if (unsafe) {
                 if (OP == kFwd) exact_forward(g, x, off, out);
                 if (OP == kDx) exact_dx(g, x, off, y, dy, out);
-                return;                                       // (the offsets gradient's finishing kernel evaluates its rows itself)
+                if (OP == kDoff) exact_doff(g, x, off, y, dy, part, smem);
+                return;
             }
         }
         if (c + 1 < c_end) commit(next, next + kQ * LDA, c + 1);
@@ -789,7 +815,6 @@ __global__ void __launch_bounds__(1024) mex_gemm_finish_doff(const __grid_consta
     for (int i = threadIdx.x; i < verdicts; i += blockDim.x) bad |= verdict[i];
     const bool unsafe = __syncthreads_or(bad) != 0;
     const size_t n = (size_t)g.R * g.M * g.K, row = (size_t)blockIdx.x * g.K;
-    const int r = blockIdx.x / g.M, m = blockIdx.x - r * g.M;
     T sum = T(0);
     const auto keep = [&](int k, T v) {
         if (normalize) part[row + k] = v;
@@ -797,11 +822,7 @@ __global__ void __launch_bounds__(1024) mex_gemm_finish_doff(const __grid_consta
         sum += v;
     };
     if (unsafe) {
-        for (int k = threadIdx.x; k < g.K; k += blockDim.x) {
-            T v = T(0);
-            for (long long i = 0; i < (long long)g.B * g.rs; ++i) v += mex_exact_doff_term(g, x, off[row + k], y, dy, r, m, k, i);
-            keep(k, v);
-        }
+        for (int k = threadIdx.x; k < g.K; k += blockDim.x) keep(k, part[row + k]);          // (whole sums: exact_doff)
     } else if (groups > 1) {                                  // (K <= 256 / groups, 256 threads)
         const int width = kGemmThreads / groups, k = threadIdx.x % width;
         T v = T(0);

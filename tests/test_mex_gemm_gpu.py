@@ -175,3 +175,26 @@ def test_gradients_behind_another_family_s_forward_pass(port, c):
         full = small.repeat_interleave(2, 2).repeat_interleave(2, 3).contiguous()
         for a, b in zip(mex_ops.mex_backward(x, off, y, small, m, pooled=True, **attrs), mex_ops.mex_backward(x, off, y, full, m, **attrs)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shape,m,blocks,regions", [((28, 64, 32, 32), 8, (4, 2, 2), 0), ((48, 32, 32, 32), 30, (32, 1, 1), 2), ((40, 12, 24, 25), 9, (12, 3, 3), 0)],
+                         ids=["short_patches", "pixels", "overlapping"])
+def test_long_sums_beyond_the_safe_spread(shape, m, blocks, regions):
+    """One offset 200 below the others, up to 115 K positions in a sum of the offsets gradient.  256 threads share them: a register of up to 450
+    terms is some 0.3 x 2^-24 x sqrt(450) = 4e-7 of its sum away from it, one that takes all terms 6e-6."""
+    strides = blocks if blocks[1] < 3 else (blocks[0], 1, 1)
+    region = dict(use_unshared_regions=True, unshared_offset_region=[regions]) if regions else dict(use_unshared_regions=False, shared_offset_region=[-1])
+    attrs = dict(softmax_mode=True, blocks=list(blocks), strides=list(strides), **region)
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x, off = torch.randn(shape, generator=gen, device="cuda"), torch.randn((max(1, regions) ** 2, m) + blocks, generator=gen, device="cuda")
+    off[-1, m // 2, 1, 0, 0] = -200.0
+    y = mex_ops.mex_forward(x.double(), off.double(), m, flags=abi.FLAG_FORCE_DIRECT, **attrs)
+    dy = torch.randn(y.shape, generator=gen, device="cuda")
+    want = mex_ops.mex_backward(x.double(), off.double(), y, dy.double(), m, flags=abi.FLAG_FORCE_DIRECT, **attrs)
+    wide = mex_ops.mex_backward(x.double(), off.double(), y, dy.double(), m, **attrs)
+    for got, ref in zip(wide, want):
+        assert float((got - ref).norm()) <= 1e-14 * float(ref.norm())
+    y = y.float()
+    want = mex_ops.mex_backward(x.double(), off.double(), y.double(), dy.double(), m, flags=abi.FLAG_FORCE_DIRECT, **attrs)
+    for got, ref in zip(mex_ops.mex_backward(x, off, y, dy, m, **attrs), want):
+        assert float((got.double() - ref).norm()) <= 1.5e-6 * float(ref.norm())
