@@ -123,7 +123,9 @@ enum { SIMNETS_SIM_L1 = 0, SIMNETS_SIM_L2 = 1 };
  * same input, offsets, descriptor and flags (SIMNETS_FLAG_MEX_DY_POOLED2 aside) and nothing has written to it
  * since, other gradient calls of that layer excepted.  The per-position maxima and the offsets tables that the
  * forward pass left there are then used as they are instead of being computed again (same values, fewer
- * launches).  Ignored where the forward pass of the shape does not leave them.  The caller owns the promise: a
+ * launches).  Ignored where the forward pass of the shape does not leave them: gradients that run on other kernels
+ * than the forward pass (layers of fewer than 48 instances) prepare the workspace again, over what the forward pass
+ * left there.  The caller owns the promise: a
  * workspace that was reused in between gives wrong gradients, not an error. */
 #define SIMNETS_FLAG_MEX_WORKSPACE_PRIMED (1u << 8)
 
@@ -294,8 +296,8 @@ SIMNETS_API int simnets_mex_forward_pool2x2(const simnets_mex_desc* d,
  *   host_out[1] != 0: a tensor-core kernel gave up on a bounded wait between its roles (about two seconds) and left
  *                     early; the exact kernels launched behind it recomputed the outputs of that call, so they are
  *                     valid, only slow.  Not expected outside SIMNETS_FLAG_MEX_TEST_EXPIRE_WAIT.
- * The words are cleared by the next call that runs the prepasses on this workspace (every call without
- * SIMNETS_FLAG_MEX_WORKSPACE_PRIMED). */
+ * The words are set anew by the next call that runs the prepasses on this workspace (every call without
+ * SIMNETS_FLAG_MEX_WORKSPACE_PRIMED, and those that ignore it). */
 SIMNETS_API int simnets_mex_workspace_status(const void* workspace, void* stream, int32_t* host_out);
 
 /* MEX forward for callers that have no scratch to give.  No counterpart in the reference: its

@@ -59,7 +59,7 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
 
 template <typename T>
 struct GemmWs {
-    int* flag;           // [2] the workspace's status words
+    int* flag;           // [2] the workspace's status words, written by the contractions of a call that ran the prepass (null in others)
     int* verdict;        // one per CTA of the parameter prepass: offsets that the factorised form cannot take
     T *mo, *lse;         // [R][M]
     T *eo;               // [R][M][K]
@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kGemmThreads, gemm_ctas<T, OP, TM>()) mex_gemm
             if (!POS && OP != kDoff && threadIdx.x < kTN) mx_s[POS ? 0 : threadIdx.x] = cmx;
             if (!POS && OP == kDoff) place_maxima(c_begin);
             const bool unsafe = gemm_unsafe(verdict, verdicts);
-            if (OP == kFwd && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) flag[threadIdx.x] = threadIdx.x == 0 && unsafe;
+            if (flag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) flag[threadIdx.x] = threadIdx.x == 0 && unsafe;
             if (unsafe) {
                 if (OP == kFwd) exact_forward(g, x, off, out);
                 if (OP == kDx) exact_dx(g, x, off, y, dy, out);
@@ -956,9 +956,11 @@ cudaError_t gemm_forward(const MexGeo& g, const T* x, const T* off, T* y, void* 
 template <typename T>
 cudaError_t gemm_backward(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* dx, T* doff, bool accumulate, void* ws, void* products, uint32_t flags,
                           cudaStream_t s) {
-    const GemmWs<T> w = carve_gemm<T>(g, ws);
-    // (a primed workspace holds what the forward pass prepared for the same input and offsets)
-    cudaError_t e = flags & SIMNETS_FLAG_MEX_WORKSPACE_PRIMED ? cudaSuccess : gemm_prepare(g, w, x, off, flags & ~uint32_t(SIMNETS_FLAG_MEX_MAXIMA_GIVEN), s);
+    GemmWs<T> w = carve_gemm<T>(g, ws);
+    // (a primed workspace holds what the forward pass prepared for the same input and offsets, and its status)
+    const bool primed = (flags & SIMNETS_FLAG_MEX_WORKSPACE_PRIMED) != 0;
+    cudaError_t e = primed ? cudaSuccess : gemm_prepare(g, w, x, off, flags & ~uint32_t(SIMNETS_FLAG_MEX_MAXIMA_GIVEN), s);
+    if (primed) w.flag = nullptr;
     if (e != cudaSuccess) return e;
     const T* rows = gemm_norm(flags) ? w.offn : off;
     if (dx != nullptr) {

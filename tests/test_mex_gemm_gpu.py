@@ -198,3 +198,28 @@ def test_long_sums_beyond_the_safe_spread(shape, m, blocks, regions):
     want = mex_ops.mex_backward(x.double(), off.double(), y.double(), dy.double(), m, flags=abi.FLAG_FORCE_DIRECT, **attrs)
     for got, ref in zip(mex_ops.mex_backward(x, off, y, dy, m, **attrs), want):
         assert float((got.double() - ref).norm()) <= 1.5e-6 * float(ref.norm())
+
+
+@pytest.mark.parametrize("dtype", [abi.F32, abi.F64], ids=["f32", "f64"])
+@pytest.mark.parametrize("c", BACKWARD_ONLY + [c for c in EDGES if c["name"] in ("overlap_72_rows", "map_2x2_split")], ids=lambda c: c["name"])
+def test_status_words_of_gradients_on_a_fresh_workspace(cuda_lib, c, dtype):
+    """A gradient call without a forward pass in front runs the prepass itself, and says what that found."""
+    t_t = torch.float32 if dtype == abi.F32 else torch.float64
+    d = cases.mex_desc(c, dtype=dtype)
+    g = abi.MexGeometry()
+    assert cuda_lib.simnets_mex_dims(C.byref(d), C.byref(g)) == 0
+    oshape = (c["shape"][0], g.channels_out_total, g.height_out, g.width_out)
+    x, off, dy = (gpu_util.dev(a, t_t) for a in cases.mex_inputs(c, (g.num_regions, g.M, g.block_c, g.block_h, g.block_w), oshape))
+    bytes_, stream, status = cuda_lib.simnets_mex_workspace_bytes(C.byref(d)), torch.cuda.current_stream().cuda_stream, (C.c_int32 * 2)(7, 7)
+    for spread, want in ((0.0, 0), (-700.0, 1)):
+        off[0, 0, 0, 0, 0] += spread
+        y = mex_ops.mex_forward(x, off, c["M"], **cases.mex_attrs(c))
+        dx, doff = torch.empty_like(x), torch.empty_like(off)
+        tensors = [C.byref(d), x.data_ptr(), off.data_ptr(), y.data_ptr(), dy.data_ptr()]
+        for call, out in ((cuda_lib.simnets_mex_input_grad, [dx.data_ptr()]), (cuda_lib.simnets_mex_offsets_grad, [doff.data_ptr()]),
+                          (cuda_lib.simnets_mex_backward, [dx.data_ptr(), doff.data_ptr()])):
+            ws = torch.full((bytes_,), 0xFF, dtype=torch.uint8, device="cuda")
+            assert call(*tensors, *out, ws.data_ptr(), bytes_, stream) == 0
+            assert cuda_lib.simnets_mex_workspace_status(ws.data_ptr(), stream, status) == 0
+            torch.cuda.synchronize()
+            assert tuple(status) == (want, 0)
