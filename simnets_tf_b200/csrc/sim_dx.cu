@@ -15,8 +15,8 @@
 // them; 19 channels in 32 rows had spent 41 % on padding), and a chunk is instances of ONE tap: its operands advance by one addition
 // each, where a cursor per staged value had cost several instructions.  256 x 64 x 32 x 32 input, 256 templates of 3x3: 4981 -> 4237 us
 // (62 -> 74 % of the pipe); 37 x 19 x 45 x 37, 100 of 5x3 at stride 2 and 1, L1:
-// 490 -> 277; 64 x 24 x 30 x 31, 90 of 3x3: 308 -> 203.  L1 adds e with the sign of d put on it, 0 selected where d is 0 or NaN: one
-// instruction per term less than multiplying by a sign (from registers 5.0 -> 5.9 T terms/s).
+// 490 -> 276; 64 x 24 x 30 x 31, 90 of 3x3: 308 -> 203.  L1 adds e with the sign of d put on it, and 0 e (NaN for an e that is no finite
+// number) where d is 0 or NaN: 256 templates of 3x3 over 256 x 64 x 32 x 32 6366 us, 8011 when a sign is multiplied by e.
 //
 // NaN pixels give 0 in the ignore_nan_input modes, and so does a pixel that no patch covers in every mode.  A tap that the
 // padding cuts off, or a step past the last one, contributes 0 * (t - x), which is NaN for an infinite x (or an infinite
@@ -32,8 +32,8 @@ namespace {
 // sign of d, 0 for 0 and NaN as in the reference
 __device__ __forceinline__ float dx_sign(float d) { return fabsf(d) > 0.f ? __uint_as_float(0x3f800000u | (__float_as_uint(d) & 0x80000000u)) : 0.f; }
 
-// e sign(d)
-__device__ __forceinline__ float dx_signed(float e, float d) { return fabsf(d) > 0.f ? __uint_as_float(__float_as_uint(e) ^ (__float_as_uint(d) & 0x80000000u)) : 0.f; }
+// e sign(d); e0 = 0 e, which is NaN where e is no finite number
+__device__ __forceinline__ float dx_signed(float e, float e0, float d) { return fabsf(d) > 0.f ? __uint_as_float(__float_as_uint(e) ^ (__float_as_uint(d) & 0x80000000u)) : e0; }
 
 // The pixels and taps of one phase along one axis: pixels first, first + stride, ... (n of them), taps r, r + stride, ... (taps
 // of them); pixel i meets tap a at output i + shift - a.
@@ -242,7 +242,10 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const float2 d = add2(splat2(t[r]), xx[r][c]), e = mul2(splat2(w[r]), g2[c]);
-                acc[r][c] = L1 ? add2(acc[r][c], make_float2(dx_signed(e.x, d.x), dx_signed(e.y, d.y))) : fma2(e, d, acc[r][c]);
+                if (L1) {
+                    const float2 e0 = mul2(e, make_float2(0.f, 0.f));
+                    acc[r][c] = add2(acc[r][c], make_float2(dx_signed(e.x, e0.x, d.x), dx_signed(e.y, e0.y, d.y)));
+                } else acc[r][c] = fma2(e, d, acc[r][c]);
             }
     };
     auto compute = [&](const float* stage, int steps) {

@@ -163,3 +163,29 @@ def test_patches_that_leave_the_image_on_every_side(port, batch, m, blocks, padd
     y = gpu_util.sim_ops.similarity_forward(*(gpu_util.dev(a) for a in (x, t, w)), **cases.sim_attrs(c)).cpu().numpy()
     cases.assert_parity(y, port.similarity_forward(d, x, t, w), port.similarity_forward(cases.sim_desc(c, dtype=gpu_util.abi.F64), *(a.astype(np.float64) for a in (x, t, w))),
                         what=c["name"])
+
+
+# ---- L1 where dy (or a weight) is no finite number and a difference is 0: 0 times it is NaN, on every kernel
+L1_MODES = [dict(fn="L1"), dict(fn="L1", flags=gpu_util.abi.FLAG_SIM_L1_SKIP_NAN)]
+
+
+def _l1_case(name, shape, M, blocks, strides, padding, seed, mode):
+    c = cases.sim_case(name, shape, M, blocks=blocks, strides=strides, padding=padding, oob=0.3, seed=seed, **mode)
+    return c, cases.sim_desc(c)
+
+
+@pytest.mark.parametrize("mode", L1_MODES, ids=["l1", "l1skip"])
+@pytest.mark.parametrize("channels", [5, 12, 17, 24, 30, 40, 48, 64, 70])
+def test_l1_input_gradients_of_a_dy_that_is_no_number(port, channels, mode):
+    """A patch of every sample is template 1, whose dy there is inf, NaN or -inf; one pixel equals a tap of infinite weight."""
+    c, d = _l1_case("dy%d" % channels, (3, channels, 9, 8), 11, (3, 2), (2, 1), (1, 0), 870 + channels, mode)
+    x, t, w, dy = cases.sim_inputs(c, port.sim_out_shape(d))
+    for n, bad in enumerate((np.inf, NAN, -np.inf)):
+        x[n, :, 3:6, 2:4] = t[1]                            # (output row 2, column 2)
+        dy[n, 1, 2, 2] = bad
+    x[0, :, 0, 6] = t[2, :, 1, 1]                           # (output row 0, column 5)
+    w[2, 0, 1, 1] = np.inf
+    dx = gpu_util.sim_ops.similarity_input_grad(*(gpu_util.dev(a) for a in (x, t, w, dy)), flags=c["flags"], **cases.sim_attrs(c)).cpu().numpy()
+    ref = port.similarity_input_grad(d, x, t, w, dy)
+    assert np.isnan(ref[:, :, 3:6, 2:4]).all() and np.isnan(ref[0, 0, 0, 6])
+    cases.assert_parity(dx, ref, what=c["name"])
