@@ -344,8 +344,8 @@ template <int MODE, int WJ> struct DwTile {
     static constexpr int SMEM = 8 * STAGE, SLOT_BYTES = 4 * (MODE == SIM_L2N_NAN ? 48 : 32) * kDpThreads;        // bytes: two stages; sums set aside
 };
 
-// a sign(d), 0 where d is 0 or NaN
-__device__ __forceinline__ float dw_signed(float a, float d) { return fabsf(d) > 0.f ? __uint_as_float(__float_as_uint(a) ^ (__float_as_uint(d) & 0x80000000u)) : 0.f; }
+// a sign(d); a0 = 0 a where d is 0 or NaN, which is NaN for an a that is no finite number
+__device__ __forceinline__ float dw_signed(float a, float a0, float d) { return fabsf(d) > 0.f ? __uint_as_float(__float_as_uint(a) ^ (__float_as_uint(d) & 0x80000000u)) : a0; }
 // the taps first .. of a block axis that leave the image, as bits (block <= 16)
 __device__ __forceinline__ uint32_t dw_missing(int first, int size) {
     const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
@@ -502,11 +502,12 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams_wide(con
                             sW[r][c] = fma2(u, d[r][c], sW[r][c]);
                         }
                 } else {
+                    const float a0[4] = {a[0] * 0.f, a[1] * 0.f, a[2] * 0.f, a[3] * 0.f};
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
 #pragma unroll
                         for (int c = 0; c < 2; ++c) {
-                            sT[r][c] = add2(sT[r][c], make_float2(dw_signed(a[r], d[r][c].x), dw_signed(a[r], d[r][c].y)));
+                            sT[r][c] = add2(sT[r][c], make_float2(dw_signed(a[r], a0[r], d[r][c].x), dw_signed(a[r], a0[r], d[r][c].y)));
                             sW[r][c] = fma2(splat2(a[r]), dp_abs2(d[r][c]), sW[r][c]);
                         }
                 }

@@ -189,3 +189,27 @@ def test_l1_input_gradients_of_a_dy_that_is_no_number(port, channels, mode):
     ref = port.similarity_input_grad(d, x, t, w, dy)
     assert np.isnan(ref[:, :, 3:6, 2:4]).all() and np.isnan(ref[0, 0, 0, 6])
     cases.assert_parity(dx, ref, what=c["name"])
+
+
+@pytest.mark.parametrize("mode", L1_MODES, ids=["l1", "l1skip"])
+@pytest.mark.parametrize("channels,m", [(3, 33), (5, 64), (6, 40), (11, 70), (30, 100), (3, 20), (2, 40)])
+def test_l1_parameter_gradients_of_a_dy_that_is_no_number(port, channels, m, mode):
+    """The first channel of a patch of every sample is that of template 1, whose dy there is inf, NaN or -inf; 64 x 32 and 64 x 64 tiles, and
+    the smaller ones of few templates or taps."""
+    c, d = _l1_case("dp%d_%d" % (channels, m), (3, channels, 9, 8), m, (3, 2), (2, 1), (1, 0), 880 + channels, mode)
+    x, t, w, dy = cases.sim_inputs(c, port.sim_out_shape(d))
+    for n, bad in enumerate((np.inf, NAN, -np.inf)):
+        x[n, 0, 3:6, 2:4] = t[1 + n, 0]                     # (output row 2, column 2)
+        dy[n, 1 + n, 2, 2] = bad
+    got = gpu_util.sim_ops.similarity_parameters_grad(*(gpu_util.dev(a) for a in (x, t, w, dy)), flags=c["flags"], **cases.sim_attrs(c))
+    ref = port.similarity_params_grad(d, x, t, w, dy)
+    assert np.isnan(ref[0][1:4, 0]).all() and np.isinf(ref[0][1, 1:]).all()
+    for g, r in zip(got, ref):
+        cases.assert_parity(g.cpu().numpy(), r, what=c["name"])
+
+
+@pytest.mark.parametrize("i", range(len(PARAM_TILES)))
+def test_l1_skipping_nan_at_the_edges_of_the_tiles(port, i):
+    shape, M, blocks, strides, padding = PARAM_TILES[i]
+    gpu_util.check_similarity(port, cases.sim_case("skip%d" % i, shape, M, blocks=blocks, strides=strides, padding=padding, oob=0.3, nan_frac=0.2, seed=890 + i, **L1_MODES[1]),
+                              f64_tiebreak=True)
