@@ -18,19 +18,28 @@ constexpr int kThreads = 256;
 
 constexpr double kLog2Pi = 1.8378770664093454835606594728112;
 
-// Deterministic block-wide sum (fixed tree), result valid in thread 0.
+// Gated launches follow a factorised kernel and work only if that one raised its flag: two CTAs per SM, since what the usual case pays is
+// their coming up (eight CTAs of 256 threads for the seven launches of a step: 16.3 us, two 12.8), of more threads, since what the other
+// case pays is how few they are.
+constexpr int kGatedThreads = 640, kGatedBwdThreads = 2 * kThreads;
+
+// Deterministic sum over kThreads threads (fixed tree), `lane` of a block of as many or of one of several such groups, which all take part;
+// the result is valid in lane 0.
 template <typename T>
-__device__ __forceinline__ T block_sum(T v, T* smem) {
-    smem[threadIdx.x] = v;
+__device__ __forceinline__ T block_sum(T v, T* smem, int lane) {
+    smem[lane] = v;
     __syncthreads();
-    for (int s = kThreads / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) smem[threadIdx.x] += smem[threadIdx.x + s];
-        __syncthreads();
+    if (lane < 32) {
+        const auto four = [&](int i) { return (smem[i] + smem[i + 128]) + (smem[i + 64] + smem[i + 192]); };
+        v = four(lane) + four(lane + 32);
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
     }
-    const T r = smem[0];
     __syncthreads();
-    return r;
+    return v;
 }
+template <typename T>
+__device__ __forceinline__ T block_sum(T v, T* smem) { return block_sum(v, smem, int(threadIdx.x)); }
 
 // ------------------------------------------------------------------ Similarity
 template <typename T>
@@ -204,21 +213,21 @@ __global__ void __launch_bounds__(kThreads) sim_dparams_direct(SimGeo g, const T
 
 // ------------------------------------------------------------------------- MEX
 template <typename T>
-__global__ void __launch_bounds__(kThreads) mex_fwd_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off, T* __restrict__ y, const int* __restrict__ gate) {
+__global__ void __launch_bounds__(kGatedThreads, 2) mex_fwd_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off, T* __restrict__ y, const int* __restrict__ gate) {
     stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.M * g.N;
-    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads)
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x)
         y[idx] = mex_exact_y(g, x, off, idx);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) mex_dx_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off,
+__global__ void __launch_bounds__(kGatedThreads, sizeof(T) == 4 ? 2 : 1) mex_dx_direct(MexGeo g, const T* __restrict__ x, const T* __restrict__ off,
                                                           const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx, const int* __restrict__ gate) {
     stream_order();
     if (gate && (gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.C * g.H * g.W;
-    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads)
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x)
         dx[idx] = mex_exact_dx(g, x, off, y, dy, idx);
 }
 
@@ -248,13 +257,13 @@ __global__ void __launch_bounds__(kThreads) mex_doff_direct(MexGeo g, const T* _
 
 // The term-by-term redo behind a factorised forward pass whose 2x2 sum pooling was produced with it: a thread redoes the four
 // outputs of one pooling window and their sum (added in window order).
-__global__ void __launch_bounds__(kThreads) mex_redo_fwd_pool(MexGeo g, const float* __restrict__ x, const float* __restrict__ off, float* __restrict__ y,
+__global__ void __launch_bounds__(kGatedThreads, 2) mex_redo_fwd_pool(MexGeo g, const float* __restrict__ x, const float* __restrict__ off, float* __restrict__ y,
                                                               float* __restrict__ pooled, const int* __restrict__ gate) {
     stream_order();
     if ((gate[0] | gate[1]) == 0) return;
     const int Hp = g.Ho / 2, Wp = g.Wo / 2;
     const long long total = (long long)g.B * g.M * g.Co * Hp * Wp;
-    for (long long i = blockIdx.x * (long long)kThreads + threadIdx.x; i < total; i += (long long)gridDim.x * kThreads) {
+    for (long long i = blockIdx.x * (long long)kGatedThreads + threadIdx.x; i < total; i += (long long)gridDim.x * kGatedThreads) {
         const int w = int(i % Wp);
         const long long ph = i / Wp, at = (ph / Hp * g.Ho + 2 * (ph % Hp)) * g.Wo + 2 * w;
         float s = 0.f;
@@ -269,31 +278,33 @@ __global__ void __launch_bounds__(kThreads) mex_redo_fwd_pool(MexGeo g, const fl
     }
 }
 
-// The same behind both gradients of a layer: one launch redoes dx and doff.
-__global__ void __launch_bounds__(kThreads) mex_redo_bwd(MexGeo g, const float* __restrict__ x, const float* __restrict__ off, const float* __restrict__ y,
+// The same behind both gradients of a layer: one launch redoes dx and doff, kThreads threads a sum.
+__global__ void __launch_bounds__(kGatedBwdThreads, 2) mex_redo_bwd(MexGeo g, const float* __restrict__ x, const float* __restrict__ off, const float* __restrict__ y,
                                                          const float* __restrict__ dy, float* __restrict__ dx, float* __restrict__ doff, int accumulate,
                                                          const int* __restrict__ gate) {
     stream_order();
-    __shared__ float smem[kThreads];
+    constexpr int kGroups = kGatedBwdThreads / kThreads;
+    __shared__ float smem[kGatedBwdThreads];
     if ((gate[0] | gate[1]) == 0) return;
     const long long total = (long long)g.B * g.C * g.H * g.W;
-    for (long long idx = blockIdx.x * (long long)kThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kThreads)
+    for (long long idx = blockIdx.x * (long long)kGatedBwdThreads + threadIdx.x; idx < total; idx += (long long)gridDim.x * kGatedBwdThreads)
         dx[idx] = mex_exact_dx(g, x, off, y, dy, idx);
-    const long long triples = (long long)g.R * g.M * g.K;
-    for (long long rmk = blockIdx.x; rmk < triples; rmk += gridDim.x) {
+    const long long triples = (long long)g.R * g.M * g.K, positions = (long long)g.B * g.rs;
+    const int group = threadIdx.x / kThreads, lane = threadIdx.x % kThreads;
+    for (long long first = (long long)blockIdx.x * kGroups; first < triples; first += (long long)gridDim.x * kGroups) {
+        const long long rmk = first + group;
         const int k = int(rmk % g.K), m = int((rmk / g.K) % g.M), r = int(rmk / ((long long)g.K * g.M));
         float sum = 0.f;
-        for (long long i = threadIdx.x; i < (long long)g.B * g.rs; i += kThreads) sum += mex_exact_doff_term(g, x, off[rmk], y, dy, r, m, k, i);
-        const float rsum = block_sum(sum, smem);
-        if (threadIdx.x == 0) doff[rmk] = accumulate ? doff[rmk] + rsum : rsum;
+        if (rmk < triples)
+            for (long long i = lane; i < positions; i += kThreads) sum += mex_exact_doff_term(g, x, off[rmk], y, dy, r, m, k, i);
+        const float rsum = block_sum(sum, smem + group * kThreads, lane);
+        if (lane == 0 && rmk < triples) doff[rmk] = accumulate ? doff[rmk] + rsum : rsum;
     }
 }
 
-// gated: the launch follows a factorised kernel and does work only if that one raised the safety flag; a grid that
-// just fills the GPU keeps the usual case (every CTA reads the flag and returns) at a few microseconds
 inline int grid_for(long long total, bool gated = false) {
-    const long long blocks = (total + kThreads - 1) / kThreads;
-    const long long cap = (long long)device_sm_count() * (gated ? 2 : 32);          // (a gated grid is there to find that nothing is to be done)
+    const int threads = gated ? kGatedThreads : kThreads;
+    const long long blocks = (total + threads - 1) / threads, cap = (long long)device_sm_count() * (gated ? 2 : 32);
     return int(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
 }
 
@@ -365,21 +376,21 @@ cudaError_t launch_mex_fwd_direct(const MexGeo& g, bool f64, const void* x, cons
     const long long total = (long long)g.B * g.M * g.N;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (in_stream_order(mex_fwd_direct<float>, grid_for(total, gate != nullptr), kThreads, 0, s)(g, (const float*)x, (const float*)off, (float*)y, gate)),
+        (in_stream_order(mex_fwd_direct<float>, grid_for(total, gate != nullptr), gate != nullptr ? kGatedThreads : kThreads, 0, s)(g, (const float*)x, (const float*)off, (float*)y, gate)),
         (in_stream_order(mex_fwd_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)off, (double*)y, gate)));
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_mex_redo_fwd_pool(const MexGeo& g, const float* x, const float* off, float* y, float* pooled, cudaStream_t s, const int* gate) {
-    in_stream_order(mex_redo_fwd_pool, grid_for((long long)g.B * g.M * g.N / 4, true), kThreads, 0, s)(g, x, off, y, pooled, gate);
+    in_stream_order(mex_redo_fwd_pool, grid_for((long long)g.B * g.M * g.N / 4, true), kGatedThreads, 0, s)(g, x, off, y, pooled, gate);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_mex_redo_bwd(const MexGeo& g, const float* x, const float* off, const float* y, const float* dy, float* dx, float* doff, bool accumulate,
                                 cudaStream_t s, const int* gate) {
-    in_stream_order(mex_redo_bwd, device_sm_count() * 2, kThreads, 0, s)(g, x, off, y, dy, dx, doff, int(accumulate), gate);
+    in_stream_order(mex_redo_bwd, device_sm_count() * 2, kGatedBwdThreads, 0, s)(g, x, off, y, dy, dx, doff, int(accumulate), gate);
     count_launch();
     return cudaGetLastError();
 }
@@ -388,7 +399,7 @@ cudaError_t launch_mex_dx_direct(const MexGeo& g, bool f64, const void* x, const
     const long long total = (long long)g.B * g.C * g.H * g.W;
     if (total == 0) return cudaSuccess;
     SIMNETS_DTYPE_SWITCH(f64,
-        (in_stream_order(mex_dx_direct<float>, grid_for(total, gate != nullptr), kThreads, 0, s)(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx, gate)),
+        (in_stream_order(mex_dx_direct<float>, grid_for(total, gate != nullptr), gate != nullptr ? kGatedThreads : kThreads, 0, s)(g, (const float*)x, (const float*)off, (const float*)y, (const float*)dy, (float*)dx, gate)),
         (in_stream_order(mex_dx_direct<double>, grid_for(total), kThreads, 0, s)(g, (const double*)x, (const double*)off, (const double*)y, (const double*)dy, (double*)dx, gate)));
     count_launch();
     return cudaGetLastError();

@@ -88,16 +88,4 @@ __host__ __device__ __forceinline__ bool mex_region_chw(const MexGeo& g, int r, 
     return c < g.Co && h < g.Ho && w < g.Wo;
 }
 
-// Position l (0 <= l < region_size) of region r -> flat output position (c*Ho + h)*Wo + w, or -1
-// when the region's footprint hangs over the edge of the output grid there.
-__host__ __device__ __forceinline__ int mex_region_position(const MexGeo& g, int r, int l) {
-    const int rw = r % g.ow, rh = (r / g.ow) % g.oh, rc = r / (g.ow * g.oh);
-    const int lw = l % g.rw, lh = (l / g.rw) % g.rh, lc = l / (g.rw * g.rh);
-    const int c = g.unshared ? lc * g.oc + rc : rc * g.rc + lc;
-    const int h = g.unshared ? lh * g.oh + rh : rh * g.rh + lh;
-    const int w = g.unshared ? lw * g.ow + rw : rw * g.rw + lw;
-    if (c >= g.Co || h >= g.Ho || w >= g.Wo) return -1;
-    return (c * g.Ho + h) * g.Wo + w;
-}
-
 }  // namespace simnets

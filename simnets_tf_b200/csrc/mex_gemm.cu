@@ -334,7 +334,7 @@ __device__ __forceinline__ bool gemm_unsafe(const int* __restrict__ verdict, int
 template <typename T>
 __device__ __noinline__ void exact_forward(const MexGeo& g, const T* x, const T* off, T* y) {
     const long long total = (long long)g.B * g.M * g.N, step = (long long)gridDim.x * gridDim.y * kGemmThreads;
-    for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kGemmThreads + threadIdx.x; i < total; i += step) y[i] = mex_exact_y(g, x, off, i);
+    for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kGemmThreads + threadIdx.x; i < total; i += step) y[i] = mex_exact_y<T, true>(g, x, off, i);
 }
 template <typename T>
 __device__ __noinline__ void exact_dx(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* dx) {

@@ -554,3 +554,29 @@ def test_results_do_not_depend_on_what_the_workspace_held(shape, M, norm, family
     for fill in (255, 127):
         for a, b in zip(run(fill), ref):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shape,m,blocks,strides,padding,pooled", [((24, 64, 32, 32), 128, (64, 1, 1), (64, 1, 1), (0, 0, 0), True), ((9, 64, 33, 31), 64, (4, 2, 2), (4, 2, 2), (0, 1, 0), False),
+                                                                   ((5, 12, 41, 40), 56, (12, 3, 3), (12, 1, 2), (0, 1, 1), False)], ids=["pixels", "short_patches", "overlapping"])
+def test_a_redone_pass_equals_the_shape_agnostic_kernels(shape, m, blocks, strides, padding, pooled):
+    """Offsets beyond the safe spread on layers whose outputs, inputs and parameters outnumber the threads of a gated launch several times: term
+    by term in the same order, so bit for bit what the kernels for any shape give."""
+    attrs = dict(softmax_mode=True, blocks=list(blocks), strides=list(strides), padding=list(padding), use_unshared_regions=pooled,
+                 unshared_offset_region=[2], shared_offset_region=[-1])
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x, off = torch.randn(shape, generator=gen, device="cuda"), torch.randn((4 if pooled else 1, m) + blocks, generator=gen, device="cuda")
+    off[-1, m // 2, 1, 0, 0] = -200.0
+    fl, direct = abi.FLAG_MEX_NO_SMALL_TILES, abi.FLAG_FORCE_DIRECT
+    y = mex_ops.mex_forward(x, off, m, flags=fl, **attrs)
+    assert torch.equal(y, mex_ops.mex_forward(x, off, m, flags=direct, **attrs))
+    dy = torch.randn(y.shape, generator=gen, device="cuda")
+    dx, doff = mex_ops.mex_input_grad(x, off, y, dy, m, flags=direct, **attrs), mex_ops.mex_offsets_grad(x, off, y, dy, m, flags=direct, **attrs)
+    assert torch.equal(mex_ops.mex_input_grad(x, off, y, dy, m, flags=fl, **attrs), dx)
+    assert torch.equal(mex_ops.mex_offsets_grad(x, off, y, dy, m, flags=fl, **attrs), doff)
+    both = mex_ops.mex_backward(x, off, y, dy, m, flags=fl, **attrs)
+    assert torch.equal(both[0], dx) and torch.equal(both[1], doff)
+    if pooled:
+        again, small = mex_ops.mex_forward_pool2(x, off, m, flags=fl, **attrs)
+        assert torch.equal(again, y)
+        want = y.view(shape[0], m, 16, 2, 16, 2)
+        assert torch.equal(small, (((want[:, :, :, 0, :, 0] + want[:, :, :, 0, :, 1]) + want[:, :, :, 1, :, 0]) + want[:, :, :, 1, :, 1]))
