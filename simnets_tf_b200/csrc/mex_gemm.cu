@@ -342,29 +342,57 @@ __device__ __noinline__ void exact_dx(const MexGeo& g, const T* x, const T* off,
     for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kGemmThreads + threadIdx.x; i < total; i += step) dx[i] = mex_exact_dx(g, x, off, y, dy, i);
 }
 
-// The sums of the offsets gradient term by term, into sums[r][m][k]: the threads of a CTA share the positions of one of them at a time, so
-// that a register adds up 1 / 256 of its B rs terms.  One thread per sum, 459 K positions under 8 instances of 4x2x2 taps: 306 ms and 1e-5
-// of the gradient's norm from float64; so 1.6 ms and 6e-7.
-template <typename T>
-__device__ __noinline__ void exact_doff(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* sums, T* red) {
-    const long long total = (long long)g.R * g.M * g.K, P = (long long)g.B * g.rs, ctas = (long long)gridDim.x * gridDim.y;
+// The sums of the offsets gradient term by term, into sums[r][m][k]: `threads` of a CTA (all or a warp) share the positions of TAPS of one
+// (r, m) at a time.
+template <typename T, int TAPS>
+__device__ __forceinline__ void exact_doff_of(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* sums, T* red, int threads) {
+    const long long P = (long long)g.B * g.rs, ctas = (long long)gridDim.x * gridDim.y;
+    const int groups = (g.K + TAPS - 1) / TAPS, per = kGemmThreads / threads, lane = threadIdx.x % threads;
     const T eps = T(g.eps), cst = T(g.cst), oob = T(g.oob);
-    for (long long i = (long long)blockIdx.y * gridDim.x + blockIdx.x; i < total; i += ctas) {
-        const int k = int(i % g.K), m = int(i / g.K % g.M), r = int(i / g.K / g.M), kw = k % g.bw, kh = k / g.bw % g.bh, kc = k / (g.bw * g.bh);
-        const long long tap = ((long long)kc * g.H + kh) * g.W + kw;
-        const T o = off[i];
-        T v = T(0);
+    for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * per + threadIdx.x / threads; i < (long long)g.R * g.M * groups; i += ctas * per) {
+        const long long row = i / groups;
+        const int k0 = int(i - row * groups) * TAPS, m = int(row % g.M), r = int(row / g.M);
+        int kc[TAPS], kh[TAPS], kw[TAPS];
+        long long tap[TAPS];
+        T o[TAPS], v[TAPS];
+#pragma unroll
+        for (int u = 0; u < TAPS; ++u) {
+            const int k = min(k0 + u, g.K - 1);
+            kw[u] = k % g.bw; kh[u] = k / g.bw % g.bh; kc[u] = k / (g.bw * g.bh);
+            tap[u] = ((long long)kc[u] * g.H + kh[u]) * g.W + kw[u];
+            o[u] = off[row * g.K + k];
+            v[u] = T(0);
+        }
 #pragma unroll 2
-        for (long long j = threadIdx.x; j < P; j += kGemmThreads) {
+        for (long long j = lane; j < P; j += threads) {
             const GemmCol c = gemm_col(g, r, j, P);
             if (c.base < 0) continue;
-            const int cc = c.c0 + kc, h = c.h0 + kh, w = c.w0 + kw;
-            const bool in = c.inside || (cc >= 0 && cc < g.C && h >= 0 && h < g.H && w >= 0 && w < g.W);
-            v += mex_weight(g, eps, cst, in ? x[c.xb + tap] : oob, o, y[c.base + (long long)m * g.N], dy[c.gbase + (long long)m * g.Ng]);
+            const T top = y[c.base + (long long)m * g.N], d = dy[c.gbase + (long long)m * g.Ng];
+#pragma unroll
+            for (int u = 0; u < TAPS; ++u) {
+                const int cc = c.c0 + kc[u], h = c.h0 + kh[u], w = c.w0 + kw[u];
+                const bool in = c.inside || (cc >= 0 && cc < g.C && h >= 0 && h < g.H && w >= 0 && w < g.W);
+                v[u] += mex_weight(g, eps, cst, in ? x[c.xb + tap[u]] : oob, o[u], top, d);
+            }
         }
-        v = row_reduce<T, true>(v, red, false);
-        if (threadIdx.x == 0) sums[i] = v;
+#pragma unroll
+        for (int u = 0; u < TAPS; ++u) {
+            const T sum = row_reduce<T, true>(v[u], red, threads == 32);
+            if (lane == 0 && k0 + u < g.K) sums[row * g.K + k0 + u] = sum;
+        }
     }
+}
+
+// A register adds up 1 / 256 of a sum's B rs terms, up to 1024 of them 1 / 32.  One thread per sum, 459 K positions under 8 instances of
+// 4x2x2 taps: 306 ms and 1e-5 of the gradient's norm from float64; so 1.6 ms and 6e-7.  A position is looked up, and its y and dy read, for
+// four taps where that leaves every CTA some (128 instances over 64 taps, 2 x 2 regions of 1024 positions: a tap per CTA 824 us, a tap per
+// warp 654, four 358).
+template <typename T>
+__device__ __noinline__ void exact_doff(const MexGeo& g, const T* x, const T* off, const T* y, const T* dy, T* sums, T* red) {
+    const int threads = (long long)g.B * g.rs <= 1024 ? 32 : kGemmThreads;
+    const long long units = (long long)gridDim.x * gridDim.y * (kGemmThreads / threads);
+    if ((long long)g.R * g.M * ((g.K + 3) / 4) >= units) exact_doff_of<T, 4>(g, x, off, y, dy, sums, red, threads);
+    else exact_doff_of<T, 1>(g, x, off, y, dy, sums, red, threads);
 }
 
 // What a CTA multiplies, in shared memory: As[2][kQ][LDA], Bs[2][kQ][LDB], step by step.  A thread's reads of them are the bound (32
