@@ -22,6 +22,7 @@
 // padding cuts off, or a step past the last one, contributes 0 * (t - x), which is NaN for an infinite x (or an infinite
 // parameter): a sum that came out NaN over a number is added up again over the taps that are there (dx_redo; the test costs 1.5 %
 // where 64 rows of channels share a tile: 128 x 64 x 32 x 32 input, 128 templates of 3x3, 1231 -> 1243 us, with kDxFold).
+#include <cmath>
 #include "kernels.cuh"
 #include "sim_exact.cuh"
 #include "tile.cuh"
@@ -118,7 +119,9 @@ __global__ void __launch_bounds__(256) sim_dx_prep(SimGeo g, int rm, int slot, i
 // of the gradient's norm against 3e-7).
 constexpr int kDxFold = 256;
 
-template <int RM, int WI, int MODE>
+// FEW: of a few templates, whose chunks of one tap would be mostly padding, a chunk is KC steps (tap, m) of whichever taps they belong to, each
+// staged with a cursor of its own.
+template <int RM, int WI, int MODE, bool FEW>
 __global__ void __launch_bounds__(DxTile<RM, WI>::T, DxTile<RM, WI>::PER_SM)
 sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, const float* __restrict__ dxp, const float* __restrict__ tm, const float* __restrict__ wt,
              const float* __restrict__ dy, float* __restrict__ dx) {
@@ -146,8 +149,8 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
     // A chunk is KC instances of one tap (fewer at the end of a tap).  The next chunk to be staged: tap (a, b) of the phase, instances
     // from m_next on.  This thread brings dy of columns s_lane (+ T), instances s_k, s_k + QSTEP, ...
     const int s_lane = threadIdx.x % TN, s_k = threadIdx.x / TN, chunks_per_tap = (g.M + KC - 1) / KC;
-    const int chunks = ph.h.taps * ph.w.taps * chunks_per_tap;
-    int a = 0, b = 0, m_next = 0, row_next = 0;                          // row_next: first row of the chunk in dxp
+    const int Q = ph.h.taps * ph.w.taps * g.M, chunks = FEW ? (Q + KC - 1) / KC : ph.h.taps * ph.w.taps * chunks_per_tap;
+    int a = 0, b = 0, m_next = FEW ? s_k : 0, row_next = 0;              // row_next: first row of the chunk in dxp; FEW: first step, and m_next this thread's
     DxPixel px[COLS];
     const float* at[COLS];
     bool ok[COLS];
@@ -158,13 +161,15 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
         col_covered[s_lane + u * T] = px[u].covered(g, ph);
     }
     auto locate = [&]() {
+        if (FEW)
+            while (m_next >= g.M) { m_next -= g.M; if (++b == ph.w.taps) { b = 0; ++a; } }
 #pragma unroll
         for (int u = 0; u < COLS; ++u) {
             const long long o = a < ph.h.taps ? px[u].at(g, a, b) : -1;
             ok[u] = o >= 0;
-            at[u] = dy + (ok[u] ? o + (long long)s_k * g.N : 0);
+            at[u] = dy + (ok[u] ? o + (long long)(FEW ? m_next : s_k) * g.N : 0);
         }
-        row_next = ((ph.rh + a * g.sh) * g.bw + ph.rw + b * g.sw) * g.M;
+        if (!FEW) row_next = ((ph.rh + a * g.sh) * g.bw + ph.rw + b * g.sw) * g.M;
     };
     if (chunks > 0) locate();
     // parameter staging: A_PER copies of 16 bytes per thread; their places inside a chunk do not change
@@ -174,9 +179,29 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
 #pragma unroll
         for (int v = 0; v < A_PER; ++v) {
             const int i = threadIdx.x + v * T, p = i / (PLANE / 4), r = i % (PLANE / 4) / (ROW / 4), e = i % (ROW / 4) * 4;
-            const bool there = m_next + r < g.M;
+            bool there = m_next + r < g.M;
+            size_t row = row_next + r;
+            if (FEW) {
+                const int q = row_next + r, tap = q / g.M, ta = tap / ph.w.taps, tb = tap - ta * ph.w.taps;
+                there = q < Q;
+                row = ((ph.rh + ta * g.sh) * g.bw + ph.rw + tb * g.sw) * g.M + q - tap * g.M;
+            }
             if (Tile::A_COPIES % T == 0 || i < Tile::A_COPIES)
-                cp_async16(stage + p * PLANE + r * ROW + e, there ? dxp + p * plane + (row_next + r) * row_floats + ct * ROW + e : dxp, there ? 16 : 0);
+                cp_async16(stage + p * PLANE + r * ROW + e, there ? dxp + p * plane + row * row_floats + ct * ROW + e : dxp, there ? 16 : 0);
+        }
+        if (FEW) {
+#pragma unroll
+            for (int s = 0; s < QPER; ++s) {
+#pragma unroll
+                for (int u = 0; u < COLS; ++u) {
+                    rb[u][s] = 0.f;
+                    if (ok[u]) { rb[u][s] = __ldg(at[u]); at[u] += (size_t)QSTEP * g.N; }
+                }
+                m_next += QSTEP;
+                if (m_next >= g.M) locate();
+            }
+            row_next += KC;
+            return;
         }
         const bool whole = m_next + KC <= g.M;
 #pragma unroll
@@ -267,7 +292,7 @@ sim_dx_tiled(const __grid_constant__ SimGeo g, const float* __restrict__ x, cons
             float* now = smem + (i & 1) * Tile::STAGE;
             float* next = smem + ((i + 1) & 1) * Tile::STAGE;
             const bool more = i + 1 < chunks;
-            const int steps = min(KC, g.M - m_now);
+            const int steps = FEW ? min(KC, Q - i * KC) : min(KC, g.M - m_now);
             if ((since += steps) > kDxFold) {
 #pragma unroll
                 for (int k = 0; k < RM * 4; ++k) {
@@ -415,30 +440,45 @@ __global__ void __launch_bounds__(kNarrowThreads) sim_dx_narrow(const __grid_con
 
 }  // namespace
 
-// The tile of a number of channels: the least padding, a tile of few rows counting for more (every row of it shares the dy values it
-// stages).
-struct DxPick { int rm, wi, slot, tiles; };
-static DxPick dx_pick(int channels) {
+// The pixels of the phase of pixel 0, which has the most.
+static long long dx_pixels(const SimGeo& g) {
+    const Axis h = dx_axis(g.H, g.bh, g.sh, g.ph, g.ph % g.sh), w = dx_axis(g.W, g.bw, g.sw, g.pw, g.pw % g.sw);
+    return (long long)g.B * h.n * w.n;
+}
+
+// The tile of a shape: the least padding of channels by rows and of a tap's templates by the halves of a chunk; a tile of few rows counts for
+// more (every row of it shares the dy values it stages), and so does the start of one, of the largest tile's long chunks above all.  An SM
+// of few warps takes as long as one of them, five times what the FP32 pipe would.  `few`: chunks that run through the taps, whose cursors take as long as thirty rows more.
+// 64 x 64 x 32 x 32 input, 3x3, in tiles of 64 rows / as picked: 1 template 58.8 / 25.1 us (few), 3 templates 58.9 / 34.4 (two tiles of 32 rows,
+// as the next two), 9 91.5 / 70.8, 17 133 / 107, 33 209 / 180; 8 x 24 x 32 x 32 under 17, L1: 62 in 64 CTAs of 24 rows,
+// 36 in 128 of 16.
+struct DxPick { int rm, wi, slot, tiles; bool few; };
+static DxPick dx_pick(const SimGeo& g) {
     static const struct { int rm, wi; } all[] = {{4, 4}, {6, 2}, {5, 2}, {4, 2}, {6, 1}, {5, 1}, {4, 1}};
-    DxPick best = {4, 4, 4, 1};
+    const double columns = double((dx_pixels(g) + 127) / 128) * g.sh * g.sw / device_sm_count();
+    DxPick best = {4, 4, 4, 1, false};
     double least = 0;
-    for (const auto& t : all) {
-        const int rows = 4 * t.rm * t.wi, tiles = (channels + rows - 1) / rows;
-        const double cost = double(tiles) * rows * (1 + 3.0 / rows);
-        if (least == 0 || cost < least) { least = cost; best = {t.rm, t.wi, t.rm == 4 ? 4 : 8, tiles}; }
-    }
+    for (const auto& t : all)
+        for (const bool few : {false, true}) {
+            if (few && (t.rm != 4 || t.wi == 4)) continue;
+            const int rows = 4 * t.rm * t.wi, tiles = (g.C + rows - 1) / rows, half = t.wi == 4 ? 8 : 4;
+            const auto each = [&](int of_rows) {
+                return (few ? double(g.M) * (of_rows + 30) : double((g.M + half - 1) / half * half) * (of_rows + 3)) + (t.wi == 4 ? 245 : 72);
+            };
+            const double all_of_it = each(rows) * std::ceil(columns * tiles), cost = std::max(all_of_it, 5 * each(4 * t.rm)) + 0.1 * all_of_it;
+            if (least == 0 || cost < least) { least = cost; best = {t.rm, t.wi, t.rm == 4 ? 4 : 8, tiles, few}; }
+        }
     return best;
 }
 size_t sim_dx_scratch_floats(const SimGeo& g) {
     if (g.C <= 8) return 0;
-    const DxPick t = dx_pick(g.C);
+    const DxPick t = dx_pick(g);
     return 2 * (size_t)g.bh * g.bw * g.M * t.tiles * 4 * t.wi * t.slot;
 }
 
 cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const float* w, const float* dy, float* dx, float* dxp, cudaStream_t s) {
     const int phases = g.sh * g.sw;
-    const Axis h = dx_axis(g.H, g.bh, g.sh, g.ph, g.ph % g.sh), v = dx_axis(g.W, g.bw, g.sw, g.pw, g.pw % g.sw);      // the phase of pixel 0 has the most pixels
-    const long long pixels = (long long)g.B * h.n * v.n;
+    const long long pixels = dx_pixels(g);
 #define DX_MODES(RUN)                            \
     switch (g.mode) {                            \
     case SIM_L1: RUN(SIM_L1); break;             \
@@ -467,28 +507,33 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
         count_launch();
         return cudaGetLastError();
     }
-    const DxPick pick = dx_pick(g.C);
+    const DxPick pick = dx_pick(g);
     const long long total = (long long)g.bh * g.bw * g.M * pick.tiles * 4 * pick.wi * pick.slot;
     in_stream_order(sim_dx_prep, int(std::min<long long>((total + 255) / 256, (long long)device_sm_count() * 8)), 256, 0, s)(g, pick.rm, pick.slot, 4 * pick.wi, pick.tiles, t, w, dxp);
     const long long blocks = (pixels + 127) / 128 * pick.tiles;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const dim3 grid{unsigned(blocks), unsigned(phases)};
     const bool folds = (long long)((g.bh + g.sh - 1) / g.sh) * ((g.bw + g.sw - 1) / g.sw) * g.M > kDxFold;         // (the most taps of a phase)
-#define DX(RM, WI, MODE)                                                                                                                      \
+#define DX_TILE(RM, WI, MODE, FEW)                                                                                                                   \
     do {                                                                                                                                      \
         using Tile = DxTile<RM, WI>;                                                                                                          \
         static SmemLimit limit;                                                                                                               \
-        const cudaError_t e = limit.raise(sim_dx_tiled<RM, WI, MODE>, Tile::SLOT_BYTES);                                                      \
+        const cudaError_t e = limit.raise(sim_dx_tiled<RM, WI, MODE, FEW>, Tile::SLOT_BYTES);                                                      \
         if (e != cudaSuccess) return e;                                                                                                       \
-        in_stream_order(sim_dx_tiled<RM, WI, MODE>, grid, Tile::T, folds ? Tile::SLOT_BYTES : 0, s)(g, x, dxp, t, w, dy, dx);                 \
+        in_stream_order(sim_dx_tiled<RM, WI, MODE, FEW>, grid, Tile::T, folds ? Tile::SLOT_BYTES : 0, s)(g, x, dxp, t, w, dy, dx);                 \
     } while (0)
-#define DX_41(MODE) DX(4, 1, MODE)
-#define DX_51(MODE) DX(5, 1, MODE)
-#define DX_61(MODE) DX(6, 1, MODE)
-#define DX_42(MODE) DX(4, 2, MODE)
-#define DX_52(MODE) DX(5, 2, MODE)
-#define DX_62(MODE) DX(6, 2, MODE)
-#define DX_44(MODE) DX(4, 4, MODE)
+#define DX_41(MODE) DX_TILE(4, 1, MODE, false)
+#define DX_51(MODE) DX_TILE(5, 1, MODE, false)
+#define DX_61(MODE) DX_TILE(6, 1, MODE, false)
+#define DX_42(MODE) DX_TILE(4, 2, MODE, false)
+#define DX_52(MODE) DX_TILE(5, 2, MODE, false)
+#define DX_62(MODE) DX_TILE(6, 2, MODE, false)
+#define DX_44(MODE) DX_TILE(4, 4, MODE, false)
+#define DX_FEW_1(MODE) DX_TILE(4, 1, MODE, true)
+#define DX_FEW_2(MODE) DX_TILE(4, 2, MODE, true)
+    if (pick.few) {
+        if (pick.wi == 1) { DX_MODES(DX_FEW_1) } else { DX_MODES(DX_FEW_2) }
+    } else
     switch (pick.wi * 8 + pick.rm) {
     case 12: DX_MODES(DX_41) break;
     case 13: DX_MODES(DX_51) break;
@@ -500,7 +545,7 @@ cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const
     }
     count_launch(2);
     return cudaGetLastError();
-#undef DX
+#undef DX_TILE
 #undef DX_MODES
 }
 

@@ -213,3 +213,21 @@ def test_l1_skipping_nan_at_the_edges_of_the_tiles(port, i):
     shape, M, blocks, strides, padding = PARAM_TILES[i]
     gpu_util.check_similarity(port, cases.sim_case("skip%d" % i, shape, M, blocks=blocks, strides=strides, padding=padding, oob=0.3, nan_frac=0.2, seed=890 + i, **L1_MODES[1]),
                               f64_tiebreak=True)
+
+
+# ---- input gradients of a few templates: chunks of eight or sixteen steps that run through the taps, in tiles of 16, 32 and 64 rows
+@pytest.mark.parametrize("infinite", [False, True], ids=["finite", "infinite"])
+@pytest.mark.parametrize("mode", MODES + L1_MODES[1:], ids=["l2", "l2n", "l2nan", "l1", "l1skip"])
+@pytest.mark.parametrize("channels,m,blocks,strides,padding", [
+    (9, 1, (1, 1), (1, 1), (0, 0)), (12, 1, (3, 3), (1, 1), (1, 1)), (16, 3, (3, 2), (2, 1), (1, 0)), (24, 2, (5, 3), (1, 1), (2, 1)), (33, 1, (2, 2), (3, 3), (0, 0)),
+    (32, 2, (3, 3), (2, 2), (1, 1)), (64, 1, (3, 3), (1, 1), (1, 1)), (64, 3, (5, 5), (1, 2), (2, 2)), (66, 5, (3, 3), (1, 1), (0, 1)), (128, 6, (3, 2), (2, 1), (1, 0)), (64, 7, (1, 1), (1, 1), (0, 0))])
+def test_input_gradients_of_a_few_templates(port, channels, m, blocks, strides, padding, mode, infinite):
+    c = cases.sim_case("few%d" % channels, (3, channels, 9, 8), m, blocks=blocks, strides=strides, padding=padding, oob=0.3, seed=900 + channels, **mode)
+    d = cases.sim_desc(c)
+    x, t, w, dy = cases.sim_inputs(c, port.sim_out_shape(d))
+    if infinite:
+        x[np.random.default_rng(m).random(x.shape) < 0.2] = np.inf
+        dy = np.abs(dy)
+    dx = gpu_util.sim_ops.similarity_input_grad(*(gpu_util.dev(a) for a in (x, t, w, dy)), flags=c["flags"], **cases.sim_attrs(c)).cpu().numpy()
+    a64 = [a.astype(np.float64) for a in (x, t, w, dy)]
+    cases.assert_parity(dx, port.similarity_input_grad(d, x, t, w, dy), port.similarity_input_grad(cases.sim_desc(c, dtype=gpu_util.abi.F64), *a64), what=c["name"])
