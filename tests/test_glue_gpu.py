@@ -8,7 +8,7 @@ import torch
 
 import cases
 import gpu_util
-from simnets_tf_b200 import abi
+from simnets_tf_b200 import abi, keras
 from simnets_tf_b200.simnet import SPECS, SimNet
 
 sim_ops = importlib.import_module("simnets_tf_b200.ops.similarity")
@@ -183,3 +183,25 @@ def test_pooled_outputs_without_a_gradient(batch):
     with torch.no_grad():
         free = net(x)
     assert torch.equal(free, net(x).detach())
+
+
+@pytest.mark.parametrize("batch", [15, 16])
+def test_the_extrema_hand_over_on_both_sides_of_its_line(batch, monkeypatch):
+    """From 2^20 values on a Similarity layer leaves the extrema of its output to the MEX layer behind it; with and without that, loss and
+    gradients are the same."""
+    spec = SPECS["cfg5"]
+    x = torch.rand(batch, 3, 32, 32, generator=torch.Generator().manual_seed(3)).cuda() - 0.5
+    labels = torch.arange(batch).cuda() % spec["classes"]
+    given = []
+    slot_of = keras.Mex.extrema_slot
+    monkeypatch.setattr(keras.Mex, "extrema_slot", lambda self, *args, **kwargs: given.append(slot_of(self, *args, **kwargs)) or given[-1])
+    outs = []
+    for fuse in (True, False):
+        net = SimNet(spec, seed=2)
+        net.fuse_extrema = fuse
+        loss = net.loss(x, labels)
+        loss.backward()
+        outs.append([loss.detach()] + [p.grad.clone() for p in net.parameters()])
+        assert len(given) == (1 if batch == 16 else 0) and None not in given
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
