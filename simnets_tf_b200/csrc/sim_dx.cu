@@ -446,12 +446,13 @@ static long long dx_pixels(const SimGeo& g) {
     return (long long)g.B * h.n * w.n;
 }
 
-// The tile of a shape: the least padding of channels by rows and of a tap's templates by the halves of a chunk; a tile of few rows counts for
-// more (every row of it shares the dy values it stages), and so does the start of one, of the largest tile's long chunks above all.  An SM
-// of few warps takes as long as one of them, five times what the FP32 pipe would.  `few`: chunks that run through the taps, whose cursors take as long as thirty rows more.
+// The tile of a shape: the least padding of channels by rows and of a tap's templates by the halves of a chunk; a row of a tile costs less the
+// more of them share the staged dy values, the start of a tile is paid too (most in the long chunks of the largest), an SM of few tiles takes
+// as long as one of its warps, and up to five tiles the busiest SM counts.  `few`: chunks that run through the taps, whose cursors take as long as
+// 13 or 42 rows more.  The weights are those that lose least against the best tile over 477 shapes timed in every tile (8 to 200 samples of 12 to
+// 200 x 32 x 32, 1 to 64 templates of 3x3 and 1x1): 1 % in the mean, 12 % less time than padding alone decides by.
 // 64 x 64 x 32 x 32 input, 3x3, in tiles of 64 rows / as picked: 1 template 58.8 / 25.1 us (few), 3 templates 58.9 / 34.4 (two tiles of 32 rows,
-// as the next two), 9 91.5 / 70.8, 17 133 / 107, 33 209 / 180; 8 x 24 x 32 x 32 under 17, L1: 62 in 64 CTAs of 24 rows,
-// 36 in 128 of 16.
+// as the next two), 9 91.5 / 70.8, 17 133 / 107; 8 x 24 x 32 x 32 under 17, L1: 62 in 64 CTAs of 24 rows, 36 in 128 of 16.
 struct DxPick { int rm, wi, slot, tiles; bool few; };
 static DxPick dx_pick(const SimGeo& g) {
     static const struct { int rm, wi; } all[] = {{4, 4}, {6, 2}, {5, 2}, {4, 2}, {6, 1}, {5, 1}, {4, 1}};
@@ -460,12 +461,12 @@ static DxPick dx_pick(const SimGeo& g) {
     double least = 0;
     for (const auto& t : all)
         for (const bool few : {false, true}) {
-            if (few && (t.rm != 4 || t.wi == 4)) continue;
+            if (few && (t.rm != 4 || t.wi == 4 || g.M > 2 || g.bh * g.bw == 1)) continue;
             const int rows = 4 * t.rm * t.wi, tiles = (g.C + rows - 1) / rows, half = t.wi == 4 ? 8 : 4;
-            const auto each = [&](int of_rows) {
-                return (few ? double(g.M) * (of_rows + 30) : double((g.M + half - 1) / half * half) * (of_rows + 3)) + (t.wi == 4 ? 245 : 72);
-            };
-            const double all_of_it = each(rows) * std::ceil(columns * tiles), cost = std::max(all_of_it, 5 * each(4 * t.rm)) + 0.1 * all_of_it;
+            const double steps = few ? double(g.M) * (rows + (t.wi == 1 ? 13 : 42)) : double((g.M + half - 1) / half * half) * (rows + 6.7) * (t.rm > 4 ? 1.03 : 1);
+            const double start = t.wi == 4 ? 245 : (t.wi == 2 ? 27 : 37), alone = t.wi == 4 ? 1 : (t.wi == 2 ? 1.1 : 1.9);
+            const double here = columns * tiles, per_sm = here < 5 ? std::ceil(here) : here;
+            const double cost = (steps + start) * (std::max(per_sm, alone) + 0.08 * per_sm);
             if (least == 0 || cost < least) { least = cost; best = {t.rm, t.wi, t.rm == 4 ? 4 : 8, tiles, few}; }
         }
     return best;
