@@ -453,13 +453,13 @@ static long long dx_pixels(const SimGeo& g) {
 // 200 x 32 x 32, 1 to 64 templates of 3x3 and 1x1): 1 % in the mean, 12 % less time than padding alone decides by.
 // 64 x 64 x 32 x 32 input, 3x3, in tiles of 64 rows / as picked: 1 template 58.8 / 25.1 us (few), 3 templates 58.9 / 34.4 (two tiles of 32 rows,
 // as the next two), 9 91.5 / 70.8, 17 133 / 107; 8 x 24 x 32 x 32 under 17, L1: 62 in 64 CTAs of 24 rows, 36 in 128 of 16.
+static const struct { int rm, wi; } kDxTiles[] = {{4, 4}, {6, 2}, {5, 2}, {4, 2}, {6, 1}, {5, 1}, {4, 1}};
 struct DxPick { int rm, wi, slot, tiles; bool few; };
 static DxPick dx_pick(const SimGeo& g) {
-    static const struct { int rm, wi; } all[] = {{4, 4}, {6, 2}, {5, 2}, {4, 2}, {6, 1}, {5, 1}, {4, 1}};
     const double columns = double((dx_pixels(g) + 127) / 128) * g.sh * g.sw / device_sm_count();
     DxPick best = {4, 4, 4, 1, false};
     double least = 0;
-    for (const auto& t : all)
+    for (const auto& t : kDxTiles)
         for (const bool few : {false, true}) {
             if (few && (t.rm != 4 || t.wi == 4 || g.M > 2 || g.bh * g.bw == 1)) continue;
             const int rows = 4 * t.rm * t.wi, tiles = (g.C + rows - 1) / rows, half = t.wi == 4 ? 8 : 4;
@@ -471,10 +471,12 @@ static DxPick dx_pick(const SimGeo& g) {
         }
     return best;
 }
+// Room for the parameters in any of the tiles: the pick follows the batch, and a workspace sized for one batch serves every smaller one.
 size_t sim_dx_scratch_floats(const SimGeo& g) {
     if (g.C <= 8) return 0;
-    const DxPick t = dx_pick(g);
-    return 2 * (size_t)g.bh * g.bw * g.M * t.tiles * 4 * t.wi * t.slot;
+    size_t row = 0;
+    for (const auto& t : kDxTiles) row = std::max(row, size_t((g.C + 4 * t.rm * t.wi - 1) / (4 * t.rm * t.wi)) * 4 * t.wi * (t.rm == 4 ? 4 : 8));
+    return 2 * (size_t)g.bh * g.bw * g.M * row;
 }
 
 cudaError_t launch_sim_dx(const SimGeo& g, const float* x, const float* t, const float* w, const float* dy, float* dx, float* dxp, cudaStream_t s) {

@@ -145,3 +145,13 @@ def test_ops_refuse_cpu_tensors():
         similarity(torch.zeros(1, 1, 4, 4), torch.zeros(2, 1, 3, 3), torch.ones(2, 1, 3, 3))
     with pytest.raises(RuntimeError, match="no CPU kernels"):
         mex(torch.zeros(1, 2, 4, 4), torch.zeros(1, 3, 2, 1, 1), 3, blocks=[2, 1, 1])
+
+
+@pytest.mark.parametrize("channels,m,blocks,strides", [(9, 1, (3, 3), (1, 1)), (24, 17, (3, 3), (1, 1)), (40, 2, (5, 3), (2, 1)), (64, 1, (1, 1), (1, 1)), (96, 33, (3, 3), (1, 1)), (200, 5, (2, 2), (2, 2))])
+def test_a_similarity_workspace_of_a_batch_serves_every_smaller_one(cuda_lib, channels, m, blocks, strides):
+    """The input gradient's tile follows the number of samples; what it needs of the workspace must not."""
+    def bytes_of(batch):
+        d = abi.make_sim_desc((batch, channels, 32, 32), m, similarity_function="L2", blocks=blocks, strides=strides, padding=(1, 1))
+        return cuda_lib.simnets_similarity_workspace_bytes(C.byref(d))
+    sizes = [bytes_of(b) for b in (1, 2, 3, 5, 8, 12, 16, 24, 40, 64, 100, 200, 512)]
+    assert sizes[0] > 0 and sizes == sorted(sizes)
