@@ -5,10 +5,11 @@
 // as a generalized GEMM with rows m, columns k and positions as the reduction index (the reference's element functors:
 // HUJI-Deep/simnets-tf include/utils/similarity_utils.hpp:64-119; no patch matrix).
 //
-// Bound: the FP32 pipe, 4 lane operations per term (5 with missing data).  A CTA of 256 threads owns 32 templates x up to
-// 64 taps, a thread 4 x 2 of them with all its sums in registers: few enough registers for 16 warps per SM, which the chain
+// Bound: the FP32 pipe, 4 lane operations per term (5 with missing data).  More than 32 templates over more than 16 taps, blocks of up to 16 x
+// 16: sim_dparams_wide, below.  The others (up to 32 templates, up to 16 taps, taller blocks): a CTA of 256 threads owns 32 or 64 templates x
+// up to 64 taps, a thread 4 x 2 of them with all its sums in registers: few enough registers for 16 warps per SM, which the chain
 // difference -> product -> sums needs (4 x 4 per thread at 12 warps stalled on that chain: FP32 pipe 53 % busy).
-// Both operands are contiguous along positions in memory and stay that way in shared memory ([row][position], rows padded by
+// There both operands are contiguous along positions in memory and stay that way in shared memory ([row][position], rows padded by
 // four floats so that eight rows of one 16-byte read hit 32 different banks): nothing is transposed, and the packed FP32
 // instructions pair two positions, so that no operand needs to be duplicated into both halves.  When the patch is short, the
 // threads cover the tile several times over and the copies split the positions of a chunk among themselves (K = 4: sixteen
@@ -33,8 +34,8 @@ struct DpTile { int k2, groups, tm, kc; };       // tap columns / 2, copies of t
 
 // Tile of a patch of K taps: the patch in n equal tiles of at most 64 taps, n the smallest that keeps nearly as many threads
 // busy as the best does (K = 36: one tile would leave 112 of 256 threads idle, three of 12 none).  Up to 32 taps a tile takes
-// 64 templates, so that a thread still stages few values per term (K = 27 at 32 templates: 906 us instead of the figure
-// below).  The chunk is long enough that every copy of the tile gets a quad of positions.
+// 64 templates, so that a thread still stages few values per term (64 templates of 27 taps over 2048 x 3 x 32 x 32, as this kernel took them: 906
+// us in tiles of 32, 760 of 64).  The chunk is long enough that every copy of the tile gets a quad of positions.
 __host__ inline DpTile dp_tile(const SimGeo& g) {
     DpTile best = {1, 1, 32, 64};
     double best_busy = 0;
@@ -332,8 +333,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams(SimGeo g
 // Operands lie [position][row], so that the packed instructions pair two TAPS: a thread owns 4 templates x 2 pairs of taps with one
 // register per sum, half of what pairing positions takes, and reads 12 values (with masks) per position for 16 terms.  A staging
 // thread brings two neighbouring rows of one position and stores them as one pair at slot pair ^ ((position >> 2) & 3) of a row of
-// 64 + 8 (32 + 8) floats: the stores of 16 positions, the 16-byte reads of eight column groups and the tensor cores' 8 x 4 fragments
-// each hit 32 different banks, and the reading loop knows position & 15 at compile time.
+// 64 + 8 (32 + 8) floats: the stores of 16 positions and the 16-byte reads of eight column groups each hit 32 different banks, and the reading loop knows position & 15 at compile time.
 constexpr int kDwTM = 64, kDwKC = 32;
 // As kDpFold; one chain per sum here, two or more there, so the chains are shorter: chunks after which a thread sets its sums aside
 __host__ inline int dw_fold(long long positions) { return positions <= 512 ? 2 : positions <= 1024 ? 4 : positions <= 4096 ? 8 : 16; }
@@ -346,11 +346,6 @@ template <int MODE, int WJ> struct DwTile {
 
 // a sign(d); a0 = 0 a where d is 0 or NaN, which is NaN for an a that is no finite number
 __device__ __forceinline__ float dw_signed(float a, float a0, float d) { return fabsf(d) > 0.f ? __uint_as_float(__float_as_uint(a) ^ (__float_as_uint(d) & 0x80000000u)) : a0; }
-// the taps first .. of a block axis that leave the image, as bits (block <= 16)
-__device__ __forceinline__ uint32_t dw_missing(int first, int size) {
-    const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
-    return 0xffffu & ~(((1u << hi) - 1u) & ~((1u << lo) - 1u));
-}
 
 template <int MODE, int WJ>
 __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams_wide(const __grid_constant__ SimGeo g, FastDiv f_N, FastDiv f_ow, int TK, const float* __restrict__ x,
@@ -428,7 +423,7 @@ __global__ void __launch_bounds__(kDpThreads, kDpCtasPerSm) sim_dparams_wide(con
         }
         // dead positions pair dy = 0 with a finite value
         const int h0 = ho * g.sh - g.ph, w0 = wo * g.sw - g.pw;
-        const int missing = live ? int(dw_missing(h0, g.H) | (dw_missing(w0, g.W) << 16)) : -1;
+        const int missing = live ? int(missing_taps(h0, g.H) | (missing_taps(w0, g.W) << 16)) : -1;
         const char* xc = reinterpret_cast<const char*>(x + (size_t)n * g.C * g.H * g.W + h0 * g.W + w0);
         const float outside = live ? oob : 0.f;
 #pragma unroll
@@ -658,7 +653,12 @@ __global__ void __launch_bounds__(512) sim_dparams_reduce(SimGeo g, int splits, 
 
 }  // namespace
 
-// Whether tiles of 64 templates x 64 (32) taps serve a shape, and how many taps such a tile takes (the patch in equal parts).
+// Whether tiles of 64 templates x 64 (32) taps serve a shape, and how many taps such a tile takes (the patch in equal parts).  Filled alike,
+// they are 1.01 to 1.33 times as fast as the smaller ones (275 shapes of 33 to 192 templates and 17 to 144 taps, 96 x C x 32 x 32; least with
+// missing data, most in L1).  Where they are filled 0.75 times as well (17 to 20 and 33 to 48 taps; 65 to 96 templates over 64 columns) both take the
+// same within 7 %, with missing data up to 12 % more here (96 templates of 13x2x2 taps 144 -> 163 us, 64 of 4x3x3 L2 63 -> 68, L1 1.00 to 1.10
+// faster).  They stay there too: the sums are shorter and in FP32 throughout (templates gradients 2.0e-7 to 3.3e-7 of their norm from
+// float64 over 96 samples, 2.3e-7 to 5.6e-7 there).
 static int dw_taps(const SimGeo& g) {
     if (g.M <= 32 || g.K <= 16 || g.bh > 16 || g.bw > 16) return 0;
     // (a term of the narrower tile costs some 15 % more staging)

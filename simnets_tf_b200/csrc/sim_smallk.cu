@@ -157,12 +157,6 @@ __global__ void __launch_bounds__(kSkThreads, 4) sim_fwd_smallk(SimGeo g, int sl
     }
 }
 
-// the taps first .. of a block axis that leave the image, as bits (block <= 16)
-__device__ __forceinline__ uint32_t sk_missing(int first, int size) {
-    const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
-    return 0xffffu & ~(((1u << hi) - 1u) & ~((1u << lo) - 1u));
-}
-
 // Parameters resident in shared memory, tiles of 128 positions streamed past them: rows = templates (TM per CTA, blockIdx.y
 // picks them), columns = positions.
 template <int MODE> struct ResidentPlanes {
@@ -220,7 +214,7 @@ __global__ void __launch_bounds__(TM * 4, TM == 64 ? 2 : 4) sim_fwd_resident(Sim
         rbase = c.base;
         const float outside = c.base >= 0 ? oob : 0.f;
         if (bits) {
-            const int missing = c.base >= 0 ? int(sk_missing(c.h0, g.H) | (sk_missing(c.w0, g.W) << 16)) : -1;
+            const int missing = c.base >= 0 ? int(missing_taps(c.h0, g.H) | (missing_taps(c.w0, g.W) << 16)) : -1;
 #pragma unroll
             for (int s = 0; s < PER; ++s) {
                 const int k = s_k + s * QSTEP;

@@ -58,11 +58,6 @@ __host__ SimWs carve(const SimGeo& g, void* base) {
 // offsets.  (Two range tests per gathered value, although a patch inside the image skipped them: 256 x 64 x 32 x 32 input, 256 templates
 // of 3x3 4134 -> 3913 us, with masks 6046 -> 5557, L1 3119 -> 2838.)
 __host__ __device__ inline bool sim_tap_bits(const SimGeo& g) { return g.bh <= 16 && g.bw <= 16 && sim_offsets_below(g, 1LL << 29); }
-// the taps of a block axis that leave the image, as bits
-__device__ __forceinline__ uint32_t sim_missing(int first, int size) {
-    const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
-    return 0xffffu & ~(((1u << hi) - 1u) & ~((1u << lo) - 1u));
-}
 
 // One block per instance m: tap-major parameter planes, the per-instance constant, and (block 0) the tap table.
 __global__ void __launch_bounds__(128) sim_prep(SimGeo g, const float* __restrict__ tm, const float* __restrict__ wt,
@@ -163,7 +158,7 @@ __global__ void __launch_bounds__(FwdTile<TM, TN>::THREADS, FwdTile<TM, TN>::PER
     const SimColumn sc = sim_column(g, j0 + s_lane, P);
     if (s_k == 0) col_base[s_lane] = sc.base;
     const bool live = sc.base >= 0;
-    const int missing = live ? int(sim_missing(sc.h0, g.H) | (sim_missing(sc.w0, g.W) << 16)) : -1;
+    const int missing = live ? int(missing_taps(sc.h0, g.H) | (missing_taps(sc.w0, g.W) << 16)) : -1;
     const float outside = live ? oob : 0.f;
     const float* xs = x + (size_t)sc.n * g.C * g.H * g.W;
     const char* xc = reinterpret_cast<const char*>(xs + sc.h0 * g.W + sc.w0);

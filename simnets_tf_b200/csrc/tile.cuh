@@ -20,6 +20,12 @@
 
 namespace simnets {
 
+// The taps of a block axis that leave the image, as bits, the first tap at `first` (blocks of up to 16): what a tap's own bit is tested against.
+__device__ __forceinline__ uint32_t missing_taps(int first, int size) {
+    const int lo = min(max(-first, 0), 16), hi = min(max(size - first, 0), 16);
+    return 0xffffu & ~(((1u << hi) - 1u) & ~((1u << lo) - 1u));
+}
+
 template <int TM_, int TN_, int KC_, int RM_, int RN_, int NA_, int NB_>
 struct TileCfg {
     static constexpr int TM = TM_, TN = TN_, KC = KC_, RM = RM_, RN = RN_, NA = NA_, NB = NB_;
