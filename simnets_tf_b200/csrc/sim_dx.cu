@@ -450,7 +450,7 @@ static long long dx_pixels(const SimGeo& g) {
 // more of them share the staged dy values, the start of a tile is paid too (most in the long chunks of the largest), an SM of few tiles takes
 // as long as one of its warps, and up to five tiles the busiest SM counts.  `few`: chunks that run through the taps, whose cursors take as long as
 // 13 or 42 rows more.  The weights are those that lose least against the best tile over 477 shapes timed in every tile (8 to 200 samples of 12 to
-// 200 x 32 x 32, 1 to 64 templates of 3x3 and 1x1): 1 % in the mean, 12 % less time than padding alone decides by.
+// 200 x 32 x 32, 1 to 64 templates of 3x3 and 1x1): 1.4 % in the mean, a tenth less time than the least padding.
 // 64 x 64 x 32 x 32 input, 3x3, in tiles of 64 rows / as picked: 1 template 58.8 / 25.1 us (few), 3 templates 58.9 / 34.4 (two tiles of 32 rows,
 // as the next two), 9 91.5 / 70.8, 17 133 / 107; 8 x 24 x 32 x 32 under 17, L1: 62 in 64 CTAs of 24 rows, 36 in 128 of 16.
 static const struct { int rm, wi; } kDxTiles[] = {{4, 4}, {6, 2}, {5, 2}, {4, 2}, {6, 1}, {5, 1}, {4, 1}};
